@@ -94,6 +94,7 @@ struct DevPairs {
 // mask; friction rows at 2 * row + k.  Slots are grouped by part and local colour, then by cut
 // colour.
 struct DevRows {
+    float4* planes;   // the ten row arrays, one allocation (15 planes of 4 x pair capacity points)
     float4* n_nrm;    // contactNormal, jacDiagABInv
     float4* n_rp1;    // relpos1CrossNormal, penetration
     float4* n_rp2;    // relpos2CrossNormal, restitution

@@ -23,6 +23,7 @@
 #include "../../include/jbgpu.h"
 #include "manifold.cuh"
 #include "mlp.cuh"
+#include "rows.cuh"
 #include "prims.cuh"
 #include "gridsync.cuh"
 #include "solver.cuh"
@@ -225,6 +226,14 @@ __device__ __forceinline__ int part_of(const DevWorld& w, const SolverBuffers& s
     return sb.worldParts ? w.world[b] : (int)(((long long)pos * sb.nParts) / sb.nFinite);
 }
 
+// The flow solver's block that holds dynamic body b's velocity (-1 when b has no position).
+__device__ __forceinline__ int flow_home(const DevWorld& w, const SolverBuffers& sb, int b) {
+    const int q = part_of(w, sb, b);
+    if (q < 0) return -1;
+    const int2 v = sb.flowPart[q];   // first block, bodies per block
+    return v.x + (sb.posOf[b] - sb.partStart[q]) / v.y;
+}
+
 __global__ void k_posof(SolverBuffers sb) {
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < sb.nFinite) sb.posOf[sb.order[s]] = s;
@@ -249,6 +258,14 @@ __global__ void k_classify(DevWorld w, DevPairs P, SolverBuffers sb) {
         if (d1) lb1 = sb.posOf[b1] - ps;
     }
     sb.candLocal[k] = lb0 | (lb1 << 16);
+    if (sb.flowOn) {
+        const int e = flow_home(w, sb, d0 ? b0 : b1);   // the block that solves it (solver_flow.cu)
+        sb.execOf[k] = e;
+        if (e >= 0) {
+            const unsigned ge = __match_any_sync(__activemask(), e);
+            if ((threadIdx.x & 31) == __ffs(ge) - 1) atomicAdd(&sb.flowCount[e], __popc(ge));
+        }
+    }
     const unsigned grp = __match_any_sync(__activemask(), q);   // one atomic per bucket and warp
     if ((threadIdx.x & 31) == __ffs(grp) - 1) atomicAdd(&sb.bucketCount[q], __popc(grp));
 }
@@ -305,13 +322,31 @@ __device__ __forceinline__ bool holds_claims(const DevWorld& w, const SolverBuff
     return (!dyn(w, b0) || __ldcg(&sb.claim[b0]) == me) && (!dyn(w, b1) || __ldcg(&sb.claim[b1]) == me);
 }
 
+// Links of a body's candidates in the order the solver takes them: a link is candidate << 1 | side
+// (0: the body is the manifold's body0).  Candidate `me` comes after `prev` (-1: it is the
+// body's first, *body); returns the body's new last link.
+JBD int link_after(const SolverBuffers& sb, int prev, int me, const int* body) {
+    if (!sb.flowOn) return -1;
+    sb.prevLink[me] = prev;
+    if (prev >= 0) sb.nextLink[prev] = me;
+    else sb.firstLink[*body] = me;
+    return me;
+}
+JBD void link_cut(const SolverBuffers& sb, int me, int body) {
+    if (!sb.flowOn) return;
+    __stcg(&sb.lastLink[body], link_after(sb, __ldcg(&sb.lastLink[body]), me, &body));
+}
+
 __global__ void __launch_bounds__(SOLVER_THREADS) k_colour(DevWorld w, DevPairs P, SolverBuffers sb) {
     unsigned barK = 0;
     const int nb = gridDim.x;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
     const int nCand = *sb.nCand;
     __shared__ int shWin, shDone, shPart;
-    for (int k = tid; k < nCand; k += nth) sb.colourOf[k] = -1;
+    for (int k = tid; k < nCand; k += nth) {
+        sb.colourOf[k] = -1;
+        if (sb.flowOn) sb.nextLink[2 * k] = sb.nextLink[2 * k + 1] = -1;
+    }
     for (int c = tid; c < sb.nParts * (MAX_LOCAL + 1); c += nth) sb.lcCount[c] = 0;
     for (int c = tid; c <= MAX_COLOURS; c += nth) sb.colourCount[c] = 0;
     if (tid == 0) { w.ctr[C_CUT_DONE] = 0; w.ctr[C_WIN0] = w.ctr[C_WIN1] = w.ctr[C_WIN2] = 0; }
@@ -321,12 +356,14 @@ __global__ void __launch_bounds__(SOLVER_THREADS) k_colour(DevWorld w, DevPairs 
     extern __shared__ unsigned long long colSmem[];
     unsigned long long* shClaim = colSmem;
     int* shTaken = (int*)(colSmem + sb.partMax);
+    int* shLast = shTaken + sb.partMax;   // link of the body's last coloured candidate
     constexpr int NONE = 0xffff;
     for (int part = next_part(w, sb, C_PART_NEXT0, &shPart); part >= 0; part = next_part(w, sb, C_PART_NEXT0, &shPart)) {
         const int s0 = sb.bucketStart[part], s1 = sb.bucketStart[part + 1];
         const int np = sb.partStart[part + 1] - sb.partStart[part];
+        const int* order0 = sb.order + sb.partStart[part];
         int* lc = sb.lcCount + part * (MAX_LOCAL + 1);
-        for (int i = threadIdx.x; i < np; i += blockDim.x) { shClaim[i] = ~0ull; shTaken[i] = -1; }
+        for (int i = threadIdx.x; i < np; i += blockDim.x) { shClaim[i] = ~0ull; shTaken[i] = -1; shLast[i] = -1; }
         if (threadIdx.x == 0) shDone = 0;
         // a thread's first COL_REG candidates (k, local bodies, coloured) stay in registers
         // through all passes; a part with more candidates than COL_REG x blockDim takes the rest
@@ -372,8 +409,8 @@ __global__ void __launch_bounds__(SOLVER_THREADS) k_colour(DevWorld w, DevPairs 
                     if ((l0 == NONE || shClaim[l0] == me) && (l1 == NONE || shClaim[l1] == me)) {
                         sb.colourOf[k] = r;
                         done |= 1u << j;
-                        if (l0 != NONE) shTaken[l0] = r;
-                        if (l1 != NONE) shTaken[l1] = r;
+                        if (l0 != NONE) { shTaken[l0] = r; shLast[l0] = link_after(sb, shLast[l0], 2 * k, order0 + l0); }
+                        if (l1 != NONE) { shTaken[l1] = r; shLast[l1] = link_after(sb, shLast[l1], 2 * k + 1, order0 + l1); }
                         myWin++;
                     }
                 }
@@ -384,8 +421,8 @@ __global__ void __launch_bounds__(SOLVER_THREADS) k_colour(DevWorld w, DevPairs 
                     const unsigned long long me = ctag(t, k);
                     if ((l0 == NONE || shClaim[l0] == me) && (l1 == NONE || shClaim[l1] == me)) {
                         sb.colourOf[k] = r;
-                        if (l0 != NONE) shTaken[l0] = r;
-                        if (l1 != NONE) shTaken[l1] = r;
+                        if (l0 != NONE) { shTaken[l0] = r; shLast[l0] = link_after(sb, shLast[l0], 2 * k, order0 + l0); }
+                        if (l1 != NONE) { shTaken[l1] = r; shLast[l1] = link_after(sb, shLast[l1], 2 * k + 1, order0 + l1); }
                         myWin++;
                     }
                 }
@@ -409,6 +446,8 @@ __global__ void __launch_bounds__(SOLVER_THREADS) k_colour(DevWorld w, DevPairs 
             for (int c = 0; c < r; c++) { st[c] = run; run += __ldcg(&lc[c]); }
             st[r] = run;
         }
+        if (sb.flowOn)
+            for (int i = threadIdx.x; i < np; i += blockDim.x) sb.lastLink[order0[i]] = shLast[i];
         __syncthreads();
     }
     // cut manifolds, grid-wide
@@ -463,8 +502,8 @@ __global__ void __launch_bounds__(SOLVER_THREADS) k_colour(DevWorld w, DevPairs 
                 if ((gb0[j] < 0 || __ldcg(&sb.claim[gb0[j]]) == me) && (gb1[j] < 0 || __ldcg(&sb.claim[gb1[j]]) == me)) {
                     sb.colourOf[gk[j]] = round;
                     gdone |= 1u << j;
-                    if (gb0[j] >= 0) sb.taken[gb0[j]] = mark;
-                    if (gb1[j] >= 0) sb.taken[gb1[j]] = mark;
+                    if (gb0[j] >= 0) { sb.taken[gb0[j]] = mark; link_cut(sb, 2 * gk[j], gb0[j]); }
+                    if (gb1[j] >= 0) { sb.taken[gb1[j]] = mark; link_cut(sb, 2 * gk[j] + 1, gb1[j]); }
                     won++;
                 }
             }
@@ -473,8 +512,8 @@ __global__ void __launch_bounds__(SOLVER_THREADS) k_colour(DevWorld w, DevPairs 
                 if (!eligible(w, P, sb, k, mark, b0, b1)) continue;
                 if (holds_claims(w, sb, b0, b1, ctag(t, k))) {
                     sb.colourOf[k] = round;
-                    if (dyn(w, b0)) sb.taken[b0] = mark;
-                    if (dyn(w, b1)) sb.taken[b1] = mark;
+                    if (dyn(w, b0)) { sb.taken[b0] = mark; link_cut(sb, 2 * k, b0); }
+                    if (dyn(w, b1)) { sb.taken[b1] = mark; link_cut(sb, 2 * k + 1, b1); }
                     won++;
                 }
             }
@@ -532,32 +571,7 @@ __global__ void k_slots(DevWorld w, DevPairs P, SolverBuffers sb, DevRows R) {
     R.slot_desc[slot] = make_int4(b0, b1, 0, lb0 | (lb1 << 16));
 }
 
-// ---- row setup (solveGroupCacheFriendlySetup, java:418-786) -------------------------------
-struct BodyV { V lin, ang, com; float im; M iw; };
-
-JBD BodyV load_body(const DevWorld& w, int b) {
-    BodyV r;
-    r.lin = mk4(w.linvel[b]);
-    r.ang = mk4(w.angvel[b]);
-    r.com = mk(w.xr0[b].w, w.xr1[b].w, w.xr2[b].w);
-    r.im = w.iloc[b].w;
-    r.iw = load_iw(w, b);
-    return r;
-}
-
-JBD void friction_row(const DevRows& R, int fi, V dir, V rp1, V rp2, const BodyV& A, const BodyV& B, float impulse) {
-    V t1 = crs(rp1, dir), t2 = crs(rp2, dir);
-    V angA = mulMv(t1, A.iw), angB = mulMv(t2, B.iw);
-    float d0 = __fadd_rn(A.im, dot(dir, crs(angA, rp1)));
-    float d1 = __fadd_rn(B.im, dot(dir, crs(angB, rp2)));
-    float jac = jdiv(1.0f, __fadd_rn(d0, d1));
-    R.f_nrm[fi] = f4(dir, jac);
-    R.f_rp1[fi] = f4(t1, impulse);
-    R.f_rp2[fi] = f4(t2, 0.0f);
-    R.f_angA[fi] = f4(angA, 0.0f);
-    R.f_angB[fi] = f4(angB, 0.0f);
-}
-
+// ---- row setup (solveGroupCacheFriendlySetup, java:418-786; the arithmetic is in rows.cuh) -----
 // Points with rows (distance <= 0) of every slot: the mask into slot_desc.z and the count into
 // slot_pt0 (scanned afterwards into the slot's first point row); 0 beyond the candidates.
 __global__ void k_point_masks(DevPairs P, DevRows R, const int* nCandPtr, int nPairs) {
@@ -584,6 +598,25 @@ __global__ void k_point_rows(DevRows R, const int* nCandPtr) {
     R.slot_desc[s] = d;
 }
 
+// Where plane `plane` (rows.cuh) of row ni is kept.
+JBD float4* row_plane(const DevRows& R, int plane, int ni) {
+    switch (plane) {
+    case RP_N: return R.n_nrm + ni;
+    case RP_N1: return R.n_rp1 + ni;
+    case RP_N2: return R.n_rp2 + ni;
+    case RP_NA: return R.n_angA + ni;
+    case RP_NB: return R.n_angB + ni;
+    }
+    const int f = (plane - RP_F) / 5, fi = ni * 2 + f;
+    switch (plane - RP_F - 5 * f) {
+    case 0: return R.f_nrm + fi;
+    case 1: return R.f_rp1 + fi;
+    case 2: return R.f_rp2 + fi;
+    case 3: return R.f_angA + fi;
+    }
+    return R.f_angB + fi;
+}
+
 // Rows are stored per point, compactly: the rows of slot s are [pt0, pt0 + popcount(mask)),
 // one normal row per point and its two friction rows at 2 * row and 2 * row + 1.
 __global__ void k_setup(DevWorld w, DevPairs P, DevRows R, const int* nCandPtr, float dt) {
@@ -598,53 +631,8 @@ __global__ void k_setup(DevWorld w, DevPairs P, DevRows R, const int* nCandPtr, 
     int ni = desc.z >> 4;
     for (int j = 0; j < 4; j++) {
         if (!(mask & (1 << j))) continue;
-        int k = p * 4 + j;
-        float4 pa = P.pA[k];
-        float dist = pa.w;
-        float4 wa = P.wA[k], wb = P.wB[k], nr = P.nrm[k], im = P.imp[k];
-        V nrm = mk(nr.x, nr.y, nr.z);
-        V rp1 = sub(mk(wa.x, wa.y, wa.z), A.com), rp2 = sub(mk(wb.x, wb.y, wb.z), B.com);
-        V angA = mulMv(crs(rp1, nrm), A.iw);
-        V angB = mulMv(crs(rp2, nrm), B.iw);
-        float d0 = __fadd_rn(A.im, dot(nrm, crs(angA, rp1)));
-        float d1 = __fadd_rn(B.im, dot(nrm, crs(angB, rp2)));
-        float jac = jdiv(1.0f, __fadd_rn(d0, d1));
-        V rp1xn = crs(rp1, nrm), rp2xn = crs(rp2, nrm);
-        V vel1 = add(crs(A.ang, rp1), A.lin);
-        V vel2 = add(crs(B.ang, rp2), B.lin);
-        V vel = sub(vel1, vel2);
-        float rel_vel = dot(nrm, vel);
-        float pen = jmin(__fadd_rn(dist, w.slop), 0.0f);
-        float rest = __fmul_rn(wb.w, -rel_vel);
-        if (rest <= 0.0f) rest = 0.0f;
-        float penVel = jdiv(-pen, dt);
-        if (rest > penVel) pen = 0.0f;
-        float imp = warm ? __fmul_rn(nr.w, w.warm) : 0.0f;
         R.pt_key[ni] = (s << 2) | j;
-        R.n_nrm[ni] = f4(nrm, jac);
-        R.n_rp1[ni] = f4(rp1xn, jdiv(__fmul_rn(-pen, w.erp), dt));   // positionalError (java:248)
-        R.n_rp2[ni] = f4(rp2xn, rest);
-        R.n_angA[ni] = f4(angA, wa.w);   // friction coefficient
-        R.n_angB[ni] = f4(angB, imp);
-        V dir1, dir2;
-        if (im.z == 0.0f) {
-            dir1 = sub(vel, scl(nrm, rel_vel));
-            float lat = len2(dir1);
-            if (lat > FLT_EPS) {
-                dir1 = scl(dir1, jdiv(1.0f, jsqrt(lat)));
-                dir2 = nor(crs(dir1, nrm));
-            } else {
-                plane_space1(nrm, dir1, dir2);
-            }
-            P.d1[k] = f4(dir1, 0.0f);
-            P.d2[k] = f4(dir2, 0.0f);
-            P.imp[k] = make_float4(im.x, im.y, 1.0f, 0.0f);
-        } else {
-            dir1 = mk4(P.d1[k]);
-            dir2 = mk4(P.d2[k]);
-        }
-        friction_row(R, ni * 2 + 0, dir1, rp1, rp2, A, B, warm ? __fmul_rn(im.x, w.warm) : 0.0f);
-        friction_row(R, ni * 2 + 1, dir2, rp1, rp2, A, B, warm ? __fmul_rn(im.y, w.warm) : 0.0f);
+        point_rows(w, P, p * 4 + j, A, B, warm, dt, [&](int plane, float4 v) { *row_plane(R, plane, ni) = v; });
         ++ni;
     }
     R.slot_im[s] = make_float2(A.im, B.im);
@@ -654,20 +642,6 @@ __global__ void k_setup(DevWorld w, DevPairs P, DevRows R, const int* nCandPtr, 
 }
 
 // ---- PGS (cooperative) ---------------------------------------------------------------------
-JBD void apply_imp(V& lin, V& ang, V n, float im, V angc, float imp) {   // SolverBody.internalApplyImpulse
-    if (im != 0.0f) {
-        V lc = scl(n, im);
-        lin.x = __fadd_rn(lin.x, __fmul_rn(imp, lc.x));
-        lin.y = __fadd_rn(lin.y, __fmul_rn(imp, lc.y));
-        lin.z = __fadd_rn(lin.z, __fmul_rn(imp, lc.z));
-        ang.x = __fadd_rn(ang.x, __fmul_rn(imp, angc.x));
-        ang.y = __fadd_rn(ang.y, __fmul_rn(imp, angc.y));
-        ang.z = __fadd_rn(ang.z, __fmul_rn(imp, angc.z));
-    }
-}
-
-enum { PH_WARM = 0, PH_NORMAL = 1, PH_FRICTION = 2 };
-
 // Largest |delta lambda| and |lambda| a thread has seen in the current iteration (the
 // residual of the residual-terminated mode).  `x > m` keeps NaN out, as the oracle does.
 struct Resid {
@@ -811,19 +785,8 @@ JBD void solve_manifold(const DevWorld& w, const DevRows& R, int s, int z, int k
                 nn = ld_ro(R.n_nrm + ni); r1 = ld_ro(R.n_rp1 + ni); r2 = ld_ro(R.n_rp2 + ni); aA = ld_ro(R.n_angA + ni);
                 aB = ld_rw(R.n_angB + ni);
             }
-            V n = mk(nn.x, nn.y, nn.z);
-            float vel1 = __fadd_rn(dot(n, l0), dot(mk(r1.x, r1.y, r1.z), a0));
-            float vel2 = __fadd_rn(dot(n, l1), dot(mk(r2.x, r2.y, r2.z), a1));
-            float rel = __fsub_rn(vel1, vel2);
-            float posErr = r1.w;          // -penetration * erp / timeStep, formed once by the setup
-            float velErr = __fsub_rn(r2.w, rel);
-            float ni1 = __fadd_rn(__fmul_rn(posErr, nn.w), __fmul_rn(velErr, nn.w));
-            float old = aB.w;
-            float sum = __fadd_rn(old, ni1);
-            float acc = 0.0f > sum ? 0.0f : sum;
-            float d = __fsub_rn(acc, old);
-            apply_imp(l0, a0, n, im0, mk(aA.x, aA.y, aA.z), d);
-            apply_imp(l1, a1, n, im1, mk(aB.x, aB.y, aB.z), -d);
+            float acc;
+            const float d = solve_normal_row(nn, r1, r2, aA, aB, aB.w, l0, a0, l1, a1, im0, im1, acc);
             aB.w = acc;
             __stcg(&R.n_angB[ni], aB);
             if (TRACK) res.add(d, acc);
@@ -860,21 +823,10 @@ JBD void solve_manifold(const DevWorld& w, const DevRows& R, int s, int z, int k
             }
             for (int f = 0; f < 2; f++) {
                 int fi = ni * 2 + f;
-                const float4 fn = fnv[f];
                 float4 r1 = r1v[f];
-                const float4 r2 = r2v[f];
-                V n = mk(fn.x, fn.y, fn.z);
-                float vel1 = __fadd_rn(dot(n, l0), dot(mk(r1.x, r1.y, r1.z), a0));
-                float vel2 = __fadd_rn(dot(n, l1), dot(mk(r2.x, r2.y, r2.z), a1));
-                float rel = __fsub_rn(vel1, vel2);
-                float j1 = __fmul_rn(-rel, fn.w);
-                float old = r1.w;
-                float acc = __fadd_rn(old, j1);
-                if (limit < acc) acc = limit;
-                else if (acc < -limit) acc = -limit;
-                j1 = __fsub_rn(acc, old);
-                apply_imp(l0, a0, n, im0, mk4(fav[f]), j1);
-                apply_imp(l1, a1, n, im1, mk4(fbv[f]), -j1);
+                float acc;
+                const float j1 = solve_friction_row(fnv[f], r1, r2v[f], fav[f], fbv[f], r1.w, limit, l0, a0, l1, a1, im0,
+                                                    im1, acc);
                 r1.w = acc;
                 __stcg(&R.f_rp1[fi], r1);
                 if (TRACK) res.add(j1, acc);
@@ -2139,7 +2091,7 @@ template <class T> static void sfree(T*& p) { if (p) cudaFree((void*)p); p = nul
 static size_t pgs_smem(const SolverBuffers& sb) {
     return (sb.partSmem ? (size_t)sb.smemCap * 32 : 0) + (size_t)3 * sb.poolPts * POOL_F4 * 16;
 }
-static size_t colour_smem(const SolverBuffers& sb) { return (size_t)sb.partMax * (sizeof(unsigned long long) + sizeof(int)); }
+static size_t colour_smem(const SolverBuffers& sb) { return (size_t)sb.partMax * (sizeof(unsigned long long) + 2 * sizeof(int)); }
 
 int solver_configure(SolverBuffers& sb, int nFinite, const std::vector<int>& worldCounts, int sms, int rangeParts,
                      int threads, int smemBodies) {
@@ -2165,17 +2117,16 @@ int solver_configure(SolverBuffers& sb, int nFinite, const std::vector<int>& wor
     int partMax = 1;
     for (int p = 0; p < parts; p++) partMax = std::max(partMax, start[p + 1] - start[p]);
     if (parts > sb.partsCap) {
-        sfree(sb.bucketCount); sfree(sb.bucketFill); sfree(sb.bucketStart);
         sfree(sb.lcCount); sfree(sb.lcFill); sfree(sb.lcStart); sfree(sb.nLocal); sfree(sb.partStart); sfree(sb.partOrder);
         size_t lc = (size_t)parts * (MAX_LOCAL + 1);
-        if (salloc(&sb.bucketCount, parts + 2) || salloc(&sb.bucketFill, parts + 2) || salloc(&sb.bucketStart, parts + 2) ||
-            salloc(&sb.lcCount, lc) || salloc(&sb.lcFill, lc) || salloc(&sb.lcStart, lc) || salloc(&sb.nLocal, parts) ||
+        if (salloc(&sb.lcCount, lc) || salloc(&sb.lcFill, lc) || salloc(&sb.lcStart, lc) || salloc(&sb.nLocal, parts) ||
             salloc(&sb.partStart, parts + 1) || salloc(&sb.partOrder, parts)) {
             sb.partsCap = 0;
             return JBGPU_ERR_CUDA;
         }
         sb.partsCap = parts;
     }
+    if (flow_plan(sb, start, sms)) return JBGPU_ERR_CUDA;
     std::vector<int> order(parts);
     for (int p = 0; p < parts; p++) order[p] = p;
     std::stable_sort(order.begin(), order.end(),
@@ -2216,13 +2167,13 @@ int solver_configure(SolverBuffers& sb, int nFinite, const std::vector<int>& wor
         return JBGPU_ERR_CUDA;
     sb.gridPgs = std::min(parts, perPgs * sms);
     sb.gridColour = std::min(parts, perColour * sms);
-    return JBGPU_OK;
+    return flow_configure(sb, sms, smemBodies) ? JBGPU_ERR_CUDA : JBGPU_OK;
 }
 
 void solver_free(SolverBuffers& sb) {
-    sfree(sb.bucketCount); sfree(sb.bucketFill); sfree(sb.bucketStart);
     sfree(sb.lcCount); sfree(sb.lcFill); sfree(sb.lcStart); sfree(sb.nLocal); sfree(sb.partStart); sfree(sb.partOrder);
     sfree(sb.orderFallback);
+    flow_free(sb);
     sb.partsCap = 0;
 }
 
@@ -2263,11 +2214,15 @@ void solve_launch_learn(const DevWorld& w, DevPairs& P, int nPairs, DevRows& R, 
         return;
     }
     const int parts = sb.nParts;
+    // the flow solver takes every solve of a fixed number of iterations without joints or learning
+    sb.flowOn = sb.flowOk && w.resTol <= 0.0f && w.numIter <= FLOW_MAX_ITERATIONS && sb.J.n == 0 && !learn.mlp &&
+                !learn.sampleX && !learn.sampleT;
     cudaMemsetAsync(sb.claim, 0xff, sizeof(unsigned long long) * w.nBodies, s);
     cudaMemsetAsync(sb.taken, 0xff, sizeof(int) * w.nBodies, s);
     cudaMemsetAsync(sb.posOf, 0xff, sizeof(int) * w.nBodies, s);
-    cudaMemsetAsync(sb.bucketCount, 0, sizeof(int) * (parts + 2), s);
-    cudaMemsetAsync(sb.bucketFill, 0, sizeof(int) * (parts + 2), s);
+    const int buckets = parts + 2 + (sb.flowOn ? sb.nFlow + 1 : 0);   // the colouring's buckets, then the flow solver's
+    cudaMemsetAsync(sb.bucketCount, 0, sizeof(int) * buckets, s);
+    cudaMemsetAsync(sb.bucketFill, 0, sizeof(int) * buckets, s);
     cudaMemsetAsync(sb.lcFill, 0, sizeof(int) * parts * (MAX_LOCAL + 1), s);
     cudaMemsetAsync(sb.colourFill, 0, sizeof(int) * (MAX_COLOURS + 1), s);
     cudaMemsetAsync(w.ctr + C_BAR_COUNT, 0, sizeof(int), s);
@@ -2275,7 +2230,7 @@ void solve_launch_learn(const DevWorld& w, DevPairs& P, int nPairs, DevRows& R, 
     cudaMemsetAsync(w.ctr + C_ISL_N, 0, sizeof(int) * 5, s);   // island statistics, part counters
     k_posof<<<gridn(sb.nFinite, 256), 256, 0, s>>>(sb); note_launch();
     k_classify<<<gridn(nPairs, 256), 256, 0, s>>>(w, P, sb); note_launch();
-    exclusive_scan(sb.bucketCount, sb.bucketStart, nullptr, parts + 2, sb.scanScratch, s);
+    exclusive_scan(sb.bucketCount, sb.bucketStart, nullptr, buckets, sb.flowScan, s);
     k_bucket_scatter<<<gridn(nPairs, 256), 256, 0, s>>>(sb); note_launch();
     {
         DevWorld wc = w;
@@ -2283,6 +2238,12 @@ void solve_launch_learn(const DevWorld& w, DevPairs& P, int nPairs, DevRows& R, 
         SolverBuffers sc = sb;
         void* args[] = {&wc, &pc, &sc};
         cudaLaunchCooperativeKernel((void*)k_colour, sb.gridColour, sb.threads, args, colour_smem(sb), s); note_launch();
+    }
+    if (sb.flowOn) {
+        if (prof) { prof->mark(PH_COLOUR, 1, s); prof->mark(PH_SETUP, 0, s); prof->mark(PH_SETUP, 1, s); prof->mark(PH_PGS, 0, s); }
+        flow_launch(w, P, nPairs, R, sb, dt, s);
+        if (prof) prof->mark(PH_PGS, 1, s);
+        return;
     }
     k_slots<<<gridn(nPairs, 256), 256, 0, s>>>(w, P, sb, R); note_launch();
     if (w.resTol > 0.0f) {        // residual mode: slots grouped by island

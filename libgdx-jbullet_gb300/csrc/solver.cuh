@@ -121,6 +121,31 @@ struct SolverBuffers {
     int gridPgs = 0;
     int threads = SOLVER_THREADS;
     DevJoints J;                  // point-to-point joints
+    // flow solver (solver_flow.cu)
+    int* execOf = nullptr;        // per candidate: the flow block that solves it
+    int* prevLink = nullptr;      // per candidate and side: link of the body's candidate before it (-1: first)
+    int* nextLink = nullptr;      // ... after it (-1: last)
+    int* firstLink = nullptr;     // per body: its first and last candidate's links, written for
+    int* lastLink = nullptr;      // bodies that have candidates
+    float4* exch = nullptr;       // per body: velocities handed from block to block, tags in .w
+    int* flowCount = nullptr;     // the nFlow + 1 entries after bucketCount / bucketFill / bucketStart
+    int* flowFill = nullptr;
+    int* flowStart = nullptr;
+    int* flowCand = nullptr;      // what a flow block needs of its candidates, grouped by block (8 ints each)
+    int* flowDesc = nullptr;      // a block's sorted slots and groups when shared memory is too small (FLOW_DESC_INTS each)
+    int2* flowPart = nullptr;     // per part: its first flow block, bodies per block
+    int* flowBody = nullptr;      // nFlow + 1 positions of the body order
+    int* flowOrder = nullptr;     // flow blocks in the order they are taken
+    void* flowScan = nullptr;     // scan scratch of the buckets
+    int* flowTop = nullptr;       // device scalars: next block, rows kept outside shared memory
+    int rowStride = 0;            // points a plane of the row arrays holds (4 x pair capacity)
+    int nFlow = 0, flowCap = 0;
+    int gridFlow = 0;
+    int flowSmem = 0;             // dynamic shared memory of a flow block
+    int flowExch = 0;             // some body's manifolds lie in two blocks
+    int flowOk = 0;               // the flow solver takes this world's parts
+    int flowOn = 0;               // ... and this solve
+    int movingStatic = 0;         // a static or kinematic body has an inverse mass (set by the world)
 };
 
 // (Re)plans the parts for nFinite ordered bodies.  worldCounts: finite bodies per batch world;
@@ -136,6 +161,16 @@ void islands_launch_select(const DevWorld& w, const DevPairs& P, int nPairs, Sol
 void solve_launch(const DevWorld& w, DevPairs& P, int nPairs, DevRows& rows, SolverBuffers& sb, float dt, cudaStream_t s,
                   const Prof* prof = nullptr);
 void solver_free(SolverBuffers& sb);
+
+// Flow solver (solver_flow.cu).  flow_plan lays out its blocks over the parts (start: nParts + 1
+// positions) and allocates the bucket tables, flow_configure chooses its launch.  Both return
+// nonzero when a CUDA call failed.
+constexpr int FLOW_DESC_INTS = 12;           // a slot's 8 ints and its group's word, kept 16-byte aligned
+constexpr int FLOW_MAX_ITERATIONS = 500000;   // its phase tags are 32 bits
+int flow_plan(SolverBuffers& sb, const std::vector<int>& start, int sms);
+int flow_configure(SolverBuffers& sb, int sms, int smemBodies);
+void flow_free(SolverBuffers& sb);
+void flow_launch(const DevWorld& w, DevPairs& P, int nPairs, DevRows& R, SolverBuffers& sb, float dt, cudaStream_t s);
 
 // Learned warm start and contact samples (solver.cu): per contact point q = slot * 4 + point,
 // 24 features (X) before the solve and the 3 converged impulses (T) after it.

@@ -197,12 +197,16 @@ void free_pairs(DevPairs& P) {
 int alloc_pair_work(jbgpu_world* w, int cap) {
     graphs_clear(w);
     DevRows& R = w->rows;
-    dfree(R.n_nrm); dfree(R.n_rp1); dfree(R.n_rp2); dfree(R.n_angA); dfree(R.n_angB);
-    dfree(R.f_nrm); dfree(R.f_rp1); dfree(R.f_rp2); dfree(R.f_angA); dfree(R.f_angB);
+    dfree(R.planes);
     dfree(R.slot_pair); dfree(R.slot_desc); dfree(R.slot_im); dfree(R.slot_pt0); dfree(R.pt_key);
     size_t c4 = (size_t)cap * 4, c8 = (size_t)cap * 8;
-    CK(dalloc(&R.n_nrm, c4)); CK(dalloc(&R.n_rp1, c4)); CK(dalloc(&R.n_rp2, c4)); CK(dalloc(&R.n_angA, c4)); CK(dalloc(&R.n_angB, c4));
-    CK(dalloc(&R.f_nrm, c8)); CK(dalloc(&R.f_rp1, c8)); CK(dalloc(&R.f_rp2, c8)); CK(dalloc(&R.f_angA, c8)); CK(dalloc(&R.f_angB, c8));
+    CK(dalloc(&R.planes, 15 * c4));
+    {
+        float4* p = R.planes;
+        for (float4** n : {&R.n_nrm, &R.n_rp1, &R.n_rp2, &R.n_angA, &R.n_angB}) { *n = p; p += c4; }
+        for (float4** f : {&R.f_nrm, &R.f_rp1, &R.f_rp2, &R.f_angA, &R.f_angB}) { *f = p; p += c8; }
+    }
+    w->sb.rowStride = (int)std::min<size_t>(c4, 0x7fffffff);
     CK(dalloc(&R.slot_pair, cap)); CK(dalloc(&R.slot_desc, cap)); CK(dalloc(&R.slot_im, cap));
     CK(dalloc(&R.slot_pt0, cap)); CK(dalloc(&R.pt_key, c4));
     SolverBuffers& S = w->sb;
@@ -212,6 +216,9 @@ int alloc_pair_work(jbgpu_world* w, int cap) {
     CK(dalloc(&S.bucket, cap)); CK(dalloc(&S.bucketList, cap));
     CK(dalloc(&S.md, cap)); CK(dalloc(&S.ml, cap)); CK(dalloc(&S.slotIsl, cap)); CK(dalloc(&S.islList, cap));
     CK(dalloc(&S.candLocal, cap));
+    dfree(S.execOf); dfree(S.prevLink); dfree(S.nextLink); dfree(S.flowCand); dfree(S.flowDesc);
+    CK(dalloc(&S.execOf, cap)); CK(dalloc(&S.prevLink, 2 * (size_t)cap)); CK(dalloc(&S.nextLink, 2 * (size_t)cap));
+    CK(dalloc(&S.flowCand, 8 * (size_t)cap)); CK(dalloc(&S.flowDesc, FLOW_DESC_INTS * (size_t)cap));
     CK(dalloc(&S.islChunk, (size_t)cap + std::max(w->capBodies, 1)));
     if (S.scanScratch) cudaFree(S.scanScratch);
     CK(cudaMalloc(&S.scanScratch, scan_scratch_bytes(cap)));
@@ -270,6 +277,8 @@ int grow_bodies(jbgpu_world* w, int need) {
     dfree(S.islConv); dfree(S.islAcc); dfree(S.islDone);
     CK(dalloc(&S.parent, nc)); CK(dalloc(&S.keepAwake, nc)); CK(dalloc(&S.inactive, nc)); CK(dalloc(&S.claim, nc));
     CK(dalloc(&S.taken, nc)); CK(dalloc(&S.posOf, nc));
+    dfree(S.firstLink); dfree(S.lastLink); dfree(S.exch);
+    CK(dalloc(&S.firstLink, nc)); CK(dalloc(&S.lastLink, nc)); CK(dalloc(&S.exch, 2 * (size_t)nc));
     CK(dalloc(&S.islCount, nc + 1)); CK(dalloc(&S.islFill, nc + 1)); CK(dalloc(&S.islStart, nc + 1));
     CK(dalloc(&S.segFlag, nc + 1)); CK(dalloc(&S.segIdx, nc + 1)); CK(dalloc(&S.islConv, nc));
     CK(dalloc(&S.islAcc, 2 * (size_t)nc)); CK(dalloc(&S.islDone, nc));
@@ -1324,8 +1333,7 @@ int jbgpu_world_destroy(jbgpu_world* w) {
     free_pairs(w->pairs[0]);
     free_pairs(w->pairs[1]);
     DevRows& R = w->rows;
-    dfree(R.n_nrm); dfree(R.n_rp1); dfree(R.n_rp2); dfree(R.n_angA); dfree(R.n_angB);
-    dfree(R.f_nrm); dfree(R.f_rp1); dfree(R.f_rp2); dfree(R.f_angA); dfree(R.f_angB);
+    dfree(R.planes);
     dfree(R.slot_pair); dfree(R.slot_desc); dfree(R.slot_im); dfree(R.slot_pt0); dfree(R.pt_key); dfree(R.nPts);
     BroadphaseBuffers& B = w->bb;
     dfree(B.bounds); dfree(B.mkeys); dfree(B.mkeys_alt); dfree(B.sortedBody); dfree(B.vals_alt);
@@ -1341,6 +1349,7 @@ int jbgpu_world_destroy(jbgpu_world* w) {
     if (N.scanScratch) cudaFree(N.scanScratch);
     SolverBuffers& V = w->sb;
     dfree(V.parent); dfree(V.keepAwake); dfree(V.inactive); dfree(V.flag); dfree(V.candIdx); dfree(V.cand); dfree(V.colourOf);
+    dfree(V.execOf); dfree(V.prevLink); dfree(V.nextLink); dfree(V.flowCand); dfree(V.flowDesc); dfree(V.firstLink); dfree(V.lastLink); dfree(V.exch);
     dfree(V.bucket); dfree(V.bucketList); dfree(V.claim); dfree(V.taken); dfree(V.posOf); dfree(V.candLocal);
     dfree(V.md); dfree(V.ml); dfree(V.slotIsl); dfree(V.islList); dfree(V.islCount); dfree(V.islFill); dfree(V.islStart);
     dfree(V.segFlag); dfree(V.segIdx); dfree(V.islChunk); dfree(V.islConv); dfree(V.islAcc); dfree(V.islDone);
@@ -1549,6 +1558,7 @@ int jbgpu_world_add_bodies(jbgpu_world* w, const jbgpu_body_desc* b, int32_t n, 
         if (d.activation_state != 0) act[i] = d.activation_state;
         float im;
         if (d.mass == 0.0f) { f |= CF_STATIC; im = 0.0f; } else im = 1.0f / d.mass;
+        if ((f & CF_KINEMATIC) && im != 0.0f) w->sb.movingStatic = 1;
         if (w->shapes[d.shape].type == JBGPU_SHAPE_STATIC_PLANE || w->shapes[d.shape].type == JBGPU_SHAPE_TRIANGLE_MESH)
             f |= CF_LISTED;
         float il[3];
