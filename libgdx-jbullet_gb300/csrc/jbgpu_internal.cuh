@@ -21,10 +21,13 @@ enum { ST_CAPACITY = 1, ST_EPA_POOL = 2, ST_TIMEOUT = 4, ST_NONFINITE = 8, ST_BA
 // Counters kept on the device (indices into DevWorld::ctr).
 enum {
     C_PAIRS = 0, C_FILL_OVERFLOW, C_EPA_QUEUE, C_GJK, C_EPA, C_SOLVE_N, C_COLOURS, C_ISLANDS,
-    C_MANIFOLDS, C_CONTACTS, C_ROWS, C_STATUS, C_BAR_COUNT, C_BAR_GEN, C_CUT_DONE, C_WIN0, C_WIN1, C_WIN2,
-    C_PGS_ITERS, C_CUT_COLOURS, C_CUT_MANIFOLDS, C_RES0, C_RES1, C_RES2, C_ISL_N, C_ISL_CONV, C_ISL_ITERS,
-    C_PART_NEXT0, C_PART_NEXT1, C_CCD_N, C_CCD_BEST, C_NCTR = 32
+    C_MANIFOLDS, C_CONTACTS, C_ROWS, C_STATUS, C_BAR_GEN, C_WIN0, C_WIN1, C_WIN2,
+    C_CUT_COLOURS, C_CUT_MANIFOLDS, C_RES0, C_RES1, C_RES2,
+    // cleared together at the start of a solve (C_SOLVE_FIRST .. C_SOLVE_LAST)
+    C_BAR_COUNT, C_PGS_ITERS, C_ISL_N, C_ISL_CONV, C_ISL_ITERS, C_PART_NEXT0, C_PART_NEXT1, C_COL_FAIL, C_CUT_DONE,
+    C_CCD_N, C_CCD_BEST, C_NCTR = 32
 };
+constexpr int C_SOLVE_FIRST = C_BAR_COUNT, C_SOLVE_COUNT = C_CUT_DONE - C_BAR_COUNT + 1;
 
 struct DevShapes {
     int* type;

@@ -258,9 +258,18 @@ __global__ void k_classify(DevWorld w, DevPairs P, SolverBuffers sb) {
         if (d1) lb1 = sb.posOf[b1] - ps;
     }
     sb.candLocal[k] = lb0 | (lb1 << 16);
+    // the candidate into its dynamic bodies' lists, for its places among theirs (first_fit_part)
+    const unsigned entry = (unsigned)k | (q == sb.nParts ? COL_CUT : 0u);
+    for (int side = 0; side < 2; side++) {
+        if (!(side ? d1 : d0)) continue;
+        const int b = side ? b1 : b0, at = atomicAdd(&sb.bodyDeg[b], 1);
+        if (at < COL_LIST) sb.bodyList[(size_t)b * COL_LIST + at] = entry;
+        else w.ctr[C_COL_FAIL] = 1;
+    }
     if (sb.flowOn) {
         const int e = flow_home(w, sb, d0 ? b0 : b1);   // the block that solves it (solver_flow.cu)
         sb.execOf[k] = e;
+        sb.candHome[k] = (unsigned char)((d0 ? 1 : 0) | (d1 && (!d0 || flow_home(w, sb, b1) == e) ? 2 : 0));
         if (e >= 0) {
             const unsigned ge = __match_any_sync(__activemask(), e);
             if ((threadIdx.x & 31) == __ffs(ge) - 1) atomicAdd(&sb.flowCount[e], __popc(ge));
@@ -300,7 +309,7 @@ JBD int next_part(const DevWorld& w, const SolverBuffers& sb, int counter, int* 
 }
 
 // ---- colouring (cooperative) ---------------------------------------------------------------
-// Each colour is grown to a maximal set by claim passes: every dynamic body is claimed by the
+// By claim passes (colour_claims; first_fit_part gives the same colours): each colour is grown to a maximal set by claim passes: every dynamic body is claimed by the
 // lowest candidate index touching it among the eligible candidates (uncoloured, no dynamic body
 // taken by the colour yet); candidates holding all their claims join the colour and take their
 // bodies; passes repeat until one adds nothing (at most MAX_SUB).  Manifolds internal to a part
@@ -337,23 +346,258 @@ JBD void link_cut(const SolverBuffers& sb, int me, int body) {
     __stcg(&sb.lastLink[body], link_after(sb, __ldcg(&sb.lastLink[body]), me, &body));
 }
 
-__global__ void __launch_bounds__(SOLVER_THREADS) k_colour(DevWorld w, DevPairs P, SolverBuffers sb) {
-    unsigned barK = 0;
+// ---- colouring as a dataflow -----------------------------------------------------------------
+// The claim passes below give every candidate the lowest colour that no earlier candidate (by
+// index) of its class - internal to a part, or cut - on one of its bodies holds, as long as no
+// colour needs more than MAX_SUB passes: a maximal independent set grown by lowest index is the
+// first in index order.  So a candidate can be coloured once the candidates before it on its two
+// bodies are: each body carries a token - the colours used so far and how many candidates have
+// passed - and a candidate takes its bodies' tokens when the count equals its place in the body's
+// list.  Tokens of a part's candidates live in shared memory, those of cut candidates in global
+// memory, 16 bytes written whole.  No barrier stands between colours or passes.
+// The token also bounds the pass in which the claim passes would have coloured its candidates: a
+// candidate joins one pass after the last earlier neighbour with a higher colour became ineligible,
+// which was at the latest when the highest of that one's earlier neighbours joined.  A bound of
+// MAX_SUB passes, a body with more than COL_LIST candidates or 64 colours send the step to the
+// claim passes (C_COL_FAIL).
+// What bounds it: the longest chain of candidates by index (21 at 1,000 boxes, 28 at 4,000 hulls),
+// each link a shared-memory or L2 round trip; the claim passes took about 50 passes of two or three
+// barriers.  Colouring phase, 1,000 boxes 233 -> 96 us, 4,000 hulls 324 -> 95, 20k bodies 303 -> 99,
+// 100k 370 -> 151, 444k in 1,024 worlds 789 -> 316.
+struct ColToken { unsigned lo, hi, jq, count; };   // colours used, latest join pass | latest of a neighbour << 8, candidates passed
+
+// The colour of a candidate that holds tokens a and b (empty for a static side), which it updates;
+// -1: no colour, or its pass may be beyond the claim passes' limit.
+JBD int take_colour(ColToken& a, ColToken& b) {
+    const unsigned long long used = (unsigned long long)(a.hi | b.hi) << 32 | (a.lo | b.lo);
+    if (used == ~0ull) return -1;
+    const int c = __ffsll((long long)~used) - 1;
+    const unsigned j0 = a.jq & 0xffu, j1 = b.jq & 0xffu, q0 = a.jq >> 8, q1 = b.jq >> 8;
+    const unsigned j = (used >> c) != 0 ? 1 + max(q0, q1) : 0, q = max(j0, j1);
+    if (j >= MAX_SUB) return -1;
+    const unsigned long long bit = 1ull << c;
+    a.lo |= (unsigned)bit; a.hi |= (unsigned)(bit >> 32);
+    b.lo |= (unsigned)bit; b.hi |= (unsigned)(bit >> 32);
+    a.jq = max(j0, j) | max(q0, q) << 8;
+    b.jq = max(j1, j) | max(q1, q) << 8;
+    a.count++;
+    b.count++;
+    return c;
+}
+
+// The places of candidate k among the candidates of its class on its bodies (rank0 | rank1 << 16).
+JBD int list_rank(const SolverBuffers& sb, int b, unsigned entry) {
+    const int n = min(sb.bodyDeg[b], COL_LIST);
+    const unsigned* l = sb.bodyList + (size_t)b * COL_LIST;
+    int r = 0;
+    for (int i = 0; i < n; i++) r += l[i] < entry && (l[i] & COL_CUT) == (entry & COL_CUT);
+    return r;
+}
+
+// Internal candidates of the part, tokens in shared memory (tok), home colours in home (2 words a
+// body).  Every thread goes over its candidates until all have passed; false when the step failed.
+JBD bool first_fit_part(const DevWorld& w, const DevPairs& P, const SolverBuffers& sb, int part, uint4* tok, unsigned* home,
+                        int* shFail, int& most) {
+    constexpr int NONE = 0xffff;
+    const int s0 = sb.bucketStart[part], s1 = sb.bucketStart[part + 1];
+    const int np = sb.partStart[part + 1] - sb.partStart[part];
+    const int* order0 = sb.order + sb.partStart[part];
+    for (int i = threadIdx.x; i < np; i += blockDim.x) {
+        tok[i] = make_uint4(0, 0, 0, 0);
+        home[2 * i] = home[2 * i + 1] = 0;
+    }
+    if (threadIdx.x == 0) *shFail = 0;
+    int ck[COL_REG], cl[COL_REG], cr[COL_REG];
+    unsigned left = 0;
+    auto ranks = [&](int k, int l) {
+        const int l0 = l & 0xffff, l1 = l >> 16 & 0xffff;
+        return (l0 != NONE ? list_rank(sb, order0[l0], (unsigned)k) : 0) |
+               (l1 != NONE ? list_rank(sb, order0[l1], (unsigned)k) : 0) << 16;
+    };
+#pragma unroll
+    for (int j = 0; j < COL_REG; j++) {
+        const int i = s0 + threadIdx.x + j * (int)blockDim.x;
+        ck[j] = i < s1 ? sb.bucketList[i] : -1;
+        cl[j] = ck[j] >= 0 ? sb.candLocal[ck[j]] : 0;
+        cr[j] = ck[j] >= 0 ? ranks(ck[j], cl[j]) : 0;
+        left += ck[j] >= 0;
+    }
+    // a part with more candidates than COL_REG x blockDim: the others through memory, their ranks in
+    // candRank, not yet coloured ones marked -1
+    const int sx = s0 + COL_REG * (int)blockDim.x;
+    for (int i = sx + threadIdx.x; i < s1; i += blockDim.x) {
+        const int k = sb.bucketList[i];
+        sb.candRank[k] = ranks(k, sb.candLocal[k]);
+        sb.colourOf[k] = -1;
+        left++;
+    }
+    __syncthreads();
+    auto attempt = [&](int k, int l, int r) {   // 1: coloured, 0: not yet, -1: failed
+        const int l0 = l & 0xffff, l1 = l >> 16 & 0xffff;
+        ColToken a{0, 0, 0, 0}, b{0, 0, 0, 0};
+        if (l0 != NONE) {
+            const uint4 t = ld_whole(tok + l0);
+            if (t.w != (unsigned)(r & 0xffff)) return 0;
+            a = ColToken{t.x, t.y, t.z, t.w};
+        }
+        if (l1 != NONE) {
+            const uint4 t = ld_whole(tok + l1);
+            if (t.w != (unsigned)(r >> 16)) return 0;
+            b = ColToken{t.x, t.y, t.z, t.w};
+        }
+        const int c = take_colour(a, b);
+        if (c < 0) return -1;
+        if (l0 != NONE) st_whole(tok + l0, make_uint4(a.lo, a.hi, a.jq, a.count));
+        if (l1 != NONE) st_whole(tok + l1, make_uint4(b.lo, b.hi, b.jq, b.count));
+        sb.colourOf[k] = c;
+        most = max(most, c + 1);
+        if (sb.flowOn) {
+            const int f = sb.candHome[k];
+            if (l0 != NONE && (f & 1)) atomicOr(&home[2 * l0 + (c >> 5)], 1u << (c & 31));
+            if (l1 != NONE && (f & 2)) atomicOr(&home[2 * l1 + (c >> 5)], 1u << (c & 31));
+        } else {
+            atomicAdd(&sb.lcCount[part * (MAX_LOCAL + 1) + c], 1);
+        }
+        return 1;
+    };
+    volatile int* fail = shFail;
+    for (int sweep = 0; left > 0 && !*fail; sweep++) {
+#pragma unroll
+        for (int j = 0; j < COL_REG; j++) {
+            if (ck[j] < 0) continue;
+            const int got = attempt(ck[j], cl[j], cr[j]);
+            if (got < 0) *fail = 1;
+            if (got > 0) { ck[j] = -1; left--; }
+        }
+        for (int i = sx + threadIdx.x; i < s1; i += blockDim.x) {
+            const int k = sb.bucketList[i];
+            if (sb.colourOf[k] >= 0) continue;
+            const int got = attempt(k, sb.candLocal[k], sb.candRank[k]);
+            if (got < 0) *fail = 1;
+            left -= got > 0;
+        }
+        if (sweep > COL_SWEEPS) { atomicOr(&w.ctr[C_STATUS], ST_TIMEOUT); *fail = 1; }
+    }
+    __syncthreads();
+    if (*fail) return false;
+    if (sb.flowOn)
+        for (int i = threadIdx.x; i < np; i += blockDim.x)
+            sb.localMask[order0[i]] = make_uint4(tok[i].x, tok[i].y, home[2 * i], home[2 * i + 1]);
+    return true;
+}
+
+// Cut candidates, grid-wide, tokens in global memory.
+JBD bool first_fit_cut(const DevWorld& w, const DevPairs& P, const SolverBuffers& sb, int c0, int c1, int tid, int nth,
+                       int& most) {
+    int ck[COL_REG], cb0[COL_REG], cb1[COL_REG], cr[COL_REG];
+    unsigned left = 0;
+    // cut candidates have two dynamic bodies, but one of them may have no place in the body order
+    auto fetch = [&](int k, int& b0, int& b1, int& r) {
+        const int p = sb.cand[k];
+        b0 = P.b0[p];
+        b1 = P.b1[p];
+        if (!dyn(w, b0)) b0 = -1;
+        if (!dyn(w, b1)) b1 = -1;
+        r = (b0 >= 0 ? list_rank(sb, b0, (unsigned)k | COL_CUT) : 0) | (b1 >= 0 ? list_rank(sb, b1, (unsigned)k | COL_CUT) : 0) << 16;
+    };
+#pragma unroll
+    for (int j = 0; j < COL_REG; j++) {
+        const int i = c0 + tid + j * nth;
+        ck[j] = i < c1 ? sb.bucketList[i] : -1;
+        cb0[j] = cb1[j] = -1;
+        cr[j] = 0;
+        if (ck[j] >= 0) { fetch(ck[j], cb0[j], cb1[j], cr[j]); left++; }
+    }
+    const int cx = c0 + COL_REG * nth;
+    for (int i = cx + tid; i < c1; i += nth) { sb.colourOf[sb.bucketList[i]] = -1; left++; }
+    auto attempt = [&](int k, int b0, int b1, int r) {
+        ColToken a{0, 0, 0, 0}, b{0, 0, 0, 0};
+        if (b0 >= 0) {
+            const uint4 t = ld_whole_gpu(sb.cutToken + b0);
+            if (t.w != (unsigned)(r & 0xffff)) return 0;
+            a = ColToken{t.x, t.y, t.z, t.w};
+        }
+        if (b1 >= 0) {
+            const uint4 t = ld_whole_gpu(sb.cutToken + b1);
+            if (t.w != (unsigned)(r >> 16)) return 0;
+            b = ColToken{t.x, t.y, t.z, t.w};
+        }
+        const int c = take_colour(a, b);
+        if (c < 0) return -1;
+        if (b0 >= 0) st_whole_gpu(sb.cutToken + b0, make_uint4(a.lo, a.hi, a.jq, a.count));
+        if (b1 >= 0) st_whole_gpu(sb.cutToken + b1, make_uint4(b.lo, b.hi, b.jq, b.count));
+        sb.colourOf[k] = c;
+        most = max(most, c + 1);
+        if (sb.flowOn) {
+            const int f = sb.candHome[k];
+            if (b0 >= 0 && (f & 1)) atomicOr(&sb.cutHome[2 * b0 + (c >> 5)], 1u << (c & 31));
+            if (b1 >= 0 && (f & 2)) atomicOr(&sb.cutHome[2 * b1 + (c >> 5)], 1u << (c & 31));
+        } else {
+            atomicAdd(&sb.colourCount[c], 1);
+        }
+        return 1;
+    };
+    for (int sweep = 0; left > 0 && !ld_acquire(&w.ctr[C_COL_FAIL]); sweep++) {
+#pragma unroll
+        for (int j = 0; j < COL_REG; j++) {
+            if (ck[j] < 0) continue;
+            const int got = attempt(ck[j], cb0[j], cb1[j], cr[j]);
+            if (got < 0) atomicExch(&w.ctr[C_COL_FAIL], 1);
+            if (got > 0) { ck[j] = -1; left--; }
+        }
+        for (int i = cx + tid; i < c1; i += nth) {
+            const int k = sb.bucketList[i];
+            if (sb.colourOf[k] >= 0) continue;
+            int b0, b1, r;
+            fetch(k, b0, b1, r);
+            const int got = attempt(k, b0, b1, r);
+            if (got < 0) atomicExch(&w.ctr[C_COL_FAIL], 1);
+            left -= got > 0;
+        }
+        if (sweep > COL_SWEEPS) { atomicOr(&w.ctr[C_STATUS], ST_TIMEOUT); atomicExch(&w.ctr[C_COL_FAIL], 1); }
+    }
+    return left == 0;
+}
+
+// The colour tables of the colour-by-colour solver from the counts (lcCount, colourCount).
+JBD void colour_tables(const SolverBuffers& sb, int tid, int nth, int cutColours) {
+    for (int part = tid; part < sb.nParts; part += nth) {
+        const int* lc = sb.lcCount + part * (MAX_LOCAL + 1);
+        int* st = sb.lcStart + part * (MAX_LOCAL + 1);
+        int run = sb.bucketStart[part], c = 0;
+        const int end = sb.bucketStart[part + 1];
+        for (; run < end; c++) { st[c] = run; run += __ldcg(&lc[c]); }
+        st[c] = run;
+        sb.nLocal[part] = c;
+    }
+    if (tid == 0) {
+        int run = sb.bucketStart[sb.nParts];
+        for (int c = 0; c < cutColours; c++) { sb.colourStart[c] = run; run += __ldcg(&sb.colourCount[c]); }
+        sb.colourStart[cutColours] = run;
+    }
+}
+
+// ---- colouring by claim passes ---------------------------------------------------------------
+// What the dataflow leaves (C_COL_FAIL).
+JBD void colour_claims(const DevWorld& w, const DevPairs& P, const SolverBuffers& sb, unsigned long long* colSmem,
+                       unsigned& barK, int tid, int nth) {
     const int nb = gridDim.x;
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
     const int nCand = *sb.nCand;
     __shared__ int shWin, shDone, shPart;
     for (int k = tid; k < nCand; k += nth) {
         sb.colourOf[k] = -1;
         if (sb.flowOn) sb.nextLink[2 * k] = sb.nextLink[2 * k + 1] = -1;
     }
+    for (int b = tid; b < w.nBodies; b += nth) {
+        sb.claim[b] = ~0ull;
+        sb.taken[b] = -1;
+    }
     for (int c = tid; c < sb.nParts * (MAX_LOCAL + 1); c += nth) sb.lcCount[c] = 0;
     for (int c = tid; c <= MAX_COLOURS; c += nth) sb.colourCount[c] = 0;
-    if (tid == 0) { w.ctr[C_CUT_DONE] = 0; w.ctr[C_WIN0] = w.ctr[C_WIN1] = w.ctr[C_WIN2] = 0; }
+    if (tid == 0) { w.ctr[C_CUT_DONE] = 0; w.ctr[C_WIN0] = w.ctr[C_WIN1] = w.ctr[C_WIN2] = 0; w.ctr[C_PART_NEXT0] = 0; }
     grid_barrier(w.ctr, nb, barK);
     // manifolds internal to the parts this block takes; the part's claims and taken marks live
     // in shared memory, indexed by the bodies' positions within the part
-    extern __shared__ unsigned long long colSmem[];
     unsigned long long* shClaim = colSmem;
     int* shTaken = (int*)(colSmem + sb.partMax);
     int* shLast = shTaken + sb.partMax;   // link of the body's last coloured candidate
@@ -538,6 +782,43 @@ __global__ void __launch_bounds__(SOLVER_THREADS) k_colour(DevWorld w, DevPairs 
         w.ctr[C_COLOURS] = round + maxLocal;
         w.ctr[C_CUT_COLOURS] = round;
         w.ctr[C_CUT_MANIFOLDS] = nCut;
+    }
+}
+
+__global__ void __launch_bounds__(SOLVER_THREADS) k_colour(DevWorld w, DevPairs P, SolverBuffers sb) {
+    extern __shared__ __align__(16) unsigned long long colSmem[];
+    __shared__ int shPart, shFail;
+    unsigned barK = 0;
+    const int nb = gridDim.x;
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
+    uint4* tok = (uint4*)colSmem;
+    unsigned* home = (unsigned*)(tok + sb.partMax);
+    int local = 0, cut = 0;   // colours
+    if (!ld_acquire(&w.ctr[C_COL_FAIL])) {   // set by k_classify: a body with too many candidates
+        bool ok = true;
+        for (int part = next_part(w, sb, C_PART_NEXT0, &shPart); part >= 0 && ok; part = next_part(w, sb, C_PART_NEXT0, &shPart))
+            ok = first_fit_part(w, P, sb, part, tok, home, &shFail, local);
+        if (!ok && threadIdx.x == 0) atomicExch(&w.ctr[C_COL_FAIL], 1);
+        const int c0 = sb.bucketStart[sb.nParts], c1 = sb.bucketStart[sb.nParts + 1];
+        if (c1 > c0) first_fit_cut(w, P, sb, c0, c1, tid, nth, cut);
+        local = __reduce_max_sync(0xffffffffu, local);
+        cut = __reduce_max_sync(0xffffffffu, cut);
+        if ((threadIdx.x & 31) == 0) {
+            if (local) atomicMax(&w.ctr[C_COLOURS], local);
+            if (cut) atomicMax(&w.ctr[C_CUT_COLOURS], cut);
+        }
+        if (tid == 0) w.ctr[C_CUT_MANIFOLDS] = c1 - c0;
+    }
+    grid_barrier(w.ctr, nb, barK);
+    if (__ldcg(&w.ctr[C_COL_FAIL])) {
+        colour_claims(w, P, sb, colSmem, barK, tid, nth);
+        return;
+    }
+    const int cuts = __ldcg(&w.ctr[C_CUT_COLOURS]);
+    if (!sb.flowOn) colour_tables(sb, tid, nth, cuts);
+    if (tid == 0) {
+        *sb.nColours = cuts;
+        w.ctr[C_COLOURS] += cuts;
     }
 }
 
@@ -2091,7 +2372,7 @@ template <class T> static void sfree(T*& p) { if (p) cudaFree((void*)p); p = nul
 static size_t pgs_smem(const SolverBuffers& sb) {
     return (sb.partSmem ? (size_t)sb.smemCap * 32 : 0) + (size_t)3 * sb.poolPts * POOL_F4 * 16;
 }
-static size_t colour_smem(const SolverBuffers& sb) { return (size_t)sb.partMax * (sizeof(unsigned long long) + 2 * sizeof(int)); }
+static size_t colour_smem(const SolverBuffers& sb) { return (size_t)sb.partMax * (sizeof(uint4) + sizeof(uint2)); }
 
 int solver_configure(SolverBuffers& sb, int nFinite, const std::vector<int>& worldCounts, int sms, int rangeParts,
                      int threads, int smemBodies) {
@@ -2144,7 +2425,8 @@ int solver_configure(SolverBuffers& sb, int nFinite, const std::vector<int>& wor
     int dev = 0, smemBlock = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&smemBlock, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
-        cudaFuncSetAttribute(k_pgs, cudaFuncAttributeMaxDynamicSharedMemorySize, smemBlock - 1024) != cudaSuccess)
+        cudaFuncSetAttribute(k_pgs, cudaFuncAttributeMaxDynamicSharedMemorySize, smemBlock - 1024) != cudaSuccess ||
+        cudaFuncSetAttribute(k_colour, cudaFuncAttributeMaxDynamicSharedMemorySize, smemBlock - 1024) != cudaSuccess)
         return JBGPU_ERR_CUDA;
     // point pools: half a block's threads in entries (a quarter with world parts, whose blocks
     // stage nothing ahead and keep more of the SM as L1), fewer or none if they would cost
@@ -2217,17 +2499,24 @@ void solve_launch_learn(const DevWorld& w, DevPairs& P, int nPairs, DevRows& R, 
     // the flow solver takes every solve of a fixed number of iterations without joints or learning
     sb.flowOn = sb.flowOk && w.resTol <= 0.0f && w.numIter <= FLOW_MAX_ITERATIONS && sb.J.n == 0 && !learn.mlp &&
                 !learn.sampleX && !learn.sampleT;
-    cudaMemsetAsync(sb.claim, 0xff, sizeof(unsigned long long) * w.nBodies, s);
-    cudaMemsetAsync(sb.taken, 0xff, sizeof(int) * w.nBodies, s);
+    cudaMemsetAsync(sb.bodyDeg, 0, sizeof(int) * w.nBodies, s);
+    if (!sb.worldParts) {   // tokens of cut candidates, and after them their home colours
+        sb.cutHome = (unsigned*)(sb.cutToken + w.nBodies);
+        cudaMemsetAsync(sb.cutToken, 0, (sizeof(uint4) + sizeof(uint2)) * (size_t)w.nBodies, s);
+    }
     cudaMemsetAsync(sb.posOf, 0xff, sizeof(int) * w.nBodies, s);
     const int buckets = parts + 2 + (sb.flowOn ? sb.nFlow + 1 : 0);   // the colouring's buckets, then the flow solver's
     cudaMemsetAsync(sb.bucketCount, 0, sizeof(int) * buckets, s);
     cudaMemsetAsync(sb.bucketFill, 0, sizeof(int) * buckets, s);
-    cudaMemsetAsync(sb.lcFill, 0, sizeof(int) * parts * (MAX_LOCAL + 1), s);
-    cudaMemsetAsync(sb.colourFill, 0, sizeof(int) * (MAX_COLOURS + 1), s);
-    cudaMemsetAsync(w.ctr + C_BAR_COUNT, 0, sizeof(int), s);
-    cudaMemsetAsync(w.ctr + C_PGS_ITERS, 0, sizeof(int), s);
-    cudaMemsetAsync(w.ctr + C_ISL_N, 0, sizeof(int) * 5, s);   // island statistics, part counters
+    if (!sb.flowOn) {
+        cudaMemsetAsync(sb.lcFill, 0, sizeof(int) * parts * (MAX_LOCAL + 1), s);
+        cudaMemsetAsync(sb.lcCount, 0, sizeof(int) * parts * (MAX_LOCAL + 1), s);
+        cudaMemsetAsync(sb.colourFill, 0, sizeof(int) * (MAX_COLOURS + 1), s);
+        cudaMemsetAsync(sb.colourCount, 0, sizeof(int) * (MAX_COLOURS + 1), s);
+    }
+    cudaMemsetAsync(w.ctr + C_SOLVE_FIRST, 0, sizeof(int) * C_SOLVE_COUNT, s);
+    cudaMemsetAsync(w.ctr + C_COLOURS, 0, sizeof(int), s);
+    cudaMemsetAsync(w.ctr + C_CUT_COLOURS, 0, sizeof(int), s);
     k_posof<<<gridn(sb.nFinite, 256), 256, 0, s>>>(sb); note_launch();
     k_classify<<<gridn(nPairs, 256), 256, 0, s>>>(w, P, sb); note_launch();
     exclusive_scan(sb.bucketCount, sb.bucketStart, nullptr, buckets, sb.flowScan, s);

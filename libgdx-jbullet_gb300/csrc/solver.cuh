@@ -8,6 +8,9 @@ constexpr int MAX_COLOURS = 1024;     // grid-wide colours of cut manifolds
 constexpr int MAX_LOCAL = 128;        // colours of the manifolds internal to one part
 constexpr int MAX_SUB = 16;
 constexpr int COL_REG = 4;            // internal-colouring candidates a thread keeps in registers           // claim passes that grow one colour towards a maximal set
+constexpr int COL_LIST = 32;          // candidates a body's list holds
+constexpr unsigned COL_CUT = 1u << 31;   // a list entry of a cut candidate
+constexpr int COL_SWEEPS = 1 << 20;   // a thread's sweeps over its candidates before it gives up
 constexpr int SOLVER_THREADS = 256;
 constexpr int PART_MAX_BODIES = 2048; // bodies of one part (velocities staged in 64 KB of shared memory)
 
@@ -71,6 +74,13 @@ struct SolverBuffers {
     int* bucket = nullptr;        // part of candidate k, nParts when cut
     int* bucketList = nullptr;    // candidates grouped by bucket
     int* candLocal = nullptr;     // per candidate: its dynamic bodies' indices within its part
+    int* bodyDeg = nullptr;       // per body: its candidates, and up to COL_LIST of them
+    unsigned* bodyList = nullptr;
+    int* candRank = nullptr;      // per candidate: its places among those of its class on its bodies
+    unsigned char* candHome = nullptr;   // ... which of its dynamic bodies live in the flow block that solves it
+    uint4* localMask = nullptr;   // per body: colours of its internal candidates, and of those solved at its home
+    uint4* cutToken = nullptr;    // per body: colouring token of its cut candidates (.xy their colours)
+    unsigned* cutHome = nullptr;  // ... colours of those solved at its home, 2 words, after the tokens
     unsigned long long* claim = nullptr;  // per body
     int* taken = nullptr;         // per body: colouring round that took it
     int* posOf = nullptr;         // per body: position in the body order (-1 none)

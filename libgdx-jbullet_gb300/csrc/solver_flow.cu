@@ -104,16 +104,42 @@ JBD void flow_side(const DevWorld& w, const SolverBuffers& sb, int k, int side, 
     r.im[side] = w.iloc[b].w;
     if (w.island[b] < 0) return;                      // static or kinematic: its velocity never changes
     unsigned f = FS_DYN;
-    const int self = 2 * k + side;
-    int prev = sb.prevLink[self], next = sb.nextLink[self];
     const int pos = sb.posOf[b], start = sb.flowBody[block], end = sb.flowBody[block + 1];
-    if (prev < 0) { f |= FS_FIRST; prev = sb.lastLink[b]; }
-    if (next < 0) { f |= FS_LAST; next = sb.firstLink[b]; }
-    const int kp = prev >> 1, kn = next >> 1;
     const bool home = pos >= start && pos < end;
-    if (!home || sb.execOf[kp] != block) f |= FS_READ_EXCH;
-    if (!home || sb.execOf[kn] != block) f |= FS_WRITE_EXCH;
-    r.place[side] = (unsigned)(home ? pos - start : 0) | (unsigned)flow_step(sb, kp) << 16;
+    bool prevHome, nextHome;   // the manifold before (after) it on this body is solved in the body's home block
+    int prevStep;
+    if (w.ctr[C_COL_FAIL]) {   // coloured by claim passes: by its links
+        const int self = 2 * k + side;
+        int prev = sb.prevLink[self], next = sb.nextLink[self];
+        if (prev < 0) { f |= FS_FIRST; prev = sb.lastLink[b]; }
+        if (next < 0) { f |= FS_LAST; next = sb.firstLink[b]; }
+        prevHome = sb.execOf[prev >> 1] == block;
+        nextHome = sb.execOf[next >> 1] == block;
+        prevStep = flow_step(sb, prev >> 1);
+    } else {                   // by the colours its body holds: internal ones in order, then cut ones
+        const uint4 lm = sb.localMask[b];
+        unsigned long long m[2] = {(unsigned long long)lm.y << 32 | lm.x, 0}, h[2] = {(unsigned long long)lm.w << 32 | lm.z, 0};
+        if (!sb.worldParts) {
+            const uint4 ct = sb.cutToken[b];
+            m[1] = (unsigned long long)ct.y << 32 | ct.x;
+            h[1] = (unsigned long long)sb.cutHome[2 * b + 1] << 32 | sb.cutHome[2 * b];
+        }
+        const int cls = sb.bucket[k] < sb.nParts ? 0 : 1, c = sb.colourOf[k];
+        const unsigned long long below = m[cls] & ((1ull << c) - 1), above = (m[cls] >> c) >> 1 << c << 1;
+        int pc = cls, nc = cls, p, q;   // class and colour of the neighbours
+        if (below) p = 63 - __clzll((long long)below);
+        else if (cls == 1 && m[0]) { pc = 0; p = 63 - __clzll((long long)m[0]); }
+        else { f |= FS_FIRST; pc = m[1] ? 1 : 0; p = 63 - __clzll((long long)m[pc]); }
+        if (above) q = __ffsll((long long)above) - 1;
+        else if (cls == 0 && m[1]) { nc = 1; q = __ffsll((long long)m[1]) - 1; }
+        else { f |= FS_LAST; nc = m[0] ? 0 : 1; q = __ffsll((long long)m[nc]) - 1; }
+        prevHome = h[pc] >> p & 1;
+        nextHome = h[nc] >> q & 1;
+        prevStep = p + (pc ? MAX_LOCAL : 0);
+    }
+    if (!home || !prevHome) f |= FS_READ_EXCH;
+    if (!home || !nextHome) f |= FS_WRITE_EXCH;
+    r.place[side] = (unsigned)(home ? pos - start : 0) | (unsigned)prevStep << 16;
     r.word[side] |= f << 24;
 }
 

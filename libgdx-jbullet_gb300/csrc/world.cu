@@ -216,6 +216,8 @@ int alloc_pair_work(jbgpu_world* w, int cap) {
     CK(dalloc(&S.bucket, cap)); CK(dalloc(&S.bucketList, cap));
     CK(dalloc(&S.md, cap)); CK(dalloc(&S.ml, cap)); CK(dalloc(&S.slotIsl, cap)); CK(dalloc(&S.islList, cap));
     CK(dalloc(&S.candLocal, cap));
+    dfree(S.candRank); dfree(S.candHome);
+    CK(dalloc(&S.candRank, cap)); CK(dalloc(&S.candHome, cap));
     dfree(S.execOf); dfree(S.prevLink); dfree(S.nextLink); dfree(S.flowCand); dfree(S.flowDesc);
     CK(dalloc(&S.execOf, cap)); CK(dalloc(&S.prevLink, 2 * (size_t)cap)); CK(dalloc(&S.nextLink, 2 * (size_t)cap));
     CK(dalloc(&S.flowCand, 8 * (size_t)cap)); CK(dalloc(&S.flowDesc, FLOW_DESC_INTS * (size_t)cap));
@@ -277,6 +279,9 @@ int grow_bodies(jbgpu_world* w, int need) {
     dfree(S.islConv); dfree(S.islAcc); dfree(S.islDone);
     CK(dalloc(&S.parent, nc)); CK(dalloc(&S.keepAwake, nc)); CK(dalloc(&S.inactive, nc)); CK(dalloc(&S.claim, nc));
     CK(dalloc(&S.taken, nc)); CK(dalloc(&S.posOf, nc));
+    dfree(S.bodyDeg); dfree(S.bodyList); dfree(S.localMask); dfree(S.cutToken);
+    CK(dalloc(&S.bodyDeg, nc)); CK(dalloc(&S.bodyList, COL_LIST * (size_t)nc)); CK(dalloc(&S.localMask, nc));
+    CK(dalloc(&S.cutToken, nc + (size_t)(nc + 1) / 2));
     dfree(S.firstLink); dfree(S.lastLink); dfree(S.exch);
     CK(dalloc(&S.firstLink, nc)); CK(dalloc(&S.lastLink, nc)); CK(dalloc(&S.exch, 2 * (size_t)nc));
     CK(dalloc(&S.islCount, nc + 1)); CK(dalloc(&S.islFill, nc + 1)); CK(dalloc(&S.islStart, nc + 1));
@@ -1349,6 +1354,7 @@ int jbgpu_world_destroy(jbgpu_world* w) {
     if (N.scanScratch) cudaFree(N.scanScratch);
     SolverBuffers& V = w->sb;
     dfree(V.parent); dfree(V.keepAwake); dfree(V.inactive); dfree(V.flag); dfree(V.candIdx); dfree(V.cand); dfree(V.colourOf);
+    dfree(V.bodyDeg); dfree(V.bodyList); dfree(V.localMask); dfree(V.cutToken); dfree(V.candRank); dfree(V.candHome);
     dfree(V.execOf); dfree(V.prevLink); dfree(V.nextLink); dfree(V.flowCand); dfree(V.flowDesc); dfree(V.firstLink); dfree(V.lastLink); dfree(V.exch);
     dfree(V.bucket); dfree(V.bucketList); dfree(V.claim); dfree(V.taken); dfree(V.posOf); dfree(V.candLocal);
     dfree(V.md); dfree(V.ml); dfree(V.slotIsl); dfree(V.islList); dfree(V.islCount); dfree(V.islFill); dfree(V.islStart);
