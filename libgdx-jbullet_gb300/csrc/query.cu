@@ -6,21 +6,28 @@
 // ray (AabbUtil2.rayAabb, accepting entries up to the closest hit so far), then a
 // SubsimplexConvexCast of a point along the ray (convex shapes) or the two triangles a
 // StaticPlaneShape spans around the ray (TriangleRaycastCallback); a hit is taken when its
-// fraction is below the closest so far.  Here one thread per ray walks the broadphase tree
-// (refit over the shapes' current aabbs) twice - counting, then writing - to list every object
-// whose aabb the ray enters before its end; then one thread per listed (ray, object) runs the
-// object's cast, so that the warps run one code path (a thread per ray walking and casting by
-// turns kept under two threads of a warp active).  An object's cast does not depend on the hits
-// before it, so the ray's answer is its smallest hit by (fraction, body, triangle), j - found by
-// a 64-bit atomicMin - unless an object before j in body order hit below j's aabb entry (then the
-// order-dependent aabb test may have skipped j): such rays, rare, are replayed in body order by a
-// block each.
+// fraction is below the closest so far.  Two paths give that answer.
+//
+// Few rays (k_ray_block): a block per ray tests every body's box, casts the objects the ray enters,
+// a thread each, and replays the reference's loop over them in body order.
+//
+// Many rays: one thread per ray walks the broadphase tree (refit over the shapes' current aabbs)
+// and lists the objects whose aabb the ray enters before its end; then, in three rounds, the
+// nearest listed objects by aabb entry are cast, a thread per (ray, object) so that the warps run
+// one code path, and what the reference is sure to skip is dropped: once object i is past, its
+// closest fraction is at most max(hit of i, aabb entry of i) - either i was cast, or it was skipped
+// because the closest was below its entry already - so an object after i in body order whose entry
+// lies above that is skipped.  An object's cast does not depend on the hits before it, so the ray's
+// answer is the smallest hit by (fraction, body, triangle), j, among those cast - unless an object
+// before j in body order hit below j's aabb entry (then the order-dependent aabb test may have
+// skipped j): such rays replay their cast objects in body order.
 #include "../../include/jbgpu.h"
 #include "gjk.cuh"
 #include "gridsync.cuh"
 #include "prims.cuh"
 #include "query.cuh"
 #include "dispatch.cuh"
+#include <algorithm>
 #include <climits>
 #include "shapes.cuh"
 
@@ -379,26 +386,24 @@ JBD bool passes_filter(const DevWorld& w, int b, int group, int mask) {   // Ray
 }
 
 // Conservative slab test for the tree's inner boxes (inflated, so that no box the exact test
-// accepts is culled).
-JBD bool slab(V o, V d, float4 mn, float4 mx) {
+// accepts is culled; the part in o covers the rounding of a far origin).  inv: 1 / d per axis,
+// formed once per ray: three divides a box were half of the walk's instructions.
+JBD V slab_inv(V d) { return mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z); }
+JBD bool slab(V o, V d, V inv, float4 mn, float4 mx) {
     float tn = -1e-3f, tf = 1.001f;
     const float lo[3] = {mn.x, mn.y, mn.z}, hi[3] = {mx.x, mx.y, mx.z};
-    const float oo[3] = {o.x, o.y, o.z}, dd[3] = {d.x, d.y, d.z};
+    const float oo[3] = {o.x, o.y, o.z}, dd[3] = {d.x, d.y, d.z}, ii[3] = {inv.x, inv.y, inv.z};
+#pragma unroll
     for (int k = 0; k < 3; k++) {
-        const float e = 1e-4f * (1.0f + fmaxf(fabsf(lo[k]), fabsf(hi[k])));
+        const float e = 1e-4f * (1.0f + fmaxf(fmaxf(fabsf(lo[k]), fabsf(hi[k])), 0.01f * fabsf(oo[k])));
         const float a = lo[k] - e, b = hi[k] + e;
-        if (dd[k] == 0.0f) {
-            if (oo[k] < a || oo[k] > b) return false;
-            continue;
-        }
-        const float inv = 1.0f / dd[k];
-        float t0 = (a - oo[k]) * inv, t1 = (b - oo[k]) * inv;
-        if (t0 > t1) { const float x = t0; t0 = t1; t1 = x; }
-        tn = fmaxf(tn, t0);
-        tf = fminf(tf, t1);
-        if (tn > tf) return false;
+        const bool flat = dd[k] == 0.0f;
+        if (flat && (oo[k] < a || oo[k] > b)) return false;
+        const float t0 = (a - oo[k]) * ii[k], t1 = (b - oo[k]) * ii[k];
+        tn = flat ? tn : fmaxf(tn, fminf(t0, t1));
+        tf = flat ? tf : fminf(tf, fmaxf(t0, t1));
     }
-    return true;
+    return !(tn > tf);
 }
 
 // A ray's candidate: a body whose aabb the ray enters before its end (rayAabb with the bound 1,
@@ -409,16 +414,15 @@ struct RayCand {
     int pad;
 };
 
-// Tree walk of one ray per thread: COUNT counts the candidates, else they are written at the
-// ray's offset (the same walk, so the same candidates in the same order).  GROW: a convex sweep's
-// path of origins, every box (node and body) grown by the sweep's cast-shape box gmin / gmax.
-template <bool COUNT, bool GROW = false>
-__global__ void __launch_bounds__(RAY_THREADS) k_ray_walk(DevWorld w, DevWorld wq, const int* sortedBody, Bvh tree,
+// Tree walk of one convex sweep's path of origins per thread, every box (node and body) grown by
+// the sweep's cast-shape box gmin / gmax: COUNT counts the candidates, else they are written at
+// the sweep's offset (the same walk, so the same candidates in the same order).
+template <bool COUNT>
+__global__ void __launch_bounds__(RAY_THREADS) k_sweep_walk(DevWorld w, DevWorld wq, const int* sortedBody, Bvh tree,
                                                          const int* wroot, const int* planeList, const int* planeStart,
                                                          const float* from, const float* to, const int* rayWorld, int n,
                                                          int nWorlds, int group, int mask, int* cnt, const int* off,
-                                                         RayCand* cand, const float4* gmin = nullptr,
-                                                         const float4* gmax = nullptr) {
+                                                         RayCand* cand, const float4* gmin, const float4* gmax) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= n) return;
     const V f = mk(from[3 * r], from[3 * r + 1], from[3 * r + 2]);
@@ -432,14 +436,13 @@ __global__ void __launch_bounds__(RAY_THREADS) k_ray_walk(DevWorld w, DevWorld w
         return;
     }
     const int base = COUNT ? 0 : off[r];
-    const float4 g0 = GROW ? gmin[r] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    const float4 g1 = GROW ? gmax[r] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const float4 g0 = gmin[r], g1 = gmax[r];
     int c = 0;
     auto consider = [&](int b) {
         if (!passes_filter(w, b, group, mask)) return;
         float enter, exit;
-        const V bmin = GROW ? add(mk4(wq.amin[b]), mk4(g0)) : mk4(wq.amin[b]);
-        const V bmax = GROW ? add(mk4(wq.amax[b]), mk4(g1)) : mk4(wq.amax[b]);
+        const V bmin = add(mk4(wq.amin[b]), mk4(g0));
+        const V bmax = add(mk4(wq.amax[b]), mk4(g1));
         if (!ray_aabb_parts(f, t, bmin, bmax, enter, exit)) return;
         if (!(enter <= jmin(1.0f, exit))) return;
         if (!COUNT) {
@@ -457,7 +460,7 @@ __global__ void __launch_bounds__(RAY_THREADS) k_ray_walk(DevWorld w, DevWorld w
         if (root & LEAF_FLAG) {
             consider(sortedBody[root & ~LEAF_FLAG]);
         } else {
-            const V d = sub(t, f);
+            const V d = sub(t, f), inv = slab_inv(d);
             int stack[RAY_STACK];
             int sp = 0;
             stack[sp++] = root;
@@ -465,14 +468,10 @@ __global__ void __launch_bounds__(RAY_THREADS) k_ray_walk(DevWorld w, DevWorld w
                 const float4* nd = tree.node + 4 * stack[--sp];
                 const float4 rec[4] = {nd[0], nd[1], nd[2], nd[3]};
                 for (int k = 0; k < 2; k++) {
-                    if (GROW) {
-                        const float4 lo = rec[2 * k], hi = rec[2 * k + 1];
-                        if (!slab(f, d, make_float4(__fadd_rn(lo.x, g0.x), __fadd_rn(lo.y, g0.y), __fadd_rn(lo.z, g0.z), 0.0f),
-                                  make_float4(__fadd_rn(hi.x, g1.x), __fadd_rn(hi.y, g1.y), __fadd_rn(hi.z, g1.z), 0.0f)))
-                            continue;
-                    } else if (!slab(f, d, rec[2 * k], rec[2 * k + 1])) {
+                    const float4 lo = rec[2 * k], hi = rec[2 * k + 1];
+                    if (!slab(f, d, inv, make_float4(__fadd_rn(lo.x, g0.x), __fadd_rn(lo.y, g0.y), __fadd_rn(lo.z, g0.z), 0.0f),
+                              make_float4(__fadd_rn(hi.x, g1.x), __fadd_rn(hi.y, g1.y), __fadd_rn(hi.z, g1.z), 0.0f)))
                         continue;
-                    }
                     const int x = __float_as_int(rec[2 * k].w);
                     if (x & LEAF_FLAG) consider(sortedBody[x & ~LEAF_FLAG]);
                     else if (sp < RAY_STACK) stack[sp++] = x;
@@ -485,84 +484,465 @@ __global__ void __launch_bounds__(RAY_THREADS) k_ray_walk(DevWorld w, DevWorld w
     if (COUNT) cnt[r] = c;
 }
 
-JBD unsigned long long hit_key(float f, int body, int sub) {    // (fraction, body, triangle) order
-    return ((unsigned long long)__float_as_uint(f) << 32) | ((unsigned long long)body << 1) | (unsigned)sub;
+JBD unsigned long long hit_key(float f, int body, int sub) {    // (fraction, body, triangle) order, -0 as 0
+    return ((unsigned long long)__float_as_uint(f + 0.0f) << 32) | ((unsigned long long)body << 1) | (unsigned)sub;
 }
 
-// One candidate per thread: the object's hits (ray_object), kept per candidate (.w = fraction,
-// -1 for none), and the ray's smallest hit key by a 64-bit atomicMin (fractions are >= 0, so
-// their bits order as the values do).
-__global__ void __launch_bounds__(RAY_THREADS) k_ray_cast(DevWorld w, const RayCand* cand, int total, const float* from,
-                                                         const float* to, float4* hitA, float4* hitB,
-                                                         unsigned long long* key) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    const RayCand c = cand[i];
-    const V f = mk(from[3 * c.ray], from[3 * c.ray + 1], from[3 * c.ray + 2]);
-    const V t = mk(to[3 * c.ray], to[3 * c.ray + 1], to[3 * c.ray + 2]);
-    ObjHits h;
-    ray_object(w, c.body, f, t, h);
-    hitA[i] = h.n > 0 ? f4(h.nrm[0], h.f[0]) : make_float4(0.0f, 0.0f, 0.0f, -1.0f);
-    hitB[i] = h.n > 1 ? f4(h.nrm[1], h.f[1]) : make_float4(0.0f, 0.0f, 0.0f, -1.0f);
-    for (int k = 0; k < h.n; k++) atomicMin(key + c.ray, hit_key(h.f[k], c.body, k));
+// ---- many rays -------------------------------------------------------------------------------
+struct RayEntry { int body; float enter; };
+
+// The walk: every leaf whose box, inflated, the ray meets goes to the ray's list (its place in the
+// tree's order, or a plane's body with PLANE_ENTRY set); cnt counts on beyond the list.  The exact
+// test of a leaf is left to k_ray_exact, a lane that is through with its ray takes the next one as
+// soon as FETCH lanes of its warp are idle, and the stack is in shared memory: with the exact test
+// in the walk and a ray to each thread 6 of 32 lanes were active, 2.6 ms for 200,000 rays in a mixed
+// level of 20,000 bodies; 0.95 ms so.
+constexpr int PLANE_ENTRY = (int)0x80000000;
+constexpr int FETCH = 8;
+__global__ void __launch_bounds__(RAY_THREADS) k_ray_list(DevWorld w, Bvh tree, const int* wroot, const int* planeList,
+                                                         const int* planeStart, const float* from, const float* to,
+                                                         const int* rayWorld, int n, int nWorlds, int* cnt, RayEntry* list,
+                                                         int listCap, int* next) {
+    __shared__ int stack[RAY_STACK][RAY_THREADS];
+    const int me = threadIdx.x, lane = me & 31;
+    int r = -1, sp = 0, c = 0;
+    RayEntry* out = nullptr;
+    V f = mk(0.0f, 0.0f, 0.0f), d = f, inv = f;
+    bool more = true;   // the batch has rays left
+    auto put = [&](int x) {
+        if (c < listCap) out[c].body = x;
+        c++;
+    };
+    while (true) {
+        const unsigned idle = __ballot_sync(0xffffffffu, sp == 0);
+        if (idle == 0xffffffffu || (more && __popc(idle) >= FETCH)) {
+            if (sp == 0 && r >= 0) cnt[r] = c;
+            if (sp == 0) r = -1;
+            if (!more) break;
+            const int leader = __ffs(idle) - 1;
+            int base = 0;
+            if (lane == leader) base = atomicAdd(next, __popc(idle));
+            base = __shfl_sync(0xffffffffu, base, leader);
+            more = base + __popc(idle) < n;
+            const int mine = base + __popc(idle & ((1u << lane) - 1u));
+            if (sp == 0 && mine < n) {
+                r = mine;
+                c = 0;
+                out = list + (size_t)r * listCap;
+                const int wi = rayWorld ? rayWorld[r] : 0;
+                if (wi < 0 || wi >= nWorlds) {   // a world the batch does not have: no candidate, flagged
+                    atomicOr(&w.ctr[C_STATUS], ST_BAD_WORLD);
+                } else {
+                    f = mk(from[3 * r], from[3 * r + 1], from[3 * r + 2]);
+                    d = sub(mk(to[3 * r], to[3 * r + 1], to[3 * r + 2]), f);
+                    inv = slab_inv(d);
+                    for (int q = planeStart[wi]; q < planeStart[wi + 1]; q++) put(planeList[q] | PLANE_ENTRY);
+                    const int root = wroot[wi];
+                    if (root != -1 && (root & LEAF_FLAG)) put(root & ~LEAF_FLAG);
+                    else if (root != -1) stack[sp++][me] = root;
+                }
+            }
+            continue;
+        }
+        if (sp > 0) {
+            const float4* nd = tree.node + 4 * stack[--sp][me];
+            const float4 rec[4] = {nd[0], nd[1], nd[2], nd[3]};
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                if (!slab(f, d, inv, rec[2 * k], rec[2 * k + 1])) continue;
+                const int x = __float_as_int(rec[2 * k].w);
+                if (x & LEAF_FLAG) put(x & ~LEAF_FLAG);
+                else if (sp < RAY_STACK) stack[sp++][me] = x;
+                else atomicOr(&w.ctr[C_STATUS], ST_CAPACITY);
+            }
+        }
+    }
 }
 
-// The candidate holding a ray's smallest hit j writes the ray's record and j's aabb entry.
-__global__ void k_ray_pick(const RayCand* cand, int total, const float4* hitA, const float4* hitB,
-                           const unsigned long long* key, const float* from, const float* to, float* enterJ,
-                           jbgpu_ray_hit* out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    const RayCand c = cand[i];
-    const unsigned long long k = key[c.ray];
-    if (k == ~0ull || (int)((k >> 1) & 0x7fffffffu) != c.body) return;
-    const float4 h = (k & 1) ? hitB[i] : hitA[i];
-    enterJ[c.ray] = c.enter;
-    jbgpu_ray_hit o;
-    o.body = c.body;
-    o.fraction = h.w;
-    o.normal[0] = h.x; o.normal[1] = h.y; o.normal[2] = h.z;
-    const V p = interp3(mk(from[3 * c.ray], from[3 * c.ray + 1], from[3 * c.ray + 2]),
-                        mk(to[3 * c.ray], to[3 * c.ray + 1], to[3 * c.ray + 2]), h.w);
-    o.point[0] = p.x; o.point[1] = p.y; o.point[2] = p.z;
-    out[c.ray] = o;
-}
-
-// j is the reference's answer unless an object before it in body order hit below j's aabb
-// entry (the reference's aabb test, bounded by the closest hit so far, could then skip j).
-__global__ void k_ray_check(const RayCand* cand, int total, const float4* hitA, const float4* hitB,
-                            const unsigned long long* key, const float* enterJ, int* undecided) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    const RayCand c = cand[i];
-    const unsigned long long k = key[c.ray];
-    if (k == ~0ull || c.body >= (int)((k >> 1) & 0x7fffffffu)) return;
-    const float e = enterJ[c.ray];
-    const float a = hitA[i].w, b = hitB[i].w;
-    if ((a >= 0.0f && a < e) || (b >= 0.0f && b < e)) undecided[c.ray] = 1;
-}
-
-// Rays without a hit get the callback's untouched record; undecided rays (and every ray when
-// the replay is forced) go to the in-order replay.
-__global__ void k_ray_finish(int n, const unsigned long long* key, const int* undecided, int replayAll,
-                             jbgpu_ray_hit* out, int* slow, int* slowCount) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+// A warp per ray: the listed leaves that pass the filter and whose box the ray enters before its
+// end stay, closed up.  A ray whose list overflowed goes to `longRays`.
+__global__ void __launch_bounds__(256) k_ray_exact(DevWorld w, DevWorld wq, const int* sortedBody, const float* from,
+                                                   const float* to, int n, int group, int mask, int* cnt, RayEntry* list,
+                                                   int listCap, int* longRays, int* longCount) {
+    const int lane = threadIdx.x & 31;
+    const int r = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (r >= n) return;
-    if (replayAll || undecided[r]) {
-        slow[atomicAdd(slowCount, 1)] = r;
+    const int m = cnt[r];
+    if (m == 0) return;
+    if (m > listCap) {
+        if (lane == 0) longRays[atomicAdd(longCount, 1)] = r;
         return;
     }
-    if (key[r] != ~0ull) return;
-    jbgpu_ray_hit o;
-    o.body = -1;
-    o.fraction = 1.0f;
-    o.normal[0] = o.normal[1] = o.normal[2] = 0.0f;
-    o.point[0] = o.point[1] = o.point[2] = 0.0f;
-    out[r] = o;
+    const V f = mk(from[3 * r], from[3 * r + 1], from[3 * r + 2]);
+    const V t = mk(to[3 * r], to[3 * r + 1], to[3 * r + 2]);
+    RayEntry* e = list + (size_t)r * listCap;
+    int kept = 0;
+    for (int c0 = 0; c0 < m; c0 += 32) {
+        const int c = c0 + lane;
+        bool in = false;
+        RayEntry x = {0, 0.0f};
+        if (c < m) {
+            const int l = e[c].body;
+            x.body = l & PLANE_ENTRY ? l & ~PLANE_ENTRY : sortedBody[l];
+            float exit;
+            in = passes_filter(w, x.body, group, mask) &&
+                 ray_aabb_parts(f, t, mk4(wq.amin[x.body]), mk4(wq.amax[x.body]), x.enter, exit) &&
+                 x.enter <= jmin(1.0f, exit);
+        }
+        const unsigned ib = __ballot_sync(0xffffffffu, in);
+        if (in) e[kept + __popc(ib & ((1u << lane) - 1u))] = x;
+        kept += __popc(ib);
+    }
+    if (lane == 0) cnt[r] = kept;
 }
 
-// The reference's loop for the undecided rays, a block per ray: every body of the ray's world in
-// index order, a chunk of SLOW_THREADS at a time evaluated in parallel (the aabb parts and the
+// The rays whose list overflowed, a warp each, a lane per child box of 16 nodes at a time and with
+// the exact test in the walk: counted, then (FILL) written at their offset.  The few rays with the
+// longest walks are here: by a thread each they took 2.6 ms however few they were.
+constexpr int LONG_WARPS = 4, LONG_STACK = 16 * RAY_STACK + 64;   // at most 16 nodes more a level of the tree
+template <bool FILL>
+__global__ void __launch_bounds__(32 * LONG_WARPS) k_ray_long(DevWorld w, DevWorld wq, const int* sortedBody, Bvh tree,
+                                                              const int* wroot, const int* planeList,
+                                                              const int* planeStart, const float* from, const float* to,
+                                                              const int* rayWorld, int group, int mask, int* cnt,
+                                                              const int* off, RayEntry* list, int listCap, RayEntry* all,
+                                                              const int* longRays, const int* longCount) {
+    __shared__ int sStack[LONG_WARPS][LONG_STACK];
+    const int lane = threadIdx.x & 31, total = *longCount;
+    int* stack = sStack[threadIdx.x >> 5];
+    for (int i = blockIdx.x * LONG_WARPS + (threadIdx.x >> 5); i < total; i += gridDim.x * LONG_WARPS) {
+        const int r = longRays[i];
+        if (FILL && cnt[r] <= listCap) continue;   // short after all: counting wrote its list
+        RayEntry* out = FILL ? all + off[r] : list + (size_t)r * listCap;
+        const V f = mk(from[3 * r], from[3 * r + 1], from[3 * r + 2]);
+        const V t = mk(to[3 * r], to[3 * r + 1], to[3 * r + 2]);
+        const V d = sub(t, f), inv = slab_inv(d);
+        const int wi = rayWorld ? rayWorld[r] : 0;
+        int c = 0, sp = 0;
+        auto consider = [&](int b) {   // by all lanes; b < 0: none
+            float enter = 0.0f, exit;
+            const bool in = b >= 0 && passes_filter(w, b, group, mask) &&
+                            ray_aabb_parts(f, t, mk4(wq.amin[b]), mk4(wq.amax[b]), enter, exit) && enter <= jmin(1.0f, exit);
+            const unsigned ib = __ballot_sync(0xffffffffu, in);
+            const int at = c + __popc(ib & ((1u << lane) - 1u));
+            if (in && (FILL || at < listCap)) out[at] = RayEntry{b, enter};
+            c += __popc(ib);
+        };
+        const int root = wroot[wi];
+        if (root != -1 && (root & LEAF_FLAG)) consider(lane == 0 ? sortedBody[root & ~LEAF_FLAG] : -1);
+        else if (root != -1) {
+            if (lane == 0) stack[0] = root;
+            sp = 1;
+        }
+        __syncwarp();
+        while (sp > 0) {
+            const int take = min(sp, 16);
+            int x = -1;
+            if (lane < 2 * take) {
+                const float4* nd = tree.node + 4 * stack[sp - 1 - (lane >> 1)] + 2 * (lane & 1);
+                const float4 mn = nd[0], mx = nd[1];
+                if (slab(f, d, inv, mn, mx)) x = __float_as_int(mn.w);
+            }
+            const bool hit = x != -1, leaf = hit && (x & LEAF_FLAG);
+            __syncwarp();
+            sp -= take;
+            const unsigned inner = __ballot_sync(0xffffffffu, hit && !leaf);
+            const int at = sp + __popc(inner & ((1u << lane) - 1u));
+            if (hit && !leaf) {
+                if (at < LONG_STACK) stack[at] = x;
+                else atomicOr(&w.ctr[C_STATUS], ST_CAPACITY);
+            }
+            sp = min(LONG_STACK, sp + __popc(inner));
+            if (__any_sync(0xffffffffu, leaf)) consider(leaf ? sortedBody[x & ~LEAF_FLAG] : -1);
+            __syncwarp();
+        }
+        for (int q = planeStart[wi]; q < planeStart[wi + 1]; q += 32)
+            consider(q + lane < planeStart[wi + 1] ? planeList[q + lane] : -1);
+        if (!FILL && lane == 0) cnt[r] = c;
+    }
+}
+
+// One cast: the ray, its candidate's place among all candidates, the body, the aabb entry.
+struct RayCast { int ray, at, body; float enter; };
+constexpr float F_UNCAST = -2.0f, F_MISS = -1.0f;   // candF: smallest hit fraction of a candidate, or these
+constexpr int RAY_ROUNDS = 3, RAY_SORT = 4;   // rays of up to RAY_SORT x 32 candidates choose by aabb entry
+__device__ constexpr int ray_round_casts(int round) { return round == 0 ? 4 : 8; }
+
+// A warp per ray: which of its candidates the next round casts - the nearest few by aabb entry that
+// are neither cast nor dropped (see the top of the file), in the last round all of them.
+__global__ void __launch_bounds__(256) k_ray_select(int n, int round, const int* cnt, const int* off, const RayEntry* list,
+                                                    int listCap, const RayEntry* all, float* candF, RayCast* casts,
+                                                    int* castCount) {
+    __shared__ int hBody[8][32], sWant[8], sBase;
+    __shared__ float hBound[8][32];
+    const float closed = __int_as_float(0x7f800000);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int r = blockIdx.x * 8 + warp;
+    const int m = r < n ? cnt[r] : 0;
+    const int o = r < n ? off[r] : 0;
+    const RayEntry* e = m <= listCap ? list + (size_t)r * listCap : all + o;
+    int hits = 0;
+    if (round == 0) {
+        for (int c = lane; c < m; c += 32) candF[o + c] = F_UNCAST;
+    } else {   // the hits so far, up to 32 of them
+        for (int c0 = 0; c0 < m && hits < 32; c0 += 32) {
+            const int c = c0 + lane;
+            const float f = c < m ? candF[o + c] : F_MISS;
+            const unsigned hb = __ballot_sync(0xffffffffu, f >= 0.0f);
+            const int at = hits + __popc(hb & ((1u << lane) - 1u));
+            if (f >= 0.0f && at < 32) {
+                hBody[warp][at] = e[c].body;
+                hBound[warp][at] = fmaxf(f, e[c].enter);
+            }
+            hits = min(32, hits + __popc(hb));
+        }
+        __syncwarp();
+    }
+    auto open = [&](int c, float& enter, int& body) {   // candidate c may still matter
+        if (c >= m || (round > 0 && candF[o + c] != F_UNCAST)) return false;
+        const RayEntry x = e[c];
+        enter = x.enter + 0.0f;
+        body = x.body;
+        for (int h = 0; h < hits; h++)
+            if (hBody[warp][h] < body && hBound[warp][h] < enter) return false;
+        return true;
+    };
+    const bool pick = round + 1 < RAY_ROUNDS && m <= 32 * RAY_SORT;
+    float en[RAY_SORT];
+    int bo[RAY_SORT];
+    int want = 0;
+    if (pick) {
+#pragma unroll
+        for (int q = 0; q < RAY_SORT; q++) {
+            en[q] = closed;
+            bo[q] = -1;
+            if (32 * q < m && open(32 * q + lane, en[q], bo[q])) want++;
+            else en[q] = closed;
+        }
+        want = min(ray_round_casts(round), __reduce_add_sync(0xffffffffu, want));
+    } else {
+        for (int c = lane; c < m; c += 32) {
+            float enter;
+            int body;
+            if (open(c, enter, body)) want++;
+        }
+        want = __reduce_add_sync(0xffffffffu, want);
+    }
+    if (lane == 0) sWant[warp] = want;   // one reservation a block: a warp's own cost as many atomics on one word
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int sum = 0;
+        for (int q = 0; q < 8; q++) {
+            const int x = sWant[q];
+            sWant[q] = sum;
+            sum += x;
+        }
+        sBase = sum ? atomicAdd(castCount + round, sum) : 0;
+    }
+    __syncthreads();
+    int base = sBase + sWant[warp];
+    if (pick) {
+        for (int k = 0; k < want; k++) {   // the nearest one left: aabb entries are >= 0, ordered as their bits
+            unsigned best = 0xffffffffu;
+#pragma unroll
+            for (int q = 0; q < RAY_SORT; q++) best = min(best, __float_as_uint(en[q]));
+            const unsigned nearest = __reduce_min_sync(0xffffffffu, best);
+            const int owner = __ffs(__ballot_sync(0xffffffffu, best == nearest)) - 1;
+            if (lane == owner) {
+                bool done = false;
+#pragma unroll
+                for (int q = 0; q < RAY_SORT; q++)
+                    if (!done && __float_as_uint(en[q]) == nearest) {
+                        casts[base + k] = RayCast{r, o + 32 * q + lane, bo[q], en[q]};
+                        en[q] = closed;
+                        done = true;
+                    }
+            }
+        }
+        return;
+    }
+    for (int c0 = 0; c0 < m && want > 0; c0 += 32) {
+        float enter = 0.0f;
+        int body = 0;
+        const bool on = open(c0 + lane, enter, body);
+        const unsigned ob = __ballot_sync(0xffffffffu, on);
+        if (on) casts[base + __popc(ob & ((1u << lane) - 1u))] = RayCast{r, o + c0 + lane, body, enter};
+        base += __popc(ob);
+    }
+}
+
+// One cast per thread: the object's hits (ray_object), kept per candidate (.w = fraction, -1 for none).
+__global__ void __launch_bounds__(RAY_THREADS) k_ray_cast(DevWorld w, const RayCast* casts, const int* count,
+                                                         const float* from, const float* to, float* candF, float4* hitA,
+                                                         float4* hitB) {
+    const int total = *count;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const RayCast c = casts[i];
+        const V f = mk(from[3 * c.ray], from[3 * c.ray + 1], from[3 * c.ray + 2]);
+        const V t = mk(to[3 * c.ray], to[3 * c.ray + 1], to[3 * c.ray + 2]);
+        ObjHits h;
+        ray_object(w, c.body, f, t, h);
+        float least = F_MISS;
+        if (h.n > 0) {
+            hitA[c.at] = f4(h.nrm[0], h.f[0]);
+            hitB[c.at] = h.n > 1 ? f4(h.nrm[1], h.f[1]) : make_float4(0.0f, 0.0f, 0.0f, F_MISS);
+            least = h.n > 1 ? fminf(h.f[0], h.f[1]) : h.f[0];
+        }
+        candF[c.at] = least;
+    }
+}
+
+JBD void write_hit(jbgpu_ray_hit* out, int body, float4 h, V from, V to) {
+    jbgpu_ray_hit o;
+    o.body = body;
+    o.fraction = body >= 0 ? h.w : 1.0f;
+    const V p = body >= 0 ? interp3(from, to, h.w) : mk(0.0f, 0.0f, 0.0f);
+    o.normal[0] = body >= 0 ? h.x : 0.0f; o.normal[1] = body >= 0 ? h.y : 0.0f; o.normal[2] = body >= 0 ? h.z : 0.0f;
+    o.point[0] = p.x; o.point[1] = p.y; o.point[2] = p.z;
+    *out = o;
+}
+
+// A warp per ray: the smallest hit j by (fraction, body, triangle) of its cast candidates.  j is the
+// reference's answer unless an object before it in body order hit below j's aabb entry (the
+// reference's aabb test, bounded by the closest hit so far, could then skip j): then the cast
+// candidates with hits are taken in body order with the closest fraction and the break at zero.
+__global__ void __launch_bounds__(256) k_ray_final(int n, const int* cnt, const int* off, const RayEntry* list, int listCap,
+                                                   const RayEntry* all, const float* candF, const float4* hitA,
+                                                   const float4* hitB, const float* from, const float* to,
+                                                   jbgpu_ray_hit* out, int* replays) {
+    const int lane = threadIdx.x & 31;
+    const int r = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (r >= n) return;
+    const int m = cnt[r], o = off[r];
+    const RayEntry* e = m <= listCap ? list + (size_t)r * listCap : all + o;
+    const V vf = mk(from[3 * r], from[3 * r + 1], from[3 * r + 2]), vt = mk(to[3 * r], to[3 * r + 1], to[3 * r + 2]);
+    unsigned long long best = ~0ull;
+    int bestAt = -1;
+    for (int c = lane; c < m; c += 32) {
+        if (!(candF[o + c] >= 0.0f)) continue;
+        const int b = e[c].body;
+        const float fb = hitB[o + c].w;
+        unsigned long long k = hit_key(hitA[o + c].w, b, 0);
+        if (fb >= 0.0f) k = min(k, hit_key(fb, b, 1));
+        if (k < best) { best = k; bestAt = c; }
+    }
+    unsigned long long j = best;
+    for (int q = 16; q > 0; q >>= 1) j = min(j, __shfl_xor_sync(0xffffffffu, j, q));
+    if (j == ~0ull) {
+        if (lane == 0) write_hit(out + r, -1, make_float4(0.0f, 0.0f, 0.0f, 0.0f), vf, vt);
+        return;
+    }
+    const int owner = __ffs(__ballot_sync(0xffffffffu, best == j)) - 1;
+    const int jb = (int)((j >> 1) & 0x7fffffffu);
+    const int jAt = __shfl_sync(0xffffffffu, bestAt, owner);
+    const float enterJ = e[jAt].enter;
+    bool skip = false;
+    for (int c = lane; c < m; c += 32) {
+        const float f = candF[o + c];
+        skip = skip || (f >= 0.0f && f < enterJ && e[c].body < jb);
+    }
+    if (!__any_sync(0xffffffffu, skip)) {
+        if (lane == 0) write_hit(out + r, jb, (j & 1) ? hitB[o + jAt] : hitA[o + jAt], vf, vt);
+        return;
+    }
+    if (lane == 0) atomicAdd(replays, 1);
+    float closest = 1.0f;
+    int body = -1, at = -1, last = -1;
+    bool second = false;
+    while (closest != 0.0f) {
+        int nb = 0x7fffffff, nc = -1;   // the next body in order with hits
+        for (int c = lane; c < m; c += 32)
+            if (candF[o + c] >= 0.0f && e[c].body > last && e[c].body < nb) { nb = e[c].body; nc = c; }
+        const int next = __reduce_min_sync(0xffffffffu, nb);
+        if (next == 0x7fffffff) break;
+        last = next;
+        nc = __shfl_sync(0xffffffffu, nc, __ffs(__ballot_sync(0xffffffffu, nb == next)) - 1);
+        if (!(e[nc].enter <= closest)) continue;   // entry <= exit holds for every candidate
+        const float fa = hitA[o + nc].w, fb = hitB[o + nc].w;
+        if (fa < closest) { closest = fa; body = next; at = nc; second = false; }
+        if (fb >= 0.0f && fb < closest) { closest = fb; body = next; at = nc; second = true; }
+    }
+    if (lane == 0)
+        write_hit(out + r, body, body < 0 ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : second ? hitB[o + at] : hitA[o + at], vf, vt);
+}
+
+// ---- few rays --------------------------------------------------------------------------------
+// A block per ray: every body of the ray's world whose box it enters, in body order, into the block's
+// list, their casts a thread each, then the reference's loop over the list by one thread.  A list
+// that overflows leaves the ray to k_rays_slow.  What bounds it: the box tests (rays x bodies) and
+// the slowest cast.
+constexpr int BLOCK_CAP = 768;
+__global__ void __launch_bounds__(SLOW_THREADS) k_ray_block(DevWorld w, DevWorld wq, const float* from, const float* to,
+                                                          const int* rayWorld, int nWorlds, int group, int mask,
+                                                          jbgpu_ray_hit* out, int* slow, int* slowCount) {
+    __shared__ int sBody[BLOCK_CAP];
+    __shared__ float sEnter[BLOCK_CAP];
+    __shared__ ObjHits sHits[BLOCK_CAP];
+    __shared__ int sWarp[SLOW_THREADS / 32];
+    const int r = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const V f = mk(from[3 * r], from[3 * r + 1], from[3 * r + 2]);
+    const V t = mk(to[3 * r], to[3 * r + 1], to[3 * r + 2]);
+    const int wi = rayWorld ? rayWorld[r] : 0;
+    if (wi < 0 || wi >= nWorlds) {   // as the walk: flagged, a miss
+        if (threadIdx.x == 0) {
+            atomicOr(&w.ctr[C_STATUS], ST_BAD_WORLD);
+            write_hit(out + r, -1, make_float4(0.0f, 0.0f, 0.0f, 0.0f), f, t);
+        }
+        return;
+    }
+    int m = 0;
+    for (int base = 0; base < w.nBodies; base += SLOW_THREADS) {
+        const int b = base + threadIdx.x;
+        float enter = 0.0f, exit;
+        const bool in = b < w.nBodies && w.world[b] == wi && passes_filter(w, b, group, mask) &&
+                        ray_aabb_parts(f, t, mk4(wq.amin[b]), mk4(wq.amax[b]), enter, exit) && enter <= jmin(1.0f, exit);
+        const unsigned ib = __ballot_sync(0xffffffffu, in);
+        if (lane == 0) sWarp[warp] = __popc(ib);
+        __syncthreads();
+        int at = m + __popc(ib & ((1u << lane) - 1u));
+        for (int q = 0; q < SLOW_THREADS / 32; q++) {
+            if (q < warp) at += sWarp[q];
+            m += sWarp[q];
+        }
+        if (in && at < BLOCK_CAP) {
+            sBody[at] = b;
+            sEnter[at] = enter;
+        }
+        __syncthreads();
+    }
+    if (m > BLOCK_CAP) {
+        if (threadIdx.x == 0) slow[atomicAdd(slowCount, 1)] = r;
+        return;
+    }
+    for (int c = threadIdx.x; c < m; c += SLOW_THREADS) ray_object(w, sBody[c], f, t, sHits[c]);
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    float closest = 1.0f;
+    int body = -1;
+    V normal = mk(0.0f, 0.0f, 0.0f);
+    for (int c = 0; c < m && closest != 0.0f; c++) {
+        if (!(sEnter[c] <= closest)) continue;   // entry <= exit holds for every one listed
+        const ObjHits& h = sHits[c];
+        for (int k = 0; k < h.n; k++)
+            if (h.f[k] < closest) {
+                closest = h.f[k];
+                body = sBody[c];
+                normal = h.nrm[k];
+            }
+    }
+    write_hit(out + r, body, f4(normal, closest), f, t);
+}
+
+__global__ void k_ray_all_slow(DevWorld w, const int* rayWorld, int nWorlds, int n, int* slow, int* slowCount) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r == 0) *slowCount = n;
+    if (r >= n) return;
+    slow[r] = r;
+    if (rayWorld && (rayWorld[r] < 0 || rayWorld[r] >= nWorlds)) atomicOr(&w.ctr[C_STATUS], ST_BAD_WORLD);
+}
+
+// The reference's loop for rays whose block list overflowed and for the forced replay, a block per
+// ray: every body of the ray's world in index order, a chunk of SLOW_THREADS at a time evaluated in parallel (the aabb parts and the
 // object's hits do not depend on the closest fraction), then replayed by one thread with the
 // closest fraction and the break at zero.
 __global__ void __launch_bounds__(SLOW_THREADS) k_rays_slow(DevWorld w, DevWorld wq, const float* from, const float* to,
@@ -739,7 +1119,7 @@ JBD bool gjk_convex_cast(const ShapeRef& sa, const Xf& fromA, V toA, const Shape
     return true;
 }
 
-int query_prepare(const DevWorld& w, BroadphaseBuffers& bb, QueryBuffers& qb, cudaStream_t s) {
+int query_prepare(const DevWorld& w, BroadphaseBuffers& bb, QueryBuffers& qb, bool tree, cudaStream_t s) {
     if (w.nBodies > qb.capBodies) {
         if (qb.qmin) cudaFree(qb.qmin);
         if (qb.qmax) cudaFree(qb.qmax);
@@ -753,6 +1133,7 @@ int query_prepare(const DevWorld& w, BroadphaseBuffers& bb, QueryBuffers& qb, cu
     }
     if (w.nBodies == 0) return JBGPU_OK;
     k_query_aabb<<<gridn(w.nBodies, 256), 256, 0, s>>>(w, qb.qmin, qb.qmax); note_launch();
+    if (!tree) return cudaGetLastError() == cudaSuccess ? JBGPU_OK : JBGPU_ERR_CUDA;
     DevWorld wq = w;
     wq.amin = qb.qmin;
     wq.amax = qb.qmax;
@@ -774,14 +1155,13 @@ int query_prepare(const DevWorld& w, BroadphaseBuffers& bb, QueryBuffers& qb, cu
     return cudaGetLastError() == cudaSuccess ? JBGPU_OK : JBGPU_ERR_CUDA;
 }
 
-static bool grow_ray_buffers(QueryBuffers& qb, int n) {
+static bool grow_ray_buffers(QueryBuffers& qb, int n, bool lists = false) {
     if (n > qb.capRays) {   // per-ray (per-sweep) buffers
-        void* old[] = {qb.slow, qb.rayCnt, qb.rayOff, qb.key, qb.enterJ, qb.undecided, qb.scanScratch};
+        void* old[] = {qb.slow, qb.rayCnt, qb.rayOff, qb.key, qb.scanScratch};
         for (void* p : old)
             if (p) cudaFree(p);
-        qb.slow = qb.rayCnt = qb.rayOff = qb.undecided = nullptr;
+        qb.slow = qb.rayCnt = qb.rayOff = nullptr;
         qb.key = nullptr;
-        qb.enterJ = nullptr;
         qb.scanScratch = nullptr;
         const int c = n > 2 * qb.capRays ? n : 2 * qb.capRays;
         qb.capRays = 0;
@@ -789,14 +1169,24 @@ static bool grow_ray_buffers(QueryBuffers& qb, int n) {
             cudaMalloc((void**)&qb.rayCnt, sizeof(int) * (size_t)c) != cudaSuccess ||
             cudaMalloc((void**)&qb.rayOff, sizeof(int) * (size_t)c) != cudaSuccess ||
             cudaMalloc((void**)&qb.key, sizeof(unsigned long long) * (size_t)c) != cudaSuccess ||
-            cudaMalloc((void**)&qb.enterJ, sizeof(float) * (size_t)c) != cudaSuccess ||
-            cudaMalloc((void**)&qb.undecided, sizeof(int) * (size_t)c) != cudaSuccess ||
             cudaMalloc(&qb.scanScratch, scan_scratch_bytes(c)) != cudaSuccess)
             return false;
         qb.capRays = c;
     }
+    if (lists) {   // per-ray candidate lists: 256 entries a ray while that stays within 512 MB, at least 8
+        const int want = (int)std::min<size_t>(256, std::max<size_t>(8, ((size_t)1 << 26) / (size_t)n));
+        if (!qb.list || (size_t)n * want > qb.listEntries) {
+            if (qb.list) cudaFree(qb.list);
+            qb.list = nullptr;
+            qb.listEntries = 0;
+            if (cudaMalloc(&qb.list, sizeof(RayEntry) * (size_t)n * want) != cudaSuccess) return false;
+            qb.listEntries = (size_t)n * want;
+        }
+        qb.listCap = want;
+    }
     if (!qb.slowCount && (cudaMalloc((void**)&qb.slowCount, sizeof(int)) != cudaSuccess ||
                           cudaMalloc((void**)&qb.candTotal, sizeof(int)) != cudaSuccess ||
+                          cudaMalloc((void**)&qb.castCount, sizeof(int) * (RAY_ROUNDS + 2)) != cudaSuccess ||
                           cudaMalloc((void**)&qb.candTotal64, sizeof(unsigned long long)) != cudaSuccess))
         return false;
     return true;
@@ -804,16 +1194,20 @@ static bool grow_ray_buffers(QueryBuffers& qb, int n) {
 
 static bool grow_cand_buffers(QueryBuffers& qb, int total) {
     if (total > qb.capCand) {
-        void* old[] = {qb.cand, qb.hitA, qb.hitB};
+        void* old[] = {qb.cand, qb.hitA, qb.hitB, qb.candBody, qb.candF};
         for (void* p : old)
             if (p) cudaFree(p);
         qb.cand = nullptr;
         qb.hitA = qb.hitB = nullptr;
+        qb.candBody = nullptr;
+        qb.candF = nullptr;
         const int c = total > 2 * qb.capCand ? total : 2 * qb.capCand;
         qb.capCand = 0;
         if (cudaMalloc((void**)&qb.cand, sizeof(RayCand) * (size_t)c) != cudaSuccess ||
             cudaMalloc((void**)&qb.hitA, sizeof(float4) * (size_t)c) != cudaSuccess ||
-            cudaMalloc((void**)&qb.hitB, sizeof(float4) * (size_t)c) != cudaSuccess)
+            cudaMalloc((void**)&qb.hitB, sizeof(float4) * (size_t)c) != cudaSuccess ||
+            cudaMalloc((void**)&qb.candBody, sizeof(RayEntry) * (size_t)c) != cudaSuccess ||
+            cudaMalloc((void**)&qb.candF, sizeof(float) * (size_t)c) != cudaSuccess)
             return false;
         qb.capCand = c;
     }
@@ -846,46 +1240,80 @@ static int candidate_total(QueryBuffers& qb, int n, cudaStream_t s, int& total) 
     return JBGPU_OK;
 }
 
+// Which path: a block per ray costs its box tests over all bodies and a fixed part worth about 4,000
+// more; the lists cost a refit, a walk by one lane, a read-back and three rounds of casts however
+// few the rays.  Measured, block / lists, us: 50 bodies 4,096 rays 170 / 234, 16,384 rays 482 / 269;
+// 2,000 bodies 4,096 rays 418 / 473, 16,384 rays 1465 / 556; 20,000 bodies 1,024 rays 538 / 1150,
+// 4,096 rays 1713 / 942.
+constexpr double RAY_BLOCK_TESTS = 3e7;
+
+bool query_rays_by_block(int bodies, int rays) { return (bodies + 4000.0) * rays <= RAY_BLOCK_TESTS; }
+
 int query_rays(const DevWorld& w, const BroadphaseBuffers& bb, QueryBuffers& qb, const float* from, const float* to,
                const int* rayWorld, int n, int group, int mask, jbgpu_ray_hit* hits, int sms, cudaStream_t s) {
     if (n <= 0) return JBGPU_OK;
     int rc;
-    if (!grow_ray_buffers(qb, n)) return JBGPU_ERR_CUDA;
-    cudaMemsetAsync(qb.slowCount, 0, sizeof(int), s);
-    cudaMemsetAsync(qb.key, 0xff, sizeof(unsigned long long) * n, s);
-    cudaMemsetAsync(qb.undecided, 0, sizeof(int) * n, s);
+    const bool byBlock = query_rays_by_block(w.nBodies, n);
+    if (!grow_ray_buffers(qb, n, !byBlock && !qb.replayAll)) return JBGPU_ERR_CUDA;
     DevWorld wq = w;
     wq.amin = qb.qmin;
     wq.amax = qb.qmax;
+    auto replay = [&]() {
+        k_rays_slow<<<sms, SLOW_THREADS, 0, s>>>(w, wq, from, to, rayWorld, group, mask, hits, qb.slow, qb.slowCount);
+        note_launch();
+        return cudaGetLastError() == cudaSuccess ? JBGPU_OK : JBGPU_ERR_CUDA;
+    };
+    if (qb.replayAll) {
+        k_ray_all_slow<<<gridn(n, 256), 256, 0, s>>>(w, rayWorld, bb.nWorlds, n, qb.slow, qb.slowCount); note_launch();
+        return replay();
+    }
+    cudaMemsetAsync(qb.slowCount, 0, sizeof(int), s);
+    if (byBlock) {
+        k_ray_block<<<n, SLOW_THREADS, 0, s>>>(w, wq, from, to, rayWorld, bb.nWorlds, group, mask, hits, qb.slow, qb.slowCount);
+        note_launch();
+        return replay();
+    }
     Bvh tree = bb.bvh;
     tree.node = qb.node;
-    if (!qb.replayAll) {
-        k_ray_walk<true><<<gridn(n, RAY_THREADS), RAY_THREADS, 0, s>>>(w, wq, bb.sortedBody, tree, bb.wroot, bb.planeList,
-                                                                        bb.planeStart, from, to, rayWorld, n, bb.nWorlds,
-                                                                        group, mask, qb.rayCnt, nullptr, nullptr);
+    const int cap = qb.listCap;
+    RayEntry* list = (RayEntry*)qb.list;
+    cudaMemsetAsync(qb.castCount, 0, sizeof(int) * (RAY_ROUNDS + 2), s);
+    int* next = qb.castCount + RAY_ROUNDS;
+    int* longCount = next + 1;
+    const int walkers = std::min(gridn(n, RAY_THREADS), sms * 6);
+    k_ray_list<<<walkers, RAY_THREADS, 0, s>>>(w, tree, bb.wroot, bb.planeList, bb.planeStart, from, to, rayWorld, n,
+                                               bb.nWorlds, qb.rayCnt, list, cap, next);
+    note_launch();
+    k_ray_exact<<<gridn(n, 8), 256, 0, s>>>(w, wq, bb.sortedBody, from, to, n, group, mask, qb.rayCnt, list, cap, qb.slow,
+                                            longCount);
+    note_launch();
+    const int longs = std::min(gridn(n, LONG_WARPS), sms * 4);
+    k_ray_long<false><<<longs, 32 * LONG_WARPS, 0, s>>>(w, wq, bb.sortedBody, tree, bb.wroot, bb.planeList, bb.planeStart,
+                                                        from, to, rayWorld, group, mask, qb.rayCnt, nullptr, list, cap,
+                                                        nullptr, qb.slow, longCount);
+    note_launch();
+    exclusive_scan(qb.rayCnt, qb.rayOff, qb.candTotal, n, qb.scanScratch, s);
+    int total = 0;
+    if ((rc = candidate_total(qb, n, s, total)) != JBGPU_OK) return rc;
+    if (!grow_cand_buffers(qb, total)) return JBGPU_ERR_CUDA;
+    RayEntry* all = (RayEntry*)qb.candBody;
+    RayCast* casts = (RayCast*)qb.cand;
+    if (total > 0) {
+        k_ray_long<true><<<longs, 32 * LONG_WARPS, 0, s>>>(w, wq, bb.sortedBody, tree, bb.wroot, bb.planeList,
+                                                           bb.planeStart, from, to, rayWorld, group, mask, qb.rayCnt,
+                                                           qb.rayOff, list, cap, all, qb.slow, longCount);
         note_launch();
-        exclusive_scan(qb.rayCnt, qb.rayOff, qb.candTotal, n, qb.scanScratch, s);
-        int total = 0;
-        if ((rc = candidate_total(qb, n, s, total)) != JBGPU_OK) return rc;
-        if (!grow_cand_buffers(qb, total)) return JBGPU_ERR_CUDA;
-        if (total > 0) {
-            RayCand* cand = (RayCand*)qb.cand;
-            k_ray_walk<false><<<gridn(n, RAY_THREADS), RAY_THREADS, 0, s>>>(w, wq, bb.sortedBody, tree, bb.wroot,
-                                                                             bb.planeList, bb.planeStart, from, to, rayWorld,
-                                                                             n, bb.nWorlds, group, mask, nullptr, qb.rayOff,
-                                                                             cand);
+        for (int round = 0; round < RAY_ROUNDS; round++) {
+            k_ray_select<<<gridn(n, 8), 256, 0, s>>>(n, round, qb.rayCnt, qb.rayOff, list, cap, all, qb.candF, casts,
+                                                     qb.castCount);
             note_launch();
-            k_ray_cast<<<gridn(total, RAY_THREADS), RAY_THREADS, 0, s>>>(w, cand, total, from, to, qb.hitA, qb.hitB, qb.key);
-            note_launch();
-            k_ray_pick<<<gridn(total, 256), 256, 0, s>>>(cand, total, qb.hitA, qb.hitB, qb.key, from, to, qb.enterJ, hits);
-            note_launch();
-            k_ray_check<<<gridn(total, 256), 256, 0, s>>>(cand, total, qb.hitA, qb.hitB, qb.key, qb.enterJ, qb.undecided);
+            k_ray_cast<<<std::min(gridn(total, RAY_THREADS), sms * 16), RAY_THREADS, 0, s>>>(
+                w, casts, qb.castCount + round, from, to, qb.candF, qb.hitA, qb.hitB);
             note_launch();
         }
     }
-    k_ray_finish<<<gridn(n, 256), 256, 0, s>>>(n, qb.key, qb.undecided, qb.replayAll, hits, qb.slow, qb.slowCount);
-    note_launch();
-    k_rays_slow<<<sms, SLOW_THREADS, 0, s>>>(w, wq, from, to, rayWorld, group, mask, hits, qb.slow, qb.slowCount);
+    k_ray_final<<<gridn(n, 8), 256, 0, s>>>(n, qb.rayCnt, qb.rayOff, list, cap, all, qb.candF, qb.hitA, qb.hitB, from, to,
+                                            hits, qb.slowCount);
     note_launch();
     return cudaGetLastError() == cudaSuccess ? JBGPU_OK : JBGPU_ERR_CUDA;
 }
@@ -1051,7 +1479,7 @@ int query_sweeps(const DevWorld& w, const BroadphaseBuffers& bb, QueryBuffers& q
     const bool walk = (long long)n >= 8LL * sms * RAY_THREADS;
     const dim3 grid(gridn(w.nBodies, 128), n < 65535 ? n : 65535);
     if (walk) {
-        k_ray_walk<true, true><<<gridn(n, RAY_THREADS), RAY_THREADS, 0, s>>>(
+        k_sweep_walk<true><<<gridn(n, RAY_THREADS), RAY_THREADS, 0, s>>>(
             w, wq, bb.sortedBody, tree, bb.wroot, bb.planeList, bb.planeStart, qb.sweepFrom, qb.sweepTo, sweepWorld, n,
             bb.nWorlds, group, mask, qb.rayCnt, nullptr, nullptr, qb.sweepMin, qb.sweepMax);
         note_launch();
@@ -1080,7 +1508,7 @@ int query_sweeps(const DevWorld& w, const BroadphaseBuffers& bb, QueryBuffers& q
         RayCand* cand = (RayCand*)qb.cand;
         if (!listed) {
             if (walk) {
-                k_ray_walk<false, true><<<gridn(n, RAY_THREADS), RAY_THREADS, 0, s>>>(
+                k_sweep_walk<false><<<gridn(n, RAY_THREADS), RAY_THREADS, 0, s>>>(
                     w, wq, bb.sortedBody, tree, bb.wroot, bb.planeList, bb.planeStart, qb.sweepFrom, qb.sweepTo, sweepWorld,
                     n, bb.nWorlds, group, mask, nullptr, qb.rayOff, cand, qb.sweepMin, qb.sweepMax);
             } else {
@@ -1352,8 +1780,8 @@ void ccd_free(CcdBuffers& cb) {
 
 void query_free(QueryBuffers& qb) {
     void* ps[] = {qb.qmin, qb.qmax, qb.node, qb.visit, qb.slow, qb.slowCount, qb.from, qb.to, qb.rayWorld, qb.hits,
-                  qb.rayCnt, qb.rayOff, qb.candTotal, qb.candTotal64, qb.key, qb.enterJ, qb.undecided, qb.scanScratch, qb.cand, qb.hitA,
-                  qb.hitB, qb.sweepMin, qb.sweepMax, qb.sweepPlane, qb.sweepFrom, qb.sweepTo};
+                  qb.rayCnt, qb.rayOff, qb.candTotal, qb.candTotal64, qb.key, qb.scanScratch, qb.cand, qb.hitA,
+                  qb.hitB, qb.list, qb.castCount, qb.candBody, qb.candF, qb.sweepMin, qb.sweepMax, qb.sweepPlane, qb.sweepFrom, qb.sweepTo};
     for (void* p : ps)
         if (p) cudaFree(p);
     qb = QueryBuffers();

@@ -16,10 +16,14 @@ struct QueryBuffers {
     int* slow = nullptr;          // rays the closest-hit shortcut cannot decide (replayed in body order)
     int* slowCount = nullptr;
     int* rayCnt = nullptr;        // per ray: candidates, their offsets, the smallest hit key,
-    int* rayOff = nullptr;        // the aabb entry of that hit's object, undecided flag
+    int* rayOff = nullptr;
     unsigned long long* key = nullptr;
-    float* enterJ = nullptr;
-    int* undecided = nullptr;
+    void* list = nullptr;         // per ray: its first listCap candidates (body, aabb entry)
+    int listCap = 0;
+    size_t listEntries = 0;
+    int* castCount = nullptr;     // casts of each round
+    void* candBody = nullptr;     // (body, aabb entry) of the candidates of rays with more than listCap
+    float* candF = nullptr;       // per candidate: not cast, missed, or its smallest hit fraction
     void* scanScratch = nullptr;
     int* candTotal = nullptr;
     unsigned long long* candTotal64 = nullptr;   // the same total in 64 bits (refuses overflowing batches)
@@ -42,9 +46,11 @@ struct QueryBuffers {
     int capSweeps = 0;
 };
 
-// Query boxes for every body and the refit tree over them; builds the broadphase tree first
-// when the body set changed since its last build.
-int query_prepare(const DevWorld& w, BroadphaseBuffers& bb, QueryBuffers& qb, cudaStream_t s);
+// Query boxes for every body and, with `tree`, the refit tree over them; builds the broadphase
+// tree first when the body set changed since its last build.
+int query_prepare(const DevWorld& w, BroadphaseBuffers& bb, QueryBuffers& qb, bool tree, cudaStream_t s);
+// Whether a batch of rays takes a block per ray (and needs no refit tree).
+bool query_rays_by_block(int bodies, int rays);
 // n rays (device buffers) against the prepared boxes; grows the replay list to n.  sms: blocks
 // of the replay kernel.
 int query_rays(const DevWorld& w, const BroadphaseBuffers& bb, QueryBuffers& qb, const float* from, const float* to,

@@ -2303,7 +2303,7 @@ int jbgpu_world_ray_test(jbgpu_world* w, const float* from, const float* to, con
     DevWorld d = dev_view(w);
     QueryBuffers& Q = w->qb;
     CK(cudaMemsetAsync(w->dw.ctr + C_STATUS, 0, sizeof(int), s));   // traversal-stack and world-id flags of this call
-    rc = query_prepare(d, w->bb, Q, s);
+    rc = query_prepare(d, w->bb, Q, !Q.replayAll && !query_rays_by_block(w->nBodies, n), s);
     if (rc) return fail(rc, "ray query preparation failed");
     const float* df = from;
     const float* dt = to;
@@ -2363,7 +2363,7 @@ int jbgpu_world_convex_sweep_test(jbgpu_world* w, int32_t shape, const float* fr
     DevWorld d = dev_view(w);
     QueryBuffers& Q = w->qb;
     CK(cudaMemsetAsync(w->dw.ctr + C_STATUS, 0, sizeof(int), s));   // traversal-stack and world-id flags of this call
-    rc = query_prepare(d, w->bb, Q, s);
+    rc = query_prepare(d, w->bb, Q, true, s);
     if (rc) return fail(rc, "sweep query preparation failed");
     if (deviceBuffers) {
         rc = query_sweeps(d, w->bb, Q, shape, from, to, sweepWorld, n, group, mask, hits, w->sms, s);
