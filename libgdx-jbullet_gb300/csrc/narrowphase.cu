@@ -111,10 +111,19 @@ __global__ void k_narrow_scatter(int nPairs, const int* cntp, const unsigned cha
 // Entries of the pass: the pairs of buckets 1..6 = the start of bucket 0's row.
 JBD int narrow_active(const int* blockOff, int nBlocks) { return blockOff[(NB_BUCKETS - 1) * nBlocks]; }
 
-// With perm: n = the grouping's pair blocks and entry i is pair perm[i]; without: n = pairs.
+// A pair to each G lanes.  With perm: n = the grouping's pair blocks and entry i is pair perm[i];
+// without: n = pairs.
+// What bounds it: the code the pairs of a warp take apart, one after the other.  In a batch that
+// leaves most of the GPU idle a pair has lanes to spare: they split a hull's vertex scan, and a warp
+// holds fewer pairs (narrow_pairs has the line and the times).  Lanes that take the next pair when
+// theirs is done, and the manifold in a pass of its own, were slower: 672 us against 475 us for
+// 600,000 pairs - lanes in step share the simplex's cases.
+template <int G>
 __global__ void __launch_bounds__(128, 4) k_narrow(DevWorld w, DevPairs P, int n, const int* perm, const int* blockOff, EpaRec* queue,
                          int* queueCount, const int* cntp) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1);
+    const unsigned gmask = (G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (lane - gl));
+    int i = (blockIdx.x * blockDim.x + threadIdx.x) / G;
     if (i >= (perm ? narrow_active(blockOff, n) : (cntp ? min(n, *cntp) : n))) return;
     int p = perm ? perm[i] : i;
     uint64_t key = P.keys[p];
@@ -126,7 +135,8 @@ __global__ void __launch_bounds__(128, 4) k_narrow(DevWorld w, DevPairs P, int n
     const int kind = pair_leaves(w, key, col0, col1, x0, x1, f, g);
     if (kind == ALG_EMPTY || kind >= ALG_CONVEX_CONCAVE) return;   // no manifold; meshes: the concave pass
     const bool fresh = !P.has[p];            // the algorithm and its manifold come with the first dispatch
-    if (fresh) P.has[p] = 1;
+    __syncwarp(gmask);
+    if (fresh && gl == 0) P.has[p] = 1;
     // The collision first, without the manifold (it reads nothing of it), so that GJK's state and
     // the manifold's 4 points are never live together: at most one point for the manifold.
     bool hit = false;
@@ -170,9 +180,10 @@ __global__ void __launch_bounds__(128, 4) k_narrow(DevWorld w, DevPairs P, int n
         md = __fmul_rn(md, md);
         {   // one counter atomic per group of converged lanes
             const unsigned am = __activemask();
-            if ((threadIdx.x & 31) == __ffs(am) - 1) atomicAdd(&w.ctr[C_GJK], __popc(am));
+            if (lane == __ffs(am) - 1) atomicAdd(&w.ctr[C_GJK], __popc(am) / G);
         }
-        GjkPart gp = gjk_part(sa, f.x, sb, g.x, md);
+        GjkPart gp = gjk_part<G>(sa, f.x, sb, g.x, md, gl, gmask);
+        if (gl != 0) return;
         if (gp.needEpa) {
             int q = atomicAdd(queueCount, 1);
             EpaRec r;
@@ -194,6 +205,7 @@ __global__ void __launch_bounds__(128, 4) k_narrow(DevWorld w, DevPairs P, int n
             hit = true;
         }
     }
+    if (gl != 0) return;
     // ManifoldResult.addContactPoint and refreshContactPoints on the pair's manifold
     Mf m;
     if (fresh) m.n = 0;
@@ -383,6 +395,20 @@ __global__ void __launch_bounds__(32) k_narrow_epa_smem(DevWorld w, DevPairs P, 
 
 static int gridn_nb(int nPairs) { return (nPairs + NB_THREADS - 1) / NB_THREADS; }
 
+// The pass over nPairs pairs (with cntp an upper bound: the pair capacity, half as large again as the
+// count or more).  Lanes to a pair, us at 1 / 4 / 32: 139 pairs (60 mixed bodies) 87 / 56 / 36; 5,134
+// (boxes) 38 / 36.5 / 56; 19,780 (boxes and hulls on a mesh) 105 / 93 / 163; 30,087 61 / 82 / 194;
+// 114,015 151 / 245 / 778.
+static void narrow_pairs(const DevWorld& w, DevPairs& P, int nPairs, NarrowBuffers& nb, const int* perm, const int* cntp,
+                         cudaStream_t s) {
+    const int n = perm ? gridn_nb(nPairs) : nPairs;
+    const int lanes = nPairs <= 32 * nb.sms ? 32 : nPairs <= 200 * nb.sms ? 4 : 1;
+    auto k = lanes == 32 ? k_narrow<32> : lanes == 4 ? k_narrow<4> : k_narrow<1>;
+    k<<<((size_t)nPairs * lanes + 127) / 128, 128, 0, s>>>(w, P, n, perm, perm ? nb.blockOff : nullptr,
+                                                          (EpaRec*)nb.queue, nb.queueCount, cntp);
+    note_launch();
+}
+
 // The three EPA tiers over a queue (queueCount on the device); ovfCount: 3 ints (the two
 // overflow lists' counts and the tier mode the last tier sets for the next step).
 static void epa_tiers(const DevWorld& w, DevPairs& P, void* queue, int* queueCount, int* ovfQueue, int* ovfQueue2,
@@ -417,11 +443,9 @@ void narrowphase_launch(const DevWorld& w, DevPairs& P, int nPairs, NarrowBuffer
     if (nPairs > 0) {
         if (nb.group) {
             narrow_group(w, P, nPairs, nb, s, cntp);
-            k_narrow<<<(nPairs + 127) / 128, 128, 0, s>>>(w, P, gridn_nb(nPairs), nb.perm, nb.blockOff,
-                                                           (EpaRec*)nb.queue, nb.queueCount, nullptr); note_launch();
+            narrow_pairs(w, P, nPairs, nb, nb.perm, nullptr, s);
         } else {
-            k_narrow<<<(nPairs + 127) / 128, 128, 0, s>>>(w, P, nPairs, nullptr, nullptr, (EpaRec*)nb.queue,
-                                                           nb.queueCount, cntp); note_launch();
+            narrow_pairs(w, P, nPairs, nb, nullptr, cntp, s);
         }
     }
     if (prof) { prof->mark(PH_NARROW, 1, s); prof->mark(PH_EPA, 0, s); }
@@ -725,8 +749,7 @@ void narrowphase_launch_static(const DevWorld& w, DevPairs& P, int nPairs, Narro
     cudaMemsetAsync(nb.queueCount, 0, sizeof(int), s);
     if (nPairs <= 0) return;
     narrow_group(w, P, nPairs, nb, s);
-    k_narrow<<<(nPairs + 127) / 128, 128, 0, s>>>(w, P, gridn_nb(nPairs), nb.perm, nb.blockOff, (EpaRec*)nb.queue,
-                                                   nb.queueCount, nullptr); note_launch();
+    narrow_pairs(w, P, nPairs, nb, nb.perm, nullptr, s);
     unsigned char* b = (unsigned char*)base;
     EpaArena ar;
     ar.fN = (float4*)(b + OFF_FN);

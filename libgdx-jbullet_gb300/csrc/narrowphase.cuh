@@ -10,6 +10,7 @@ constexpr int NB_BUCKETS = 11;   // narrowphase algorithm buckets (pairs grouped
 struct NarrowBuffers {
     void* queue = nullptr;        // EpaRec per queued pair (pair capacity)
     int* queueCount = nullptr;
+    int sms = 1;
     int slots = 0;                // EPA blocks, striding over the queue
     int* ovfQueue = nullptr;      // queries the 192-face tier left to the full-capacity tier
     int* ovfCount = nullptr;      // 3 ints: that list's count, ovfQueue2's count, the tier mode

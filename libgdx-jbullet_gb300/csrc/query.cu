@@ -135,10 +135,7 @@ JBD bool subsimplex_ray(const ShapeRef& sb, const Xf& tB, V from, V to, float& f
             w = sub(supA, supB);
             n = v;
         }
-        s.lastW = w;                                 // addVertex
-        s.needsUpdate = true;
-        s.W[s.nv] = w; s.P[s.nv] = supA; s.Q[s.nv] = supB;
-        s.nv++;
+        sx_add(s, w, supA, supB);
         const bool ok = sx_update(s);                // closest(v)
         v = s.cV;
         dist2 = ok ? len2(v) : 0.0f;
@@ -275,10 +272,7 @@ JBD bool subsimplex_cast(const ShapeRef& sa, const Xf& fromA, V toA, const Shape
             w = sub(supA, supB);
             n = v;
         }
-        s.lastW = w;                                 // addVertex
-        s.needsUpdate = true;
-        s.W[s.nv] = w; s.P[s.nv] = supA; s.Q[s.nv] = supB;
-        s.nv++;
+        sx_add(s, w, supA, supB);
         const bool ok = sx_update(s);                // closest(v)
         v = s.cV;
         dist2 = ok ? len2(v) : 0.0f;

@@ -1300,6 +1300,7 @@ int jbgpu_world_create(const jbgpu_config* cfg, jbgpu_world** out) {
              CK(cudaMemset(S.nCand, 0, sizeof(int))); CK(cudaMemset(S.nColours, 0, sizeof(int)));
              NarrowBuffers& N = w->nb;
              N.slots = w->sms * 2;
+             N.sms = w->sms;
              if (narrowphase_configure()) return fail(JBGPU_ERR_CUDA, "EPA shared-memory size");
              CK(dalloc(&N.queueCount, 1));
              CK(dalloc(&N.ovfCount, 3));
