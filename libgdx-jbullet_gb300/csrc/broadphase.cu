@@ -31,20 +31,28 @@ __device__ __forceinline__ float ord2f(unsigned u) {
     return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
 }
 
-// Scene bounds of finite aabb centres (ordered-int atomics).
+// Scene bounds of finite aabb centres (ordered-int atomics, one a warp).  By whole warps; i >= nBodies:
+// none.
+JBD void box_centre_bounds(const DevWorld& w, int i, unsigned* s) {
+    unsigned lo[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, hi[3] = {0u, 0u, 0u};
+    if (i < w.nBodies && !(w.flags[i] & CF_LISTED)) {
+        float4 a = w.amin[i], b = w.amax[i];
+        float c[3] = {0.5f * (a.x + b.x), 0.5f * (a.y + b.y), 0.5f * (a.z + b.z)};
+        for (int k = 0; k < 3; k++) lo[k] = hi[k] = f2ord(c[k]);
+    }
+    for (int k = 0; k < 3; k++) {
+        const unsigned mn = __reduce_min_sync(0xffffffffu, lo[k]), mx = __reduce_max_sync(0xffffffffu, hi[k]);
+        if ((threadIdx.x & 31) == 0) {
+            atomicMin(&s[k], mn);
+            atomicMax(&s[3 + k], mx);
+        }
+    }
+}
 __global__ void k_bounds(DevWorld w, unsigned* bnd) {
     __shared__ unsigned s[6];
     if (threadIdx.x < 6) s[threadIdx.x] = (threadIdx.x < 3) ? 0xffffffffu : 0u;
     __syncthreads();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < w.nBodies && !(w.flags[i] & CF_LISTED)) {
-        float4 a = w.amin[i], b = w.amax[i];
-        float c[3] = {0.5f * (a.x + b.x), 0.5f * (a.y + b.y), 0.5f * (a.z + b.z)};
-        for (int k = 0; k < 3; k++) {
-            atomicMin(&s[k], f2ord(c[k]));
-            atomicMax(&s[3 + k], f2ord(c[k]));
-        }
-    }
+    box_centre_bounds(w, blockIdx.x * blockDim.x + threadIdx.x, s);
     __syncthreads();
     if (threadIdx.x < 3) atomicMin(&bnd[threadIdx.x], s[threadIdx.x]);
     else if (threadIdx.x < 6) atomicMax(&bnd[threadIdx.x], s[threadIdx.x]);
@@ -59,11 +67,8 @@ __device__ __forceinline__ unsigned expand_bits(unsigned v) {
 }
 
 // key = world << 32 | morton30 for finite bodies; planes get the all-ones key (sorted last).
-__global__ void k_morton(DevWorld w, const unsigned* bnd, uint64_t* keys, int* vals) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= w.nBodies) return;
-    vals[i] = i;
-    if (w.flags[i] & CF_LISTED) { keys[i] = ~0ull; return; }
+JBD uint64_t morton_key(const DevWorld& w, const unsigned* bnd, int i) {
+    if (w.flags[i] & CF_LISTED) return ~0ull;
     float lo[3], hi[3];
     for (int k = 0; k < 3; k++) { lo[k] = ord2f(bnd[k]); hi[k] = ord2f(bnd[3 + k]); }
     float4 a = w.amin[i], b = w.amax[i];
@@ -76,7 +81,71 @@ __global__ void k_morton(DevWorld w, const unsigned* bnd, uint64_t* keys, int* v
         q[k] = min((unsigned)(t * 1024.0f), 1023u);
     }
     unsigned m = (expand_bits(q[0]) << 2) | (expand_bits(q[1]) << 1) | expand_bits(q[2]);
-    keys[i] = ((uint64_t)(unsigned)w.world[i] << 32) | m;
+    return ((uint64_t)(unsigned)w.world[i] << 32) | m;
+}
+__global__ void k_morton(DevWorld w, const unsigned* bnd, uint64_t* keys, int* vals) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= w.nBodies) return;
+    vals[i] = i;
+    keys[i] = morton_key(w, bnd, i);
+}
+
+// Bounds, keys and the stable sort by key in one block, for up to ORDER_SMALL bodies: a bitonic
+// network over key and body in one word (the world above ORDER_WORLD_BITS would not fit), R words a
+// thread in registers, exchanged by shuffles within a warp and through shared memory beyond it.  The
+// general path is 15 launches and more (four or five radix passes), some 2.5 us each however few the
+// bodies.
+constexpr int ORDER_SMALL = 4096, ORDER_THREADS = 1024, ORDER_WORLD_BITS = 21;
+template <int R>
+__global__ void __launch_bounds__(ORDER_THREADS) k_order_small(DevWorld w, uint64_t* keys, int* vals) {
+    __shared__ uint64_t sx[ORDER_SMALL];
+    __shared__ unsigned bnd[6];
+    const int n = w.nBodies, tid = threadIdx.x, threads = blockDim.x, size = R * threads;
+    if (tid < 6) bnd[tid] = tid < 3 ? 0xffffffffu : 0u;
+    __syncthreads();
+    for (int r = 0; r < R; r++) box_centre_bounds(w, r * threads + tid, bnd);
+    __syncthreads();
+    uint64_t x[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int i = tid * R + r;
+        uint64_t m = ~0ull << 12;   // listed bodies and the padding behind them last
+        if (i < n && !(w.flags[i] & CF_LISTED)) {
+            const uint64_t key = morton_key(w, bnd, i);
+            m = ((key >> 32) << 42) | ((key & 0x3fffffffu) << 12);
+        }
+        x[r] = m | (unsigned)i;
+    }
+    for (int k = 2; k <= size; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            if (j >= 32 * R) {
+                __syncthreads();
+#pragma unroll
+                for (int r = 0; r < R; r++) sx[tid * R + r] = x[r];
+                __syncthreads();
+            }
+            uint64_t y[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                if (j >= 32 * R) y[r] = sx[(tid * R + r) ^ j];
+                else if (j >= R) y[r] = __shfl_xor_sync(0xffffffffu, x[r], j / R);
+                else y[r] = R > 2 && j == 2 ? x[(r ^ 2) & (R - 1)] : x[(r ^ 1) & (R - 1)];
+            }
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const int e = tid * R + r;
+                const bool least = ((e & j) == 0) == ((e & k) == 0);
+                x[r] = least == (x[r] < y[r]) ? x[r] : y[r];
+            }
+        }
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int e = tid * R + r;
+        if (e >= n) continue;
+        const int i = (int)(x[r] & 0xfffu);
+        vals[e] = i;
+        keys[e] = w.flags[i] & CF_LISTED ? ~0ull : ((x[r] >> 42) << 32) | ((x[r] >> 12) & 0x3fffffffu);
+    }
 }
 
 __device__ __forceinline__ int delta(const uint64_t* k, int n, int i, int j) {
@@ -411,66 +480,269 @@ __global__ void k_segment_sort_long(const int* off, const int* cnt, int* partner
     }
 }
 
-// Carry manifolds of persisting pairs (binary search in last step's sorted keys: within the
-// owner's segment when last step's per-owner offsets are at hand, else over all of them).
-__global__ void k_persist(DevWorld w, DevPairs nw, DevPairs old, int nNew, int nOld, const int* offPrev, const int* newCnt,
-                          const int* oldCnt) {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (newCnt) nNew = min(nNew, *newCnt);
-    if (oldCnt) nOld = min(nOld, *oldCnt);
-    if (p >= nNew) return;
-    uint64_t key = nw.keys[p];
-    int lo = 0, hi = nOld - 1, found = -1;
-    if (offPrev) {
-        const int o = key_owner(key);
-        lo = offPrev[o];
-        hi = min(offPrev[o + 1], nOld) - 1;
-    }
-    while (lo <= hi) {
-        int mid = (lo + hi) >> 1;
-        uint64_t k = old.keys[mid];
-        if (k == key) { found = mid; break; }
-        if (k < key) lo = mid + 1; else hi = mid - 1;
-    }
-    int a = key_owner(key), b = key_partner(key);
-    if (found >= 0 && old.has[found]) {
-        int n = old.n[found];
-        nw.has[p] = 1;
-        nw.n[p] = n;
-        nw.b0[p] = old.b0[found];
-        nw.b1[p] = old.b1[found];
-        for (int j = 0; j < n; j++) {
-            int s = found * 4 + j, d = p * 4 + j;
-            nw.pA[d] = old.pA[s]; nw.pB[d] = old.pB[s]; nw.wA[d] = old.wA[s]; nw.wB[d] = old.wB[s];
-            nw.nrm[d] = old.nrm[s]; nw.imp[d] = old.imp[s]; nw.d1[d] = old.d1[s]; nw.d2[d] = old.d2[s];
+// Carry the manifold of the lane's pair p over when it persists: its key is searched in
+// old.keys[lo .. hi].  The warp then copies its pairs' points together, a lane a point (four lanes
+// read a pair's 64 bytes of each array): a lane a pair, every lane on lines of its own, took 347 us
+// for 1.9 million pairs, @PW us so.  By whole warps.
+JBD void persist_warp(const DevWorld& w, DevPairs& nw, const DevPairs& old, bool valid, int p, uint64_t key, int lo, int hi) {
+    const int lane = threadIdx.x & 31;
+    int found = -1, n = 0;
+    if (valid) {
+        while (lo <= hi) {
+            int mid = (lo + hi) >> 1;
+            uint64_t k = old.keys[mid];
+            if (k == key) { found = mid; break; }
+            if (k < key) lo = mid + 1; else hi = mid - 1;
         }
-    } else {
-        nw.has[p] = 0;
-        nw.n[p] = 0;
         int mb0, mb1;
-        manifold_bodies(a, b, w.sh.type[w.shape[min(a, b)]], w.sh.type[w.shape[max(a, b)]], mb0, mb1);
+        const int has = found >= 0 && old.has[found] ? 1 : 0;
+        if (has) {
+            n = old.n[found];
+            mb0 = old.b0[found];
+            mb1 = old.b1[found];
+        } else {
+            const int a = key_owner(key), b = key_partner(key);
+            manifold_bodies(a, b, w.sh.type[w.shape[min(a, b)]], w.sh.type[w.shape[max(a, b)]], mb0, mb1);
+        }
+        nw.has[p] = has;
+        nw.n[p] = n;
         nw.b0[p] = mb0;
         nw.b1[p] = mb1;
+    }
+    unsigned left = __ballot_sync(0xffffffffu, n > 0);
+    while (left) {   // eight pairs with points at a time
+        unsigned m = left;
+        int src = -1;
+        for (int q = 0; q < 8 && m; q++, m &= m - 1)
+            if (q == lane >> 2) src = __ffs(m) - 1;
+        left = m;
+        const int from = max(src, 0);
+        const int so = __shfl_sync(0xffffffffu, found, from), d0 = __shfl_sync(0xffffffffu, p, from);
+        const int cnt = __shfl_sync(0xffffffffu, n, from);
+        if (src >= 0 && (lane & 3) < cnt) {
+            const size_t s = (size_t)so * 4 + (lane & 3), d = (size_t)d0 * 4 + (lane & 3);
+            const float4 x0 = old.pA[s], x1 = old.pB[s], x2 = old.wA[s], x3 = old.wB[s];
+            const float4 x4 = old.nrm[s], x5 = old.imp[s], x6 = old.d1[s], x7 = old.d2[s];
+            nw.pA[d] = x0; nw.pB[d] = x1; nw.wA[d] = x2; nw.wB[d] = x3;
+            nw.nrm[d] = x4; nw.imp[d] = x5; nw.d1[d] = x6; nw.d2[d] = x7;
+        }
+    }
+}
+
+// The range of old.keys that can hold a key of owner o: its segment of last step's per-owner offsets
+// when they are at hand, else all of them.
+JBD void persist_range(const int* offPrev, int nOld, int o, int& lo, int& hi) {
+    lo = offPrev ? offPrev[o] : 0;
+    hi = (offPrev ? min(offPrev[o + 1], nOld) : nOld) - 1;
+}
+
+__global__ void k_persist(DevWorld w, DevPairs nw, DevPairs old, int nNew, int nOld, const int* offPrev, const int* newCnt,
+                          const int* oldCnt) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (newCnt) nNew = min(nNew, *newCnt);
+    if (oldCnt) nOld = min(nOld, *oldCnt);
+    if ((p & ~31) >= nNew) return;   // whole warps
+    const bool valid = p < nNew;
+    const uint64_t key = valid ? nw.keys[p] : 0;
+    int lo = 0, hi = -1;
+    if (valid) persist_range(offPrev, nOld, key_owner(key), lo, hi);
+    persist_warp(w, nw, old, valid, p, key, lo, hi);
+}
+
+// ---- direct pairs ----------------------------------------------------------------------------
+// Small worlds without the tree: a warp per owner tests the bodies of its world that can be its
+// partners - listed bodies (planes, meshes) and finite bodies of a higher index - 32 at a time in
+// index order, so that its keys come out sorted.  What the tree costs instead, however small the
+// world: a chain of dependent launches (sort, topology, refit, two traversals, two segment sorts),
+// a refit that climbs the tree one node at a time and a walk by a single lane.
+// The eight owners of a block are neighbours in the list and share its boxes, DIRECT_TILE at a time
+// in shared memory with the next tile's on their way: with every warp reading its own from L2 the
+// count of 4,000 hulls took 69 us, @H us so.
+constexpr int DIRECT_THREADS = 256, DIRECT_TILE = 256;
+struct DirectTile {
+    float mn[3][DIRECT_TILE], mx[3][DIRECT_TILE];
+    int body[DIRECT_TILE];
+    int end;
+};
+
+// f(j, hit) by all lanes of the owner's warp for 32 candidates j (hit: overlapping, filter passed) at a
+// time, ascending.  q: the owner's place in the list; called by whole blocks, `active` per warp.
+template <class F>
+JBD void direct_partners(const DevWorld& w, const DirectList& dl, const int* planeList, const int* planeStart, int q,
+                         bool active, DirectTile& t, F&& f) {
+    const int lane = threadIdx.x & 31, tid = threadIdx.x;
+    const int first = q - (tid >> 5) + 1;   // the block's first owner + 1
+    int i = 0, end = 0;
+    float4 a0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), a1 = a0;
+    if (tid == 0) t.end = 0;
+    __syncthreads();
+    if (active) {
+        i = dl.body[q];
+        const int wi = w.world[i];
+        end = dl.end[wi];
+        a0 = w.amin[i];
+        a1 = w.amax[i];
+        if (lane == 0) atomicMax(&t.end, end);
+        for (int k = planeStart[wi]; k < planeStart[wi + 1]; k += 32) {   // listed bodies before i
+            const int j = k + lane < planeStart[wi + 1] ? planeList[k + lane] : i;
+            f(j, j < i && ovl(a0, a1, w.amin[j], w.amax[j]) && filt(w, i, j));
+        }
+    }
+    __syncthreads();
+    const int last = t.end;
+    int j = 0;
+    float4 b0, b1;
+    auto load = [&](int base) {
+        if (base + tid >= last) return;
+        j = dl.body[base + tid];
+        b0 = w.amin[j];
+        b1 = w.amax[j];
+    };
+    load(first);
+    for (int base = first; base < last; base += DIRECT_TILE) {            // every body after i
+        if (base + tid < last) {
+            t.mn[0][tid] = b0.x; t.mn[1][tid] = b0.y; t.mn[2][tid] = b0.z;
+            t.mx[0][tid] = b1.x; t.mx[1][tid] = b1.y; t.mx[2][tid] = b1.z;
+            t.body[tid] = j;
+        }
+        __syncthreads();
+        load(base + DIRECT_TILE);
+        if (base < end) {
+            unsigned hits = 0;   // of the lane, a bit per 32 boxes; no branch between the loads
+#pragma unroll
+            for (int c = 0; c < DIRECT_TILE / 32; c++) {
+                const int e = 32 * c + lane, k = base + e;
+                const bool hit = (k > q) & (k < end) & (a0.x <= t.mx[0][e]) & (a1.x >= t.mn[0][e]) & (a0.y <= t.mx[1][e]) &
+                                 (a1.y >= t.mn[1][e]) & (a0.z <= t.mx[2][e]) & (a1.z >= t.mn[2][e]);
+                hits |= hit ? 1u << c : 0u;
+            }
+            for (unsigned any = __reduce_or_sync(0xffffffffu, hits); any; any &= any - 1) {
+                const int c = __ffs(any) - 1, other = t.body[32 * c + lane];
+                f(other, ((hits >> c) & 1) && filt(w, i, other));
+            }
+        }
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(DIRECT_THREADS) k_direct_count(DevWorld w, DirectList dl, const int* planeList,
+                                                                 const int* planeStart, int* cnt, int* tcount, int* kept) {
+    __shared__ DirectTile t;
+    const int lane = threadIdx.x & 31;
+    const int q = (blockIdx.x * DIRECT_THREADS + threadIdx.x) >> 5;
+    const int i = q < w.nBodies ? dl.body[q] : w.nBodies;   // the entry past the bodies counts none
+    const bool active = q < w.nBodies && !(w.flags[i] & CF_LISTED);
+    int c = 0, found = 0;
+    direct_partners(w, dl, planeList, planeStart, q, active, t, [&](int j, bool hit) {
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        const int d = found + __popc(m & ((1u << lane) - 1u));
+        if (hit && d < DIRECT_CACHE) kept[(size_t)i * DIRECT_CACHE + d] = j;
+        found += __popc(m);
+        if (hit && w.hasCompound) c += pair_subs(w.sh, w.shape[i], w.shape[j]);
+    });
+    if (w.hasCompound) c = __reduce_add_sync(0xffffffffu, c);
+    else c = found;
+    if (lane == 0 && q <= w.nBodies) {
+        cnt[i] = c;
+        if (q < w.nBodies) tcount[i] = found;
+    }
+}
+
+// The concave pass's candidates, bounded (see k_plane_pairs).
+__global__ void k_mesh_bound(DevWorld w, const int* planeList, const int* planeStart, int* candBound) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= w.nBodies || (w.flags[i] & CF_LISTED)) return;
+    const int wi = w.world[i];
+    for (int k = planeStart[wi]; k < planeStart[wi + 1]; k++) {
+        const int p = planeList[k];
+        if (!ovl(w.amin[i], w.amax[i], w.amin[p], w.amax[p]) || !filt(w, i, p)) continue;
+        const int c = mesh_candidates(w, i, p);
+        if (c) atomicAdd(candBound, c);
+    }
+}
+
+// Keys and persistence of an owner's pairs: the partners the count kept, or tested again when there
+// were more.  With compounds the keys go by child combination, then by partner.
+__global__ void __launch_bounds__(DIRECT_THREADS) k_direct_fill(DevWorld w, DirectList dl, const int* planeList,
+                                                                const int* planeStart, const int* off, const int* tcount,
+                                                                const int* kept, int* partners, DevPairs nw, DevPairs old,
+                                                                int capacity, int nOld, const int* offPrev,
+                                                                const int* oldCnt) {
+    __shared__ DirectTile t;
+    const int lane = threadIdx.x & 31;
+    const int q = (blockIdx.x * DIRECT_THREADS + threadIdx.x) >> 5;
+    const int i = q < w.nBodies ? dl.body[q] : 0;
+    int o = 0, c = 0, found = 0;
+    if (q < w.nBodies && !(w.flags[i] & CF_LISTED)) {
+        o = off[i];
+        c = off[i + 1] - o;
+        found = tcount[i];
+        if (o + c > capacity) c = 0;
+    }
+    const uint64_t owner = (uint64_t)(unsigned)i << 32;
+    const bool again = c > 0 && found > DIRECT_CACHE;
+    const int* list = again ? partners + o : kept + (size_t)i * DIRECT_CACHE;
+    if (__syncthreads_or(again)) {
+        int at = o;
+        direct_partners(w, dl, planeList, planeStart, q, again, t, [&](int j, bool hit) {
+            const unsigned m = __ballot_sync(0xffffffffu, hit);
+            if (hit) partners[at + __popc(m & ((1u << lane) - 1u))] = j;
+            at += __popc(m);
+        });
+        __syncwarp();
+    }
+    if (c == 0) return;
+    if (oldCnt) nOld = min(nOld, *oldCnt);
+    int lo, hi;
+    persist_range(offPrev, nOld, i, lo, hi);
+    int at = o;
+    for (int sub = 0; at < o + c; sub++) {
+        const int before = at;
+        for (int k = 0; k < found; k += 32) {
+            const int j = k + lane < found ? list[k + lane] : -1;
+            const bool put = j >= 0 && (sub == 0 || sub < pair_subs(w.sh, w.shape[i], w.shape[j]));
+            const unsigned m = __ballot_sync(0xffffffffu, put);
+            const int p = at + __popc(m & ((1u << lane) - 1u));
+            const uint64_t key = owner | ((unsigned)sub << 24) | (unsigned)j;
+            if (put) nw.keys[p] = key;
+            persist_warp(w, nw, old, put, p, key, lo, hi);
+            at += __popc(m);
+        }
+        if (at == before) break;
     }
 }
 
 static inline int gridn(int n, int b) { return (n + b - 1) / b; }
 
-// The tree over the Morton order is rebuilt every rebuildInterval steps and only refitted to the
-// new AABBs in between: a refitted tree bounds every body exactly, so the traversal finds the
-// same pair set whatever the tree's shape; only its cost depends on how stale the order is.
-// The tree over the finite bodies' current w.amin/w.amax: Morton keys of the box centres (the
-// batch world in the high bits), radix sort, world leaf ranges, Karras topology.  Boxes are
-// written by a refit.
-void broadphase_build_tree(const DevWorld& w, BroadphaseBuffers& bb, cudaStream_t s) {
-    const int n = w.nBodies, nf = bb.nFinite;
+// The bodies' Morton order is renewed every rebuildInterval steps, and with it the tree's topology;
+// in between the tree is only refitted to the new AABBs: a refitted tree bounds every body exactly,
+// so the traversal finds the same pair set whatever the tree's shape; only its cost depends on how
+// stale the order is.
+// The order: Morton keys of the current w.amin/w.amax centres (the batch world in the high bits),
+// sorted.
+void broadphase_order(const DevWorld& w, BroadphaseBuffers& bb, cudaStream_t s) {
+    const int n = w.nBodies;
     bb.built = true;
+    bb.treeBuilt = false;
     bb.sinceBuild = 0;
+    if (n <= ORDER_SMALL && bb.worldBits <= ORDER_WORLD_BITS) {
+        int size = 32;
+        while (size < n) size <<= 1;
+        auto k = size <= ORDER_THREADS ? k_order_small<1> : size == 2 * ORDER_THREADS ? k_order_small<2> : k_order_small<4>;
+        k<<<1, std::min(size, ORDER_THREADS), 0, s>>>(w, bb.mkeys, bb.sortedBody); note_launch();
+        return;
+    }
     cudaMemsetAsync(bb.bounds, 0, sizeof(unsigned) * 6, s);
     cudaMemsetAsync(bb.bounds, 0xff, sizeof(unsigned) * 3, s);
     k_bounds<<<gridn(n, 256), 256, 0, s>>>(w, bb.bounds); note_launch();
     k_morton<<<gridn(n, 256), 256, 0, s>>>(w, bb.bounds, bb.mkeys, bb.sortedBody); note_launch();
     radix_sort_pairs(bb.mkeys, bb.sortedBody, bb.mkeys_alt, bb.vals_alt, n, 32 + bb.worldBits, bb.sortScratch, s);
+}
+
+// The tree over the current order: world leaf ranges, Karras topology.  Boxes are written by a refit.
+void broadphase_topology(BroadphaseBuffers& bb, cudaStream_t s) {
+    const int nf = bb.nFinite;
+    bb.treeBuilt = true;
     if (nf > 0) {
         cudaMemsetAsync(bb.wstart, 0xff, sizeof(int) * bb.nWorlds, s);
         cudaMemsetAsync(bb.wend, 0xff, sizeof(int) * bb.nWorlds, s);
@@ -496,11 +768,25 @@ void broadphase_refit_into(const DevWorld& wq, const BroadphaseBuffers& bb, floa
     k_refit<<<gridn(nf, 256), 256, 0, s>>>(wq, bb.sortedBody, nf, t); note_launch();
 }
 
+bool broadphase_rebuilds(const BroadphaseBuffers& bb) { return !(bb.built && bb.sinceBuild + 1 < bb.rebuildInterval); }
+
 void broadphase_run_count(const DevWorld& w, BroadphaseBuffers& bb, cudaStream_t s) {
-    int n = w.nBodies;
-    if (bb.built && bb.sinceBuild + 1 < bb.rebuildInterval) {
+    const int n = w.nBodies, nf = bb.nFinite;
+    if (broadphase_rebuilds(bb)) {
+        broadphase_order(w, bb, s);
+        if (!bb.direct) broadphase_topology(bb, s);
+    } else {
         bb.sinceBuild++;
-        int nf = bb.nFinite;
+    }
+    cudaMemsetAsync(bb.candBound, 0, sizeof(int), s);
+    if (bb.direct) {
+        k_direct_count<<<gridn(n + 1, DIRECT_THREADS / 32), DIRECT_THREADS, 0, s>>>(w, bb.list, bb.planeList, bb.planeStart,
+                                                                                    bb.cnt, bb.tcount, bb.kept);
+        note_launch();
+        if (bb.meshes) {
+            k_mesh_bound<<<gridn(n, 128), 128, 0, s>>>(w, bb.planeList, bb.planeStart, bb.candBound); note_launch();
+        }
+    } else {
         cudaMemsetAsync(bb.cnt, 0, sizeof(int) * (n + 1), s);
         if (nf > 1) {
             cudaMemsetAsync(bb.bvh.visit, 0, sizeof(int) * (nf - 1), s);
@@ -508,32 +794,26 @@ void broadphase_run_count(const DevWorld& w, BroadphaseBuffers& bb, cudaStream_t
             k_traverse<false><<<gridn(nf, 128), 128, 0, s>>>(w, bb.sortedBody, nf, bb.bvh, bb.wroot, bb.cnt, nullptr,
                                                               nullptr, nullptr, 0, bb.tcount, bb.tcache); note_launch();
         }
-        cudaMemsetAsync(bb.candBound, 0, sizeof(int), s);
         if (bb.nPlanes > 0)
             k_plane_pairs<false><<<gridn(n, 256), 256, 0, s>>>(w, bb.planeList, bb.planeStart, bb.cnt, nullptr, nullptr,
                                                                 nullptr, 0, bb.candBound); note_launch();
-        exclusive_scan(bb.cnt, bb.off, bb.total, n + 1, bb.scanScratch, s);
-        return;
     }
-    broadphase_build_tree(w, bb, s);
-    int nf = bb.nFinite;
-    cudaMemsetAsync(bb.cnt, 0, sizeof(int) * (n + 1), s);
-    if (nf > 0) {
-        if (nf > 1) {
-            cudaMemsetAsync(bb.bvh.visit, 0, sizeof(int) * (nf - 1), s);
-            k_refit<<<gridn(nf, 256), 256, 0, s>>>(w, bb.sortedBody, nf, bb.bvh); note_launch();
-            k_traverse<false><<<gridn(nf, 128), 128, 0, s>>>(w, bb.sortedBody, nf, bb.bvh, bb.wroot, bb.cnt, nullptr,
-                                                              nullptr, nullptr, 0, bb.tcount, bb.tcache); note_launch();
-        }
-    }
-    cudaMemsetAsync(bb.candBound, 0, sizeof(int), s);
-    if (bb.nPlanes > 0)
-        k_plane_pairs<false><<<gridn(n, 256), 256, 0, s>>>(w, bb.planeList, bb.planeStart, bb.cnt, nullptr, nullptr,
-                                                            nullptr, 0, bb.candBound); note_launch();
     exclusive_scan(bb.cnt, bb.off, bb.total, n + 1, bb.scanScratch, s);
 }
 
-void broadphase_run_fill(const DevWorld& w, BroadphaseBuffers& bb, DevPairs& nw, int capacity, cudaStream_t s) {
+// Count and fill, us, tree / direct: 60 bodies 85 / 30, 1,000 131 / 40, 4,000 hulls 287 / 100, 256
+// worlds of 17 bodies 169 / 85; 20,000 252 / 312; 1,024 worlds of 433 bodies 710 / 1184 - the count
+// pays for 32 tests at a time (steps) and the fill for a warp an owner.
+bool broadphase_direct(const std::vector<int>& bodies, const std::vector<int>& finite) {
+    double steps = 0.0, owners = 0.0;
+    for (size_t k = 0; k < bodies.size(); k++) {
+        steps += finite[k] * (1.0 + bodies[k] / 64.0);
+        owners += finite[k];
+    }
+    return owners <= 32768.0 && steps <= 1.0e6;
+}
+
+static void tree_fill(const DevWorld& w, BroadphaseBuffers& bb, DevPairs& nw, int capacity, cudaStream_t s) {
     int n = w.nBodies, nf = bb.nFinite;
     cudaMemsetAsync(bb.cursor, 0, sizeof(int) * (n + 1), s);
     // counts are recovered from the offsets: cnt[i] = off[i+1] - off[i]
@@ -557,12 +837,20 @@ void broadphase_run_fill(const DevWorld& w, BroadphaseBuffers& bb, DevPairs& nw,
     note_launch();
 }
 
-void broadphase_persist(const DevWorld& w, BroadphaseBuffers& bb, DevPairs& nw, const DevPairs& old, int nNew, int nOld,
-                        cudaStream_t s, const int* newCnt, const int* oldCnt) {
-    if (nNew > 0) {
-        k_persist<<<gridn(nNew, 256), 256, 0, s>>>(w, nw, old, nNew, nOld, bb.offPrevValid ? bb.offPrev : nullptr, newCnt,
-                                                    oldCnt);
+void broadphase_fill(const DevWorld& w, BroadphaseBuffers& bb, DevPairs& nw, const DevPairs& old, int capacity, int nNew,
+                     int nOld, cudaStream_t s, const int* newCnt, const int* oldCnt) {
+    const int* offPrev = bb.offPrevValid ? bb.offPrev : nullptr;
+    if (bb.direct) {
+        k_direct_fill<<<gridn(w.nBodies, DIRECT_THREADS / 32), DIRECT_THREADS, 0, s>>>(
+            w, bb.list, bb.planeList, bb.planeStart, bb.off, bb.tcount, bb.kept, bb.partners, nw, old, capacity, nOld,
+            offPrev, oldCnt);
         note_launch();
+    } else {
+        tree_fill(w, bb, nw, capacity, s);
+        if (nNew > 0) {
+            k_persist<<<gridn(nNew, 256), 256, 0, s>>>(w, nw, old, nNew, nOld, offPrev, newCnt, oldCnt);
+            note_launch();
+        }
     }
     std::swap(bb.off, bb.offPrev);   // this step's offsets index the pair array the next step persists from
     bb.offPrevValid = true;

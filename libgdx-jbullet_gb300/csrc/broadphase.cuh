@@ -1,4 +1,6 @@
 #pragma once
+#include <vector>
+
 #include "jbgpu_internal.cuh"
 
 namespace jbg {
@@ -21,11 +23,24 @@ struct Bvh {           // Karras radix tree over nf sorted leaves; internal node
 
 constexpr int TRAV_CACHE = 64;         // pairs a counting traversal keeps for the filling one
 
+constexpr int DIRECT_CACHE = 256;      // the same of the direct count; more and the fill tests again
+
+struct DirectList {    // every body, grouped by world in index order
+    int* body = nullptr;
+    int* pos = nullptr;    // per body: its place in `body`
+    int* end = nullptr;    // per world: the end of its group
+};
+
 struct BroadphaseBuffers {
     int nFinite = 0, nPlanes = 0, nWorlds = 1, worldBits = 0;
     int rebuildInterval = 1;             // rebuild the tree every this many steps, refit in between
     int sinceBuild = 0;                  // steps since the last build
-    bool built = false;                  // the tree matches the current body set
+    bool built = false;                  // the Morton order matches the current body set
+    bool treeBuilt = false;              // the tree's topology matches that order
+    bool direct = false;                 // pairs by testing a world's bodies directly
+    DirectList list;
+    int* kept = nullptr;                 // per body: the first DIRECT_CACHE partners its count found
+    bool meshes = false;                 // some listed body is a triangle mesh
     unsigned* bounds = nullptr;          // 6 ordered-int scene bounds
     uint64_t* mkeys = nullptr;           // morton keys (sorted in place)
     uint64_t* mkeys_alt = nullptr;
@@ -52,12 +67,18 @@ struct BroadphaseBuffers {
     int* tcache = nullptr;               // per sorted leaf: the first TRAV_CACHE partners' sorted leaves
 };
 
-void broadphase_build_tree(const DevWorld& w, BroadphaseBuffers& bb, cudaStream_t s);
+void broadphase_order(const DevWorld& w, BroadphaseBuffers& bb, cudaStream_t s);
+void broadphase_topology(BroadphaseBuffers& bb, cudaStream_t s);
 void broadphase_refit_into(const DevWorld& wq, const BroadphaseBuffers& bb, float4* node, int* visit, cudaStream_t s);
+// Whether the next count renews the Morton order.
+bool broadphase_rebuilds(const BroadphaseBuffers& bb);
+// Whether worlds of these many bodies (all, finite) find their pairs without the tree.
+bool broadphase_direct(const std::vector<int>& bodies, const std::vector<int>& finite);
 void broadphase_run_count(const DevWorld& w, BroadphaseBuffers& bb, cudaStream_t s);
-void broadphase_run_fill(const DevWorld& w, BroadphaseBuffers& bb, DevPairs& nw, int capacity, cudaStream_t s);
-// newCnt / oldCnt (nullable): the pair counts on the device, nNew / nOld then being upper bounds.
-void broadphase_persist(const DevWorld& w, BroadphaseBuffers& bb, DevPairs& nw, const DevPairs& old, int nNew, int nOld,
-                        cudaStream_t s, const int* newCnt = nullptr, const int* oldCnt = nullptr);
+// Keys of the counted pairs into nw (room for `capacity`), the manifolds of persisting pairs carried
+// over from old.  newCnt / oldCnt (nullable): the pair counts on the device, nNew / nOld then being
+// upper bounds.
+void broadphase_fill(const DevWorld& w, BroadphaseBuffers& bb, DevPairs& nw, const DevPairs& old, int capacity, int nNew,
+                     int nOld, cudaStream_t s, const int* newCnt = nullptr, const int* oldCnt = nullptr);
 
 }  // namespace jbg

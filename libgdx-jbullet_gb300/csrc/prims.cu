@@ -13,6 +13,9 @@ namespace {
 constexpr int SCAN_BLOCK = 1024;
 constexpr int SCAN_ITEMS = 4;
 constexpr int SCAN_TILE = SCAN_BLOCK * SCAN_ITEMS;
+// Up to this many tiles (8 million values) a tile's carry is summed by its own block: one launch less
+// than a scan of the tile sums apart, about 3 us in every scan of a step.
+constexpr int SCAN_CARRY_TILES = 2048;
 constexpr int RS_THREADS = 256;
 constexpr int RS_ROUNDS = 16;
 constexpr int RS_TILE = RS_THREADS * RS_ROUNDS;
@@ -43,7 +46,8 @@ __device__ __forceinline__ int block_inclusive_scan(int v, int* smem) {
     return v;
 }
 
-__global__ void k_scan_tiles(const int* in, int* out, int* tileSums, int n) {
+// total (nullable): written when one tile holds all values.
+__global__ void k_scan_tiles(const int* in, int* out, int* tileSums, int n, int* total) {
     __shared__ int smem[32];
     int base = blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_ITEMS;
     int v[SCAN_ITEMS];
@@ -52,7 +56,10 @@ __global__ void k_scan_tiles(const int* in, int* out, int* tileSums, int n) {
     int incl = block_inclusive_scan(sum, smem);
     int run = incl - sum;
     for (int k = 0; k < SCAN_ITEMS; k++) { if (base + k < n) out[base + k] = run; run += v[k]; }
-    if (threadIdx.x == blockDim.x - 1) tileSums[blockIdx.x] = incl;
+    if (threadIdx.x == blockDim.x - 1) {
+        if (gridDim.x > 1) tileSums[blockIdx.x] = incl;
+        else if (total) *total = incl;
+    }
 }
 
 // Single block: exclusive scan of m values in place (m arbitrary, looped in chunks of 1024).
@@ -81,6 +88,23 @@ __global__ void k_scan_add(int* out, const int* tileSums, int n) {
         if (base + k < n) out[base + k] += add;
 }
 
+// The same from the tiles' own sums: every block adds up those before its tile.
+__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_carry(int* out, const int* tileSums, int n, int* total) {
+    __shared__ int smem[32];
+    __shared__ int before;
+    int v = 0;
+    for (int k = threadIdx.x; k < (int)blockIdx.x; k += SCAN_BLOCK) v += tileSums[k];
+    const int sum = block_inclusive_scan(v, smem);
+    if (threadIdx.x == SCAN_BLOCK - 1) {
+        before = sum;
+        if (blockIdx.x == gridDim.x - 1 && total) *total = sum + tileSums[blockIdx.x];
+    }
+    __syncthreads();
+    const int add = before, base = blockIdx.x * SCAN_TILE;
+    for (int k = threadIdx.x; k < SCAN_TILE; k += SCAN_BLOCK)
+        if (base + k < n) out[base + k] += add;
+}
+
 size_t scan_scratch_bytes(int n) { return sizeof(int) * (size_t)((n + SCAN_TILE - 1) / SCAN_TILE + 1); }
 
 void exclusive_scan(const int* in, int* out, int* total, int n, void* scratch, cudaStream_t s) {
@@ -90,9 +114,14 @@ void exclusive_scan(const int* in, int* out, int* total, int n, void* scratch, c
     }
     int tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
     int* sums = (int*)scratch;
-    k_scan_tiles<<<tiles, SCAN_BLOCK, 0, s>>>(in, out, sums, n); note_launch();
+    k_scan_tiles<<<tiles, SCAN_BLOCK, 0, s>>>(in, out, sums, n, total); note_launch();
+    if (tiles == 1) return;
+    if (tiles <= SCAN_CARRY_TILES) {
+        k_scan_carry<<<tiles, SCAN_BLOCK, 0, s>>>(out, sums, n, total); note_launch();
+        return;
+    }
     k_scan_single<<<1, SCAN_BLOCK, 0, s>>>(sums, tiles, total); note_launch();
-    if (tiles > 1) { k_scan_add<<<tiles, 256, 0, s>>>(out, sums, n); note_launch(); }
+    k_scan_add<<<tiles, 256, 0, s>>>(out, sums, n); note_launch();
 }
 
 // ---- radix sort ---------------------------------------------------------------------------

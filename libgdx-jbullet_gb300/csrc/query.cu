@@ -1131,7 +1131,8 @@ int query_prepare(const DevWorld& w, BroadphaseBuffers& bb, QueryBuffers& qb, bo
     DevWorld wq = w;
     wq.amin = qb.qmin;
     wq.amax = qb.qmax;
-    if (!bb.built) broadphase_build_tree(wq, bb, s);
+    if (!bb.built) broadphase_order(wq, bb, s);
+    if (!bb.treeBuilt) broadphase_topology(bb, s);
     const int nodes = bb.nFinite > 1 ? bb.nFinite - 1 : 1;
     if (nodes > qb.capNodes) {
         if (qb.node) cudaFree(qb.node);

@@ -388,6 +388,7 @@ int sync_shapes(jbgpu_world* w) {
 int sync_planes(jbgpu_world* w) {
     if (!w->planesDirty) return JBGPU_OK;
     BroadphaseBuffers& B = w->bb;
+    B.meshes = false;
     int nw = 1;
     for (int i = 0; i < w->nBodies; i++) nw = std::max(nw, w->hWorld[i] + 1);
     std::vector<std::vector<int>> per(nw);
@@ -395,7 +396,11 @@ int sync_planes(jbgpu_world* w) {
     std::vector<int> finite(nw, 0);
     unsigned kinds = 0;                 // convex shape kinds present
     for (int i = 0; i < w->nBodies; i++) {
-        if (w->hFlags[i] & CF_LISTED) { per[w->hWorld[i]].push_back(i); np++; }
+        if (w->hFlags[i] & CF_LISTED) {
+            per[w->hWorld[i]].push_back(i);
+            np++;
+            B.meshes = B.meshes || w->shapes[w->hShape[i]].type == SHAPE_MESH;
+        }
         else {
             nf++;
             finite[w->hWorld[i]]++;
@@ -409,7 +414,7 @@ int sync_planes(jbgpu_world* w) {
     for (int k = 0; k < nw; k++) { start[k] = (int)list.size(); list.insert(list.end(), per[k].begin(), per[k].end()); }
     start[nw] = (int)list.size();
     dfree(B.planeList); dfree(B.planeStart); dfree(B.wstart); dfree(B.wend); dfree(B.wroot); dfree(B.bounds); dfree(B.total);
-    dfree(B.candBound); dfree(B.segLong);
+    dfree(B.candBound); dfree(B.segLong); dfree(B.list.body); dfree(B.list.pos); dfree(B.list.end); dfree(B.kept);
     CK(dalloc(&B.planeList, std::max<size_t>(1, list.size()))); CK(dalloc(&B.planeStart, nw + 1));
     CK(dalloc(&B.wstart, nw)); CK(dalloc(&B.wend, nw)); CK(dalloc(&B.wroot, nw)); CK(dalloc(&B.bounds, 6)); CK(dalloc(&B.total, 1));
     CK(dalloc(&B.candBound, 1)); CK(dalloc(&B.segLong, 1));
@@ -423,7 +428,20 @@ int sync_planes(jbgpu_world* w) {
     B.worldBits = nw > 1 ? bits : 0;
     w->nWorlds = nw;
     w->worldFinite = finite;
-    w->bb.built = false;
+    std::vector<int> pos(std::max(w->nBodies, 1)), end(nw + 1, 0), body(std::max(w->nBodies, 1)), bodies(nw, 0);
+    for (int i = 0; i < w->nBodies; i++) bodies[w->hWorld[i]]++;
+    for (int k = 0; k < nw; k++) end[k + 1] = end[k] + bodies[k];   // group starts, advanced to the ends below
+    for (int i = 0; i < w->nBodies; i++) {
+        pos[i] = end[w->hWorld[i]]++;
+        body[pos[i]] = i;
+    }
+    B.direct = broadphase_direct(bodies, finite);
+    if (B.direct) CK(dalloc(&B.kept, (size_t)DIRECT_CACHE * body.size()));
+    CK(dalloc(&B.list.body, body.size())); CK(dalloc(&B.list.pos, pos.size())); CK(dalloc(&B.list.end, nw));
+    CK(cudaMemcpy(B.list.body, body.data(), sizeof(int) * body.size(), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(B.list.pos, pos.data(), sizeof(int) * pos.size(), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(B.list.end, end.data(), sizeof(int) * nw, cudaMemcpyHostToDevice));
+    w->bb.built = w->bb.treeBuilt = false;
     w->solverDirty = true;
     w->orderValid = false;
     w->planesDirty = false;
@@ -478,8 +496,7 @@ int stage_pairs_fill(jbgpu_world* w, int total) {
     if (w->hasMesh && concave_reserve(w->nb, w->capRows, w->candBound, s) < 0)
         return fail(JBGPU_ERR_CUDA, "concave pass buffers");
     w->prof.mark(PH_PAIR_FILL, 0, s);
-    broadphase_run_fill(d, w->bb, w->pairs[nxt], w->capRows, s);
-    broadphase_persist(d, w->bb, w->pairs[nxt], w->pairs[w->cur], total, w->nPairs, s);
+    broadphase_fill(d, w->bb, w->pairs[nxt], w->pairs[w->cur], w->capRows, total, w->nPairs, s);
     w->prof.mark(PH_PAIR_FILL, 1, s);
     w->cur = nxt;
     w->nPairs = total;
@@ -757,8 +774,8 @@ uint64_t fbits64(float f) { uint32_t u; std::memcpy(&u, &f, 4); return u; }
 int single_step_graph(jbgpu_world* w, float dt) {
     cudaStream_t s = w->stream;
     BroadphaseBuffers& B = w->bb;
-    const bool rebuild = !(B.built && B.sinceBuild + 1 < B.rebuildInterval);
-    const bool builtBefore = B.built;
+    const bool rebuild = broadphase_rebuilds(B);
+    const bool builtBefore = B.built, treeBefore = B.treeBuilt;
     const int ageBefore = B.sinceBuild;
     const uint64_t ka[8] = {1, (uint64_t)rebuild, (uint64_t)(uintptr_t)B.off, (uint64_t)(uintptr_t)B.offPrev,
                             fbits64(dt), 0, 0, 0};
@@ -774,12 +791,13 @@ int single_step_graph(jbgpu_world* w, float dt) {
     }, captured);
     if (rc == GRAPH_FALLBACK) {            // nothing ran: undo the capture's host side
         B.built = builtBefore;
+        B.treeBuilt = treeBefore;
         B.sinceBuild = ageBefore;
         return GRAPH_FALLBACK;
     }
     if (rc) return rc;
     if (!captured) {                       // what broadphase_run_count does on the host
-        if (rebuild) { B.built = true; B.sinceBuild = 0; }
+        if (rebuild) { B.built = true; B.treeBuilt = !B.direct; B.sinceBuild = 0; }
         else B.sinceBuild++;
     }
     w->orderValid = true;
@@ -813,8 +831,7 @@ int single_step_graph(jbgpu_world* w, float dt) {
         DevWorld d = dev_view(w);
         w->pairCountDev = cnt;
         struct Reset { jbgpu_world* w; ~Reset() { w->pairCountDev = nullptr; } } reset{w};
-        broadphase_run_fill(d, B, w->pairs[nxt], bound, s);
-        broadphase_persist(d, B, w->pairs[nxt], w->pairs[old], bound, w->capPairs[old], s, B.total, cnt);
+        broadphase_fill(d, B, w->pairs[nxt], w->pairs[old], bound, bound, w->capPairs[old], s, B.total, cnt);
         CK(cudaMemcpyAsync(cnt, B.total, sizeof(int), cudaMemcpyDeviceToDevice, s));
         int r = narrow_and_islands(w, cnt);   // ... and read the count from the device
         if (r) return r;
@@ -839,7 +856,7 @@ int single_step_graph(jbgpu_world* w, float dt) {
     }
     w->nPairs = total;
     if (rc) return rc;
-    if (!captured) {                       // broadphase_persist's host side
+    if (!captured) {                       // broadphase_fill's host side
         std::swap(B.off, B.offPrev);
         B.offPrevValid = true;
     }
@@ -1348,7 +1365,7 @@ int jbgpu_world_destroy(jbgpu_world* w) {
     dfree(B.bvh.left); dfree(B.bvh.right); dfree(B.bvh.lo); dfree(B.bvh.hi); dfree(B.bvh.parent); dfree(B.bvh.leafParent);
     dfree(B.bvh.visit); dfree(B.bvh.node); dfree(B.tcount); dfree(B.tcache); dfree(B.wstart); dfree(B.wend); dfree(B.wroot);
     dfree(B.planeList); dfree(B.planeStart); dfree(B.cnt); dfree(B.off); dfree(B.offPrev); dfree(B.cursor); dfree(B.total); dfree(B.partners);
-    dfree(B.candBound); dfree(B.segLong);
+    dfree(B.candBound); dfree(B.segLong); dfree(B.list.body); dfree(B.list.pos); dfree(B.list.end); dfree(B.kept);
     NarrowBuffers& N = w->nb;
     if (N.queue) cudaFree(N.queue);
     dfree(N.queueCount); dfree(N.ovfQueue); dfree(N.ovfQueue2); dfree(N.ovfCount); dfree(N.pairBucket); dfree(N.perm); dfree(N.blockOff);
