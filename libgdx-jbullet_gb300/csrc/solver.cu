@@ -1538,16 +1538,42 @@ JBD void body_impulse(V& lin, V& ang, float im, const M& iw, V impulse, V relPos
     ang = add(ang, mulMv(crs(relPos, impulse), iw));
 }
 
+// Where a joint's bodies keep their velocities: global memory, or (local) the block's shared memory at
+// their place in the one part; listed bodies (planes, meshes) stay in global memory.
+struct JointVel {
+    bool local = false;
+    float4 *sl = nullptr, *sa = nullptr;
+    const int* posOf = nullptr;
+    __device__ __forceinline__ void load(const DevWorld& w, int b, V& l, V& a) const {
+        if (local && !(w.flags[b] & CF_LISTED)) {
+            const int i = posOf[b];
+            l = mk4(sl[i]);
+            a = mk4(sa[i]);
+        } else {
+            gload(w, b, l, a);
+        }
+    }
+    __device__ __forceinline__ void store(const DevWorld& w, int b, V l, V a) const {
+        if (local && !(w.flags[b] & CF_LISTED)) {
+            const int i = posOf[b];
+            sl[i] = f4(l, 0.0f);
+            sa[i] = f4(a, 0.0f);
+        } else {
+            gstore(w, b, l, a);
+        }
+    }
+};
+
 // Point2PointConstraint.solveConstraint (java:103-171) of joint j on the bodies' velocities in
 // global memory: per axis, impulse = depth tau / dt / Adiag - damping relVel / Adiag, clamped,
 // applied to both bodies.
-JBD void joint_solve(const DevWorld& w, const DevJoints& J, int j, float dt) {
+JBD void joint_solve(const DevWorld& w, const DevJoints& J, const JointVel& at, int j, float dt) {
     const int a = J.a[j], b = J.b[j];
     const float4 q1 = J.r1[j], q2 = J.r2[j], dp = J.dep[j], st = J.set[j];
     const V r1 = mk(q1.x, q1.y, q1.z), r2 = mk(q2.x, q2.y, q2.z);
     V vA, wA, vB = mk(0.0f, 0.0f, 0.0f), wB = mk(0.0f, 0.0f, 0.0f);
-    gload(w, a, vA, wA);
-    if (b >= 0) gload(w, b, vB, wB);
+    at.load(w, a, vA, wA);
+    if (b >= 0) at.load(w, b, vB, wB);
     const float imA = w.iloc[a].w, imB = b >= 0 ? w.iloc[b].w : 0.0f;
     const M IA = load_iw(w, a);
     M IB;
@@ -1572,8 +1598,8 @@ JBD void joint_solve(const DevWorld& w, const DevJoints& J, int j, float dt) {
         body_impulse(vB, wB, imB, IB, scl(iv, -1.0f), r2);
         set_coord(n, i, 0.0f);
     }
-    if (imA != 0.0f) gstore(w, a, vA, wA);
-    if (b >= 0 && imB != 0.0f) gstore(w, b, vB, wB);
+    if (imA != 0.0f) at.store(w, a, vA, wA);
+    if (b >= 0 && imB != 0.0f) at.store(w, b, vB, wB);
     __stcg(J.imp + j, acc);
 }
 
@@ -1590,11 +1616,11 @@ JBD void torque_impulse(V& ang, float im, const M& iw, V t) {
 // them: the relative angular velocity orthogonal to the hinge axes and the axes' misalignment
 // removed by torque impulses, the limit with its clamped accumulated impulse, the motor clipped
 // per solve.
-JBD void hinge_solve(const DevWorld& w, const DevJoints& J, int j, float dt) {
+JBD void hinge_solve(const DevWorld& w, const DevJoints& J, const JointVel& at, int j, float dt) {
     const int a = J.a[j], b = J.b[j], kind = J.kind[j];
     V vA, wA, vB = mk(0.0f, 0.0f, 0.0f), wB = mk(0.0f, 0.0f, 0.0f);
-    gload(w, a, vA, wA);
-    if (b >= 0) gload(w, b, vB, wB);
+    at.load(w, a, vA, wA);
+    if (b >= 0) at.load(w, b, vB, wB);
     const float imA = w.iloc[a].w, imB = b >= 0 ? w.iloc[b].w : 0.0f;
     const M IA = load_iw(w, a), IB = joint_iw(w, b);
     const float4* H = J.hs + JOINT_STEP_F4 * j;
@@ -1657,8 +1683,8 @@ JBD void hinge_solve(const DevWorld& w, const DevJoints& J, int j, float dt) {
         torque_impulse(wA, imA, IA, add(motorImp, zero));
         torque_impulse(wB, imB, IB, sub(scl(motorImp, -1.0f), zero));
     }
-    if (imA != 0.0f) gstore(w, a, vA, wA);
-    if (b >= 0 && imB != 0.0f) gstore(w, b, vB, wB);
+    if (imA != 0.0f) at.store(w, a, vA, wA);
+    if (b >= 0 && imB != 0.0f) at.store(w, b, vB, wB);
     __stcg(J.imp + j, acc);
     __stcg(&J.hs[JOINT_STEP_F4 * j + 5].y, accLimit);
 }
@@ -1668,11 +1694,11 @@ JBD void hinge_solve(const DevWorld& w, const DevJoints& J, int j, float dt) {
 // (TranslationalLimitMotor.java:70-150) per limited linear axis, on the velocities as the earlier
 // axes left them, then RotationalLimitMotor.solveAngularLimits (RotationalLimitMotor.java:135-203)
 // per angular axis whose limit or motor applies.
-JBD void d6_solve(const DevWorld& w, const DevJoints& J, int j, float dt) {
+JBD void d6_solve(const DevWorld& w, const DevJoints& J, const JointVel& at, int j, float dt) {
     const int a = J.a[j], b = J.b[j];
     V vA, wA, vB = mk(0.0f, 0.0f, 0.0f), wB = mk(0.0f, 0.0f, 0.0f);
-    gload(w, a, vA, wA);
-    if (b >= 0) gload(w, b, vB, wB);
+    at.load(w, a, vA, wA);
+    if (b >= 0) at.load(w, b, vB, wB);
     const float imA = w.iloc[a].w, imB = b >= 0 ? w.iloc[b].w : 0.0f;
     const M IA = load_iw(w, a), IB = joint_iw(w, b);
     const float4* S = J.d6set + D6_SET_F4 * j;
@@ -1738,8 +1764,8 @@ JBD void d6_solve(const DevWorld& w, const DevJoints& J, int j, float dt) {
         torque_impulse(wA, imA, IA, mi);
         torque_impulse(wB, imB, IB, scl(mi, -1.0f));
     }
-    if (imA != 0.0f) gstore(w, a, vA, wA);
-    if (b >= 0 && imB != 0.0f) gstore(w, b, vB, wB);
+    if (imA != 0.0f) at.store(w, a, vA, wA);
+    if (b >= 0 && imB != 0.0f) at.store(w, b, vB, wB);
     __stcg(H + 11, accL);
     __stcg(H + 12, accA);
 }
@@ -1747,11 +1773,11 @@ JBD void d6_solve(const DevWorld& w, const DevJoints& J, int j, float dt) {
 // ConeTwistConstraint.solveConstraint (ConeTwistConstraint.java:267-368): the hinge's linear rows,
 // then the swing and twist limits with clamped accumulated impulses, both from the angular
 // velocities as the linear rows left them.
-JBD void cone_solve(const DevWorld& w, const DevJoints& J, int j, float dt) {
+JBD void cone_solve(const DevWorld& w, const DevJoints& J, const JointVel& at, int j, float dt) {
     const int a = J.a[j], b = J.b[j], kind = J.kind[j];
     V vA, wA, vB = mk(0.0f, 0.0f, 0.0f), wB = mk(0.0f, 0.0f, 0.0f);
-    gload(w, a, vA, wA);
-    if (b >= 0) gload(w, b, vB, wB);
+    at.load(w, a, vA, wA);
+    if (b >= 0) at.load(w, b, vB, wB);
     const float imA = w.iloc[a].w, imB = b >= 0 ? w.iloc[b].w : 0.0f;
     const M IA = load_iw(w, a), IB = joint_iw(w, b);
     float4* H = J.hs + JOINT_STEP_F4 * j;
@@ -1790,20 +1816,20 @@ JBD void cone_solve(const DevWorld& w, const DevJoints& J, int j, float dt) {
         torque_impulse(wA, imA, IA, imp);
         torque_impulse(wB, imB, IB, scl(imp, -1.0f));
     }
-    if (imA != 0.0f) gstore(w, a, vA, wA);
-    if (b >= 0 && imB != 0.0f) gstore(w, b, vB, wB);
+    if (imA != 0.0f) at.store(w, a, vA, wA);
+    if (b >= 0 && imB != 0.0f) at.store(w, b, vB, wB);
     __stcg(J.imp + j, acc);
     __stcg(H + 6, lim);
 }
 
 // SliderConstraint.solveConstraintInt (SliderConstraint.java:528-685) on the bodies in the roles
 // the setup gave them.
-JBD void slider_solve(const DevWorld& w, const DevJoints& J, int j, float dt) {
+JBD void slider_solve(const DevWorld& w, const DevJoints& J, const JointVel& at, int j, float dt) {
     const bool useA = J.set[j].x != 0.0f;
     const int ia = useA ? J.a[j] : J.b[j], ib = useA ? J.b[j] : J.a[j];
     V vA = mk(0.0f, 0.0f, 0.0f), wA = vA, vB = vA, wB = vA;
-    if (ia >= 0) gload(w, ia, vA, wA);
-    if (ib >= 0) gload(w, ib, vB, wB);
+    if (ia >= 0) at.load(w, ia, vA, wA);
+    if (ib >= 0) at.load(w, ib, vB, wB);
     const float imA = ia >= 0 ? w.iloc[ia].w : 0.0f, imB = ib >= 0 ? w.iloc[ib].w : 0.0f;
     const M IA = joint_iw(w, ia), IB = joint_iw(w, ib);
     const float4* P = J.d6set + D6_SET_F4 * j;
@@ -1877,8 +1903,8 @@ JBD void slider_solve(const DevWorld& w, const DevJoints& J, int j, float dt) {
         torque_impulse(wA, imA, IA, mi);
         torque_impulse(wB, imB, IB, scl(mi, -1.0f));
     }
-    if (ia >= 0 && imA != 0.0f) gstore(w, ia, vA, wA);
-    if (ib >= 0 && imB != 0.0f) gstore(w, ib, vB, wB);
+    if (ia >= 0 && imA != 0.0f) at.store(w, ia, vA, wA);
+    if (ib >= 0 && imB != 0.0f) at.store(w, ib, vB, wB);
     __stcg(H + 8, acc);
 }
 
@@ -2041,6 +2067,20 @@ JBD void island_residuals(const DevWorld& w, const SolverBuffers& sb, int flag, 
     }
 }
 
+// One colour of joints (those of processed islands): no two share a body.
+JBD void joint_colour(const DevWorld& w, const SolverBuffers& sb, int c, const JointVel& at, int first, int stride, float dt) {
+    for (int q = sb.J.colStart[c] + first; q < sb.J.colStart[c + 1]; q += stride) {
+        const int j = sb.J.order[q];
+        if (!sb.J.act[j]) continue;
+        const int jt = sb.J.kind[j] & JK_TYPE;
+        if (jt == JOINT_HINGE) hinge_solve(w, sb.J, at, j, dt);
+        else if (jt == JOINT_6DOF) d6_solve(w, sb.J, at, j, dt);
+        else if (jt == JOINT_CONE) cone_solve(w, sb.J, at, j, dt);
+        else if (jt == JOINT_SLIDER) slider_solve(w, sb.J, at, j, dt);
+        else joint_solve(w, sb.J, at, j, dt);
+    }
+}
+
 // Phases: warm start, then iterations of (normal rows, friction rows): numIterations of them,
 // or, with a residual tolerance, until every island's residual is within it (at most maxIter;
 // the rows of an island stop once it converges).  Within a phase the parts' internal
@@ -2114,8 +2154,47 @@ __global__ void __launch_bounds__(SOLVER_THREADS, 2) k_pgs(DevWorld w, DevPairs 
     }
     if (nSlots == 0 && sb.J.n == 0) return;
     const bool contacts = nSlots > 0;   // else only joints (the colouring did not run this step)
-    if (tid == 0) for (int k = 0; k < 3; k++) w.ctr[C_RES0 + k] = 0;
     Staged st;
+    if (nb == 1 && sb.nParts == 1 && nCut == 0 && !byRes && smem && sb.partMax <= sb.smemCap) {
+        // One part with joints, one block: its velocities stay in shared memory through every phase of
+        // joints and contacts, and a phase ends with the block's barrier.  With the part staged in and
+        // out around every phase and a grid barrier of one block, 64 chains of 8 took
+        // 190 us, 75 us so.
+        PartView v = part_view(sb, 0);
+        if (!contacts) v.nLoc = 0;
+        JointVel at;
+        at.local = true;
+        at.sl = sl;
+        at.sa = sa;
+        at.posOf = sb.posOf;
+        stage_in(w, sb, v, sl, sa);
+        if (!contacts)
+            for (int i = threadIdx.x; i < v.np; i += blockDim.x) sb.posOf[sb.order[i]] = i;
+        __syncthreads();
+        for (int ph = 0; ph < 1 + 2 * maxIt; ph++) {
+            const int kind = ph == 0 ? PH_WARM : (ph & 1 ? PH_NORMAL : PH_FRICTION);
+            if (kind == PH_NORMAL)
+                for (int c = 0; c < sb.J.nCol; c++) {
+                    joint_colour(w, sb, c, at, threadIdx.x, blockDim.x, dt);
+                    __syncthreads();
+                }
+            st = Staged();
+            for (int c = 0; c < v.nLoc; c++) {
+                const bool last = c + 1 == v.nLoc;
+                if (threadIdx.x == 0) shPoolTop[(step + 2) % 3] = 0;
+                local_colour(w, R, sb, v.lcs[c], v.lcs[c + 1], kind, true, sl, sa, rc,
+                             last ? 0 : v.lcs[c + 1] + (int)threadIdx.x, last ? 0 : v.lcs[c + 2], kind, pool(step),
+                             pool(step + 1), st);
+                __syncthreads();
+                ++step;
+            }
+        }
+        stage_out(w, sb, v, sl, sa);
+        if (tid == 0 && maxIt > 0) atomicMax(&w.ctr[C_PGS_ITERS], maxIt);
+        for (int s = tid; s < nSlots; s += nth) writeback_slot(P, R, s);
+        return;
+    }
+    if (tid == 0) for (int k = 0; k < 3; k++) w.ctr[C_RES0 + k] = 0;
     int it = -1;          // -1: the warm-start phase
     for (;;) {
         for (int sub = 0; sub < (it < 0 ? 1 : 2); sub++) {
@@ -2124,17 +2203,7 @@ __global__ void __launch_bounds__(SOLVER_THREADS, 2) k_pgs(DevWorld w, DevPairs 
                 // the joints of processed islands, before the iteration's contact rows
                 // (SequentialImpulseConstraintSolver.java:823-842), colour by colour
                 for (int c = 0; c < sb.J.nCol; c++) {
-                    const int j0 = sb.J.colStart[c], j1 = sb.J.colStart[c + 1];
-                    for (int q = j0 + spread; q < j1; q += nth) {
-                        const int j = sb.J.order[q];
-                        if (!sb.J.act[j]) continue;
-                        const int jt = sb.J.kind[j] & JK_TYPE;
-                        if (jt == JOINT_HINGE) hinge_solve(w, sb.J, j, dt);
-                        else if (jt == JOINT_6DOF) d6_solve(w, sb.J, j, dt);
-                        else if (jt == JOINT_CONE) cone_solve(w, sb.J, j, dt);
-                        else if (jt == JOINT_SLIDER) slider_solve(w, sb.J, j, dt);
-                        else joint_solve(w, sb.J, j, dt);
-                    }
+                    joint_colour(w, sb, c, JointVel(), spread, nth, dt);
                     grid_barrier(w.ctr, nb, barK);
                 }
             }
