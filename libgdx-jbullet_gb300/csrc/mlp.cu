@@ -16,7 +16,7 @@ int set_last_error(int code, const char* msg);   // world.cu
 using namespace jbg;
 
 struct jbgpu_mlp {
-    int device = 0;
+    int device = 0, sms = 1;
     cudaStream_t s = nullptr;
     float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr, *norm = nullptr, *loss = nullptr;
     __nv_bfloat16 *w1 = nullptr, *w2 = nullptr, *w3 = nullptr;
@@ -69,99 +69,122 @@ JBD int mlp_load_inputs(MlpSmem& S, const MlpDev& M, const float* X, const int* 
     return valid;
 }
 
-// One 64-sample tile of a mini-batch: forward, loss, backward, gradients added into grad.
-// coef = 2 / (batch samples x outputs): the derivative of the batch-mean squared error.
-__global__ void __launch_bounds__(MLP_THREADS) k_mlp_train(MlpDev M, const float* X, const float* T, const int* idx,
-                                                            int first, int count, float coef, float* grad, float* loss) {
+// c * gelu' as bf16 into dz (rows m0.., columns n0.. of the warp) and its column sums into b.
+template <int NT>
+JBD void mlp_dz(const float (&c)[NT][4], const float (&grad)[NT][4], __nv_bfloat16 (*dz)[MLP_LDH], float (&b)[NT][2], int m0,
+                int n0) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int q = 0; q < NT; q++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const __nv_bfloat16 x = __float2bfloat16_rn(c[q][2 * h] * grad[q][2 * h]);
+            const __nv_bfloat16 y = __float2bfloat16_rn(c[q][2 * h + 1] * grad[q][2 * h + 1]);
+            *(uint32_t*)&dz[m0 + g + 8 * h][n0 + 8 * q + 2 * t] = pack_bf16(x, y);
+            b[q][0] += __bfloat162float(x);
+            b[q][1] += __bfloat162float(y);
+        }
+}
+
+JBD void red_add2(float* p, float a, float b) {   // p 8-byte aligned
+    asm volatile("red.relaxed.gpu.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(a), "f"(b) : "memory");
+}
+
+// 64-sample tiles of a mini-batch: forward, loss, backward; the block's gradients stay in registers over
+// its tiles and are added into grad at the end.  coef = 2 / (batch samples x outputs): the derivative of
+// the batch-mean squared error.
+// What bounds it: the length of one tile's chain, five products deep with a block barrier between.
+// Operands gathered element by element from rows on the same banks, gelu' worked out again and a
+// quarter as many warps took 55 us for 256 tiles; 21 us so.
+__global__ void __launch_bounds__(MLP_TRAIN_THREADS) k_mlp_train(MlpDev M, const float* X, const float* T, const int* idx,
+                                                                  int first, int count, float coef, float* grad,
+                                                                  float* loss) {
+    constexpr int WARPS = MLP_TRAIN_THREADS / 32, NT = MlpTiles<WARPS>::NT;
     extern __shared__ __align__(16) unsigned char mlpSmem[];
     MlpSmem& S = *reinterpret_cast<MlpSmem*>(mlpSmem);
-    const int tileFirst = first + blockIdx.x * MLP_TILE;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int m0 = warp * 16;
+    const int m0 = (warp & 3) * 16, n0 = (warp >> 2) * 8 * NT;
+    const int tiles = (count + MLP_TILE - 1) / MLP_TILE;
     mlp_load_weights(S, M);
-    const int valid = mlp_load_inputs(S, M, X, idx, tileFirst, first + count);
-    __syncthreads();
-    mlp_forward(S, M);
-    // loss and dY (FP32 kept in S.y, BF16 copy padded to 16 columns in S.dy)
-    float part = 0.0f;
-    for (int e = threadIdx.x; e < MLP_TILE * MLP_OUTP; e += blockDim.x) {
-        int i = e / MLP_OUTP, o = e % MLP_OUTP;
-        float d = 0.0f;
-        if (i < valid && o < MLP_OUT) {
-            int row = idx ? idx[tileFirst + i] : tileFirst + i;
-            float tn = (T[(size_t)row * MLP_OUT + o] - M.norm[2 * MLP_IN + o]) / M.norm[2 * MLP_IN + MLP_OUT + o];
-            float r = S.y[i][o] - tn;
-            part += r * r;
-            d = coef * r;
+    float lossSum = 0.0f;
+    float b3 = 0.0f;                        // lane o of warp 0: db3[o]
+    float b1[NT][2] = {}, b2[NT][2] = {};   // the lane's columns n0 + 8 q + 2 t + e, its rows alone
+    float w3[2][4] = {}, w2[NT][4] = {}, w1[2][4] = {};
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int tileFirst = first + tile * MLP_TILE;
+        const int valid = mlp_load_inputs(S, M, X, idx, tileFirst, first + count);
+        __syncthreads();
+        MlpTiles<WARPS> G;
+        mlp_forward<WARPS>(S, M, G);
+        // loss and dY (FP32 kept in S.y, BF16 copy padded to 16 columns in S.dy)
+        for (int e = threadIdx.x; e < MLP_TILE * MLP_OUTP; e += blockDim.x) {
+            int i = e / MLP_OUTP, o = e % MLP_OUTP;
+            float d = 0.0f;
+            if (i < valid && o < MLP_OUT) {
+                int row = idx ? idx[tileFirst + i] : tileFirst + i;
+                float tn = (T[(size_t)row * MLP_OUT + o] - M.norm[2 * MLP_IN + o]) / M.norm[2 * MLP_IN + MLP_OUT + o];
+                float r = S.y[i][o] - tn;
+                lossSum += r * r;
+                d = coef * r;
+            }
+            S.dy[i][o] = __float2bfloat16_rn(d);
+            if (o < MLP_OUT) S.y[i][o] = d;
         }
-        S.dy[i][o] = __float2bfloat16_rn(d);
-        if (o < MLP_OUT) S.y[i][o] = d;
-    }
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    if (lane == 0 && part != 0.0f) atomicAdd(loss, part * coef * 0.5f);
-    __syncthreads();
-    // dW3 = dY^T H2 (16 padded rows x 64), warps split the columns
-    for (int n0 = warp * 16; n0 < warp * 16 + 16; n0 += 8) {
-        float c[4];
-        warp_gemm(c, 0, n0, MLP_TILE, [&](int o, int k) { return S.dy[k][o]; }, [&](int k, int n) { return S.h2[k][n]; });
-        for (int q = 0; q < 4; q++) {
-            int o = g + (q >> 1) * 8, n = n0 + 2 * t + (q & 1);
-            if (o < MLP_OUT) atomicAdd(&grad[MLP_OFF_W3 + o * MLP_H + n], c[q]);
+        __syncthreads();
+        // dZ2 = (dY W3) * gelu'(Z2)
+        {
+            float c[NT][4] = {};
+            warp_gemm<NT, MLP_OUTP, false, true>(c, &S.dy[m0][0], MLP_LDO, &S.w3[0][n0], MLP_LDH);
+            mlp_dz(c, G.g2, S.dz2, b2, m0, n0);
         }
-    }
-    if (threadIdx.x < MLP_OUT) {
-        float sdb = 0.0f;
-        for (int i = 0; i < MLP_TILE; i++) sdb += S.y[i][threadIdx.x];
-        atomicAdd(&grad[MLP_OFF_B3 + threadIdx.x], sdb);
-    }
-    // dZ2 = (dY W3) * gelu'(Z2)
-    for (int n0 = 0; n0 < MLP_H; n0 += 8) {
-        float c[4];
-        warp_gemm(c, m0, n0, MLP_OUTP, [&](int i, int k) { return S.dy[i][k]; }, [&](int k, int n) { return S.w3[k][n]; });
-        for (int q = 0; q < 4; q++) {
-            int i = m0 + g + (q >> 1) * 8, n = n0 + 2 * t + (q & 1);
-            S.dz2[i][n] = __float2bfloat16_rn(c[q] * gelu_grad(S.z2[i][n]));
+        // dW3 = dY^T H2 (16 padded rows), the columns over the warps by twos of tiles
+        if (warp < 4) warp_gemm<2, MLP_TILE, true, true>(w3, &S.dy[0][0], MLP_LDO, &S.h2[0][16 * warp], MLP_LDH);
+        else if (warp == 4 && lane < MLP_OUT)
+            for (int i = 0; i < MLP_TILE; i++) b3 += S.y[i][lane];
+        __syncthreads();
+        // dZ1 = (dZ2 W2) * gelu'(Z1); dW2 = dZ2^T H1
+        {
+            float c[NT][4] = {};
+            warp_gemm<NT, MLP_H, false, true>(c, &S.dz2[m0][0], MLP_LDH, &S.w2[0][n0], MLP_LDH);
+            mlp_dz(c, G.g1, S.dz1, b1, m0, n0);
         }
+        warp_gemm<NT, MLP_TILE, true, true>(w2, &S.dz2[0][m0], MLP_LDH, &S.h1[0][n0], MLP_LDH);
+        __syncthreads();
+        // dW1 = dZ1^T X: 16 columns a warp
+        warp_gemm<2, MLP_TILE, true, true>(w1, &S.dz1[0][m0], MLP_LDH, &S.x[0][16 * (warp >> 2)], MLP_LDX);
+        __syncthreads();
     }
-    __syncthreads();
-    // dW2 = dZ2^T H1 (rows split over warps), db2
-    for (int n0 = 0; n0 < MLP_H; n0 += 8) {
-        float c[4];
-        warp_gemm(c, m0, n0, MLP_TILE, [&](int i, int k) { return S.dz2[k][i]; }, [&](int k, int n) { return S.h1[k][n]; });
-        for (int q = 0; q < 4; q++) {
-            int i = m0 + g + (q >> 1) * 8, n = n0 + 2 * t + (q & 1);
-            atomicAdd(&grad[MLP_OFF_W2 + i * MLP_H + n], c[q]);
-        }
-    }
-    if (threadIdx.x < MLP_H) {
-        float sdb = 0.0f;
-        for (int i = 0; i < MLP_TILE; i++) sdb += __bfloat162float(S.dz2[i][threadIdx.x]);
-        atomicAdd(&grad[MLP_OFF_B2 + threadIdx.x], sdb);
-    }
-    // dZ1 = (dZ2 W2) * gelu'(Z1)
-    for (int n0 = 0; n0 < MLP_H; n0 += 8) {
-        float c[4];
-        warp_gemm(c, m0, n0, MLP_H, [&](int i, int k) { return S.dz2[i][k]; }, [&](int k, int n) { return S.w2[k][n]; });
-        for (int q = 0; q < 4; q++) {
-            int i = m0 + g + (q >> 1) * 8, n = n0 + 2 * t + (q & 1);
-            S.dz1[i][n] = __float2bfloat16_rn(c[q] * gelu_grad(S.z1[i][n]));
+    for (int o = 16; o > 0; o >>= 1) lossSum += __shfl_xor_sync(0xffffffffu, lossSum, o);
+    if (lane == 0 && lossSum != 0.0f) atomicAdd(loss, lossSum * coef * 0.5f);
+    if (warp == 4 && lane < MLP_OUT) atomicAdd(&grad[MLP_OFF_B3 + lane], b3);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int i = g + 8 * h;
+#pragma unroll
+        for (int q = 0; q < NT; q++)
+            red_add2(&grad[MLP_OFF_W2 + (m0 + i) * MLP_H + n0 + 8 * q + 2 * t], w2[q][2 * h], w2[q][2 * h + 1]);
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const int n = 16 * (warp >> 2) + 8 * q + 2 * t;
+            if (n < MLP_IN) red_add2(&grad[MLP_OFF_W1 + (m0 + i) * MLP_IN + n], w1[q][2 * h], w1[q][2 * h + 1]);
+            if (warp < 4 && i < MLP_OUT)
+                red_add2(&grad[MLP_OFF_W3 + i * MLP_H + 16 * warp + 8 * q + 2 * t], w3[q][2 * h], w3[q][2 * h + 1]);
         }
     }
-    __syncthreads();
-    // dW1 = dZ1^T X (24 of 32 padded columns), db1
-    for (int n0 = 0; n0 < MLP_IN; n0 += 8) {
-        float c[4];
-        warp_gemm(c, m0, n0, MLP_TILE, [&](int i, int k) { return S.dz1[k][i]; }, [&](int k, int n) { return S.x[k][n]; });
-        for (int q = 0; q < 4; q++) {
-            int i = m0 + g + (q >> 1) * 8, n = n0 + 2 * t + (q & 1);
-            atomicAdd(&grad[MLP_OFF_W1 + i * MLP_IN + n], c[q]);
+#pragma unroll
+    for (int q = 0; q < NT; q++)
+#pragma unroll
+        for (int e = 0; e < 2; e++)
+            for (int o = 4; o < 32; o <<= 1) {   // over the rows g
+                b1[q][e] += __shfl_xor_sync(0xffffffffu, b1[q][e], o);
+                b2[q][e] += __shfl_xor_sync(0xffffffffu, b2[q][e], o);
+            }
+    if (g == 0)
+#pragma unroll
+        for (int q = 0; q < NT; q++) {
+            red_add2(&grad[MLP_OFF_B1 + n0 + 8 * q + 2 * t], b1[q][0], b1[q][1]);
+            red_add2(&grad[MLP_OFF_B2 + n0 + 8 * q + 2 * t], b2[q][0], b2[q][1]);
         }
-    }
-    if (threadIdx.x < MLP_H) {
-        float sdb = 0.0f;
-        for (int i = 0; i < MLP_TILE; i++) sdb += __bfloat162float(S.dz1[i][threadIdx.x]);
-        atomicAdd(&grad[MLP_OFF_B1 + threadIdx.x], sdb);
-    }
 }
 
 // Raw features -> raw outputs (y = y' * outScale + outMean) for `count` rows.
@@ -172,7 +195,8 @@ __global__ void __launch_bounds__(MLP_THREADS) k_mlp_forward(MlpDev M, const flo
     for (int first = blockIdx.x * MLP_TILE; first < count; first += gridDim.x * MLP_TILE) {
         const int valid = mlp_load_inputs(S, M, X, nullptr, first, count);
         __syncthreads();
-        mlp_forward(S, M);
+        MlpTiles<MLP_THREADS / 32> G;
+        mlp_forward<MLP_THREADS / 32>(S, M, G);
         for (int e = threadIdx.x; e < valid * MLP_OUT; e += blockDim.x) {
             int i = e / MLP_OUT, o = e % MLP_OUT;
             Y[(size_t)(first + i) * MLP_OUT + o] = S.y[i][o] * M.norm[2 * MLP_IN + MLP_OUT + o] + M.norm[2 * MLP_IN + o];
@@ -225,7 +249,7 @@ int ensure_io(jbgpu_mlp* h, int n) {
 void launch_train_batch(jbgpu_mlp* h, const float* X, const float* T, const int* idx, int first, int count) {
     int tiles = (count + MLP_TILE - 1) / MLP_TILE;
     float coef = 2.0f / (float)(count * MLP_OUT);
-    k_mlp_train<<<tiles, MLP_THREADS, mlp_smem_bytes(), h->s>>>(mlp_view(h), X, T, idx, first, count, coef, h->g, h->loss);
+    k_mlp_train<<<std::min(tiles, 2 * h->sms), MLP_TRAIN_THREADS, mlp_smem_bytes(), h->s>>>(mlp_view(h), X, T, idx, first, count, coef, h->g, h->loss);
     note_launch();
 }
 
@@ -247,6 +271,7 @@ int jbgpu_mlp_create(int32_t device, uint64_t seed, jbgpu_mlp** out) {
         return set_last_error(JBGPU_ERR_CUDA, cudaGetErrorString(e));
     };
     cudaError_t e;
+    if ((e = cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess) return fail(e);
     if ((e = cudaStreamCreateWithFlags(&h->s, cudaStreamNonBlocking)) != cudaSuccess) return fail(e);
     if ((e = cudaMalloc(&h->p, sizeof(float) * MLP_NPARAM)) != cudaSuccess) return fail(e);
     if ((e = cudaMalloc(&h->g, sizeof(float) * MLP_NPARAM)) != cudaSuccess) return fail(e);

@@ -2401,7 +2401,8 @@ __global__ void __launch_bounds__(MLP_THREADS) k_mlp_warmstart(DevWorld w, DevPa
             }
         }
         __syncthreads();
-        mlp_forward(S, M);
+        MlpTiles<MLP_THREADS / 32> G;
+        mlp_forward<MLP_THREADS / 32>(S, M, G);
         if (threadIdx.x < MLP_TILE) {
             const int q = first + threadIdx.x;
             if (q < nq) {
