@@ -18,7 +18,9 @@ using namespace jbg;
 struct jbgpu_mlp {
     int device = 0, sms = 1;
     cudaStream_t s = nullptr;
-    float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr, *norm = nullptr, *loss = nullptr;
+    float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr, *norm = nullptr;
+    float* loss = nullptr;                // behind the gradient: both are cleared and read together
+    float* hostGrad = nullptr;            // pinned: gradient and loss
     __nv_bfloat16 *w1 = nullptr, *w2 = nullptr, *w3 = nullptr;
     float *X = nullptr, *T = nullptr;     // training set on the device
     int n = 0, cap = 0;
@@ -274,11 +276,12 @@ int jbgpu_mlp_create(int32_t device, uint64_t seed, jbgpu_mlp** out) {
     if ((e = cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess) return fail(e);
     if ((e = cudaStreamCreateWithFlags(&h->s, cudaStreamNonBlocking)) != cudaSuccess) return fail(e);
     if ((e = cudaMalloc(&h->p, sizeof(float) * MLP_NPARAM)) != cudaSuccess) return fail(e);
-    if ((e = cudaMalloc(&h->g, sizeof(float) * MLP_NPARAM)) != cudaSuccess) return fail(e);
+    if ((e = cudaMalloc(&h->g, sizeof(float) * (MLP_NPARAM + 1))) != cudaSuccess) return fail(e);
+    h->loss = h->g + MLP_NPARAM;
+    if ((e = cudaMallocHost(&h->hostGrad, sizeof(float) * (MLP_NPARAM + 1))) != cudaSuccess) return fail(e);
     if ((e = cudaMalloc(&h->m, sizeof(float) * MLP_NPARAM)) != cudaSuccess) return fail(e);
     if ((e = cudaMalloc(&h->v, sizeof(float) * MLP_NPARAM)) != cudaSuccess) return fail(e);
     if ((e = cudaMalloc(&h->norm, sizeof(float) * MLP_NORM)) != cudaSuccess) return fail(e);
-    if ((e = cudaMalloc(&h->loss, sizeof(float))) != cudaSuccess) return fail(e);
     if ((e = cudaMalloc(&h->w1, sizeof(__nv_bfloat16) * MLP_H * MLP_INP)) != cudaSuccess) return fail(e);
     if ((e = cudaMalloc(&h->w2, sizeof(__nv_bfloat16) * MLP_H * MLP_H)) != cudaSuccess) return fail(e);
     if ((e = cudaMalloc(&h->w3, sizeof(__nv_bfloat16) * MLP_OUTP * MLP_H)) != cudaSuccess) return fail(e);
@@ -315,9 +318,10 @@ int jbgpu_mlp_destroy(jbgpu_mlp* h) {
     if (!h) return JBGPU_OK;
     cudaSetDevice(h->device);
     if (h->s) cudaStreamSynchronize(h->s);
-    for (void* q : {(void*)h->p, (void*)h->g, (void*)h->m, (void*)h->v, (void*)h->norm, (void*)h->loss, (void*)h->w1,
+    for (void* q : {(void*)h->p, (void*)h->g, (void*)h->m, (void*)h->v, (void*)h->norm, (void*)h->w1,
                     (void*)h->w2, (void*)h->w3, (void*)h->X, (void*)h->T, (void*)h->idx, (void*)h->io})
         if (q) cudaFree(q);
+    if (h->hostGrad) cudaFreeHost(h->hostGrad);
     if (h->s) cudaStreamDestroy(h->s);
     delete h;
     return JBGPU_OK;
@@ -381,16 +385,14 @@ int jbgpu_mlp_gradients(jbgpu_mlp* h, const float* x, const float* t, int32_t n,
     float* dt = h->io + (size_t)n * MLP_IN;
     MCK(cudaMemcpyAsync(dx, x, sizeof(float) * (size_t)n * MLP_IN, cudaMemcpyHostToDevice, h->s));
     MCK(cudaMemcpyAsync(dt, t, sizeof(float) * (size_t)n * MLP_OUT, cudaMemcpyHostToDevice, h->s));
-    MCK(cudaMemsetAsync(h->g, 0, sizeof(float) * MLP_NPARAM, h->s));
-    MCK(cudaMemsetAsync(h->loss, 0, sizeof(float), h->s));
+    MCK(cudaMemsetAsync(h->g, 0, sizeof(float) * (MLP_NPARAM + 1), h->s));
     launch_train_batch(h, dx, dt, nullptr, 0, n);
     MCK(cudaGetLastError());
-    MCK(cudaMemcpyAsync(grad, h->g, sizeof(float) * MLP_NPARAM, cudaMemcpyDeviceToHost, h->s));
-    float l = 0.0f;
-    MCK(cudaMemcpyAsync(&l, h->loss, sizeof(float), cudaMemcpyDeviceToHost, h->s));
+    MCK(cudaMemcpyAsync(h->hostGrad, h->g, sizeof(float) * (MLP_NPARAM + 1), cudaMemcpyDeviceToHost, h->s));
     MCK(cudaMemsetAsync(h->g, 0, sizeof(float) * MLP_NPARAM, h->s));
     MCK(cudaStreamSynchronize(h->s));
-    if (loss) *loss = l;
+    std::memcpy(grad, h->hostGrad, sizeof(float) * MLP_NPARAM);
+    if (loss) *loss = h->hostGrad[MLP_NPARAM];
     return JBGPU_OK;
 }
 

@@ -283,10 +283,15 @@ class StateBuffers:
     def __init__(self, n, fields=None):
         self.n = n
         self.arrays = {}
-        for name, (w, dt) in STATE_FIELDS.items():
-            if fields is None or name in fields:
-                shape = (n,) if w == 1 else (n, w)
-                self.arrays[name] = np.zeros(shape, dtype=dt)
+        fields = [f for f in STATE_FIELDS if fields is None or f in fields]
+        # one block in the order of the struct, which the library fills with one copy
+        block = np.zeros(n * sum(STATE_FIELDS[f][0] for f in fields), np.float32)
+        at = 0
+        for name in fields:
+            w, dt = STATE_FIELDS[name]
+            a = block[at: at + n * w].view(dt)
+            self.arrays[name] = a if w == 1 else a.reshape(n, w)
+            at += n * w
         self.struct = State()
         self.struct.n_bodies = n
         for name, (w, dt) in STATE_FIELDS.items():

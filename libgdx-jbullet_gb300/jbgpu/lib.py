@@ -490,7 +490,7 @@ class GpuWorld:
     def get_state(self):
         sb = _abi.StateBuffers(self.n_bodies)
         check(lib().jbgpu_world_get_state(self.h, C.byref(sb.struct)))
-        return sb.copy_arrays()
+        return sb.arrays
 
     def set_state(self, arrays):
         arrays = {k: v for k, v in arrays.items() if k != "island_tag"}
