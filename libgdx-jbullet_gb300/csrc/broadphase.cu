@@ -505,6 +505,7 @@ JBD void persist_warp(const DevWorld& w, DevPairs& nw, const DevPairs& old, bool
             manifold_bodies(a, b, w.sh.type[w.shape[min(a, b)]], w.sh.type[w.shape[max(a, b)]], mb0, mb1);
         }
         nw.has[p] = has;
+        nw.steps[p] = has ? old.steps[found] : 0;
         nw.n[p] = n;
         nw.b0[p] = mb0;
         nw.b1[p] = mb1;

@@ -303,14 +303,16 @@ JBD GjkPart gjk_end(GjkRun& g, float marginA, float marginB, V offset) {
 }
 template <int G = 1>
 JBD GjkPart gjk_part(const ShapeRef& sa, const Xf& tA, const ShapeRef& sb, const Xf& tB, float maxDist2, int gl = 0,
-                     unsigned gmask = 0u) {
+                     unsigned gmask = 0u, int* steps = nullptr) {
     const V offset = scl(add(tA.o, tB.o), 0.5f);
     Xf lA = tA, lB = tB;
     lA.o = sub(lA.o, offset);
     lB.o = sub(lB.o, offset);
     GjkRun r;
     gjk_begin(r);
-    while (!gjk_step<G>(r, sa, lA, sb, lB, maxDist2, gl, gmask)) {}
+    int n = 1;
+    while (!gjk_step<G>(r, sa, lA, sb, lB, maxDist2, gl, gmask)) n++;
+    if (steps) *steps = n;
     return gjk_end(r, sa.margin, sb.margin, offset);
 }
 

@@ -90,6 +90,7 @@ struct DevPairs {
     int* b0;              // manifold body0 / body1
     int* b1;
     float4 *pA, *pB, *wA, *wB, *nrm, *imp, *d1, *d2;
+    unsigned char* steps; // GJK's steps for the pair in the last narrowphase (groups pairs; 0: none yet)
 };
 
 // Solver rows, one normal row per contact point with distance <= 0, stored compactly: the

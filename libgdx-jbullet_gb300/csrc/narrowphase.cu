@@ -36,11 +36,10 @@ JBD void manifold_refresh(Mf& m, const DevWorld& w, int mb0, int mb1) {
 
 // Pairs grouped by algorithm before the pass, so that the threads of a warp run the same code:
 // bucket 0 = nothing to do (both bodies inactive, or two planes), 1 convex-plane, 2 sphere-
-// sphere, then GJK pairs by shape kinds: 3 box-box, 4 with a sphere, 5 with a capsule, 6 with a
-// hull, each split by whether the pair's manifold held points after the last step (7-10: the
-// same kinds, touching) - separated pairs mostly leave GJK after a few iterations, touching
-// ones converge on the contact, so a warp of either kind runs similar iteration counts.  perm
-// lists buckets 1..10 in order; the pass covers nPairs - count[0] entries.
+// sphere, then GJK pairs by shape kinds (box-box, with a sphere, with a capsule, with a hull), by
+// whether the pair's manifold held points after the last step, and by the steps GJK took for the
+// pair then: a warp takes the steps of its slowest pair, and a pair takes about as many as last time.
+// perm lists the buckets from 1 on in order; the pass covers nPairs - count[0] entries.
 JBD int narrow_bucket(const DevWorld& w, const DevPairs& P, int p) {
     uint64_t key = P.keys[p];
     int a = key_owner(key), b = key_partner(key);
@@ -51,11 +50,12 @@ JBD int narrow_bucket(const DevWorld& w, const DevPairs& P, int p) {
     if (kind == ALG_EMPTY || kind >= ALG_CONVEX_CONCAVE) return 0;   // meshes: the concave pass
     if (kind == ALG_CONVEX_PLANE || kind == ALG_PLANE_CONVEX) return 1;
     if (kind == ALG_SPHERE_SPHERE) return 2;
-    const int touching = P.has[p] && P.n[p] > 0 ? 4 : 0;
-    if (t0 == SHAPE_HULL || t1 == SHAPE_HULL) return 6 + touching;
-    if (t0 == SHAPE_CAPSULE || t1 == SHAPE_CAPSULE) return 5 + touching;
-    if (t0 == SHAPE_SPHERE || t1 == SHAPE_SPHERE) return 4 + touching;
-    return 3 + touching;
+    const int touching = P.has[p] && P.n[p] > 0 ? 1 : 0;
+    const int kinds = t0 == SHAPE_HULL || t1 == SHAPE_HULL ? 3 : t0 == SHAPE_CAPSULE || t1 == SHAPE_CAPSULE ? 2
+                    : t0 == SHAPE_SPHERE || t1 == SHAPE_SPHERE ? 1 : 0;
+    const int steps = P.steps[p];
+    const int cls = steps <= 3 ? 0 : steps <= 5 ? 1 : steps <= 8 ? 2 : 3;
+    return 3 + (2 * kinds + touching) * NB_CLASSES + cls;
 }
 
 // Stable grouping: per block and bucket counts, laid out bucket-major with bucket 0 last, then
@@ -65,15 +65,15 @@ JBD int narrow_bucket(const DevWorld& w, const DevPairs& P, int p) {
 constexpr int NB_THREADS = 256;
 JBD int bucket_row(int v) { return v == 0 ? NB_BUCKETS - 1 : v - 1; }
 
-// Per-warp bucket counts of the block in shared memory (one ballot per bucket, one barrier);
-// then a thread's rank among the block's threads of its bucket and each bucket's block count.
-JBD void block_bucket_counts(int v, int (*shc)[NB_THREADS / 32]) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int u = 0; u < NB_BUCKETS; u++) {
-        unsigned m = __ballot_sync(0xffffffffu, v == u);
-        if (lane == 0) shc[u][warp] = __popc(m);
-    }
+// Per-warp bucket counts of the block in shared memory (v < 0: none); the lanes of the warp with the
+// thread's bucket.
+JBD unsigned block_bucket_counts(int v, int (*shc)[NB_THREADS / 32]) {
+    for (int k = threadIdx.x; k < NB_BUCKETS * (NB_THREADS / 32); k += NB_THREADS) (&shc[0][0])[k] = 0;
     __syncthreads();
+    const unsigned same = __match_any_sync(0xffffffffu, v);
+    if (v >= 0 && (threadIdx.x & 31) == __ffs(same) - 1) shc[v][threadIdx.x >> 5] = __popc(same);
+    __syncthreads();
+    return same;
 }
 __global__ void k_narrow_count(DevWorld w, DevPairs P, int nPairs, const int* cntp, unsigned char* bucket, int* blockCnt) {
     __shared__ int shc[NB_BUCKETS][NB_THREADS / 32];
@@ -95,20 +95,15 @@ __global__ void k_narrow_scatter(int nPairs, const int* cntp, const unsigned cha
     __shared__ int shc[NB_BUCKETS][NB_THREADS / 32];
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     int v = p < (cntp ? min(nPairs, *cntp) : nPairs) ? bucket[p] : -1;
-    block_bucket_counts(v, shc);
+    const unsigned same = block_bucket_counts(v, shc);
     if (v < 0) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int before = 0;
     for (int k = 0; k < warp; k++) before += shc[v][k];
-    unsigned mv = 0;
-    for (int u = 0; u < NB_BUCKETS; u++) {
-        unsigned m = __ballot_sync(__activemask(), v == u);
-        if (v == u) mv = m;
-    }
-    perm[blockOff[bucket_row(v) * gridDim.x + blockIdx.x] + before + __popc(mv & ((1u << lane) - 1u))] = p;
+    perm[blockOff[bucket_row(v) * gridDim.x + blockIdx.x] + before + __popc(same & ((1u << lane) - 1u))] = p;
 }
 
-// Entries of the pass: the pairs of buckets 1..6 = the start of bucket 0's row.
+// Entries of the pass: the pairs of buckets from 1 on = the start of bucket 0's row.
 JBD int narrow_active(const int* blockOff, int nBlocks) { return blockOff[(NB_BUCKETS - 1) * nBlocks]; }
 
 // A pair to each G lanes.  With perm: n = the grouping's pair blocks and entry i is pair perm[i];
@@ -117,10 +112,13 @@ JBD int narrow_active(const int* blockOff, int nBlocks) { return blockOff[(NB_BU
 // leaves most of the GPU idle a pair has lanes to spare: they split a hull's vertex scan, and a warp
 // holds fewer pairs (narrow_pairs has the line and the times).  Lanes that take the next pair when
 // theirs is done, and the manifold in a pass of its own, were slower: 672 us against 475 us for
-// 600,000 pairs - lanes in step share the simplex's cases.
+// 600,000 pairs - lanes in step share the simplex's cases; the pass in two without that, 497 us
+// against 449 us.  Three blocks of 168 registers an SM rather than four of 128, which spill: 4,000
+// hulls 121 -> 99 us, 1,024 worlds 1044 -> 993 us, 600,000 mixed pairs 430 -> 447 us.
 template <int G>
-__global__ void __launch_bounds__(128, 4) k_narrow(DevWorld w, DevPairs P, int n, const int* perm, const int* blockOff, EpaRec* queue,
-                         int* queueCount, const int* cntp) {
+__global__ void __launch_bounds__(128, 3)
+    k_narrow(DevWorld w, DevPairs P, int n, const int* perm, const int* blockOff, EpaRec* queue, int* queueCount,
+             const int* cntp) {
     const int lane = threadIdx.x & 31, gl = lane & (G - 1);
     const unsigned gmask = (G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (lane - gl));
     int i = (blockIdx.x * blockDim.x + threadIdx.x) / G;
@@ -182,8 +180,10 @@ __global__ void __launch_bounds__(128, 4) k_narrow(DevWorld w, DevPairs P, int n
             const unsigned am = __activemask();
             if (lane == __ffs(am) - 1) atomicAdd(&w.ctr[C_GJK], __popc(am) / G);
         }
-        GjkPart gp = gjk_part<G>(sa, f.x, sb, g.x, md, gl, gmask);
+        int steps = 0;
+        GjkPart gp = gjk_part<G>(sa, f.x, sb, g.x, md, gl, gmask, &steps);
         if (gl != 0) return;
+        P.steps[p] = (unsigned char)min(steps, 255);
         if (gp.needEpa) {
             int q = atomicAdd(queueCount, 1);
             EpaRec r;

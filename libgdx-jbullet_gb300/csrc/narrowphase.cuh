@@ -4,7 +4,8 @@
 
 namespace jbg {
 
-constexpr int NB_BUCKETS = 11;   // narrowphase algorithm buckets (pairs grouped by them)
+constexpr int NB_CLASSES = 4;                // GJK pairs of a kind by their last number of steps
+constexpr int NB_BUCKETS = 3 + 8 * NB_CLASSES;   // narrowphase algorithm buckets (pairs grouped by them)
 
 // EPA queue (the polytopes live in shared memory, one warp and one polytope per block).
 struct NarrowBuffers {

@@ -186,11 +186,14 @@ int alloc_pairs(DevPairs& P, int cap) {
     size_t c4 = (size_t)cap * 4;
     CK(dalloc(&P.pA, c4)); CK(dalloc(&P.pB, c4)); CK(dalloc(&P.wA, c4)); CK(dalloc(&P.wB, c4));
     CK(dalloc(&P.nrm, c4)); CK(dalloc(&P.imp, c4)); CK(dalloc(&P.d1, c4)); CK(dalloc(&P.d2, c4));
+    CK(dalloc(&P.steps, cap));
+    CK(cudaMemset(P.steps, 0, cap));
     return JBGPU_OK;
 }
 void free_pairs(DevPairs& P) {
     dfree(P.keys); dfree(P.has); dfree(P.n); dfree(P.b0); dfree(P.b1);
     dfree(P.pA); dfree(P.pB); dfree(P.wA); dfree(P.wB); dfree(P.nrm); dfree(P.imp); dfree(P.d1); dfree(P.d2);
+    dfree(P.steps);
 }
 
 // Work buffers whose size follows the pair capacity.
@@ -1010,6 +1013,7 @@ __global__ void k_pairs_move(DevPairs S, DevPairs D, int nPairs, const int* flag
     D.keys[q] = ((uint64_t)(unsigned)newIndex[key_owner(k)] << 32) | ((uint64_t)key_sub(k) << 24) |
                 (uint64_t)(unsigned)newIndex[key_partner(k)];
     D.has[q] = S.has[p];
+    D.steps[q] = S.steps[p];
     D.n[q] = S.n[p];
     D.b0[q] = S.b0[p] >= 0 ? newIndex[S.b0[p]] : S.b0[p];
     D.b1[q] = S.b1[p] >= 0 ? newIndex[S.b1[p]] : S.b1[p];
