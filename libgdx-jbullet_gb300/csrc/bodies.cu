@@ -20,9 +20,7 @@ __global__ void k_apply_gravity(DevWorld w) {
 
 // predictUnconstraintMotion (DiscreteDynamicsWorld.java:741-767):
 // RigidBody.integrateVelocities + applyDamping (dynamics/RigidBody.java:246-299,323-342)
-__global__ void k_predict(DevWorld w, float dt) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= w.nBodies) return;
+JBD void predict_body(const DevWorld& w, int i, float dt) {
     if (is_static_or_kin(w.flags[i]) || !is_active_state(w.act[i])) return;
     const float MAX_ANGVEL = __fmul_rn(SIMD_2_PI, 0.25f);
     float im = w.iloc[i].w;
@@ -44,11 +42,14 @@ __global__ void k_predict(DevWorld w, float dt) {
     w.linvel[i] = f4(lv, 0.0f);
     w.angvel[i] = f4(av, 0.0f);
 }
-
-// CollisionWorld.updateSingleAabb (collision/dispatch/CollisionWorld.java:195-229)
-__global__ void k_aabb(DevWorld w) {
+__global__ void k_predict(DevWorld w, float dt) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= w.nBodies) return;
+    predict_body(w, i, dt);
+}
+
+// CollisionWorld.updateSingleAabb (collision/dispatch/CollisionWorld.java:195-229)
+JBD void update_aabb(const DevWorld& w, int i) {
     int act = w.act[i];
     if (!is_active_state(act)) return;
     Xf t = load_xf(w, i);
@@ -65,12 +66,15 @@ __global__ void k_aabb(DevWorld w) {
         w.act[i] = set_activation(act, DISABLE_SIMULATION);
     }
 }
+__global__ void k_aabb(DevWorld w) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= w.nBodies) return;
+    update_aabb(w, i);
+}
 
 // integrateTransforms (DiscreteDynamicsWorld.java:679-739), CCD off; then
 // RigidBody.setCenterOfMassTransform -> updateInertiaTensor (dynamics/RigidBody.java:344-354,449-459)
-__global__ void k_integrate(DevWorld w, float dt) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= w.nBodies) return;
+JBD void integrate_body(const DevWorld& w, int i, float dt) {
     w.hitf[i] = 1.0f;
     if (!is_active_state(w.act[i]) || is_static_or_kin(w.flags[i])) return;
     Xf t = load_xf(w, i);
@@ -83,12 +87,15 @@ __global__ void k_integrate(DevWorld w, float dt) {
     w.iw1[i] = f4(iw.r[1], 0.0f);
     w.iw2[i] = f4(iw.r[2], 0.0f);
 }
+__global__ void k_integrate(DevWorld w, float dt) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= w.nBodies) return;
+    integrate_body(w, i, dt);
+}
 
 // updateActivationState (DiscreteDynamicsWorld.java:475-512) with RigidBody.updateDeactivation /
 // wantsSleeping (dynamics/RigidBody.java:543-576)
-__global__ void k_activation(DevWorld w, float dt) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= w.nBodies) return;
+JBD void update_activation(const DevWorld& w, int i, float dt) {
     int act = w.act[i];
     float dtime = w.deact[i];
     V lv = mk4(w.linvel[i]), av = mk4(w.angvel[i]);
@@ -121,6 +128,11 @@ __global__ void k_activation(DevWorld w, float dt) {
     }
     w.act[i] = act;
     w.deact[i] = dtime;
+}
+__global__ void k_activation(DevWorld w, float dt) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= w.nBodies) return;
+    update_activation(w, i, dt);
 }
 
 __global__ void k_clear_forces(DevWorld w) {   // DiscreteDynamicsWorld.clearForces (java:226-236)
@@ -197,6 +209,25 @@ void launch_predict(const DevWorld& w, float dt, cudaStream_t s) {
 }
 void launch_aabb(const DevWorld& w, cudaStream_t s) {
     if (w.nBodies) { k_aabb<<<grid_for(w.nBodies, 256), 256, 0, s>>>(w); note_launch(); }
+}
+// Phases that follow one another body by body, in one launch.
+__global__ void k_predict_aabb(DevWorld w, float dt) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= w.nBodies) return;
+    predict_body(w, i, dt);
+    update_aabb(w, i);
+}
+__global__ void k_integrate_activation(DevWorld w, float dt) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= w.nBodies) return;
+    integrate_body(w, i, dt);
+    update_activation(w, i, dt);
+}
+void launch_predict_aabb(const DevWorld& w, float dt, cudaStream_t s) {
+    if (w.nBodies) { k_predict_aabb<<<grid_for(w.nBodies, 256), 256, 0, s>>>(w, dt); note_launch(); }
+}
+void launch_integrate_activation(const DevWorld& w, float dt, cudaStream_t s) {
+    if (w.nBodies) { k_integrate_activation<<<grid_for(w.nBodies, 256), 256, 0, s>>>(w, dt); note_launch(); }
 }
 void launch_integrate(const DevWorld& w, float dt, cudaStream_t s) {
     if (w.nBodies) { k_integrate<<<grid_for(w.nBodies, 256), 256, 0, s>>>(w, dt); note_launch(); }

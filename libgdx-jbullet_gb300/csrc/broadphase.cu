@@ -779,7 +779,7 @@ void broadphase_run_count(const DevWorld& w, BroadphaseBuffers& bb, cudaStream_t
     } else {
         bb.sinceBuild++;
     }
-    cudaMemsetAsync(bb.candBound, 0, sizeof(int), s);
+    if (bb.meshes) cudaMemsetAsync(bb.candBound, 0, sizeof(int), s);   // else it stays 0
     if (bb.direct) {
         k_direct_count<<<gridn(n + 1, DIRECT_THREADS / 32), DIRECT_THREADS, 0, s>>>(w, bb.list, bb.planeList, bb.planeStart,
                                                                                     bb.cnt, bb.tcount, bb.kept);

@@ -59,7 +59,7 @@ struct BroadphaseBuffers {
     int* offPrev = nullptr;              // last step's off: the old pairs of owner o are [offPrev[o], offPrev[o + 1])
     bool offPrevValid = false;           // offPrev matches the previous pair array
     int* cursor = nullptr;               // fill cursors (n + 1)
-    int* total = nullptr;                // device total pair count
+    int* total = nullptr;                // device total pair count, and behind it candBound
     int* segLong = nullptr;              // device: owners whose partner segments the warp pass sorts
     int* candBound = nullptr;            // device: the concave pass's candidates, bounded by the count pass
     int* partners = nullptr;             // CSR partner lists (pair capacity)

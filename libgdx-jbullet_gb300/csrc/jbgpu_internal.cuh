@@ -20,13 +20,19 @@ enum { ST_CAPACITY = 1, ST_EPA_POOL = 2, ST_TIMEOUT = 4, ST_NONFINITE = 8, ST_BA
 
 // Counters kept on the device (indices into DevWorld::ctr).
 enum {
-    C_PAIRS = 0, C_FILL_OVERFLOW, C_EPA_QUEUE, C_GJK, C_EPA, C_SOLVE_N, C_COLOURS, C_ISLANDS,
+    C_PAIRS = 0, C_FILL_OVERFLOW,
+    // cleared together before a narrowphase (C_NARROW_FIRST, C_NARROW_COUNT of them)
+    C_EPA_QUEUE, C_EPA_OVF0, C_EPA_OVF1, C_GJK, C_EPA,
+    C_SOLVE_N, C_COLOURS,
+    // cleared together before the islands
+    C_ISLANDS,
     C_MANIFOLDS, C_CONTACTS, C_ROWS, C_STATUS, C_BAR_GEN, C_WIN0, C_WIN1, C_WIN2,
     C_CUT_COLOURS, C_CUT_MANIFOLDS, C_RES0, C_RES1, C_RES2,
     // cleared together at the start of a solve (C_SOLVE_FIRST .. C_SOLVE_LAST)
     C_BAR_COUNT, C_PGS_ITERS, C_ISL_N, C_ISL_CONV, C_ISL_ITERS, C_PART_NEXT0, C_PART_NEXT1, C_COL_FAIL, C_CUT_DONE,
-    C_CCD_N, C_CCD_BEST, C_NCTR = 32
+    C_CCD_N, C_CCD_BEST, C_NCTR = 36
 };
+constexpr int C_NARROW_FIRST = C_EPA_QUEUE, C_NARROW_COUNT = C_EPA - C_EPA_QUEUE + 1;
 constexpr int C_SOLVE_FIRST = C_BAR_COUNT, C_SOLVE_COUNT = C_CUT_DONE - C_BAR_COUNT + 1;
 
 struct DevShapes {
@@ -218,6 +224,8 @@ struct BroadphaseScratch;   // world.cu owns the buffers; broadphase.cu reads th
 void launch_apply_gravity(const DevWorld& w, cudaStream_t s);
 void launch_predict(const DevWorld& w, float dt, cudaStream_t s);
 void launch_aabb(const DevWorld& w, cudaStream_t s);
+void launch_predict_aabb(const DevWorld& w, float dt, cudaStream_t s);        // the two in one launch
+void launch_integrate_activation(const DevWorld& w, float dt, cudaStream_t s);
 void launch_integrate(const DevWorld& w, float dt, cudaStream_t s);
 void launch_activation(const DevWorld& w, float dt, cudaStream_t s);
 void launch_clear_forces(const DevWorld& w, cudaStream_t s);

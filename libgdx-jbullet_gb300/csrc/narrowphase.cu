@@ -366,15 +366,15 @@ __global__ void __launch_bounds__(32 * WARPS) k_narrow_epa_tier(DevWorld w, DevP
 
 
 // Full-capacity tier over the queries the 192-face tier could not finish.
-// c: the tier counters (c[0] counts list); block 0 also sets the tier mode of the next step.
+// c[0] counts list, c[1] the queries tier 1 left; block 0 also sets the tier mode of the next step.
 __global__ void __launch_bounds__(32) k_narrow_epa_smem(DevWorld w, DevPairs P, const EpaRec* queue, const int* list,
-                                                       int* c, const int* queueCount, int tier2Warps,
+                                                       const int* c, int* mode, const int* queueCount, int tier2Warps,
                                                        const int2* cand, float4* res) {
     extern __shared__ float4 epaSmem[];
     int n = c[0];
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        const int q = *queueCount, m = c[2];
-        c[2] = m > 0 ? m - 1 : ((q > tier2Warps && 3 * c[1] > q) ? EPA_T1_SKIP_STEPS : 0);
+        const int q = *queueCount, m = *mode;
+        *mode = m > 0 ? m - 1 : ((q > tier2Warps && 3 * c[1] > q) ? EPA_T1_SKIP_STEPS : 0);
     }
     EpaSlot sl;
     sl.fN = epaSmem;
@@ -409,21 +409,22 @@ static void narrow_pairs(const DevWorld& w, DevPairs& P, int nPairs, NarrowBuffe
     note_launch();
 }
 
-// The three EPA tiers over a queue (queueCount on the device); ovfCount: 3 ints (the two
-// overflow lists' counts and the tier mode the last tier sets for the next step).
+// The three EPA tiers over a queue (queueCount on the device, at most maxQueue); ovfCount: the two
+// overflow lists' counts, cleared by the caller; mode: the tier mode the last tier sets for the next step.
 static void epa_tiers(const DevWorld& w, DevPairs& P, void* queue, int* queueCount, int* ovfQueue, int* ovfQueue2,
-                      int* ovfCount, int slots, const int2* cand, float4* res, cudaStream_t s) {
-    cudaMemsetAsync(ovfCount, 0, sizeof(int) * 2, s);
-    EPA_T1_KERNEL<<<slots, 32 * EPA_T1_WARPS, EPA_T1_SMEM_BYTES, s>>>(
-        w, P, (const EpaRec*)queue, nullptr, queueCount, ovfQueue2, ovfCount + 1, ovfCount + 2, queueCount,
-        slots * EPA_T2_WARPS, cand, res);
+                      int* ovfCount, int* mode, int slots, int maxQueue, const int2* cand, float4* res, cudaStream_t s) {
+    const int tier2Warps = slots * EPA_T2_WARPS;
+    if (maxQueue > tier2Warps) {   // else tier 1 is skipped whatever the queue holds
+        EPA_T1_KERNEL<<<slots, 32 * EPA_T1_WARPS, EPA_T1_SMEM_BYTES, s>>>(w, P, (const EpaRec*)queue, nullptr, queueCount,
+                                                                          ovfQueue2, ovfCount + 1, mode, queueCount,
+                                                                          tier2Warps, cand, res);
+        note_launch();
+    }
+    EPA_T2_KERNEL<<<std::min(slots, (maxQueue + EPA_T2_WARPS - 1) / EPA_T2_WARPS), 32 * EPA_T2_WARPS, EPA_T2_SMEM_BYTES, s>>>(
+        w, P, (const EpaRec*)queue, ovfQueue2, ovfCount + 1, ovfQueue, ovfCount, mode, queueCount, tier2Warps, cand, res);
     note_launch();
-    EPA_T2_KERNEL<<<slots, 32 * EPA_T2_WARPS, EPA_T2_SMEM_BYTES, s>>>(
-        w, P, (const EpaRec*)queue, ovfQueue2, ovfCount + 1, ovfQueue, ovfCount, ovfCount + 2, queueCount,
-        slots * EPA_T2_WARPS, cand, res);
-    note_launch();
-    k_narrow_epa_smem<<<slots, 32, EPA_SMEM_BYTES, s>>>(w, P, (const EpaRec*)queue, ovfQueue, ovfCount, queueCount,
-                                                        slots * EPA_T2_WARPS, cand, res);
+    k_narrow_epa_smem<<<std::min(slots, maxQueue), 32, EPA_SMEM_BYTES, s>>>(w, P, (const EpaRec*)queue, ovfQueue, ovfCount,
+                                                                            mode, queueCount, tier2Warps, cand, res);
     note_launch();
 }
 
@@ -439,7 +440,7 @@ static void narrow_group(const DevWorld& w, DevPairs& P, int nPairs, NarrowBuffe
 void narrowphase_launch(const DevWorld& w, DevPairs& P, int nPairs, NarrowBuffers& nb, cudaStream_t s,
                         const Prof* prof, const int* cntp) {
     if (prof) prof->mark(PH_NARROW, 0, s);
-    cudaMemsetAsync(nb.queueCount, 0, sizeof(int), s);
+    cudaMemsetAsync(w.ctr + C_NARROW_FIRST, 0, sizeof(int) * C_NARROW_COUNT, s);
     if (nPairs > 0) {
         if (nb.group) {
             narrow_group(w, P, nPairs, nb, s, cntp);
@@ -449,7 +450,8 @@ void narrowphase_launch(const DevWorld& w, DevPairs& P, int nPairs, NarrowBuffer
         }
     }
     if (prof) { prof->mark(PH_NARROW, 1, s); prof->mark(PH_EPA, 0, s); }
-    if (nPairs > 0) epa_tiers(w, P, nb.queue, nb.queueCount, nb.ovfQueue, nb.ovfQueue2, nb.ovfCount, nb.slots, nullptr, nullptr, s);
+    if (nPairs > 0) epa_tiers(w, P, nb.queue, nb.queueCount, nb.ovfQueue, nb.ovfQueue2, nb.ovfCount, nb.tierMode, nb.slots, nPairs, nullptr,
+                              nullptr, s);
     if (prof) prof->mark(PH_EPA, 1, s);
 }
 
@@ -650,12 +652,12 @@ static void concave_passes(const DevWorld& w, DevPairs& P, int nPairs, const int
     exclusive_scan(nb.meshCnt, nb.meshOff, nb.meshTotal, nPairs, nb.meshScan, s);
     if (haveCandidates) {
         k_mesh_fill<<<blocks, 128, 0, s>>>(w, P, nb.meshList, nb.meshOff, nb.cand, nb.capCand); note_launch();
-        cudaMemsetAsync(nb.candCount, 0, sizeof(int), s);
+        cudaMemsetAsync(nb.candCount, 0, sizeof(int) * 3, s);
         k_mesh_gjk<<<(nb.capCand + 127) / 128, 128, 0, s>>>(w, P, nb.cand, nb.meshTotal, nb.capCand, nb.candRes,
                                                             (EpaRec*)nb.candQueue, nb.candCount);
         note_launch();
-        epa_tiers(w, P, nb.candQueue, nb.candCount, nb.candOvf, nb.candOvf2, nb.candCount + 1, nb.slots, nb.cand,
-                  nb.candRes, s);
+        epa_tiers(w, P, nb.candQueue, nb.candCount, nb.candOvf, nb.candOvf2, nb.candCount + 1, nb.candCount + 3, nb.slots,
+                  nb.capCand, nb.cand, nb.candRes, s);
     }
     k_mesh_merge<<<blocks, 128, 0, s>>>(w, P, nb.meshList, nb.meshCnt, nb.meshOff, nb.candRes); note_launch();
 }
@@ -746,7 +748,7 @@ int epa_static_scratch(int device, void** base) {
 
 void narrowphase_launch_static(const DevWorld& w, DevPairs& P, int nPairs, NarrowBuffers& nb, void* base, int slots,
                                cudaStream_t s) {
-    cudaMemsetAsync(nb.queueCount, 0, sizeof(int), s);
+    cudaMemsetAsync(w.ctr + C_NARROW_FIRST, 0, sizeof(int) * C_NARROW_COUNT, s);
     if (nPairs <= 0) return;
     narrow_group(w, P, nPairs, nb, s);
     narrow_pairs(w, P, nPairs, nb, nb.perm, nullptr, s);

@@ -10,11 +10,12 @@ constexpr int NB_BUCKETS = 3 + 8 * NB_CLASSES;   // narrowphase algorithm bucket
 // EPA queue (the polytopes live in shared memory, one warp and one polytope per block).
 struct NarrowBuffers {
     void* queue = nullptr;        // EpaRec per queued pair (pair capacity)
-    int* queueCount = nullptr;
+    int* queueCount = nullptr;    // (among the world's counters, as ovfCount)
     int sms = 1;
     int slots = 0;                // EPA blocks, striding over the queue
     int* ovfQueue = nullptr;      // queries the 192-face tier left to the full-capacity tier
-    int* ovfCount = nullptr;      // 3 ints: that list's count, ovfQueue2's count, the tier mode
+    int* ovfCount = nullptr;      // 2 ints: that list's count, ovfQueue2's count
+    int* tierMode = nullptr;
     int* ovfQueue2 = nullptr;     // queries the 96-face tier left to the 192-face tier
     unsigned char* pairBucket = nullptr;   // algorithm bucket per pair (pair capacity)
     int* perm = nullptr;          // pairs grouped by bucket (pair capacity)

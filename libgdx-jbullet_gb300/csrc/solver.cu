@@ -57,9 +57,10 @@ __device__ __forceinline__ void uf_unite(int* parent, int a, int b, int* ctr) {
     atomicOr(&ctr[C_STATUS], ST_TIMEOUT);
 }
 
-__global__ void k_uf_init(int n, int* parent) {
+__global__ void k_uf_init(DevWorld w, int* parent) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) parent[i] = i;
+    if (i < 4) w.ctr[C_ISLANDS + i] = 0;   // islands, manifolds, contacts, rows
+    if (i < w.nBodies) parent[i] = i;
 }
 
 // Unions in rounds over the pairs (sampling, as in the Afforest connected-components
@@ -99,6 +100,68 @@ __global__ void k_joint_union(DevWorld w, SolverBuffers sb) {
 __global__ void k_uf_compress(int n, int* parent) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) parent[i] = uf_find(parent, i);
+}
+
+// Islands of a small world, unions to awake flags, by one block with the parents in shared memory: the
+// general path is a chain of ten launches, 45 us for 60 bodies.
+constexpr int ISL_SMALL_BODIES = 8192, ISL_SMALL_PAIRS = 8192, ISL_SMALL_THREADS = 1024;
+__device__ __forceinline__ int uf_find_shared(volatile int* parent, int x) {
+    int p = parent[x];
+    while (p != x) {
+        const int gp = parent[p];
+        if (gp != p) atomicCAS((int*)&parent[x], p, gp);   // path halving
+        x = p;
+        p = parent[x];
+    }
+    return x;
+}
+__device__ __forceinline__ void uf_unite_shared(int* parent, int a, int b, int* ctr) {
+    for (int it = 0; it < 1 << 20; it++) {
+        a = uf_find_shared(parent, a);
+        b = uf_find_shared(parent, b);
+        if (a == b) return;
+        if (a > b) { const int t = a; a = b; b = t; }
+        if (atomicCAS(&parent[b], b, a) == b) return;
+    }
+    atomicOr(&ctr[C_STATUS], ST_TIMEOUT);
+}
+__global__ void __launch_bounds__(ISL_SMALL_THREADS) k_islands_small(DevWorld w, DevPairs P, int nPairs, const int* cntp,
+                                                                     SolverBuffers sb) {
+    __shared__ int parent[ISL_SMALL_BODIES];
+    __shared__ unsigned char keep[ISL_SMALL_BODIES];
+    __shared__ int islands;
+    const int n = w.nBodies, tid = threadIdx.x;
+    if (tid < 4) w.ctr[C_ISLANDS + tid] = 0;
+    if (tid == 0) islands = 0;
+    for (int i = tid; i < n; i += ISL_SMALL_THREADS) {
+        parent[i] = i;
+        keep[i] = 0;
+    }
+    if (cntp) nPairs = min(nPairs, *cntp);
+    __syncthreads();
+    for (int p = tid; p < nPairs; p += ISL_SMALL_THREADS) {
+        const uint64_t key = P.keys[p];
+        const int a = key_owner(key), b = key_partner(key);
+        if (merges_islands(w.flags[a]) && merges_islands(w.flags[b])) uf_unite_shared(parent, a, b, w.ctr);
+    }
+    for (int j = tid; j < sb.J.n; j += ISL_SMALL_THREADS) {   // as k_joint_union
+        const int a = sb.J.a[j], b = sb.J.b[j];
+        if (b < 0 || is_static_or_kin(w.flags[a]) || is_static_or_kin(w.flags[b])) continue;
+        if (is_active_state(w.act[a]) || is_active_state(w.act[b])) uf_unite_shared(parent, a, b, w.ctr);
+    }
+    __syncthreads();
+    for (int i = tid; i < n; i += ISL_SMALL_THREADS) {
+        const int isl = is_static_or_kin(w.flags[i]) ? -1 : uf_find_shared(parent, i);
+        w.island[i] = isl;
+        sb.inactive[i] = 0;
+        if (isl < 0) continue;
+        if (isl == i) atomicAdd(&islands, 1);
+        const int a = w.act[i];
+        if (a == ACTIVE_TAG || a == DISABLE_DEACTIVATION) keep[isl] = 1;
+    }
+    __syncthreads();
+    for (int i = tid; i < n; i += ISL_SMALL_THREADS) sb.keepAwake[i] = keep[i];
+    if (tid == 0) w.ctr[C_ISLANDS] = islands;
 }
 
 __global__ void k_islands(DevWorld w, int* parent, int* keepAwake, int* inactive) {
@@ -156,17 +219,14 @@ __global__ void k_select(DevWorld w, DevPairs P, int nPairs, const int* cntp, co
     flag[p] = f;
 }
 
-__global__ void k_compact(int nPairs, const int* flag, const int* idx, int* cand) {
+// Candidates in pair order; the manifold counts (has, points) of the counters.
+__global__ void k_compact(DevPairs P, int nPairs, const int* cntp, const int* flag, const int* idx, int* cand, int* ctr) {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p < nPairs && flag[p]) cand[idx[p]] = p;
-}
-
-// Manifold counts (has, points) for the counters.
-__global__ void k_count_manifolds(DevPairs P, int nPairs, const int* cntp, int* ctr) {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
     int m = 0, c = 0;
     if (p < (cntp ? min(nPairs, *cntp) : nPairs) && P.has[p]) { m = 1; c = P.n[p]; }
-    for (int o = 16; o > 0; o >>= 1) { m += __shfl_down_sync(0xffffffffu, m, o); c += __shfl_down_sync(0xffffffffu, c, o); }
+    m = __reduce_add_sync(0xffffffffu, m);
+    c = __reduce_add_sync(0xffffffffu, c);
     if ((threadIdx.x & 31) == 0 && (m || c)) { atomicAdd(&ctr[C_MANIFOLDS], m); atomicAdd(&ctr[C_CONTACTS], c); }
 }
 
@@ -177,7 +237,11 @@ __global__ void k_count_manifolds(DevPairs P, int nPairs, const int* cntp, int* 
 void islands_launch_unions(const DevWorld& w, const DevPairs& P, int nPairs, SolverBuffers& sb, cudaStream_t s,
                            const int* cntp) {
     int n = w.nBodies;
-    k_uf_init<<<gridn(n, 256), 256, 0, s>>>(n, sb.parent); note_launch();
+    if (n <= ISL_SMALL_BODIES && nPairs <= ISL_SMALL_PAIRS) {
+        k_islands_small<<<1, ISL_SMALL_THREADS, 0, s>>>(w, P, nPairs, cntp, sb); note_launch();
+        return;
+    }
+    k_uf_init<<<gridn(std::max(n, 4), 256), 256, 0, s>>>(w, sb.parent); note_launch();
     if (nPairs > 0) {
         for (int r = 0; r < UF_ROUNDS; r++) {
             if (r > 0) { k_uf_compress<<<gridn(n, 256), 256, 0, s>>>(n, sb.parent); note_launch(); }
@@ -198,8 +262,7 @@ void islands_launch_select(const DevWorld& w, const DevPairs& P, int nPairs, Sol
     if (nPairs > 0) {
         k_select<<<gridn(nPairs, 256), 256, 0, s>>>(w, P, nPairs, cntp, sb.inactive, sb.flag); note_launch();
         exclusive_scan(sb.flag, sb.candIdx, sb.nCand, nPairs, sb.scanScratch, s);
-        k_compact<<<gridn(nPairs, 256), 256, 0, s>>>(nPairs, sb.flag, sb.candIdx, sb.cand); note_launch();
-        k_count_manifolds<<<gridn(nPairs, 256), 256, 0, s>>>(P, nPairs, cntp, w.ctr); note_launch();
+        k_compact<<<gridn(nPairs, 256), 256, 0, s>>>(P, nPairs, cntp, sb.flag, sb.candIdx, sb.cand, w.ctr); note_launch();
     } else {
         cudaMemsetAsync(sb.nCand, 0, sizeof(int), s);
     }
@@ -234,9 +297,30 @@ __device__ __forceinline__ int flow_home(const DevWorld& w, const SolverBuffers&
     return v.x + (sb.posOf[b] - sb.partStart[q]) / v.y;
 }
 
-__global__ void k_posof(SolverBuffers sb) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < sb.nFinite) sb.posOf[sb.order[s]] = s;
+// Everything a solve starts from zero, and the bodies' places in the order (-1: listed bodies), in one
+// launch: a dozen memsets took about 1.5 us each.
+__global__ void k_solve_clear(DevWorld w, SolverBuffers sb, int buckets) {
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    for (int i = tid; i < w.nBodies; i += stride) {
+        sb.bodyDeg[i] = 0;
+        if (w.flags[i] & CF_LISTED) sb.posOf[i] = -1;
+        if (!sb.worldParts) {
+            sb.cutToken[i] = make_uint4(0, 0, 0, 0);
+            sb.cutHome[2 * i] = sb.cutHome[2 * i + 1] = 0;
+        }
+        if (sb.flowOn && sb.flowExch) sb.exch[2 * i] = sb.exch[2 * i + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    for (int s = tid; s < sb.nFinite; s += stride) sb.posOf[sb.order[s]] = s;
+    for (int b = tid; b < buckets; b += stride) sb.bucketCount[b] = sb.bucketFill[b] = 0;
+    if (!sb.flowOn) {
+        for (int c = tid; c < sb.nParts * (MAX_LOCAL + 1); c += stride) sb.lcFill[c] = sb.lcCount[c] = 0;
+        for (int c = tid; c <= MAX_COLOURS; c += stride) sb.colourFill[c] = sb.colourCount[c] = 0;
+    }
+    if (tid < C_SOLVE_COUNT) w.ctr[C_SOLVE_FIRST + tid] = 0;
+    if (tid == 0) {
+        w.ctr[C_ROWS] = w.ctr[C_COLOURS] = w.ctr[C_CUT_COLOURS] = 0;
+        if (sb.flowOn) sb.flowTop[0] = sb.flowTop[1] = 0;
+    }
 }
 
 // Bucket of candidate k: the part holding all its dynamic bodies, else nParts (cut).
@@ -2544,6 +2628,7 @@ void solve_launch(const DevWorld& w, DevPairs& P, int nPairs, DevRows& R, Solver
 void solve_launch_learn(const DevWorld& w, DevPairs& P, int nPairs, DevRows& R, SolverBuffers& sb, float dt,
                         cudaStream_t s, const Prof* prof, const SolverLearn& learn) {
     if (prof) prof->mark(PH_COLOUR, 0, s);
+    if (nPairs <= 0 || sb.nFinite <= 0 || sb.nParts <= 0) cudaMemsetAsync(w.ctr + C_ROWS, 0, sizeof(int), s);
     if (nPairs <= 0 || sb.nFinite <= 0 || sb.nParts <= 0) {
         cudaMemsetAsync(sb.nColours, 0, sizeof(int), s);
         cudaMemsetAsync(sb.nCand, 0, sizeof(int), s);
@@ -2569,25 +2654,9 @@ void solve_launch_learn(const DevWorld& w, DevPairs& P, int nPairs, DevRows& R, 
     // the flow solver takes every solve of a fixed number of iterations without joints or learning
     sb.flowOn = sb.flowOk && w.resTol <= 0.0f && w.numIter <= FLOW_MAX_ITERATIONS && sb.J.n == 0 && !learn.mlp &&
                 !learn.sampleX && !learn.sampleT;
-    cudaMemsetAsync(sb.bodyDeg, 0, sizeof(int) * w.nBodies, s);
-    if (!sb.worldParts) {   // tokens of cut candidates, and after them their home colours
-        sb.cutHome = (unsigned*)(sb.cutToken + w.nBodies);
-        cudaMemsetAsync(sb.cutToken, 0, (sizeof(uint4) + sizeof(uint2)) * (size_t)w.nBodies, s);
-    }
-    cudaMemsetAsync(sb.posOf, 0xff, sizeof(int) * w.nBodies, s);
+    if (!sb.worldParts) sb.cutHome = (unsigned*)(sb.cutToken + w.nBodies);   // behind the tokens of cut candidates
     const int buckets = parts + 2 + (sb.flowOn ? sb.nFlow + 1 : 0);   // the colouring's buckets, then the flow solver's
-    cudaMemsetAsync(sb.bucketCount, 0, sizeof(int) * buckets, s);
-    cudaMemsetAsync(sb.bucketFill, 0, sizeof(int) * buckets, s);
-    if (!sb.flowOn) {
-        cudaMemsetAsync(sb.lcFill, 0, sizeof(int) * parts * (MAX_LOCAL + 1), s);
-        cudaMemsetAsync(sb.lcCount, 0, sizeof(int) * parts * (MAX_LOCAL + 1), s);
-        cudaMemsetAsync(sb.colourFill, 0, sizeof(int) * (MAX_COLOURS + 1), s);
-        cudaMemsetAsync(sb.colourCount, 0, sizeof(int) * (MAX_COLOURS + 1), s);
-    }
-    cudaMemsetAsync(w.ctr + C_SOLVE_FIRST, 0, sizeof(int) * C_SOLVE_COUNT, s);
-    cudaMemsetAsync(w.ctr + C_COLOURS, 0, sizeof(int), s);
-    cudaMemsetAsync(w.ctr + C_CUT_COLOURS, 0, sizeof(int), s);
-    k_posof<<<gridn(sb.nFinite, 256), 256, 0, s>>>(sb); note_launch();
+    k_solve_clear<<<std::min(gridn(std::max(w.nBodies, buckets), 256), 2048), 256, 0, s>>>(w, sb, buckets); note_launch();
     k_classify<<<gridn(nPairs, 256), 256, 0, s>>>(w, P, sb); note_launch();
     exclusive_scan(sb.bucketCount, sb.bucketStart, nullptr, buckets, sb.flowScan, s);
     k_bucket_scatter<<<gridn(nPairs, 256), 256, 0, s>>>(sb); note_launch();

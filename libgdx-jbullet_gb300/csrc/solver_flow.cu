@@ -676,8 +676,6 @@ void flow_free(SolverBuffers& sb) {
 
 void flow_launch(const DevWorld& w, DevPairs& P, int nPairs, DevRows& R, SolverBuffers& sb, float dt, cudaStream_t s) {
     k_flow_gather<<<(nPairs + 255) / 256, 256, 0, s>>>(w, P, sb); note_launch();
-    cudaMemsetAsync(sb.flowTop, 0, sizeof(int) * 2, s);
-    if (sb.flowExch) cudaMemsetAsync(sb.exch, 0, sizeof(float4) * 2 * (size_t)w.nBodies, s);
     DevWorld wc = w;
     DevPairs pc = P;
     DevRows rc = R;

@@ -417,10 +417,12 @@ int sync_planes(jbgpu_world* w) {
     for (int k = 0; k < nw; k++) { start[k] = (int)list.size(); list.insert(list.end(), per[k].begin(), per[k].end()); }
     start[nw] = (int)list.size();
     dfree(B.planeList); dfree(B.planeStart); dfree(B.wstart); dfree(B.wend); dfree(B.wroot); dfree(B.bounds); dfree(B.total);
-    dfree(B.candBound); dfree(B.segLong); dfree(B.list.body); dfree(B.list.pos); dfree(B.list.end); dfree(B.kept);
+    dfree(B.segLong); dfree(B.list.body); dfree(B.list.pos); dfree(B.list.end); dfree(B.kept);
     CK(dalloc(&B.planeList, std::max<size_t>(1, list.size()))); CK(dalloc(&B.planeStart, nw + 1));
-    CK(dalloc(&B.wstart, nw)); CK(dalloc(&B.wend, nw)); CK(dalloc(&B.wroot, nw)); CK(dalloc(&B.bounds, 6)); CK(dalloc(&B.total, 1));
-    CK(dalloc(&B.candBound, 1)); CK(dalloc(&B.segLong, 1));
+    CK(dalloc(&B.wstart, nw)); CK(dalloc(&B.wend, nw)); CK(dalloc(&B.wroot, nw)); CK(dalloc(&B.bounds, 6)); CK(dalloc(&B.total, 2));
+    B.candBound = B.total + 1;
+    CK(cudaMemset(B.total, 0, sizeof(int) * 2));
+    CK(dalloc(&B.segLong, 1));
     if (!list.empty()) CK(cudaMemcpy(B.planeList, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(B.planeStart, start.data(), sizeof(int) * (nw + 1), cudaMemcpyHostToDevice));
     B.nFinite = nf;
@@ -482,11 +484,10 @@ int stage_pairs(jbgpu_world* w) {
     broadphase_run_count(d, w->bb, s);
     w->orderValid = true;
     w->prof.mark(PH_PAIR_COUNT, 1, s);
-    CK(cudaMemcpyAsync(w->hostPinned, w->bb.total, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(w->hostPinned + 2, w->bb.candBound, sizeof(int), cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(w->hostPinned + 1, w->bb.total, sizeof(int) * 2, cudaMemcpyDeviceToHost, s));   // and candBound
     CK(cudaStreamSynchronize(s));
     w->candBound = w->hostPinned[2];
-    return stage_pairs_fill(w, *w->hostPinned);
+    return stage_pairs_fill(w, w->hostPinned[1]);
 }
 
 // The pair stage after the count: buffers for `total` pairs, fill, persistence.
@@ -545,7 +546,6 @@ int run_stage(jbgpu_world* w, int stage, float dt) {
     case JBGPU_STAGE_AABB: P.mark(PH_AABB, 0, s); launch_aabb(d, s); P.mark(PH_AABB, 1, s); break;
     case JBGPU_STAGE_PAIRS: { int rc = stage_pairs(w); if (rc) return rc; break; }
     case JBGPU_STAGE_NARROWPHASE:
-        CK(cudaMemsetAsync(w->dw.ctr + C_GJK, 0, sizeof(int) * 2, s));
         narrowphase_launch(d, w->pairs[w->cur], w->nPairs, w->nb, s, &P);
         if (w->hasMesh) {
             P.mark(PH_CONCAVE, 0, s);
@@ -556,14 +556,12 @@ int run_stage(jbgpu_world* w, int stage, float dt) {
         break;
     case JBGPU_STAGE_ISLANDS:
         P.mark(PH_ISLANDS, 0, s);
-        CK(cudaMemsetAsync(w->dw.ctr + C_ISLANDS, 0, sizeof(int) * 4, s));
         islands_launch(d, w->pairs[w->cur], w->nPairs, w->sb, s);
         P.mark(PH_ISLANDS, 1, s);
         break;
     case JBGPU_STAGE_SOLVE: {
         int rc = prepare_solver(w);
         if (rc) return rc;
-        CK(cudaMemsetAsync(w->dw.ctr + C_ROWS, 0, sizeof(int), s));
         SolverLearn learn;
         MlpDev md;
         if (w->mlp) {
@@ -698,10 +696,8 @@ int narrow_and_islands(jbgpu_world* w, const int* cntp = nullptr) {
     DevWorld d = dev_view(w);
     CK(cudaEventRecord(w->evFork, s));
     CK(cudaStreamWaitEvent(a, w->evFork, 0));
-    CK(cudaMemsetAsync(w->dw.ctr + C_ISLANDS, 0, sizeof(int) * 4, a));
     islands_launch_unions(d, w->pairs[w->cur], w->nPairs, w->sb, a, cntp);
     CK(cudaEventRecord(w->evJoin, a));
-    CK(cudaMemsetAsync(w->dw.ctr + C_GJK, 0, sizeof(int) * 2, s));
     narrowphase_launch(d, w->pairs[w->cur], w->nPairs, w->nb, s, &w->prof, cntp);
     if (w->hasMesh) {   // buffers reserved for the count pass's bound (stage_pairs_fill, single_step_graph)
         w->prof.mark(PH_CONCAVE, 0, s);
@@ -785,11 +781,9 @@ int single_step_graph(jbgpu_world* w, float dt) {
     bool captured = false;
     int rc = capture_or_replay(w, ka, [&]() -> int {
         DevWorld d = dev_view(w);
-        launch_predict(d, dt, s);
-        launch_aabb(d, s);
+        launch_predict_aabb(d, dt, s);
         broadphase_run_count(d, B, s);
-        CK(cudaMemcpyAsync(w->hostPinned + 1, B.total, sizeof(int), cudaMemcpyDeviceToHost, s));
-        CK(cudaMemcpyAsync(w->hostPinned + 2, B.candBound, sizeof(int), cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(w->hostPinned + 1, B.total, sizeof(int) * 2, cudaMemcpyDeviceToHost, s));   // and candBound
         return JBGPU_OK;
     }, captured);
     if (rc == GRAPH_FALLBACK) {            // nothing ran: undo the capture's host side
@@ -838,10 +832,13 @@ int single_step_graph(jbgpu_world* w, float dt) {
         CK(cudaMemcpyAsync(cnt, B.total, sizeof(int), cudaMemcpyDeviceToDevice, s));
         int r = narrow_and_islands(w, cnt);   // ... and read the count from the device
         if (r) return r;
-        static const int rest[] = {JBGPU_STAGE_SOLVE, JBGPU_STAGE_INTEGRATE, JBGPU_STAGE_ACTIVATION};
-        for (int st : rest)
-            if ((r = run_stage(w, st, dt))) return r;
-        return JBGPU_OK;
+        if ((r = run_stage(w, JBGPU_STAGE_SOLVE, dt))) return r;
+        if (!w->ccdOn) {
+            launch_integrate_activation(dev_view(w), dt, s);
+            return JBGPU_OK;
+        }
+        if ((r = run_stage(w, JBGPU_STAGE_INTEGRATE, dt))) return r;
+        return run_stage(w, JBGPU_STAGE_ACTIVATION, dt);
     }, captured);
     if (rc == GRAPH_FALLBACK) {            // the count ran; the rest with launches
         B.off = offBefore;
@@ -1348,9 +1345,10 @@ int jbgpu_world_create(const jbgpu_config* cfg, jbgpu_world** out) {
              N.slots = w->sms * 2;
              N.sms = w->sms;
              if (narrowphase_configure()) return fail(JBGPU_ERR_CUDA, "EPA shared-memory size");
-             CK(dalloc(&N.queueCount, 1));
-             CK(dalloc(&N.ovfCount, 3));
-             CK(cudaMemset(N.ovfCount, 0, sizeof(int) * 3));
+             N.queueCount = d.ctr + C_EPA_QUEUE;
+             N.ovfCount = d.ctr + C_EPA_OVF0;
+             CK(dalloc(&N.tierMode, 1));
+             CK(cudaMemset(N.tierMode, 0, sizeof(int)));
 
              return grow_bodies(w, std::max(1, c.initial_body_capacity));
          }()) != JBGPU_OK) {
@@ -1394,10 +1392,10 @@ int jbgpu_world_destroy(jbgpu_world* w) {
     dfree(B.bvh.left); dfree(B.bvh.right); dfree(B.bvh.lo); dfree(B.bvh.hi); dfree(B.bvh.parent); dfree(B.bvh.leafParent);
     dfree(B.bvh.visit); dfree(B.bvh.node); dfree(B.tcount); dfree(B.tcache); dfree(B.wstart); dfree(B.wend); dfree(B.wroot);
     dfree(B.planeList); dfree(B.planeStart); dfree(B.cnt); dfree(B.off); dfree(B.offPrev); dfree(B.cursor); dfree(B.total); dfree(B.partners);
-    dfree(B.candBound); dfree(B.segLong); dfree(B.list.body); dfree(B.list.pos); dfree(B.list.end); dfree(B.kept);
+    dfree(B.segLong); dfree(B.list.body); dfree(B.list.pos); dfree(B.list.end); dfree(B.kept);
     NarrowBuffers& N = w->nb;
     if (N.queue) cudaFree(N.queue);
-    dfree(N.queueCount); dfree(N.ovfQueue); dfree(N.ovfQueue2); dfree(N.ovfCount); dfree(N.pairBucket); dfree(N.perm); dfree(N.blockOff);
+    dfree(N.tierMode); dfree(N.ovfQueue); dfree(N.ovfQueue2); dfree(N.pairBucket); dfree(N.perm); dfree(N.blockOff);
     if (N.scanScratch) cudaFree(N.scanScratch);
     SolverBuffers& V = w->sb;
     dfree(V.parent); dfree(V.keepAwake); dfree(V.inactive); dfree(V.flag); dfree(V.candIdx); dfree(V.cand); dfree(V.colourOf);
@@ -1824,7 +1822,6 @@ int jbgpu_world_narrowphase_static(jbgpu_world* w, int32_t epa_slots) {
     if (epa_static_scratch(w->device, &base)) return fail(JBGPU_ERR_CUDA, "cudaGetSymbolAddress of the static EPA scratch");
     cudaStream_t s = w->stream;
     CK(cudaMemsetAsync(w->dw.ctr + C_STATUS, 0, sizeof(int), s));
-    CK(cudaMemsetAsync(w->dw.ctr + C_GJK, 0, sizeof(int) * 2, s));
     narrowphase_launch_static(dev_view(w), w->pairs[w->cur], w->nPairs, w->nb, base, epa_slots, s);
     CK(cudaGetLastError());
     return check_status(w);
