@@ -869,7 +869,7 @@ JBD void colour_claims(const DevWorld& w, const DevPairs& P, const SolverBuffers
     }
 }
 
-__global__ void __launch_bounds__(SOLVER_THREADS) k_colour(DevWorld w, DevPairs P, SolverBuffers sb) {
+__global__ void __launch_bounds__(COLOUR_THREADS) k_colour(DevWorld w, DevPairs P, SolverBuffers sb) {
     extern __shared__ __align__(16) unsigned long long colSmem[];
     __shared__ int shPart, shFail;
     unsigned barK = 0;
@@ -2151,6 +2151,68 @@ JBD void island_residuals(const DevWorld& w, const SolverBuffers& sb, int flag, 
     }
 }
 
+// Every part through all phases on its own, with no grid barrier: fixed iterations, no cut manifold, no
+// joints.  pool(c): the point pool of step c, tops: its three counters.
+template <class Pool>
+JBD void pgs_parts_alone(const DevWorld& w, const DevPairs& P, const DevRows& R, const SolverBuffers& sb, int counter, int maxIt,
+                         float4* sl, float4* sa, int* tops, Pool pool) {
+    const bool smem = sb.partSmem != 0;
+    ResCtl rc;
+    int step = 0;
+    __shared__ int shPart;
+    int itMax = 0;
+    for (int part = next_part(w, sb, counter, &shPart); part >= 0; part = next_part(w, sb, counter, &shPart)) {
+        const PartView v = part_view(sb, part);
+        const bool psm = smem && v.np <= sb.smemCap;
+        if (psm) stage_in(w, sb, v, sl, sa);
+        __syncthreads();
+        // (small world parts: the next steps' slots are not staged, their pools are too small
+        // for a block's manifolds and staging measured slower there)
+        const int nl = v.nLoc;
+        Staged st;
+        auto run = [&](int kind, int c) {
+            if (threadIdx.x == 0) tops[(step + 2) % 3] = 0;
+            local_colour(w, R, sb, v.lcs[c], v.lcs[c + 1], kind, psm, sl, sa, rc, 0, 0, kind, pool(step),
+                         pool(step + 1), st);
+            __syncthreads();
+            ++step;
+        };
+        for (int c = 0; c < nl; c++) run(PH_WARM, c);
+        int it = 0;
+        for (; it < maxIt && nl > 0; it++) {
+            for (int c = 0; c < nl; c++) run(PH_NORMAL, c);
+            for (int c = 0; c < nl; c++) run(PH_FRICTION, c);
+        }
+        if (it > itMax) itMax = it;
+        if (psm) stage_out(w, sb, v, sl, sa);
+        for (int s = sb.bucketStart[part] + threadIdx.x; s < sb.bucketStart[part + 1]; s += blockDim.x)
+            writeback_slot(P, R, s);
+        __syncthreads();
+    }
+    if (threadIdx.x == 0 && itMax > 0) atomicMax(&w.ctr[C_PGS_ITERS], itMax);
+}
+
+// World parts with fixed iterations and no joints (k_pgs takes over when the colouring left manifolds
+// to cut colours).  What bounds it is the largest worlds' chain of colours: a colour of 2,048 bodies holds
+// some 320 manifolds, two rounds of 256 threads but one of 384, and this path alone fits in the 80
+// registers that two such blocks an SM leave.  1,024 worlds of up to 2,048 bodies: solver phase
+// 2120 -> 1572 us (3 blocks of 256 threads 2523, 2 of 512 2243; pools of 48 entries 1639, of 64 2071: the
+// rest of the SM is L1).
+__global__ void __launch_bounds__(WORLD_THREADS, 2) k_pgs_worlds(DevWorld w, DevPairs P, DevRows R, SolverBuffers sb) {
+    extern __shared__ float4 smv[];
+    __shared__ int tops[3];
+    if (*sb.nColours != 0) return;
+    if (threadIdx.x < 3) tops[threadIdx.x] = 0;
+    float4* poolBase = smv + (sb.partSmem ? 2 * sb.smemCap : 0);
+    pgs_parts_alone(w, P, R, sb, C_PART_NEXT1, w.numIter, smv, smv + sb.smemCap, tops, [&](int c) {
+        PointPool pp;
+        pp.cap = WORLD_POOL;
+        pp.e = poolBase + (size_t)(c % 3) * WORLD_POOL * POOL_F4;
+        pp.top = &tops[c % 3];
+        return pp;
+    });
+}
+
 // One colour of joints (those of processed islands): no two share a body.
 JBD void joint_colour(const DevWorld& w, const SolverBuffers& sb, int c, const JointVel& at, int first, int stride, float dt) {
     for (int q = sb.J.colStart[c] + first; q < sb.J.colStart[c + 1]; q += stride) {
@@ -2203,37 +2265,8 @@ __global__ void __launch_bounds__(SOLVER_THREADS, 2) k_pgs(DevWorld w, DevPairs 
     rc.on = byRes;
     int step = 0;           // colour steps this block has run (the pool alternates with it)
     if (nCut == 0 && !byRes && sb.J.n == 0) {
-        __shared__ int shPart;
-        int itMax = 0;
-        for (int part = next_part(w, sb, C_PART_NEXT1, &shPart); part >= 0; part = next_part(w, sb, C_PART_NEXT1, &shPart)) {
-            const PartView v = part_view(sb, part);
-            const bool psm = smem && v.np <= sb.smemCap;
-            if (psm) stage_in(w, sb, v, sl, sa);
-            __syncthreads();
-            // (small world parts: the next steps' slots are not staged, their pools are too small
-            // for a block's manifolds and staging measured slower there)
-            const int nl = v.nLoc;
-            Staged st;
-            auto run = [&](int kind, int c) {
-                if (threadIdx.x == 0) shPoolTop[(step + 2) % 3] = 0;
-                local_colour(w, R, sb, v.lcs[c], v.lcs[c + 1], kind, psm, sl, sa, rc, 0, 0, kind, pool(step),
-                             pool(step + 1), st);
-                __syncthreads();
-                ++step;
-            };
-            for (int c = 0; c < nl; c++) run(PH_WARM, c);
-            int it = 0;
-            for (; it < maxIt && nl > 0; it++) {
-                for (int c = 0; c < nl; c++) run(PH_NORMAL, c);
-                for (int c = 0; c < nl; c++) run(PH_FRICTION, c);
-            }
-            if (it > itMax) itMax = it;
-            if (psm) stage_out(w, sb, v, sl, sa);
-            for (int s = sb.bucketStart[part] + threadIdx.x; s < sb.bucketStart[part + 1]; s += blockDim.x)
-                writeback_slot(P, R, s);
-            __syncthreads();
-        }
-        if (threadIdx.x == 0 && itMax > 0) atomicMax(&w.ctr[C_PGS_ITERS], itMax);
+        if (sb.gridWorlds) return;   // k_pgs_worlds solved them
+        pgs_parts_alone(w, P, R, sb, C_PART_NEXT1, maxIt, sl, sa, shPoolTop, pool);
         return;
     }
     if (nSlots == 0 && sb.J.n == 0) return;
@@ -2523,8 +2556,8 @@ template <class T> static cudaError_t salloc(T** p, size_t n) {
 }
 template <class T> static void sfree(T*& p) { if (p) cudaFree((void*)p); p = nullptr; }
 
-static size_t pgs_smem(const SolverBuffers& sb) {
-    return (sb.partSmem ? (size_t)sb.smemCap * 32 : 0) + (size_t)3 * sb.poolPts * POOL_F4 * 16;
+static size_t pgs_smem(const SolverBuffers& sb, int poolPts) {
+    return (sb.partSmem ? (size_t)sb.smemCap * 32 : 0) + (size_t)3 * poolPts * POOL_F4 * 16;
 }
 static size_t colour_smem(const SolverBuffers& sb) { return (size_t)sb.partMax * (sizeof(uint4) + sizeof(uint2)); }
 
@@ -2580,28 +2613,37 @@ int solver_configure(SolverBuffers& sb, int nFinite, const std::vector<int>& wor
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&smemBlock, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
         cudaFuncSetAttribute(k_pgs, cudaFuncAttributeMaxDynamicSharedMemorySize, smemBlock - 1024) != cudaSuccess ||
+        cudaFuncSetAttribute(k_pgs_worlds, cudaFuncAttributeMaxDynamicSharedMemorySize, smemBlock - 1024) != cudaSuccess ||
         cudaFuncSetAttribute(k_colour, cudaFuncAttributeMaxDynamicSharedMemorySize, smemBlock - 1024) != cudaSuccess)
         return JBGPU_ERR_CUDA;
+    // more threads for world parts, unless the caller chose: see k_pgs_worlds; k_colour's too where a part
+    // has enough candidates for them (1,024 worlds of up to 2,048 bodies 284 -> 182 us, one world of 1,000
+    // boxes 85 -> 60 us; 256 worlds of up to 128 bodies 39 -> 44 us, the 304 parts of 100,000 bodies 128 -> 135)
+    const bool wider = sb.worldParts && threads == SOLVER_THREADS;
+    sb.worldThreads = wider ? WORLD_THREADS : threads;
+    sb.colourThreads = wider && partMax > 768 ? COLOUR_THREADS : threads;
     // point pools: half a block's threads in entries (a quarter with world parts, whose blocks
     // stage nothing ahead and keep more of the SM as L1), fewer or none if they would cost
-    // occupancy
-    int perPgs = 0, perColour = 0, perBare = 0;
+    // occupancy; WORLD_POOL in k_pgs_worlds
+    int perPgs = 0, perColour = 0, perBare = 0, perWorlds = 0;
     sb.poolPts = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perBare, k_pgs, threads, pgs_smem(sb)) != cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perBare, k_pgs, threads, pgs_smem(sb, 0)) != cudaSuccess)
         return JBGPU_ERR_CUDA;
     for (int pts = sb.worldParts ? threads / 4 : threads / 2; pts >= 16; pts /= 2) {
         sb.poolPts = pts;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perPgs, k_pgs, threads, pgs_smem(sb)) != cudaSuccess)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perPgs, k_pgs, threads, pgs_smem(sb, pts)) != cudaSuccess)
             return JBGPU_ERR_CUDA;
         if (perPgs >= perBare) break;
         sb.poolPts = 0;
     }
-    size_t smem = pgs_smem(sb);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perPgs, k_pgs, threads, smem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perColour, k_colour, threads, colour_smem(sb)) != cudaSuccess ||
-        perPgs < 1 || perColour < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perPgs, k_pgs, threads, pgs_smem(sb, sb.poolPts)) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perWorlds, k_pgs_worlds, sb.worldThreads, pgs_smem(sb, WORLD_POOL)) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perColour, k_colour, sb.colourThreads, colour_smem(sb)) != cudaSuccess ||
+        perPgs < 1 || perColour < 1 || perWorlds < 1)
         return JBGPU_ERR_CUDA;
     sb.gridPgs = std::min(parts, perPgs * sms);
+    sb.gridWorlds = sb.worldParts ? std::min(parts, perWorlds * sms) : 0;
     sb.gridColour = std::min(parts, perColour * sms);
     return flow_configure(sb, sms, smemBodies) ? JBGPU_ERR_CUDA : JBGPU_OK;
 }
@@ -2643,9 +2685,10 @@ void solve_launch_learn(const DevWorld& w, DevPairs& P, int nPairs, DevRows& R, 
             DevPairs pc = P;
             DevRows rc = R;
             SolverBuffers sc = sb;
+            sc.gridWorlds = 0;
             float dtc = dt;
             void* args[] = {&wc, &pc, &rc, &sc, &dtc};
-            cudaLaunchCooperativeKernel((void*)k_pgs, sb.gridPgs, sb.threads, args, pgs_smem(sb), s); note_launch();
+            cudaLaunchCooperativeKernel((void*)k_pgs, sb.gridPgs, sb.threads, args, pgs_smem(sb, sb.poolPts), s); note_launch();
         }
         if (prof) prof->mark(PH_PGS, 1, s);
         return;
@@ -2665,7 +2708,7 @@ void solve_launch_learn(const DevWorld& w, DevPairs& P, int nPairs, DevRows& R, 
         DevPairs pc = P;
         SolverBuffers sc = sb;
         void* args[] = {&wc, &pc, &sc};
-        cudaLaunchCooperativeKernel((void*)k_colour, sb.gridColour, sb.threads, args, colour_smem(sb), s); note_launch();
+        cudaLaunchCooperativeKernel((void*)k_colour, sb.gridColour, sb.colourThreads, args, colour_smem(sb), s); note_launch();
     }
     if (sb.flowOn) {
         if (prof) { prof->mark(PH_COLOUR, 1, s); prof->mark(PH_SETUP, 0, s); prof->mark(PH_SETUP, 1, s); prof->mark(PH_PGS, 0, s); }
@@ -2712,7 +2755,11 @@ void solve_launch_learn(const DevWorld& w, DevPairs& P, int nPairs, DevRows& R, 
         SolverBuffers sc = sb;
         float dtc = dt;
         void* args[] = {&wc, &pc, &rc, &sc, &dtc};
-        cudaLaunchCooperativeKernel((void*)k_pgs, sb.gridPgs, sb.threads, args, pgs_smem(sb), s); note_launch();
+        if (sb.J.n > 0 || w.resTol > 0.0f) sc.gridWorlds = 0;
+        if (sc.gridWorlds) {
+            k_pgs_worlds<<<sc.gridWorlds, sb.worldThreads, pgs_smem(sb, WORLD_POOL), s>>>(wc, pc, rc, sc); note_launch();
+        }
+        cudaLaunchCooperativeKernel((void*)k_pgs, sb.gridPgs, sb.threads, args, pgs_smem(sb, sb.poolPts), s); note_launch();
     }
     if (prof) prof->mark(PH_PGS, 1, s);
     if (learn.sampleT) {

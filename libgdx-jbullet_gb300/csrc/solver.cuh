@@ -12,6 +12,9 @@ constexpr int COL_LIST = 32;          // candidates a body's list holds
 constexpr unsigned COL_CUT = 1u << 31;   // a list entry of a cut candidate
 constexpr int COL_SWEEPS = 1 << 20;   // a thread's sweeps over its candidates before it gives up
 constexpr int SOLVER_THREADS = 256;
+constexpr int WORLD_THREADS = 384;    // k_pgs_worlds, and the entries of its point pools
+constexpr int WORLD_POOL = 16;
+constexpr int COLOUR_THREADS = 512;   // k_colour of world parts (the others: SOLVER_THREADS)
 constexpr int PART_MAX_BODIES = 2048; // bodies of one part (velocities staged in 64 KB of shared memory)
 
 // Solver parts.  Dynamic bodies are split into parts of consecutive positions in a body order
@@ -130,6 +133,8 @@ struct SolverBuffers {
     int gridColour = 0;           // co-resident blocks of the cooperative kernels
     int gridPgs = 0;
     int threads = SOLVER_THREADS;
+    int worldThreads = WORLD_THREADS, colourThreads = SOLVER_THREADS;
+    int gridWorlds = 0;           // blocks of k_pgs_worlds (0: not world parts)
     DevJoints J;                  // point-to-point joints
     // flow solver (solver_flow.cu)
     int* execOf = nullptr;        // per candidate: the flow block that solves it

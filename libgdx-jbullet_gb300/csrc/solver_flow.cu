@@ -657,9 +657,9 @@ int flow_configure(SolverBuffers& sb, int sms, int smemBodies) {
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_flow, flow_threads(sb), sb.flowSmem) != cudaSuccess) return 1;
     sb.gridFlow = std::min(sb.nFlow, blocks * sms);
     // Past about 512 bodies a resident block the blocks come in so many rounds, each as long as the
-    // longest chain of its manifolds, that the colour-by-colour solver's wider blocks win: 146k bodies
-    // in 1,000 worlds 630 us against its 900, 131k in 500 larger ones 835 against 821, 248k in 1,000
-    // 1330-1500 against 1243, 444k in 1,024 3094 against 2426.
+    // longest chain of its manifolds, that the colour-by-colour solver's wider blocks win.  Flow / by colour
+    // with its setup, us: 57k bodies in 1,024 worlds 345 / 685, 128k in 256 larger ones 1032 / 1240, 152k in
+    // 1,024 854 / 1013; 444k in 1,024 3094 / 1891.
     const bool wide = sb.worldParts && sb.nFinite > 512 * blocks * sms;
     sb.flowOk = !wide && most <= sb.gridFlow && !sb.movingStatic && (smemBodies <= 0 || sb.partMax <= smemBodies) &&
                 (size_t)sb.partMax * 32 + FLOW_HIST_BYTES <= (size_t)sb.flowSmem;
