@@ -115,10 +115,13 @@ JBD void mesh_quantize(V p, V bmin, V bmax, V q, int out[3]) {
 
 // ConvexTriangleCallback's query of a convex leaf c against the mesh leaf t: c's box in the mesh's
 // space widened by the mesh margin (setTimeStepAndCounters, ConvexTriangleCallback.java:82-104),
-// quantized, and the mesh's tree walked as OptimizedBvh.walkStacklessQuantizedTree does
-// (OptimizedBvh.java:940-997).  Returns the triangles found; the first `room` of them are written
-// as (p, triangle) in walk order to out when out is given.
-JBD int mesh_walk(const DevWorld& w, const Leaf& c, const Leaf& t, int p, int2* out, int room = 0) {
+// quantized.
+struct MeshQuery {
+    int lo[3], hi[3];
+    const int4* nodes;
+    int count;
+};
+JBD MeshQuery mesh_query(const DevWorld& w, const Leaf& c, const Leaf& t) {
     const DevShapes& sh = w.sh;
     const Xf convexInTri = xf_mul(xf_inverse(t.x), c.x);
     V mn, mx;
@@ -128,23 +131,64 @@ JBD int mesh_walk(const DevWorld& w, const Leaf& c, const Leaf& t, int p, int2* 
     mn = sub(mn, mk(mt, mt, mt));
     const float4* q = sh.mesh_q + 3 * t.shape;
     const V bmin = mk4(q[0]), bmax = mk4(q[1]), quant = mk4(q[2]);
-    int qa[3], qb[3];
-    mesh_quantize(mn, bmin, bmax, quant, qa);
-    mesh_quantize(mx, bmin, bmax, quant, qb);
-    const int4* nodes = sh.mesh_nodes + sh.mesh_node_off[t.shape];
-    const int nn = sh.mesh_node_cnt[t.shape];
+    MeshQuery r;
+    mesh_quantize(mn, bmin, bmax, quant, r.lo);
+    mesh_quantize(mx, bmin, bmax, quant, r.hi);
+    r.nodes = sh.mesh_nodes + sh.mesh_node_off[t.shape];
+    r.count = sh.mesh_node_cnt[t.shape];
+    return r;
+}
+JBD bool mesh_overlaps(const MeshQuery& q, int4 nd) {
+    const int n0 = nd.x & 0xFFFF, n1 = (nd.x >> 16) & 0xFFFF, n2 = nd.y & 0xFFFF;
+    const int m0 = (nd.y >> 16) & 0xFFFF, m1 = nd.z & 0xFFFF, m2 = (nd.z >> 16) & 0xFFFF;
+    return !(q.lo[0] > m0 || q.hi[0] < n0) && !(q.lo[2] > m2 || q.hi[2] < n2) && !(q.lo[1] > m1 || q.hi[1] < n1);
+}
+
+// The mesh's tree walked as OptimizedBvh.walkStacklessQuantizedTree does (OptimizedBvh.java:940-997).
+// Returns the triangles found.
+JBD int mesh_walk(const DevWorld& w, const Leaf& c, const Leaf& t) {
+    const MeshQuery q = mesh_query(w, c, t);
     int found = 0;
-    for (int cur = 0; cur < nn;) {
-        const int4 nd = nodes[cur];
-        const int n0 = nd.x & 0xFFFF, n1 = (nd.x >> 16) & 0xFFFF, n2 = nd.y & 0xFFFF;
-        const int m0 = (nd.y >> 16) & 0xFFFF, m1 = nd.z & 0xFFFF, m2 = (nd.z >> 16) & 0xFFFF;
-        const bool ov = !(qa[0] > m0 || qb[0] < n0) && !(qa[2] > m2 || qb[2] < n2) && !(qa[1] > m1 || qb[1] < n1);
-        const bool leaf = nd.w >= 0;
-        if (leaf && ov) {
-            if (out && found < room) out[found] = make_int2(p, nd.w & ((1 << 21) - 1));
-            ++found;
-        }
+    for (int cur = 0; cur < q.count;) {
+        const int4 nd = q.nodes[cur];
+        const bool ov = mesh_overlaps(q, nd), leaf = nd.w >= 0;
+        if (leaf && ov) ++found;
         cur += (ov || leaf) ? 1 : max(1, -nd.w);
+    }
+    return found;
+}
+
+// The same by a warp, 32 consecutive nodes at a time: a node is walked when no inner node before it
+// that fails the test skips past it (a skipped node's own skip ends within its ancestor's).  The first
+// `room` triangles are written as (p, triangle) in walk order to out when out is given.
+JBD int mesh_walk_warp(const DevWorld& w, const Leaf& c, const Leaf& t, int p, int2* out, int room = 0) {
+    const MeshQuery q = mesh_query(w, c, t);
+    const int lane = threadIdx.x & 31;
+    int found = 0;
+    for (int cur = 0; cur < q.count;) {
+        const int at = cur + lane;
+        int next = 0;   // where the walk goes on after this node
+        int4 nd = make_int4(0, 0, 0, 0);
+        bool hit = false;
+        if (at < q.count) {
+            nd = q.nodes[at];
+            const bool ov = mesh_overlaps(q, nd), leaf = nd.w >= 0;
+            hit = leaf && ov;
+            next = at + ((ov || leaf) ? 1 : max(1, -nd.w));
+        }
+        int reach = next;   // the furthest of this node and those before it
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, reach, o);
+            if (lane >= o) reach = max(reach, v);
+        }
+        const int before = __shfl_up_sync(0xffffffffu, reach, 1);
+        hit = hit && (lane == 0 || before <= at);
+        const unsigned hb = __ballot_sync(0xffffffffu, hit);
+        const int k = found + __popc(hb & ((1u << lane) - 1u));
+        if (hit && out && k < room) out[k] = make_int2(p, nd.w & ((1 << 21) - 1));
+        found += __popc(hb);
+        cur = __shfl_sync(0xffffffffu, reach, 31);
     }
     return found;
 }
@@ -152,7 +196,8 @@ JBD int mesh_walk(const DevWorld& w, const Leaf& c, const Leaf& t, int p, int2* 
 // The triangle candidates the concave pass will list for body i against the listed mesh body m
 // (every convex leaf of i: its compound children, or itself): the bound the pair count pass
 // sums so that the candidate buffer is sized before the narrowphase.
-JBD int mesh_candidates(const DevWorld& w, int i, int m) {
+template <class Walk>
+JBD int mesh_candidates(const DevWorld& w, int i, int m, Walk&& walk) {
     const int si = w.shape[i], sm = w.shape[m];
     if (w.sh.type[sm] != SHAPE_MESH) return 0;
     Leaf t;
@@ -163,7 +208,7 @@ JBD int mesh_candidates(const DevWorld& w, int i, int m) {
     const int ti = w.sh.type[si];
     if (ti == SHAPE_COMPOUND) {
         int n = 0;
-        for (int k = 0; k < w.sh.child_cnt[si]; k++) n += mesh_walk(w, compound_child(w.sh, si, k, xi, i), t, 0, nullptr);
+        for (int k = 0; k < w.sh.child_cnt[si]; k++) n += walk(compound_child(w.sh, si, k, xi, i), t);
         return n;
     }
     if (!shape_is_convex(ti)) return 0;
@@ -171,7 +216,7 @@ JBD int mesh_candidates(const DevWorld& w, int i, int m) {
     c.shape = si;
     c.x = xi;
     c.body = i;
-    return mesh_walk(w, c, t, 0, nullptr);
+    return walk(c, t);
 }
 
 }  // namespace jbg

@@ -489,10 +489,10 @@ JBD bool concave_pair(const DevWorld& w, const DevPairs& P, int p, int& col0, in
     return true;
 }
 
-// Per pair: the ConvexTriangleCallback's manifold on first contact, the candidate count, and the
-// pair appended to the list of mesh pairs (list[0] counts them; the fill and the merge run over
-// the list, a thread per mesh pair, in whatever order the appends landed - pairs are independent).
-__global__ void k_mesh_count(DevWorld w, DevPairs P, int nPairs, const int* cntp, int* cnt, int* list) {
+// Per pair: the ConvexTriangleCallback's manifold on first contact and the pair appended to the list of
+// mesh pairs (list[0] counts them; the walks run over the list, a warp per mesh pair, the merge a thread
+// each, in whatever order the appends landed - pairs are independent).
+__global__ void k_mesh_list(DevWorld w, DevPairs P, int nPairs, const int* cntp, int* cnt, int* list) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= nPairs) return;
     int col0, col1;
@@ -501,31 +501,44 @@ __global__ void k_mesh_count(DevWorld w, DevPairs P, int nPairs, const int* cntp
     const bool mine = p < (cntp ? min(nPairs, *cntp) : nPairs) && concave_pair(w, P, p, col0, col1, x0, x1, c, t);
     const unsigned act = __activemask();
     const unsigned m = __ballot_sync(act, mine);
-    if (!mine) {
-        cnt[p] = 0;
-        return;
-    }
+    cnt[p] = 0;   // k_mesh_count writes the mesh pairs' own
+    if (!mine) return;
     const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
     int base = 0;
     if (lane == leader) base = atomicAdd(list, __popc(m));
     base = __shfl_sync(m, base, leader);
     list[1 + base + __popc(m & ((1u << lane) - 1u))] = p;
     if (!P.has[p]) { P.has[p] = 1; P.n[p] = 0; }
-    cnt[p] = mesh_walk(w, c, t, p, nullptr);
+}
+
+__global__ void __launch_bounds__(128) k_mesh_count(DevWorld w, DevPairs P, const int* list, int* cnt) {
+    const int total = list[0];
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < total; i += (gridDim.x * blockDim.x) >> 5) {
+        const int p = list[1 + i];
+        int col0, col1;
+        Xf x0, x1;
+        Leaf c, t;
+        concave_pair(w, P, p, col0, col1, x0, x1, c, t);
+        const int n = mesh_walk_warp(w, c, t, p, nullptr);
+        if ((threadIdx.x & 31) == 0) cnt[p] = n;
+    }
 }
 
 // The pair's candidates in walk order at its offset; cap: the candidate buffer's capacity (sized
 // from the count pass's bound; a pair that would run past it flags ST_CAPACITY).
-__global__ void k_mesh_fill(DevWorld w, DevPairs P, const int* list, const int* off, int2* cand, int cap) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= list[0]) return;
-    const int p = list[1 + i];
-    int col0, col1;
-    Xf x0, x1;
-    Leaf c, t;
-    concave_pair(w, P, p, col0, col1, x0, x1, c, t);
-    const int room = cap - off[p];
-    if (mesh_walk(w, c, t, p, cand + off[p], room) > room) atomicOr(&w.ctr[C_STATUS], ST_CAPACITY);
+__global__ void __launch_bounds__(128) k_mesh_fill(DevWorld w, DevPairs P, const int* list, const int* off, int2* cand,
+                                                   int cap) {
+    const int total = list[0];
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < total; i += (gridDim.x * blockDim.x) >> 5) {
+        const int p = list[1 + i];
+        int col0, col1;
+        Xf x0, x1;
+        Leaf c, t;
+        concave_pair(w, P, p, col0, col1, x0, x1, c, t);
+        const int room = cap - off[p];
+        const int n = mesh_walk_warp(w, c, t, p, cand + off[p], room);
+        if ((threadIdx.x & 31) == 0 && n > room) atomicOr(&w.ctr[C_STATUS], ST_CAPACITY);
+    }
 }
 
 // Per candidate: GjkPairDetector between the convex object and the triangle (ConvexConvex
@@ -641,17 +654,23 @@ int concave_reserve(NarrowBuffers& nb, int pairCap, int candCap, cudaStream_t s)
     return moved;
 }
 
+// Lists the mesh pairs and counts their candidates.
+static void mesh_count(const DevWorld& w, DevPairs& P, int nPairs, const int* cntp, NarrowBuffers& nb, cudaStream_t s) {
+    cudaMemsetAsync(nb.meshList, 0, sizeof(int), s);
+    k_mesh_list<<<(nPairs + 127) / 128, 128, 0, s>>>(w, P, nPairs, cntp, nb.meshCnt, nb.meshList); note_launch();
+    k_mesh_count<<<std::min((nPairs + 3) / 4, 16 * nb.sms), 128, 0, s>>>(w, P, nb.meshList, nb.meshCnt); note_launch();
+}
+
 // The pass on reserved buffers with every count on the device: nPairs bounds the pair count (cntp:
 // the device count, or null for exactly nPairs) and the candidate buffer holds the count pass's
 // bound.  Grids are sized by the capacities; kernels read the counts.
 static void concave_passes(const DevWorld& w, DevPairs& P, int nPairs, const int* cntp, NarrowBuffers& nb, cudaStream_t s,
                            bool haveCandidates) {
     const int blocks = (nPairs + 127) / 128;
-    cudaMemsetAsync(nb.meshList, 0, sizeof(int), s);
-    k_mesh_count<<<blocks, 128, 0, s>>>(w, P, nPairs, cntp, nb.meshCnt, nb.meshList); note_launch();
+    mesh_count(w, P, nPairs, cntp, nb, s);
     exclusive_scan(nb.meshCnt, nb.meshOff, nb.meshTotal, nPairs, nb.meshScan, s);
     if (haveCandidates) {
-        k_mesh_fill<<<blocks, 128, 0, s>>>(w, P, nb.meshList, nb.meshOff, nb.cand, nb.capCand); note_launch();
+        k_mesh_fill<<<std::min((nPairs + 3) / 4, 16 * nb.sms), 128, 0, s>>>(w, P, nb.meshList, nb.meshOff, nb.cand, nb.capCand); note_launch();
         cudaMemsetAsync(nb.candCount, 0, sizeof(int) * 3, s);
         k_mesh_gjk<<<(nb.capCand + 127) / 128, 128, 0, s>>>(w, P, nb.cand, nb.meshTotal, nb.capCand, nb.candRes,
                                                             (EpaRec*)nb.candQueue, nb.candCount);
@@ -676,8 +695,7 @@ int concave_launch(const DevWorld& w, DevPairs& P, int nPairs, const int* cntp, 
     if (nPairs <= 0) return 0;
     if (concave_reserve(nb, nPairs, 0, s) < 0) return 1;
     // the exact candidate count first (the stage path: no bound from a count pass of this step)
-    cudaMemsetAsync(nb.meshList, 0, sizeof(int), s);
-    k_mesh_count<<<(nPairs + 127) / 128, 128, 0, s>>>(w, P, nPairs, cntp, nb.meshCnt, nb.meshList); note_launch();
+    mesh_count(w, P, nPairs, cntp, nb, s);
     exclusive_scan(nb.meshCnt, nb.meshOff, nb.meshTotal, nPairs, nb.meshScan, s);
     if (cudaMemcpyAsync(hostTotal, nb.meshTotal, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
