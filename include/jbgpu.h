@@ -609,8 +609,8 @@ int jbgpu_world_get_transforms(jbgpu_world* world, float* transforms);
  * reference's CProfileManager table, linearmath/CProfileManager.java:41-100).  Phases:
  * 0 predict, 1 aabb, 2 pair count (bounds, morton, sort, tree, count, scan), 3 pair fill
  * (fill, sort, persist), 4 narrowphase GJK pass, 5 EPA pass, 6 islands, 7 colouring,
- * 8 solver setup, 9 PGS, 10 integrate, 11 activation, 12 gravity + clear forces, 13 the
- * triangle-mesh pass of the narrowphase (worlds with meshes). */
+ * 8 solver setup (within 9 where the flow solver runs), 9 PGS, 10 integrate, 11 activation,
+ * 12 gravity + clear forces, 13 the triangle-mesh pass of the narrowphase (worlds with meshes). */
 #define JBGPU_NUM_PHASES 14
 int jbgpu_world_set_profiling(jbgpu_world* world, int32_t max_steps);   /* 0 turns it off */
 /* Sum of each phase's device milliseconds over the profiled steps so far (waits for them).

@@ -13,7 +13,8 @@
 //   manifold (the reference's algorithm lifetime, HashedOverlappingPairCache.java:222-228) is
 //   carried over.
 // Static planes (infinite aabb, StaticPlaneShape.java:124-128) stay out of the tree; each
-// finite body tests the planes of its world directly.
+// finite body tests the planes of its world directly.  Small worlds test all their bodies so
+// (direct pairs, below) and keep of these steps the order, 1 and 2, for the solver's parts.
 #include <utility>
 
 #include "broadphase.cuh"

@@ -1,7 +1,7 @@
 // Narrowphase: CollisionDispatcher.dispatchAllCollisionPairs for every overlapping pair
 // (collision/dispatch/CollisionDispatcher.java:252-257, DefaultNearCallback.java:39-66).
 //
-// Pass 1 (one thread per pair): needsCollision, algorithm creation (the pair's manifold),
+// Pass 1 (a lane per pair, more in small batches): needsCollision, algorithm creation (the pair's manifold),
 // then sphere-sphere (SphereSphereCollisionAlgorithm.java:73-134), convex-plane
 // (ConvexPlaneCollisionAlgorithm.java:75-136) or convex-convex GJK
 // (ConvexConvexAlgorithm.java:90-139), adding at most one point and refreshing the

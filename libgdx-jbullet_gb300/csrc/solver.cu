@@ -17,7 +17,9 @@
 // share a dynamic body.  Every phase (warm start, then numIterations x normal rows, friction
 // rows) runs the parts' local colours with their velocities in shared memory, then the cut
 // colours: the reference solver run on the manifolds sorted by (part, colour) with cut
-// manifolds last, the order hook of SequentialImpulseConstraintSolver.java:769-779.
+// manifolds last, the order hook of SequentialImpulseConstraintSolver.java:769-779.  Most solves keep
+// that order without its phases, manifold by manifold as their bodies' velocities arrive
+// (solver_flow.cu).
 #include <algorithm>
 #include <cstdlib>
 #include "../../include/jbgpu.h"
