@@ -3,7 +3,9 @@
 // Radix pass = three kernels: per-tile digit histograms (shared-memory atomics), one
 // single-block exclusive scan over the digit-major histogram table, and a scatter that
 // ranks keys stably inside each tile with warp match masks and writes them to their
-// global digit offsets.  Tiles are 4096 keys (256 threads x 16 rounds).
+// global digit offsets.  Tiles are 256 threads x 4 rounds, or 16 rounds for many keys.
+#include <algorithm>
+
 #include <cuda_runtime.h>
 #include "prims.cuh"
 
@@ -17,8 +19,10 @@ constexpr int SCAN_TILE = SCAN_BLOCK * SCAN_ITEMS;
 // than a scan of the tile sums apart, about 3 us in every scan of a step.
 constexpr int SCAN_CARRY_TILES = 2048;
 constexpr int RS_THREADS = 256;
-constexpr int RS_ROUNDS = 16;
-constexpr int RS_TILE = RS_THREADS * RS_ROUNDS;
+// A round is a chain of four block barriers, so a tile's length is the pass's time while the tiles leave SMs
+// idle: 15,000 keys 26 us a scatter in tiles of 16 rounds, 9 us in tiles of 4.  Past RS_MANY keys the
+// longer tiles keep the histogram table, and with it the scan, a quarter as long.
+constexpr int RS_FEW_ROUNDS = 4, RS_MANY_ROUNDS = 16, RS_MANY = 1 << 19;
 constexpr int RS_BINS = 256;
 constexpr int RS_WARPS = RS_THREADS / 32;
 }
@@ -125,11 +129,12 @@ void exclusive_scan(const int* in, int* out, int* total, int n, void* scratch, c
 }
 
 // ---- radix sort ---------------------------------------------------------------------------
+template <int RS_ROUNDS>
 __global__ void k_rs_hist(const uint64_t* keys, int n, int shift, int* hist, int tiles) {
     __shared__ int bins[RS_BINS];
     bins[threadIdx.x] = 0;
     __syncthreads();
-    int base = blockIdx.x * RS_TILE;
+    int base = blockIdx.x * RS_THREADS * RS_ROUNDS;
     for (int r = 0; r < RS_ROUNDS; r++) {
         int i = base + r * RS_THREADS + threadIdx.x;
         if (i < n) atomicAdd(&bins[(int)((keys[i] >> shift) & 0xff)], 1);
@@ -138,6 +143,7 @@ __global__ void k_rs_hist(const uint64_t* keys, int n, int shift, int* hist, int
     hist[threadIdx.x * tiles + blockIdx.x] = bins[threadIdx.x];   // digit-major
 }
 
+template <int RS_ROUNDS>
 __global__ void k_rs_scatter(const uint64_t* keys, const int* vals, uint64_t* okeys, int* ovals, int n, int shift,
                              const int* hist, int tiles) {
     __shared__ int warpCnt[RS_WARPS][RS_BINS];
@@ -145,7 +151,7 @@ __global__ void k_rs_scatter(const uint64_t* keys, const int* vals, uint64_t* ok
     int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     digitBase[threadIdx.x] = hist[threadIdx.x * tiles + blockIdx.x];
     const unsigned lt = (1u << lane) - 1u;
-    int base = blockIdx.x * RS_TILE;
+    int base = blockIdx.x * RS_THREADS * RS_ROUNDS;
     for (int r = 0; r < RS_ROUNDS; r++) {
         for (int k = threadIdx.x; k < RS_WARPS * RS_BINS; k += RS_THREADS) (&warpCnt[0][0])[k] = 0;
         __syncthreads();
@@ -173,15 +179,22 @@ __global__ void k_rs_scatter(const uint64_t* keys, const int* vals, uint64_t* ok
     }
 }
 
+static int rs_tiles(int n) {
+    const int tile = RS_THREADS * (n > RS_MANY ? RS_MANY_ROUNDS : RS_FEW_ROUNDS);
+    return (n + tile - 1) / tile;
+}
+
+// (for any count up to n: the tiles of RS_MANY keys are more than those of somewhat more keys)
 size_t sort_scratch_bytes(int n) {
-    int tiles = (n + RS_TILE - 1) / RS_TILE;
+    const int tiles = n > RS_MANY ? std::max(rs_tiles(n), rs_tiles(RS_MANY)) : rs_tiles(n);
     return sizeof(int) * ((size_t)tiles * RS_BINS + 16) + scan_scratch_bytes(tiles * RS_BINS);
 }
 
 void radix_sort_pairs(uint64_t* keys, int* vals, uint64_t* keys_alt, int* vals_alt, int n, int bits, void* scratch,
                       cudaStream_t s) {
     if (n <= 1) return;
-    int tiles = (n + RS_TILE - 1) / RS_TILE;
+    const int tiles = rs_tiles(n);
+    const bool many = n > RS_MANY;
     int* hist = (int*)scratch;
     void* scanScratch = (void*)(hist + (size_t)tiles * RS_BINS + 16);
     int passes = (bits + 7) / 8;
@@ -189,9 +202,12 @@ void radix_sort_pairs(uint64_t* keys, int* vals, uint64_t* keys_alt, int* vals_a
     int *va = vals, *vb = vals_alt;
     for (int p = 0; p < passes; p++) {
         int shift = 8 * p;
-        k_rs_hist<<<tiles, RS_THREADS, 0, s>>>(ka, n, shift, hist, tiles); note_launch();
+        (many ? k_rs_hist<RS_MANY_ROUNDS> : k_rs_hist<RS_FEW_ROUNDS>)<<<tiles, RS_THREADS, 0, s>>>(ka, n, shift, hist, tiles);
+        note_launch();
         exclusive_scan(hist, hist, nullptr, tiles * RS_BINS, scanScratch, s);
-        k_rs_scatter<<<tiles, RS_THREADS, 0, s>>>(ka, va, kb, vb, n, shift, hist, tiles); note_launch();
+        (many ? k_rs_scatter<RS_MANY_ROUNDS> : k_rs_scatter<RS_FEW_ROUNDS>)<<<tiles, RS_THREADS, 0, s>>>(
+            ka, va, kb, vb, n, shift, hist, tiles);
+        note_launch();
         uint64_t* tk = ka; ka = kb; kb = tk;
         int* tv = va; va = vb; vb = tv;
     }
