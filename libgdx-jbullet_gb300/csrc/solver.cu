@@ -301,7 +301,7 @@ __device__ __forceinline__ int flow_home(const DevWorld& w, const SolverBuffers&
 
 // Everything a solve starts from zero, and the bodies' places in the order (-1: listed bodies), in one
 // launch: a dozen memsets took about 1.5 us each.
-__global__ void k_solve_clear(DevWorld w, SolverBuffers sb, int buckets) {
+__global__ void k_solve_clear(DevWorld w, SolverBuffers sb, int buckets, int* slotPt0, int nPairs) {
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     for (int i = tid; i < w.nBodies; i += stride) {
         sb.bodyDeg[i] = 0;
@@ -315,6 +315,7 @@ __global__ void k_solve_clear(DevWorld w, SolverBuffers sb, int buckets) {
     for (int s = tid; s < sb.nFinite; s += stride) sb.posOf[sb.order[s]] = s;
     for (int b = tid; b < buckets; b += stride) sb.bucketCount[b] = sb.bucketFill[b] = 0;
     if (!sb.flowOn) {
+        for (int p = tid; p < nPairs; p += stride) slotPt0[p] = 0;   // beyond the candidates it stays so
         for (int c = tid; c < sb.nParts * (MAX_LOCAL + 1); c += stride) sb.lcFill[c] = sb.lcCount[c] = 0;
         for (int c = tid; c <= MAX_COLOURS; c += stride) sb.colourFill[c] = sb.colourCount[c] = 0;
     }
@@ -935,35 +936,16 @@ __global__ void k_slots(DevWorld w, DevPairs P, SolverBuffers sb, DevRows R) {
         if (dyn(w, b0)) lb0 = sb.posOf[b0] - ps;
         if (dyn(w, b1)) lb1 = sb.posOf[b1] - ps;
     }
-    R.slot_desc[slot] = make_int4(b0, b1, 0, lb0 | (lb1 << 16));
+    int mask = 0;   // the points with distance <= 0; their count is scanned into the slot's first row
+    for (int j = 0, n = P.n[p]; j < n; j++)
+        if (P.pA[p * 4 + j].w <= 0.0f) mask |= 1 << j;
+    R.slot_pt0[slot] = __popc(mask);
+    R.slot_desc[slot] = make_int4(b0, b1, mask, lb0 | (lb1 << 16));
 }
 
 // ---- row setup (solveGroupCacheFriendlySetup, java:418-786; the arithmetic is in rows.cuh) -----
-// Points with rows (distance <= 0) of every slot: the mask into slot_desc.z and the count into
-// slot_pt0 (scanned afterwards into the slot's first point row); 0 beyond the candidates.
-__global__ void k_point_masks(DevPairs P, DevRows R, const int* nCandPtr, int nPairs) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nPairs) return;
-    int cnt = 0;
-    if (s < *nCandPtr) {
-        int p = R.slot_pair[s];
-        int n = P.n[p], mask = 0;
-        for (int j = 0; j < n; j++)
-            if (P.pA[p * 4 + j].w <= 0.0f) mask |= 1 << j;
-        R.slot_desc[s].z = mask;
-        cnt = __popc(mask);
-    }
-    R.slot_pt0[s] = cnt;
-}
-
-// slot_desc.z = first point row << 4 | point mask (after the scan of the counts).
-__global__ void k_point_rows(DevRows R, const int* nCandPtr) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= *nCandPtr) return;
-    int4 d = R.slot_desc[s];
-    d.z = (R.slot_pt0[s] << 4) | (d.z & 15);
-    R.slot_desc[s] = d;
-}
+// slot_desc.z holds the slot's point mask from k_slots; k_setup puts the first point row above it
+// (slot_pt0, scanned).
 
 // Where plane `plane` (rows.cuh) of row ni is kept.
 JBD float4* row_plane(const DevRows& R, int plane, int ni) {
@@ -992,6 +974,8 @@ __global__ void k_setup(DevWorld w, DevPairs P, DevRows R, const int* nCandPtr, 
     if (s >= nSlots) return;
     int p = R.slot_pair[s];
     int4 desc = R.slot_desc[s];
+    desc.z = (R.slot_pt0[s] << 4) | (desc.z & 15);
+    R.slot_desc[s].z = desc.z;
     BodyV A = load_body(w, desc.x), B = load_body(w, desc.y);
     const bool warm = (w.solverMode & 4) != 0;
     const int mask = desc.z & 15;
@@ -2701,7 +2685,9 @@ void solve_launch_learn(const DevWorld& w, DevPairs& P, int nPairs, DevRows& R, 
                 !learn.sampleX && !learn.sampleT;
     if (!sb.worldParts) sb.cutHome = (unsigned*)(sb.cutToken + w.nBodies);   // behind the tokens of cut candidates
     const int buckets = parts + 2 + (sb.flowOn ? sb.nFlow + 1 : 0);   // the colouring's buckets, then the flow solver's
-    k_solve_clear<<<std::min(gridn(std::max(w.nBodies, buckets), 256), 2048), 256, 0, s>>>(w, sb, buckets); note_launch();
+    k_solve_clear<<<std::min(gridn(std::max(w.nBodies, buckets), 256), 2048), 256, 0, s>>>(w, sb, buckets, R.slot_pt0,
+                                                                                                nPairs);
+    note_launch();
     k_classify<<<gridn(nPairs, 256), 256, 0, s>>>(w, P, sb); note_launch();
     exclusive_scan(sb.bucketCount, sb.bucketStart, nullptr, buckets, sb.flowScan, s);
     k_bucket_scatter<<<gridn(nPairs, 256), 256, 0, s>>>(sb); note_launch();
@@ -2734,9 +2720,7 @@ void solve_launch_learn(const DevWorld& w, DevPairs& P, int nPairs, DevRows& R, 
         k_isl_segments<<<gridn(n, 256), 256, 0, s>>>(sb, n); note_launch();
     }
     if (prof) { prof->mark(PH_COLOUR, 1, s); prof->mark(PH_SETUP, 0, s); }
-    k_point_masks<<<gridn(nPairs, 256), 256, 0, s>>>(P, R, sb.nCand, nPairs); note_launch();
     exclusive_scan(R.slot_pt0, R.slot_pt0, R.nPts, nPairs, sb.scanScratch, s);
-    k_point_rows<<<gridn(nPairs, 256), 256, 0, s>>>(R, sb.nCand); note_launch();
     k_setup<<<gridn(nPairs, 128), 128, 0, s>>>(w, P, R, sb.nCand, dt); note_launch();
     if (learn.sampleX) {
         k_contact_features<<<std::min(gridn(nPairs * 4, 256), 4096), 256, 0, s>>>(w, P, R, R.nPts, learn.sampleX);
