@@ -185,9 +185,7 @@ __global__ void k_island_awake(DevWorld w, int* keepAwake) {
     if (a == ACTIVE_TAG || a == DISABLE_DEACTIVATION) keepAwake[isl] = 1;
 }
 
-__global__ void k_island_sleep(DevWorld w, const int* keepAwake, int* inactive) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= w.nBodies) return;
+JBD void island_sleep(const DevWorld& w, const int* keepAwake, int* inactive, int i) {
     int isl = w.island[i];
     if (isl < 0) return;
     int a = w.act[i];
@@ -196,29 +194,67 @@ __global__ void k_island_sleep(DevWorld w, const int* keepAwake, int* inactive) 
     w.act[i] = a;
     if (!is_active_state(a)) inactive[isl] = 1;
 }
+__global__ void k_island_sleep(DevWorld w, const int* keepAwake, int* inactive) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < w.nBodies) island_sleep(w, keepAwake, inactive, i);
+}
 
 // Candidate manifolds: in islandmanifold, island processed, at least one point with distance <= 0.
+JBD bool selected(const DevWorld& w, const DevPairs& P, const int* inactive, int p) {
+    if (!P.has[p]) return false;
+    int b0 = P.b0[p], b1 = P.b1[p];
+    int a0 = w.act[b0], a1 = w.act[b1];
+    int f0 = w.flags[b0], f1 = w.flags[b1];
+    bool resp = !(f0 & CF_NO_CONTACT_RESPONSE) && !(f1 & CF_NO_CONTACT_RESPONSE) &&
+                (!is_static_or_kin(f0) || !is_static_or_kin(f1));
+    if ((a0 == ISLAND_SLEEPING && a1 == ISLAND_SLEEPING) || !resp) return false;
+    int isl = w.island[b0] >= 0 ? w.island[b0] : w.island[b1];
+    if (inactive[isl]) return false;
+    int n = P.n[p];
+    for (int j = 0; j < n; j++)
+        if (P.pA[p * 4 + j].w <= 0.0f) return true;
+    return false;
+}
 __global__ void k_select(DevWorld w, DevPairs P, int nPairs, const int* cntp, const int* inactive, int* flag) {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= nPairs) return;
     if (cntp && p >= *cntp) { flag[p] = 0; return; }   // past the device pair count: not a candidate
-    int f = 0;
-    if (P.has[p]) {
-        int b0 = P.b0[p], b1 = P.b1[p];
-        int a0 = w.act[b0], a1 = w.act[b1];
-        int f0 = w.flags[b0], f1 = w.flags[b1];
-        bool resp = !(f0 & CF_NO_CONTACT_RESPONSE) && !(f1 & CF_NO_CONTACT_RESPONSE) &&
-                    (!is_static_or_kin(f0) || !is_static_or_kin(f1));
-        if ((a0 != ISLAND_SLEEPING || a1 != ISLAND_SLEEPING) && resp) {
-            int isl = w.island[b0] >= 0 ? w.island[b0] : w.island[b1];
-            if (!inactive[isl]) {
-                int n = P.n[p];
-                for (int j = 0; j < n; j++)
-                    if (P.pA[p * 4 + j].w <= 0.0f) { f = 1; break; }
-            }
+    flag[p] = selected(w, P, inactive, p) ? 1 : 0;
+}
+
+// Sleep decisions, selection, candidates and counts of a small world by one block: four launches of some
+// 4 us each otherwise.
+constexpr int SMALL_BODIES = 4096, SMALL_PAIRS = 2048, SMALL_THREADS = 1024;
+__global__ void __launch_bounds__(SMALL_THREADS) k_select_small(DevWorld w, DevPairs P, int nPairs, const int* cntp,
+                                                                SolverBuffers sb) {
+    __shared__ int sCount[SMALL_THREADS / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int i = tid; i < w.nBodies; i += SMALL_THREADS) island_sleep(w, sb.keepAwake, sb.inactive, i);
+    if (cntp) nPairs = min(nPairs, *cntp);
+    __syncthreads();
+    int found = 0, manifolds = 0, points = 0;
+    for (int base = 0; base < nPairs; base += SMALL_THREADS) {
+        const int p = base + tid;
+        const bool on = p < nPairs && selected(w, P, sb.inactive, p);
+        if (p < nPairs && P.has[p]) { manifolds++; points += P.n[p]; }
+        const unsigned m = __ballot_sync(0xffffffffu, on);
+        if (lane == 0) sCount[warp] = __popc(m);
+        __syncthreads();
+        int at = found + __popc(m & ((1u << lane) - 1u));
+        for (int q = 0; q < SMALL_THREADS / 32; q++) {
+            if (q < warp) at += sCount[q];
+            found += sCount[q];
         }
+        if (on) sb.cand[at] = p;
+        __syncthreads();
     }
-    flag[p] = f;
+    manifolds = __reduce_add_sync(0xffffffffu, manifolds);
+    points = __reduce_add_sync(0xffffffffu, points);
+    if (lane == 0 && manifolds) {
+        atomicAdd(&w.ctr[C_MANIFOLDS], manifolds);
+        atomicAdd(&w.ctr[C_CONTACTS], points);
+    }
+    if (tid == 0) *sb.nCand = found;
 }
 
 // Candidates in pair order; the manifold counts (has, points) of the counters.
@@ -260,6 +296,10 @@ void islands_launch_unions(const DevWorld& w, const DevPairs& P, int nPairs, Sol
 void islands_launch_select(const DevWorld& w, const DevPairs& P, int nPairs, SolverBuffers& sb, cudaStream_t s,
                            const int* cntp) {
     int n = w.nBodies;
+    if (n <= SMALL_BODIES && nPairs <= SMALL_PAIRS) {
+        k_select_small<<<1, SMALL_THREADS, 0, s>>>(w, P, nPairs, cntp, sb); note_launch();
+        return;
+    }
     k_island_sleep<<<gridn(n, 256), 256, 0, s>>>(w, sb.keepAwake, sb.inactive); note_launch();
     if (nPairs > 0) {
         k_select<<<gridn(nPairs, 256), 256, 0, s>>>(w, P, nPairs, cntp, sb.inactive, sb.flag); note_launch();
@@ -301,8 +341,7 @@ __device__ __forceinline__ int flow_home(const DevWorld& w, const SolverBuffers&
 
 // Everything a solve starts from zero, and the bodies' places in the order (-1: listed bodies), in one
 // launch: a dozen memsets took about 1.5 us each.
-__global__ void k_solve_clear(DevWorld w, SolverBuffers sb, int buckets, int* slotPt0, int nPairs) {
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+JBD void solve_clear(const DevWorld& w, const SolverBuffers& sb, int buckets, int* slotPt0, int nPairs, int tid, int stride) {
     for (int i = tid; i < w.nBodies; i += stride) {
         sb.bodyDeg[i] = 0;
         if (w.flags[i] & CF_LISTED) sb.posOf[i] = -1;
@@ -326,11 +365,12 @@ __global__ void k_solve_clear(DevWorld w, SolverBuffers sb, int buckets, int* sl
     }
 }
 
+__global__ void k_solve_clear(DevWorld w, SolverBuffers sb, int buckets, int* slotPt0, int nPairs) {
+    solve_clear(w, sb, buckets, slotPt0, nPairs, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
 // Bucket of candidate k: the part holding all its dynamic bodies, else nParts (cut).
-__global__ void k_classify(DevWorld w, DevPairs P, SolverBuffers sb) {
-    int nCand = *sb.nCand;
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nCand) return;
+JBD void classify(const DevWorld& w, const DevPairs& P, const SolverBuffers& sb, int k) {
     int p = sb.cand[k];
     int b0 = P.b0[p], b1 = P.b1[p];
     bool d0 = dyn(w, b0), d1 = dyn(w, b1);
@@ -366,6 +406,11 @@ __global__ void k_classify(DevWorld w, DevPairs P, SolverBuffers sb) {
     if ((threadIdx.x & 31) == __ffs(grp) - 1) atomicAdd(&sb.bucketCount[q], __popc(grp));
 }
 
+__global__ void k_classify(DevWorld w, DevPairs P, SolverBuffers sb) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < *sb.nCand) classify(w, P, sb, k);
+}
+
 // Fill position of a lane among the lanes of its warp with the same key: the group's leader
 // takes the group's places from *ctr with one atomic.
 JBD int group_take(int* ctr, int key) {
@@ -377,12 +422,36 @@ JBD int group_take(int* ctr, int key) {
     return base + __popc(grp & ((1u << lane) - 1u));
 }
 
-__global__ void k_bucket_scatter(SolverBuffers sb) {
-    int nCand = *sb.nCand;
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nCand) return;
+JBD void bucket_scatter(const SolverBuffers& sb, int k) {
     int b = sb.bucket[k];
     sb.bucketList[sb.bucketStart[b] + group_take(&sb.bucketFill[b], b)] = k;
+}
+__global__ void k_bucket_scatter(SolverBuffers sb) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < *sb.nCand) bucket_scatter(sb, k);
+}
+
+// Clear, classification, bucket starts and lists of a small world by one block (buckets <= its threads).
+__global__ void __launch_bounds__(SMALL_THREADS) k_prepare_small(DevWorld w, DevPairs P, SolverBuffers sb, int buckets,
+                                                                 int* slotPt0, int nPairs) {
+    __shared__ int sSum[SMALL_THREADS / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nCand = *sb.nCand;
+    solve_clear(w, sb, buckets, slotPt0, nPairs, tid, SMALL_THREADS);
+    __syncthreads();
+    for (int k = tid; k < nCand; k += SMALL_THREADS) classify(w, P, sb, k);
+    __syncthreads();
+    const int own = tid < buckets ? __ldcg(&sb.bucketCount[tid]) : 0;   // counted by atomics
+    int v = own;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+    }
+    if (lane == 31) sSum[warp] = v;
+    __syncthreads();
+    for (int q = 0; q < warp; q++) v += sSum[q];
+    if (tid < buckets) sb.bucketStart[tid] = v - own;
+    __syncthreads();
+    for (int k = tid; k < nCand; k += SMALL_THREADS) bucket_scatter(sb, k);
 }
 
 // Blocks take parts largest first from a shared counter (ctr[counter], cleared before the
@@ -2685,12 +2754,16 @@ void solve_launch_learn(const DevWorld& w, DevPairs& P, int nPairs, DevRows& R, 
                 !learn.sampleX && !learn.sampleT;
     if (!sb.worldParts) sb.cutHome = (unsigned*)(sb.cutToken + w.nBodies);   // behind the tokens of cut candidates
     const int buckets = parts + 2 + (sb.flowOn ? sb.nFlow + 1 : 0);   // the colouring's buckets, then the flow solver's
-    k_solve_clear<<<std::min(gridn(std::max(w.nBodies, buckets), 256), 2048), 256, 0, s>>>(w, sb, buckets, R.slot_pt0,
+    if (w.nBodies <= SMALL_BODIES && nPairs <= SMALL_PAIRS && buckets <= SMALL_THREADS) {
+        k_prepare_small<<<1, SMALL_THREADS, 0, s>>>(w, P, sb, buckets, R.slot_pt0, nPairs); note_launch();
+    } else {
+        k_solve_clear<<<std::min(gridn(std::max(w.nBodies, buckets), 256), 2048), 256, 0, s>>>(w, sb, buckets, R.slot_pt0,
                                                                                                 nPairs);
-    note_launch();
-    k_classify<<<gridn(nPairs, 256), 256, 0, s>>>(w, P, sb); note_launch();
-    exclusive_scan(sb.bucketCount, sb.bucketStart, nullptr, buckets, sb.flowScan, s);
-    k_bucket_scatter<<<gridn(nPairs, 256), 256, 0, s>>>(sb); note_launch();
+        note_launch();
+        k_classify<<<gridn(nPairs, 256), 256, 0, s>>>(w, P, sb); note_launch();
+        exclusive_scan(sb.bucketCount, sb.bucketStart, nullptr, buckets, sb.flowScan, s);
+        k_bucket_scatter<<<gridn(nPairs, 256), 256, 0, s>>>(sb); note_launch();
+    }
     {
         DevWorld wc = w;
         DevPairs pc = P;
