@@ -1127,11 +1127,11 @@ int query_prepare(const DevWorld& w, BroadphaseBuffers& bb, QueryBuffers& qb, bo
     }
     if (w.nBodies == 0) return JBGPU_OK;
     k_query_aabb<<<gridn(w.nBodies, 256), 256, 0, s>>>(w, qb.qmin, qb.qmax); note_launch();
-    if (!tree) return cudaGetLastError() == cudaSuccess ? JBGPU_OK : JBGPU_ERR_CUDA;
     DevWorld wq = w;
     wq.amin = qb.qmin;
     wq.amax = qb.qmax;
-    if (!bb.built) broadphase_order(wq, bb, s);
+    if (!bb.built) broadphase_order(wq, bb, s);   // with or without the tree: the solver's parts follow the order
+    if (!tree) return cudaGetLastError() == cudaSuccess ? JBGPU_OK : JBGPU_ERR_CUDA;
     if (!bb.treeBuilt) broadphase_topology(bb, s);
     const int nodes = bb.nFinite > 1 ? bb.nFinite - 1 : 1;
     if (nodes > qb.capNodes) {

@@ -84,3 +84,22 @@ def test_ray_paths_batched_worlds(gpu_lib, oracle_lib, n):
     world = rng.integers(0, 4, n).astype(np.int32)
     assert _same(o.ray_test(frm, to, world=world), g.ray_test(frm, to, world=world))
     g.close()
+
+
+@pytest.mark.gpu
+def test_rays_before_the_first_step_leave_the_same_order(gpu_lib):
+    """A query on bodies added since the last step fixes the order the solver's parts follow, whichever
+    path the rays take: a world of several parts steps the same after few rays and after many."""
+    sc = scenes.small_mixed(2600, seed=3, region=(14.0, 16.0, 14.0))
+    rng = np.random.Generator(np.random.PCG64(2))
+    worlds = [GpuWorld(sc), GpuWorld(sc)]
+    for g, n in zip(worlds, (3, 12000)):
+        frm = rng.uniform((-7, 0, -7), (7, 16, 7), (n, 3)).astype(F)
+        to = rng.uniform((-7, 0, -7), (7, 16, 7), (n, 3)).astype(F)
+        g.ray_test(frm, to)
+        for _ in range(40):
+            g.step(sc.dt)
+    assert worlds[0].counters()["cut_manifolds"] > 0
+    assert not H.compare_state(worlds[0].get_state(), worlds[1].get_state())
+    for g in worlds:
+        g.close()
