@@ -774,14 +774,17 @@ void broadphase_refit_into(const DevWorld& wq, const BroadphaseBuffers& bb, floa
 
 bool broadphase_rebuilds(const BroadphaseBuffers& bb) { return !(bb.built && bb.sinceBuild + 1 < bb.rebuildInterval); }
 
+// A query on bodies changed since the last step makes the order and, when it needs none, leaves the tree.
+bool broadphase_makes_tree(const BroadphaseBuffers& bb) {
+    return !bb.direct && (!bb.treeBuilt || broadphase_rebuilds(bb));
+}
+
 void broadphase_run_count(const DevWorld& w, BroadphaseBuffers& bb, cudaStream_t s) {
     const int n = w.nBodies, nf = bb.nFinite;
-    if (broadphase_rebuilds(bb)) {
-        broadphase_order(w, bb, s);
-        if (!bb.direct) broadphase_topology(bb, s);
-    } else {
-        bb.sinceBuild++;
-    }
+    const bool tree = broadphase_makes_tree(bb);
+    if (broadphase_rebuilds(bb)) broadphase_order(w, bb, s);
+    else bb.sinceBuild++;
+    if (tree) broadphase_topology(bb, s);
     if (bb.meshes) cudaMemsetAsync(bb.candBound, 0, sizeof(int), s);   // else it stays 0
     if (bb.direct) {
         k_direct_count<<<gridn(n + 1, DIRECT_THREADS / 32), DIRECT_THREADS, 0, s>>>(w, bb.list, bb.planeList, bb.planeStart,

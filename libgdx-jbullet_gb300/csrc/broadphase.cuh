@@ -72,6 +72,8 @@ void broadphase_topology(BroadphaseBuffers& bb, cudaStream_t s);
 void broadphase_refit_into(const DevWorld& wq, const BroadphaseBuffers& bb, float4* node, int* visit, cudaStream_t s);
 // Whether the next count renews the Morton order.
 bool broadphase_rebuilds(const BroadphaseBuffers& bb);
+// Whether it makes the tree's topology (its order changed, or a query made the order alone).
+bool broadphase_makes_tree(const BroadphaseBuffers& bb);
 // Whether worlds of these many bodies (all, finite) find their pairs without the tree.
 bool broadphase_direct(const std::vector<int>& bodies, const std::vector<int>& finite);
 void broadphase_run_count(const DevWorld& w, BroadphaseBuffers& bb, cudaStream_t s);

@@ -721,7 +721,7 @@ int narrow_and_islands(jbgpu_world* w, const int* cntp = nullptr) {
 // the solver, integration and activation.  B's kernels read the pair count from the device
 // (w.ctr[C_PAIRS], the broadphase total) and are sized by the pair capacity.  Launches bake
 // their pointers and host-side arguments, so each graph is kept per arrangement of the
-// alternating buffers (pair arrays, per-owner offsets), the tree path (rebuild or refit) and dt;
+// alternating buffers (pair arrays, per-owner offsets), the tree path (order, topology or refit) and dt;
 // anything else that changes a buffer or an argument clears them all (graphs_clear).  The host
 // state the launch functions change while a graph is captured (tree age, offset swap) is
 // changed by hand when the graph is replayed.
@@ -773,11 +773,11 @@ uint64_t fbits64(float f) { uint32_t u; std::memcpy(&u, &f, 4); return u; }
 int single_step_graph(jbgpu_world* w, float dt) {
     cudaStream_t s = w->stream;
     BroadphaseBuffers& B = w->bb;
-    const bool rebuild = broadphase_rebuilds(B);
+    const bool rebuild = broadphase_rebuilds(B), makesTree = broadphase_makes_tree(B);
     const bool builtBefore = B.built, treeBefore = B.treeBuilt;
     const int ageBefore = B.sinceBuild;
     const uint64_t ka[8] = {1, (uint64_t)rebuild, (uint64_t)(uintptr_t)B.off, (uint64_t)(uintptr_t)B.offPrev,
-                            fbits64(dt), 0, 0, 0};
+                            fbits64(dt), (uint64_t)makesTree, 0, 0};
     bool captured = false;
     int rc = capture_or_replay(w, ka, [&]() -> int {
         DevWorld d = dev_view(w);
@@ -794,8 +794,9 @@ int single_step_graph(jbgpu_world* w, float dt) {
     }
     if (rc) return rc;
     if (!captured) {                       // what broadphase_run_count does on the host
-        if (rebuild) { B.built = true; B.treeBuilt = !B.direct; B.sinceBuild = 0; }
+        if (rebuild) { B.built = true; B.treeBuilt = false; B.sinceBuild = 0; }
         else B.sinceBuild++;
+        if (makesTree) B.treeBuilt = true;
     }
     w->orderValid = true;
     CK(cudaStreamSynchronize(s));
