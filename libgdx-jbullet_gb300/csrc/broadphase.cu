@@ -747,10 +747,10 @@ void broadphase_order(const DevWorld& w, BroadphaseBuffers& bb, cudaStream_t s) 
 void broadphase_topology(BroadphaseBuffers& bb, cudaStream_t s) {
     const int nf = bb.nFinite;
     bb.treeBuilt = true;
+    cudaMemsetAsync(bb.wroot, 0xff, sizeof(int) * bb.nWorlds, s);   // no root: worlds of listed bodies alone
     if (nf > 0) {
         cudaMemsetAsync(bb.wstart, 0xff, sizeof(int) * bb.nWorlds, s);
         cudaMemsetAsync(bb.wend, 0xff, sizeof(int) * bb.nWorlds, s);
-        cudaMemsetAsync(bb.wroot, 0xff, sizeof(int) * bb.nWorlds, s);
         k_world_ranges<<<gridn(nf, 256), 256, 0, s>>>(bb.mkeys, nf, bb.wstart, bb.wend, bb.wroot); note_launch();
         if (nf > 1) {
             cudaMemsetAsync(bb.bvh.parent, 0xff, sizeof(int) * (nf - 1), s);
