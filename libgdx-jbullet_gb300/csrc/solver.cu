@@ -943,14 +943,18 @@ JBD void colour_claims(const DevWorld& w, const DevPairs& P, const SolverBuffers
 
 __global__ void __launch_bounds__(COLOUR_THREADS) k_colour(DevWorld w, DevPairs P, SolverBuffers sb) {
     extern __shared__ __align__(16) unsigned long long colSmem[];
-    __shared__ int shPart, shFail;
+    __shared__ int shPart, shFail, shClaims;
     unsigned barK = 0;
     const int nb = gridDim.x;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
+    // Set by k_classify (a body with too many candidates) or by a block of this launch already under way:
+    // one read a block, as barriers lie on the path it chooses.
+    if (threadIdx.x == 0) shClaims = (int)ld_acquire(&w.ctr[C_COL_FAIL]);
+    __syncthreads();
     uint4* tok = (uint4*)colSmem;
     unsigned* home = (unsigned*)(tok + sb.partMax);
     int local = 0, cut = 0;   // colours
-    if (!ld_acquire(&w.ctr[C_COL_FAIL])) {   // set by k_classify: a body with too many candidates
+    if (!shClaims) {
         bool ok = true;
         for (int part = next_part(w, sb, C_PART_NEXT0, &shPart); part >= 0 && ok; part = next_part(w, sb, C_PART_NEXT0, &shPart))
             ok = first_fit_part(w, P, sb, part, tok, home, &shFail, local);
