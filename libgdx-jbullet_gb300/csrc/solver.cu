@@ -2331,11 +2331,12 @@ __global__ void __launch_bounds__(SOLVER_THREADS, 2) k_pgs(DevWorld w, DevPairs 
     if (nSlots == 0 && sb.J.n == 0) return;
     const bool contacts = nSlots > 0;   // else only joints (the colouring did not run this step)
     Staged st;
-    if (nb == 1 && sb.nParts == 1 && nCut == 0 && !byRes && smem && sb.partMax <= sb.smemCap) {
+    if (nb == 1 && sb.nParts == 1 && nCut == 0 && !byRes && smem && sb.partMax <= sb.smemCap && !sb.movingStatic) {
         // One part with joints, one block: its velocities stay in shared memory through every phase of
         // joints and contacts, and a phase ends with the block's barrier.  With the part staged in and
         // out around every phase and a grid barrier of one block, 64 chains of 8 took
-        // 190 us, 75 us so.
+        // 190 us, 75 us so.  (Not with a kinematic body that keeps its mass: contacts have its velocity
+        // in global memory, where every phase must find what the joints made of it.)
         PartView v = part_view(sb, 0);
         if (!contacts) v.nLoc = 0;
         JointVel at;
