@@ -2622,7 +2622,7 @@ static size_t pgs_smem(const SolverBuffers& sb, int poolPts) {
 static size_t colour_smem(const SolverBuffers& sb) { return (size_t)sb.partMax * (sizeof(uint4) + sizeof(uint2)); }
 
 int solver_configure(SolverBuffers& sb, int nFinite, const std::vector<int>& worldCounts, int sms, int rangeParts,
-                     int threads, int smemBodies) {
+                     int threads, int smemBodies, cudaStream_t s) {
     sb.threads = threads;
     int maxWorld = 0;
     for (int c : worldCounts) maxWorld = std::max(maxWorld, c);
@@ -2654,13 +2654,14 @@ int solver_configure(SolverBuffers& sb, int nFinite, const std::vector<int>& wor
         }
         sb.partsCap = parts;
     }
-    if (flow_plan(sb, start, sms)) return JBGPU_ERR_CUDA;
+    if (flow_plan(sb, start, sms, s)) return JBGPU_ERR_CUDA;
     std::vector<int> order(parts);
     for (int p = 0; p < parts; p++) order[p] = p;
     std::stable_sort(order.begin(), order.end(),
                      [&](int a, int b) { return start[a + 1] - start[a] > start[b + 1] - start[b]; });
-    if (cudaMemcpy(sb.partStart, start.data(), sizeof(int) * (parts + 1), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(sb.partOrder, order.data(), sizeof(int) * parts, cudaMemcpyHostToDevice) != cudaSuccess)
+    if (cudaMemcpyAsync(sb.partStart, start.data(), sizeof(int) * (parts + 1), cudaMemcpyHostToDevice, s) != cudaSuccess ||
+        cudaMemcpyAsync(sb.partOrder, order.data(), sizeof(int) * parts, cudaMemcpyHostToDevice, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess)
         return JBGPU_ERR_CUDA;
     sb.nFinite = nFinite;
     sb.nParts = parts;

@@ -167,7 +167,7 @@ struct SolverBuffers {
 // rangeParts > 0 asks for that many range parts; threads per block of the colouring and PGS;
 // smemBodies > 0 caps the parts whose velocities are staged in shared memory.
 int solver_configure(SolverBuffers& sb, int nFinite, const std::vector<int>& worldCounts, int sms, int rangeParts,
-                     int threads, int smemBodies);
+                     int threads, int smemBodies, cudaStream_t s);
 void islands_launch(const DevWorld& w, const DevPairs& P, int nPairs, SolverBuffers& sb, cudaStream_t s);
 void islands_launch_unions(const DevWorld& w, const DevPairs& P, int nPairs, SolverBuffers& sb, cudaStream_t s,
                            const int* cntp);
@@ -182,7 +182,7 @@ void solver_free(SolverBuffers& sb);
 // nonzero when a CUDA call failed.
 constexpr int FLOW_DESC_INTS = 12;           // a slot's 8 ints and its group's word, kept 16-byte aligned
 constexpr int FLOW_MAX_ITERATIONS = 500000;   // its phase tags are 32 bits
-int flow_plan(SolverBuffers& sb, const std::vector<int>& start, int sms);
+int flow_plan(SolverBuffers& sb, const std::vector<int>& start, int sms, cudaStream_t s);
 int flow_configure(SolverBuffers& sb, int sms, int smemBodies);
 void flow_free(SolverBuffers& sb);
 void flow_launch(const DevWorld& w, DevPairs& P, int nPairs, DevRows& R, SolverBuffers& sb, float dt, cudaStream_t s);

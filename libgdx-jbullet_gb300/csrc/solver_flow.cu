@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, FLOW_BLOCKS) k_flow(DevWorld w, 
 template <class T> static cudaError_t falloc(T** p, size_t n) { return cudaMalloc((void**)p, sizeof(T) * (n ? n : 1)); }
 template <class T> static void ffree(T*& p) { if (p) cudaFree((void*)p); p = nullptr; }
 
-int flow_plan(SolverBuffers& sb, const std::vector<int>& start, int sms) {
+int flow_plan(SolverBuffers& sb, const std::vector<int>& start, int sms, cudaStream_t s) {
     const int parts = (int)start.size() - 1;
     std::vector<int2> part(parts);
     std::vector<int> body, size(parts), order;
@@ -637,9 +637,10 @@ int flow_plan(SolverBuffers& sb, const std::vector<int>& start, int sms) {
     sb.nFlow = nFlow;
     sb.flowExch = !sb.worldParts || nFlow > parts;
     sb.gridFlow = sb.worldParts ? most : nFlow;   // blocks that wait on one another; flow_configure adds the rest
-    return cudaMemcpy(sb.flowPart, part.data(), sizeof(int2) * parts, cudaMemcpyHostToDevice) != cudaSuccess ||
-           cudaMemcpy(sb.flowBody, body.data(), sizeof(int) * (nFlow + 1), cudaMemcpyHostToDevice) != cudaSuccess ||
-           cudaMemcpy(sb.flowOrder, order.data(), sizeof(int) * nFlow, cudaMemcpyHostToDevice) != cudaSuccess;
+    return cudaMemcpyAsync(sb.flowPart, part.data(), sizeof(int2) * parts, cudaMemcpyHostToDevice, s) != cudaSuccess ||
+           cudaMemcpyAsync(sb.flowBody, body.data(), sizeof(int) * (nFlow + 1), cudaMemcpyHostToDevice, s) != cudaSuccess ||
+           cudaMemcpyAsync(sb.flowOrder, order.data(), sizeof(int) * nFlow, cudaMemcpyHostToDevice, s) != cudaSuccess ||
+           cudaStreamSynchronize(s) != cudaSuccess;
 }
 
 static int flow_threads(const SolverBuffers& sb) { return sb.threads < SOLVER_THREADS ? sb.threads : FLOW_THREADS; }

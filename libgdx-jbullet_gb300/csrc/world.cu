@@ -180,14 +180,14 @@ int num_sms_of(int dev) {
     return s > 0 ? s : 1;
 }
 
-int alloc_pairs(DevPairs& P, int cap) {
+int alloc_pairs(DevPairs& P, int cap, cudaStream_t s) {
     CK(dalloc(&P.keys, cap)); CK(dalloc(&P.has, cap)); CK(dalloc(&P.n, cap));
     CK(dalloc(&P.b0, cap)); CK(dalloc(&P.b1, cap));
     size_t c4 = (size_t)cap * 4;
     CK(dalloc(&P.pA, c4)); CK(dalloc(&P.pB, c4)); CK(dalloc(&P.wA, c4)); CK(dalloc(&P.wB, c4));
     CK(dalloc(&P.nrm, c4)); CK(dalloc(&P.imp, c4)); CK(dalloc(&P.d1, c4)); CK(dalloc(&P.d2, c4));
     CK(dalloc(&P.steps, cap));
-    CK(cudaMemset(P.steps, 0, cap));
+    CK(cudaMemsetAsync(P.steps, 0, cap, s));
     return JBGPU_OK;
 }
 void free_pairs(DevPairs& P) {
@@ -303,7 +303,7 @@ int ensure_pair_capacity(jbgpu_world* w, int buf, int need) {
     if (need > w->capPairs[buf]) {
         graphs_clear(w);
         free_pairs(w->pairs[buf]);
-        int rc = alloc_pairs(w->pairs[buf], nc);
+        int rc = alloc_pairs(w->pairs[buf], nc, w->stream);
         if (rc) return rc;
         w->capPairs[buf] = nc;
     }
@@ -421,10 +421,11 @@ int sync_planes(jbgpu_world* w) {
     CK(dalloc(&B.planeList, std::max<size_t>(1, list.size()))); CK(dalloc(&B.planeStart, nw + 1));
     CK(dalloc(&B.wstart, nw)); CK(dalloc(&B.wend, nw)); CK(dalloc(&B.wroot, nw)); CK(dalloc(&B.bounds, 6)); CK(dalloc(&B.total, 2));
     B.candBound = B.total + 1;
-    CK(cudaMemset(B.total, 0, sizeof(int) * 2));
+    cudaStream_t s = w->stream;
+    CK(cudaMemsetAsync(B.total, 0, sizeof(int) * 2, s));
     CK(dalloc(&B.segLong, 1));
-    if (!list.empty()) CK(cudaMemcpy(B.planeList, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(B.planeStart, start.data(), sizeof(int) * (nw + 1), cudaMemcpyHostToDevice));
+    if (!list.empty()) CK(cudaMemcpyAsync(B.planeList, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(B.planeStart, start.data(), sizeof(int) * (nw + 1), cudaMemcpyHostToDevice, s));
     B.nFinite = nf;
     B.nPlanes = np;
     B.nWorlds = nw;
@@ -443,9 +444,10 @@ int sync_planes(jbgpu_world* w) {
     B.direct = broadphase_direct(bodies, finite);
     if (B.direct) CK(dalloc(&B.kept, (size_t)DIRECT_CACHE * body.size()));
     CK(dalloc(&B.list.body, body.size())); CK(dalloc(&B.list.pos, pos.size())); CK(dalloc(&B.list.end, nw));
-    CK(cudaMemcpy(B.list.body, body.data(), sizeof(int) * body.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(B.list.pos, pos.data(), sizeof(int) * pos.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(B.list.end, end.data(), sizeof(int) * nw, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(B.list.body, body.data(), sizeof(int) * body.size(), cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(B.list.pos, pos.data(), sizeof(int) * pos.size(), cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(B.list.end, end.data(), sizeof(int) * nw, cudaMemcpyHostToDevice, s));
+    CK(cudaStreamSynchronize(s));   // the lists above are this function's
     w->bb.built = w->bb.treeBuilt = false;
     w->solverDirty = true;
     w->orderValid = false;
@@ -516,7 +518,7 @@ int prepare_solver(jbgpu_world* w) {
     if (w->solverDirty) {
         graphs_clear(w);
         int rc = solver_configure(S, nf, w->worldFinite, w->sms, w->cfg.solver_parts,
-                                  w->cfg.solver_threads ? w->cfg.solver_threads : SOLVER_THREADS, w->cfg.solver_smem_bodies);
+                                  w->cfg.solver_threads ? w->cfg.solver_threads : SOLVER_THREADS, w->cfg.solver_smem_bodies, w->stream);
         if (rc) return fail(rc, "solver part tables");
         w->solverDirty = false;
     }
@@ -621,7 +623,7 @@ int sync_joints(jbgpu_world* w) {
         CK(dalloc(&J.d6set, D6_SET_F4 * (size_t)c));
         CK(dalloc(&J.order, c)); CK(dalloc(&J.colStart, c + 1)); CK(dalloc(&J.r1, c)); CK(dalloc(&J.r2, c));
         CK(dalloc(&J.dep, c)); CK(dalloc(&J.imp, c)); CK(dalloc(&J.act, c));
-        CK(cudaMemset(J.imp, 0, sizeof(float) * c));
+        CK(cudaMemsetAsync(J.imp, 0, sizeof(float) * c, w->stream));
         w->capJoints = c;
     }
     auto dynBody = [&](int b) { return b >= 0 && !(w->hFlags[b] & (CF_STATIC | CF_KINEMATIC)); };
@@ -1329,7 +1331,7 @@ int jbgpu_world_create(const jbgpu_config* cfg, jbgpu_world** out) {
     d.slop = c.linear_slop;
     d.solverMode = c.solver_mode;
     int rc;
-    if (cudaMalloc(&d.ctr, sizeof(int) * C_NCTR) != cudaSuccess || cudaMemset(d.ctr, 0, sizeof(int) * C_NCTR) != cudaSuccess ||
+    if (cudaMalloc(&d.ctr, sizeof(int) * C_NCTR) != cudaSuccess || cudaMemsetAsync(d.ctr, 0, sizeof(int) * C_NCTR, w->stream) != cudaSuccess ||
         cudaMallocHost(&w->hostPinned, sizeof(int) * 64) != cudaSuccess) {
         delete w;
         return fail(JBGPU_ERR_CUDA, "counter allocation");
@@ -1340,8 +1342,8 @@ int jbgpu_world_create(const jbgpu_config* cfg, jbgpu_world** out) {
              CK(dalloc(&S.colourStart, MAX_COLOURS + 1)); CK(dalloc(&S.nCand, 1)); CK(dalloc(&S.nColours, 1));
              CK(dalloc(&S.nIslChunks, 1));
              CK(dalloc(&w->rows.nPts, 1));
-             CK(cudaMemset(w->rows.nPts, 0, sizeof(int)));
-             CK(cudaMemset(S.nCand, 0, sizeof(int))); CK(cudaMemset(S.nColours, 0, sizeof(int)));
+             CK(cudaMemsetAsync(w->rows.nPts, 0, sizeof(int), w->stream));
+             CK(cudaMemsetAsync(S.nCand, 0, sizeof(int), w->stream)); CK(cudaMemsetAsync(S.nColours, 0, sizeof(int), w->stream));
              NarrowBuffers& N = w->nb;
              N.slots = w->sms * 2;
              N.sms = w->sms;
@@ -1349,7 +1351,7 @@ int jbgpu_world_create(const jbgpu_config* cfg, jbgpu_world** out) {
              N.queueCount = d.ctr + C_EPA_QUEUE;
              N.ovfCount = d.ctr + C_EPA_OVF0;
              CK(dalloc(&N.tierMode, 1));
-             CK(cudaMemset(N.tierMode, 0, sizeof(int)));
+             CK(cudaMemsetAsync(N.tierMode, 0, sizeof(int), w->stream));
 
              return grow_bodies(w, std::max(1, c.initial_body_capacity));
          }()) != JBGPU_OK) {
@@ -1688,8 +1690,8 @@ int jbgpu_world_remove_bodies(jbgpu_world* w, const int32_t* bodies, int32_t n) 
     CK(dalloc(&dFrom, std::max(nNew, 1)));
     CK(dalloc(&dNew, nOld));
     CK(cudaMalloc(&tmp, sizeof(float4) * std::max(nNew, 1)));
-    CK(cudaMemcpy(dFrom, from.data(), sizeof(int) * nNew, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(dNew, newIndex.data(), sizeof(int) * nOld, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(dFrom, from.data(), sizeof(int) * nNew, cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(dNew, newIndex.data(), sizeof(int) * nOld, cudaMemcpyHostToDevice, s));
     DevWorld& d = w->dw;
     int rc = 0;
     using namespace removal;
@@ -1834,16 +1836,18 @@ int jbgpu_world_set_ccd(jbgpu_world* w, const int32_t* bodies, const float* thr,
         if (bodies[k] < 0 || bodies[k] >= w->nBodies) return fail(JBGPU_ERR_INVALID_ARGUMENT, "bad body index");
     if (n == 0) return JBGPU_OK;
     CK(cudaSetDevice(w->device));
-    CK(cudaStreamSynchronize(w->stream));
+    cudaStream_t s = w->stream;
     std::vector<float> t(w->nBodies), r(w->nBodies);
-    CK(cudaMemcpy(t.data(), w->dw.ccdThr, sizeof(float) * w->nBodies, cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(r.data(), w->dw.ccdRad, sizeof(float) * w->nBodies, cudaMemcpyDeviceToHost));
+    CK(cudaMemcpyAsync(t.data(), w->dw.ccdThr, sizeof(float) * w->nBodies, cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(r.data(), w->dw.ccdRad, sizeof(float) * w->nBodies, cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
     for (int k = 0; k < n; k++) {
         t[bodies[k]] = thr[k];
         r[bodies[k]] = rad[k];
     }
-    CK(cudaMemcpy(w->dw.ccdThr, t.data(), sizeof(float) * w->nBodies, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(w->dw.ccdRad, r.data(), sizeof(float) * w->nBodies, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(w->dw.ccdThr, t.data(), sizeof(float) * w->nBodies, cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(w->dw.ccdRad, r.data(), sizeof(float) * w->nBodies, cudaMemcpyHostToDevice, s));
+    CK(cudaStreamSynchronize(s));
     bool on = false;
     for (float v : t) on = on || v != 0.0f;
     if (on != w->ccdOn) graphs_clear(w);   // the integrate stage's launches change
@@ -1856,21 +1860,23 @@ int jbgpu_world_set_ccd(jbgpu_world* w, const int32_t* bodies, const float* thr,
 static int body_gravity(jbgpu_world* w, const int32_t* bodies, const float* acc, int32_t n, bool all) {
     if (w->nBodies == 0) return JBGPU_OK;
     CK(cudaSetDevice(w->device));
-    CK(cudaStreamSynchronize(w->stream));
+    cudaStream_t s = w->stream;
     std::vector<float4> il(w->nBodies), g(w->nBodies);
-    CK(cudaMemcpy(il.data(), w->dw.iloc, sizeof(float4) * w->nBodies, cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(g.data(), w->dw.gravity, sizeof(float4) * w->nBodies, cudaMemcpyDeviceToHost));
+    CK(cudaMemcpyAsync(il.data(), w->dw.iloc, sizeof(float4) * w->nBodies, cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(g.data(), w->dw.gravity, sizeof(float4) * w->nBodies, cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
     const int m = all ? w->nBodies : n;
     for (int k = 0; k < m; k++) {
         const int i = all ? k : bodies[k];
         const float* a = all ? acc : acc + 3 * k;
         const float im = il[i].w;
         if (im != 0.0f) {
-            const float s = 1.0f / im;
-            g[i] = make_float4(a[0] * s, a[1] * s, a[2] * s, 0.0f);
+            const float inv = 1.0f / im;
+            g[i] = make_float4(a[0] * inv, a[1] * inv, a[2] * inv, 0.0f);
         }
     }
-    CK(cudaMemcpy(w->dw.gravity, g.data(), sizeof(float4) * w->nBodies, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(w->dw.gravity, g.data(), sizeof(float4) * w->nBodies, cudaMemcpyHostToDevice, s));
+    CK(cudaStreamSynchronize(s));
     return JBGPU_OK;
 }
 
@@ -2686,6 +2692,8 @@ int jbgpu_world_counters(jbgpu_world* w, jbgpu_counters* c) {
     int nc = 0;
     CK(cudaMemcpyAsync(h, w->dw.ctr, sizeof(int) * C_NCTR, cudaMemcpyDeviceToHost, w->stream));
     CK(cudaMemcpyAsync(&nc, w->sb.nCand, sizeof(int), cudaMemcpyDeviceToHost, w->stream));
+    int replays = 0;
+    if (w->qb.slowCount) CK(cudaMemcpyAsync(&replays, w->qb.slowCount, sizeof(int), cudaMemcpyDeviceToHost, w->stream));
     CK(cudaStreamSynchronize(w->stream));
     std::memset(c, 0, sizeof(*c));
     c->steps = w->steps;
@@ -2707,9 +2715,7 @@ int jbgpu_world_counters(jbgpu_world* w, jbgpu_counters* c) {
     c->solver_islands_converged = h[C_ISL_CONV];
     c->solver_island_iterations = h[C_ISL_ITERS];
     c->ccd_clamped = w->ccdOn ? h[C_CCD_N] : 0;
-    if (w->qb.slowCount) {
-        CK(cudaMemcpy(&c->ray_replays, w->qb.slowCount, sizeof(int), cudaMemcpyDeviceToHost));
-    }
+    c->ray_replays = replays;
     return JBGPU_OK;
 }
 
