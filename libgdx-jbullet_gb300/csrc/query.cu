@@ -26,6 +26,7 @@
 #include "gridsync.cuh"
 #include "prims.cuh"
 #include "query.cuh"
+#include "ray_lists.cuh"
 #include "dispatch.cuh"
 #include <algorithm>
 #include <climits>
@@ -1150,7 +1151,7 @@ int query_prepare(const DevWorld& w, BroadphaseBuffers& bb, QueryBuffers& qb, bo
     return cudaGetLastError() == cudaSuccess ? JBGPU_OK : JBGPU_ERR_CUDA;
 }
 
-static bool grow_ray_buffers(QueryBuffers& qb, int n, bool lists = false) {
+static bool grow_ray_buffers(QueryBuffers& qb, int n, bool lists = false, int bodies = 0) {
     if (n > qb.capRays) {   // per-ray (per-sweep) buffers
         void* old[] = {qb.slow, qb.rayCnt, qb.rayOff, qb.key, qb.scanScratch};
         for (void* p : old)
@@ -1168,16 +1169,19 @@ static bool grow_ray_buffers(QueryBuffers& qb, int n, bool lists = false) {
             return false;
         qb.capRays = c;
     }
-    if (lists) {   // per-ray candidate lists: 256 entries a ray while that stays within 512 MB, at least 8
-        const int want = (int)std::min<size_t>(256, std::max<size_t>(8, ((size_t)1 << 26) / (size_t)n));
-        if (!qb.list || (size_t)n * want > qb.listEntries) {
+    if (lists) {
+        qb.listCap = ray_list_fit(n, bodies, qb.listEntries, [&](size_t entries) {
             if (qb.list) cudaFree(qb.list);
             qb.list = nullptr;
             qb.listEntries = 0;
-            if (cudaMalloc(&qb.list, sizeof(RayEntry) * (size_t)n * want) != cudaSuccess) return false;
-            qb.listEntries = (size_t)n * want;
-        }
-        qb.listCap = want;
+            if (cudaMalloc(&qb.list, sizeof(RayEntry) * entries) != cudaSuccess) {
+                cudaGetLastError();
+                return false;
+            }
+            qb.listEntries = entries;
+            return true;
+        });
+        if (!qb.listCap) return false;
     }
     if (!qb.slowCount && (cudaMalloc((void**)&qb.slowCount, sizeof(int)) != cudaSuccess ||
                           cudaMalloc((void**)&qb.candTotal, sizeof(int)) != cudaSuccess ||
@@ -1249,7 +1253,7 @@ int query_rays(const DevWorld& w, const BroadphaseBuffers& bb, QueryBuffers& qb,
     if (n <= 0) return JBGPU_OK;
     int rc;
     const bool byBlock = query_rays_by_block(w.nBodies, n);
-    if (!grow_ray_buffers(qb, n, !byBlock && !qb.replayAll)) return JBGPU_ERR_CUDA;
+    if (!grow_ray_buffers(qb, n, !byBlock && !qb.replayAll, w.nBodies)) return JBGPU_ERR_CUDA;
     DevWorld wq = w;
     wq.amin = qb.qmin;
     wq.amax = qb.qmax;
