@@ -148,8 +148,8 @@ struct jbgpu_world {
     int* hostPinned = nullptr;
     Prof prof;
     int* profHist = nullptr;      // per profiled step: device counters + solver manifolds
-    float* ioStage = nullptr;     // device staging for apply_forces, get_transforms and get_state (STATE_TOTAL words per body)
-    int capIo = 0;
+    float* ioStage = nullptr;     // device staging for apply_forces, get_transforms (12 words a body) and get_state
+    size_t capIo = 0;             // words
     // learned warm start and training samples
     jbgpu_mlp* mlp = nullptr;     // not owned
     bool learnReady = false;      // warm-start kernel configured
@@ -946,12 +946,13 @@ __global__ void k_pack_transforms(DevWorld w, float* out);
 __global__ void k_pack_interpolated(DevWorld w, float t, float* out);
 
 namespace {
-int ensure_io(jbgpu_world* w) {
-    if (w->capIo >= w->nBodies && w->ioStage) return JBGPU_OK;
+int ensure_io(jbgpu_world* w, int words) {   // room for so many words a body
+    if ((size_t)words * w->nBodies <= w->capIo) return JBGPU_OK;
     if (w->ioStage) cudaFree(w->ioStage);
     w->ioStage = nullptr;
-    int c = std::max(w->nBodies, w->capBodies);
-    CK(cudaMalloc(&w->ioStage, sizeof(float) * STATE_TOTAL * (size_t)std::max(c, 1)));
+    w->capIo = 0;
+    const size_t c = (size_t)words * std::max(w->nBodies, w->capBodies);
+    CK(cudaMalloc(&w->ioStage, sizeof(float) * c));
     w->capIo = c;
     return JBGPU_OK;
 }
@@ -2477,7 +2478,7 @@ int jbgpu_world_get_state(jbgpu_world* w, jbgpu_state* st) {
     const size_t n = (size_t)w->nBodies;
     st->n_bodies = w->nBodies;
     if (n == 0) return JBGPU_OK;
-    int rc = ensure_io(w);
+    int rc = ensure_io(w, STATE_TOTAL);
     if (rc) return rc;
     cudaStream_t s = w->stream;
     k_pack_state<<<(w->nBodies + 127) / 128, 128, 0, s>>>(dev_view(w), w->ioStage); note_launch();
@@ -2723,7 +2724,7 @@ int jbgpu_world_apply_forces(jbgpu_world* w, const float* force, const float* to
     if (!w) return fail(JBGPU_ERR_INVALID_ARGUMENT, "null world");
     if (w->nBodies == 0 || (!force && !torque)) return JBGPU_OK;
     CK(cudaSetDevice(w->device));
-    int rc = ensure_io(w);
+    int rc = ensure_io(w, 12);
     if (rc) return rc;
     size_t n3 = (size_t)w->nBodies * 3;
     cudaStream_t s = w->stream;
@@ -2739,7 +2740,7 @@ int jbgpu_world_get_transforms(jbgpu_world* w, float* out) {
     if (!w || !out) return fail(JBGPU_ERR_INVALID_ARGUMENT, "null");
     if (w->nBodies == 0) return JBGPU_OK;
     CK(cudaSetDevice(w->device));
-    int rc = ensure_io(w);
+    int rc = ensure_io(w, 12);
     if (rc) return rc;
     cudaStream_t s = w->stream;
     DevWorld d = dev_view(w);
@@ -2754,7 +2755,7 @@ int jbgpu_world_get_interpolated_transforms(jbgpu_world* w, float* out) {
     if (!w || !out) return fail(JBGPU_ERR_INVALID_ARGUMENT, "null");
     if (w->nBodies == 0) return JBGPU_OK;
     CK(cudaSetDevice(w->device));
-    int rc = ensure_io(w);
+    int rc = ensure_io(w, 12);
     if (rc) return rc;
     cudaStream_t s = w->stream;
     k_pack_interpolated<<<(w->nBodies + 255) / 256, 256, 0, s>>>(dev_view(w), w->localTime, w->ioStage); note_launch();
