@@ -2483,15 +2483,23 @@ int jbgpu_world_get_state(jbgpu_world* w, jbgpu_state* st) {
     cudaStream_t s = w->stream;
     k_pack_state<<<(w->nBodies + 127) / 128, 128, 0, s>>>(dev_view(w), w->ioStage); note_launch();
     CK(cudaGetLastError());
-    // the fields in the stage's order; fields that follow one another at the caller's too go in one copy
+    // The fields in the stage's order; fields that follow one another at the caller's too go in one copy, but
+    // not where a copy could run past the end of a registered allocation, which is an error.
+    auto pageable = [](const void* p) {
+        cudaPointerAttributes a;
+        if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeUnregistered;
+        cudaGetLastError();
+        return false;
+    };
     void* const dst[] = {st->transform, st->linear_velocity, st->angular_velocity, st->inv_inertia_world, st->total_force,
                          st->total_torque, st->aabb, st->activation_state, st->deactivation_time, st->island_tag};
     size_t at = 0;
     for (int f = 0; f < 10;) {
         const size_t from = at;
         char* const to = (char*)dst[f];
+        const bool join = to && pageable(to);
         do at += n * STATE_WORDS[f++];
-        while (to && f < 10 && (char*)dst[f] == to + 4 * (at - from));
+        while (join && f < 10 && (char*)dst[f] == to + 4 * (at - from) && pageable(dst[f]));
         if (to) CK(cudaMemcpyAsync(to, w->ioStage + from, 4 * (at - from), cudaMemcpyDeviceToHost, s));
     }
     CK(cudaStreamSynchronize(s));
