@@ -39,6 +39,7 @@ single-world workload runs an independent replica per rank.  Weak scaling; rank 
 line.
 """
 import argparse
+import datetime
 import json
 import os
 import subprocess
@@ -126,14 +127,16 @@ class Dist:
 
 
 class ClockSampler:
-    """nvidia-smi clock/throttle sampling during the timed region."""
-    Q = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,clocks_event_reasons.hw_slowdown,"
+    """nvidia-smi clock/throttle sampling.  The sampler runs from start(); what it reports is sampled from
+    mark(), the beginning of the timed region, on (by nvidia-smi's own time stamps)."""
+    Q = ("timestamp,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,clocks_event_reasons.hw_slowdown,"
          "clocks_event_reasons.hw_thermal_slowdown,clocks_event_reasons.sw_thermal_slowdown,"
          "clocks_event_reasons.sw_power_cap")
 
     def __init__(self, device):
         self.device = device
         self.proc = None
+        self.since = None
         self.path = os.path.join("/tmp", "jbgpu_clocks_%d_%d.csv" % (os.getpid(), device))
 
     def start(self):
@@ -144,25 +147,20 @@ class ClockSampler:
         except Exception:
             self.proc = None
 
+    def mark(self):
+        self.since = datetime.datetime.now()
+
     def stop(self):
         if not self.proc:
             return None
-        time.sleep(0.25)
+        time.sleep(0.45)   # at least one sample after a short region
         self.proc.terminate()
         try:
             self.proc.wait(timeout=5)
         except Exception:
             self.proc.kill()
         self.f.close()
-        rows = []
-        for line in open(self.path):
-            parts = [x.strip() for x in line.split(",")]
-            if len(parts) < 9:
-                continue
-            try:
-                rows.append((float(parts[1]), float(parts[2]), float(parts[3]), parts[5:9]))
-            except ValueError:
-                continue
+        rows = self.rows(open(self.path))
         if not rows:
             return None
         sm = np.array([r[0] for r in rows])
@@ -172,6 +170,21 @@ class ClockSampler:
         reasons = sorted({names[i] for r in rows for i, v in enumerate(r[3]) if v.lower() == "active"})
         return {"sm_mhz": float(np.median(load)), "sm_max_mhz": float(max(r[1] for r in rows)), "reasons": reasons,
                 "samples": len(rows), "power_w_max": float(pw.max())}
+
+    def rows(self, lines):
+        out = []
+        for line in lines:
+            parts = [x.strip() for x in line.split(",")]
+            if len(parts) < 9:
+                continue
+            try:
+                at = datetime.datetime.strptime(parts[0], "%Y/%m/%d %H:%M:%S.%f")
+                row = (float(parts[1]), float(parts[2]), float(parts[3]), parts[5:9])
+            except ValueError:
+                continue
+            if self.since is None or at >= self.since:
+                out.append(row)
+        return out
 
 
 def peaks():
@@ -482,13 +495,14 @@ def run_ours(args, dist):
     w = GpuWorld(sc, config=cfg)
     if args.graph:
         w.set_graph(True)
-    # the sampler is up before the timed region: its start-up holds the driver while buffers grow there
+    # the sampler is up before the untimed steps: its start-up holds the driver
     clk = ClockSampler(dist.local)
     clk.start()
     advance(w, sc, S + W)
     dist.barrier()
     w.synchronize()
     l0 = lib.launch_count()
+    clk.mark()
     t0 = time.perf_counter()
     w.timer_start()
     for _ in range(K):
