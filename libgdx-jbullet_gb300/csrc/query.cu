@@ -770,8 +770,8 @@ __global__ void __launch_bounds__(256) k_ray_select(int n, int round, const int*
 __global__ void __launch_bounds__(RAY_THREADS) k_ray_cast(DevWorld w, const RayCast* casts, const int* count,
                                                          const float* from, const float* to, float* candF, float4* hitA,
                                                          float4* hitB) {
-    const int total = *count;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const unsigned total = (unsigned)*count;   // below 2^31: with int the last stride could run past it
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const RayCast c = casts[i];
         const V f = mk(from[3 * c.ray], from[3 * c.ray + 1], from[3 * c.ray + 2]);
         const V t = mk(to[3 * c.ray], to[3 * c.ray + 1], to[3 * c.ray + 2]);
