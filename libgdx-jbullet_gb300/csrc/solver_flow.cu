@@ -37,7 +37,10 @@ constexpr int FLOW_QUADS = 8;                         // manifolds of a group: f
 // this kernel, setup and solve: 100k pile 1193 / 1226 / 1276 us, 1,000 boxes in pieces of 128
 // 364 / 374 / 412 us); three blocks leave each a third less room for rows (1341 and 447 us).
 constexpr int FLOW_THREADS = 256, FLOW_BLOCKS = 2;
-constexpr int FLOW_SPIN_LIMIT = 1 << 21;              // polls; each takes about half a microsecond
+// Polls of a wait, about half a microsecond each, for every FLOW_SPIN_ITERATIONS iterations or part of
+// them: a world's first piece can wait for another world's whole solve before a block is free for its second.
+constexpr int FLOW_SPIN_LIMIT = 1 << 21, FLOW_SPIN_ITERATIONS = 512;
+static_assert((long long)FLOW_SPIN_LIMIT * (FLOW_MAX_ITERATIONS / FLOW_SPIN_ITERATIONS + 1) < 0x7fffffff, "an int counts them");
 }
 
 // 16 bytes written and read whole, between blocks (global memory) and within one (shared memory),
@@ -304,6 +307,7 @@ JBD void flow_phases(const DevWorld& w, const SolverBuffers& sb, const FlowRows&
     const bool odd = lane & 1;
     const float4* const still = odd ? w.angvel : w.linvel;
     const int nPhases = 1 + 2 * w.numIter;
+    const int spinLimit = FLOW_SPIN_LIMIT * (w.numIter / FLOW_SPIN_ITERATIONS + 1);
     const int* const groupFar = (const int*)(descFar + 2 * (size_t)n);
     const unsigned half = odd ? 16u * (unsigned)np : 0u;
     // lanes beyond a group's slots take its last slot's words with nothing to read, solve or write
@@ -351,7 +355,7 @@ JBD void flow_phases(const DevWorld& w, const SolverBuffers& sb, const FlowRows&
                 waitOut = waitOut && !there;
                 if (!__any_sync(0xffffffffu, waitIn || waitOut)) break;
                 if ((++spins & 1023) == 0) {
-                    const bool give = spins >= FLOW_SPIN_LIMIT;
+                    const bool give = spins >= spinLimit;
                     if (give && lane == 0) atomicOr(&w.ctr[C_STATUS], ST_TIMEOUT);
                     dead = __any_sync(0xffffffffu, give || (ld_acquire(&w.ctr[C_STATUS]) & ST_TIMEOUT) != 0);
                 }
