@@ -1076,36 +1076,27 @@ JBD bool gjk_convex_cast(const ShapeRef& sa, const Xf& fromA, V toA, const Shape
                          V& normal, V& hitPoint) {
     const V r = sub(sub(toA, fromA.o), sub(tB.o, tB.o));
     float lambda = 0.0f, lastLambda = 0.0f;
-    int numIter = 0;
     bool has = false;
-    float cdist = 1e30f;
-    V cn = mk(0.0f, 0.0f, 0.0f), cp = cn;
+    float dist = 1e30f;
+    V n = mk(0.0f, 0.0f, 0.0f), c = n;
     Xf iA = fromA, iB = tB;
-    auto collect = [&]() {
+    for (int numIter = 0;;) {   // one copy of GJK for the first distance and those along the way
         const GjkPart g = gjk_part(sa, iA, sb, iB, SIMD_INFINITY);
-        if (g.isValid && g.distance < cdist) {
+        if (g.isValid && g.distance < dist) {
             has = true;
-            cn = g.normalInB;
-            cp = add(g.pointOnB, g.offset);
-            cdist = g.distance;
+            n = g.normalInB;
+            c = add(g.pointOnB, g.offset);
+            dist = g.distance;
         }
-    };
-    collect();
-    if (!has) return false;
-    V c = cp, n = cn;
-    float dist = cdist;
-    while (dist > 0.001f) {
+        if (!has) return false;
+        if (numIter > 0 && dist < 0.0f) { fraction = lastLambda; normal = n; hitPoint = c; return true; }
+        if (!(dist > 0.001f)) break;
         if (++numIter > 32) return false;
         lambda = __fsub_rn(lambda, jdiv(dist, dot(r, n)));
         if (lambda > 1.0f || lambda < 0.0f || lambda <= lastLambda) return false;
         lastLambda = lambda;
         iA.o = interp3(fromA.o, toA, lambda);
         iB.o = interp3(tB.o, tB.o, lambda);
-        collect();
-        if (cdist < 0.0f) { fraction = lastLambda; normal = cn; hitPoint = cp; return true; }
-        c = cp;
-        n = cn;
-        dist = cdist;
     }
     if (dot(n, r) >= -0.04f) return false;   // DispatcherInfo.allowedCcdPenetration
     fraction = lambda;
