@@ -1,5 +1,5 @@
-// Solver rows of one contact point and their Gauss-Seidel updates
-// (SequentialImpulseConstraintSolver.java:234-346, 418-786), shared by the solver's kernels.
+// Solver rows of one contact point (SequentialImpulseConstraintSolver.java:418-786), shared by the solver's
+// kernels.
 #pragma once
 #include "jbgpu_internal.cuh"
 
@@ -102,43 +102,6 @@ JBD void apply_imp(V& lin, V& ang, V n, float im, V angc, float imp) {   // Solv
         ang.y = __fadd_rn(ang.y, __fmul_rn(imp, angc.y));
         ang.z = __fadd_rn(ang.z, __fmul_rn(imp, angc.z));
     }
-}
-
-// resolveSingleCollisionCombinedCacheFriendly (java:234-284) on velocities in registers; returns
-// the impulse change and leaves the new accumulated impulse in acc.
-JBD float solve_normal_row(float4 nn, float4 r1, float4 r2, float4 aA, float4 aB, float old, V& l0, V& a0, V& l1, V& a1,
-                           float im0, float im1, float& acc) {
-    V n = mk(nn.x, nn.y, nn.z);
-    float vel1 = __fadd_rn(dot(n, l0), dot(mk(r1.x, r1.y, r1.z), a0));
-    float vel2 = __fadd_rn(dot(n, l1), dot(mk(r2.x, r2.y, r2.z), a1));
-    float rel = __fsub_rn(vel1, vel2);
-    float posErr = r1.w;          // -penetration * erp / timeStep, formed once by the setup
-    float velErr = __fsub_rn(r2.w, rel);
-    float ni1 = __fadd_rn(__fmul_rn(posErr, nn.w), __fmul_rn(velErr, nn.w));
-    float sum = __fadd_rn(old, ni1);
-    acc = 0.0f > sum ? 0.0f : sum;
-    float d = __fsub_rn(acc, old);
-    apply_imp(l0, a0, n, im0, mk(aA.x, aA.y, aA.z), d);
-    apply_imp(l1, a1, n, im1, mk(aB.x, aB.y, aB.z), -d);
-    return d;
-}
-
-// resolveSingleFrictionCacheFriendly (java:286-346) of one friction row, limit = the normal
-// impulse times the friction coefficient.
-JBD float solve_friction_row(float4 fn, float4 r1, float4 r2, float4 aA, float4 aB, float old, float limit, V& l0, V& a0,
-                             V& l1, V& a1, float im0, float im1, float& acc) {
-    V n = mk(fn.x, fn.y, fn.z);
-    float vel1 = __fadd_rn(dot(n, l0), dot(mk(r1.x, r1.y, r1.z), a0));
-    float vel2 = __fadd_rn(dot(n, l1), dot(mk(r2.x, r2.y, r2.z), a1));
-    float rel = __fsub_rn(vel1, vel2);
-    float j1 = __fmul_rn(-rel, fn.w);
-    acc = __fadd_rn(old, j1);
-    if (limit < acc) acc = limit;
-    else if (acc < -limit) acc = -limit;
-    j1 = __fsub_rn(acc, old);
-    apply_imp(l0, a0, n, im0, mk(aA.x, aA.y, aA.z), j1);
-    apply_imp(l1, a1, n, im1, mk(aB.x, aB.y, aB.z), -j1);
-    return j1;
 }
 
 enum { PH_WARM = 0, PH_NORMAL = 1, PH_FRICTION = 2 };

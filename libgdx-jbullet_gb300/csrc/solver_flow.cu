@@ -253,7 +253,7 @@ JBD float clamp_friction(float acc, float limit) {
 // The rows of a warp's manifolds in one phase, four lanes each: the warp runs `most` points, a lane
 // whose manifold has fewer repeats its last one without effect (no lane leaves the path).  r: row 0
 // (normal, warm start) or 1 (friction) of the first point, loaded ahead, as the next point's is
-// while one is solved.  The arithmetic is that of solve_normal_row and solve_friction_row.
+// while one is solved.  The arithmetic is that of the reference's rows (java:234-346).
 template <bool NEAR, int KIND>
 JBD void flow_solve(const FlowRows& F, int idx, int npt, int most, RowPart r, FlowLane& L) {
     const int last = idx + max(npt, 1) - 1;
