@@ -1230,14 +1230,14 @@ static int candidate_total(QueryBuffers& qb, int n, cudaStream_t s, int& total) 
     return JBGPU_OK;
 }
 
-// Which path: a block per ray costs its box tests over all bodies and a fixed part worth about 4,000
+// Which path: a block per ray costs its box tests over all bodies and a fixed part worth about 1,600
 // more; the lists cost a refit, a walk by one lane, a read-back and three rounds of casts however
-// few the rays.  Measured, block / lists, us: 50 bodies 4,096 rays 170 / 234, 16,384 rays 482 / 269;
-// 2,000 bodies 4,096 rays 418 / 473, 16,384 rays 1465 / 556; 20,000 bodies 1,024 rays 538 / 1150,
-// 4,096 rays 1713 / 942.
-constexpr double RAY_BLOCK_TESTS = 3e7;
+// few the rays.  Measured with host buffers, block / lists, us: 50 bodies 4,096 rays 206 / 212, 6,000 rays
+// 284 / 231; 2,000 bodies 1,500 rays 223 / 282, 3,000 rays 389 / 327; 6,000 bodies 768 rays 261 / 311, 1,500
+// rays 447 / 312; 20,000 bodies 256 rays 272 / 356, 512 rays 460 / 335; 60,000 bodies 32 rays 405 / 393.
+constexpr double RAY_BLOCK_TESTS = 7.2e6, RAY_BLOCK_FIXED = 1600.0;
 
-bool query_rays_by_block(int bodies, int rays) { return (bodies + 4000.0) * rays <= RAY_BLOCK_TESTS; }
+bool query_rays_by_block(int bodies, int rays) { return (bodies + RAY_BLOCK_FIXED) * rays <= RAY_BLOCK_TESTS; }
 
 int query_rays(const DevWorld& w, const BroadphaseBuffers& bb, QueryBuffers& qb, const float* from, const float* to,
                const int* rayWorld, int n, int group, int mask, jbgpu_ray_hit* hits, int sms, cudaStream_t s) {
