@@ -261,7 +261,8 @@ typedef struct jbgpu_counters {
     int32_t solver_islands;   /* residual mode: islands with solver rows in the last solve */
     int32_t solver_islands_converged;  /* ... of which reached the residual */
     int32_t solver_island_iterations;  /* ... sum over them of the iterations they took */
-    int32_t ray_replays;      /* rays of the last jbgpu_world_ray_test replayed in body order */
+    int32_t ray_replays;      /* rays of the last jbgpu_world_ray_test replayed in body order (of a batch with a block
+                               * per ray, where every ray is taken so, those whose list overflowed) */
     int32_t ccd_clamped;      /* bodies of the last integrateTransforms that ran a CCD sweep
                                  (BulletStats.gNumClampedCcdMotions for one step) */
 } jbgpu_counters;

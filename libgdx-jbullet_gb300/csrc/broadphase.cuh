@@ -27,7 +27,6 @@ constexpr int DIRECT_CACHE = 256;      // the same of the direct count; more and
 
 struct DirectList {    // every body, grouped by world in index order
     int* body = nullptr;
-    int* pos = nullptr;    // per body: its place in `body`
     int* end = nullptr;    // per world: the end of its group
 };
 

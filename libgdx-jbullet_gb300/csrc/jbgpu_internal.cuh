@@ -28,7 +28,7 @@ enum {
     C_ISLANDS,
     C_MANIFOLDS, C_CONTACTS, C_ROWS, C_STATUS, C_BAR_GEN, C_WIN0, C_WIN1, C_WIN2,
     C_CUT_COLOURS, C_CUT_MANIFOLDS, C_RES0, C_RES1, C_RES2,
-    // cleared together at the start of a solve (C_SOLVE_FIRST .. C_SOLVE_LAST)
+    // cleared together at the start of a solve (C_SOLVE_FIRST, C_SOLVE_COUNT of them)
     C_BAR_COUNT, C_PGS_ITERS, C_ISL_N, C_ISL_CONV, C_ISL_ITERS, C_PART_NEXT0, C_PART_NEXT1, C_COL_FAIL, C_CUT_DONE,
     C_CCD_N, C_CCD_BEST, C_NCTR = 36
 };

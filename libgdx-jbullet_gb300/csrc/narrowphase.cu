@@ -113,8 +113,8 @@ JBD int narrow_active(const int* blockOff, int nBlocks) { return blockOff[(NB_BU
 // holds fewer pairs (narrow_pairs has the line and the times).  Lanes that take the next pair when
 // theirs is done, and the manifold in a pass of its own, were slower: 672 us against 475 us for
 // 600,000 pairs - lanes in step share the simplex's cases; the pass in two without that, 497 us
-// against 449 us.  Three blocks of 168 registers an SM rather than four of 128, which spill: 4,000
-// hulls 121 -> 99 us, 1,024 worlds 1044 -> 993 us, 600,000 mixed pairs 430 -> 447 us.
+// against 449 us.  Three blocks of 168 registers an SM (16 bytes a thread spilled) rather than four of
+// 128 (148 bytes): 4,000 hulls 121 -> 99 us, 1,024 worlds 1044 -> 993 us; 600,000 mixed pairs lose, 430 -> 447 us.
 template <int G>
 __global__ void __launch_bounds__(128, 3)
     k_narrow(DevWorld w, DevPairs P, int n, const int* perm, const int* blockOff, EpaRec* queue, int* queueCount,
@@ -396,7 +396,8 @@ __global__ void __launch_bounds__(32) k_narrow_epa_smem(DevWorld w, DevPairs P, 
 static int gridn_nb(int nPairs) { return (nPairs + NB_THREADS - 1) / NB_THREADS; }
 
 // The pass over nPairs pairs (with cntp an upper bound: the pair capacity, half as large again as the
-// count or more).  Lanes to a pair, us at 1 / 4 / 32: 139 pairs (60 mixed bodies) 87 / 56 / 36; 5,134
+// count or more, and as large as it ever was: a world keeps the forms for the most pairs it has held, as it
+// does the launches for large worlds in solver.cu).  Lanes to a pair, us at 1 / 4 / 32: 139 pairs (60 mixed bodies) 87 / 56 / 36; 5,134
 // (boxes) 38 / 36.5 / 56; 19,780 (boxes and hulls on a mesh) 105 / 93 / 163; 30,087 61 / 82 / 194;
 // 114,015 151 / 245 / 778.
 static void narrow_pairs(const DevWorld& w, DevPairs& P, int nPairs, NarrowBuffers& nb, const int* perm, const int* cntp,

@@ -13,11 +13,11 @@ struct QueryBuffers {
     float4* node = nullptr;       // the broadphase tree's topology refit over qmin / qmax
     int* visit = nullptr;
     int capNodes = 0;
-    int* slow = nullptr;          // rays the closest-hit shortcut cannot decide (replayed in body order)
-    int* slowCount = nullptr;
-    int* rayCnt = nullptr;        // per ray: candidates, their offsets, the smallest hit key,
+    int* slow = nullptr;          // rays for k_rays_slow (block lists that overflowed, the forced replay) or k_ray_long
+    int* slowCount = nullptr;     // rays replayed in body order
+    int* rayCnt = nullptr;        // per ray (sweep): its candidates and their offset,
     int* rayOff = nullptr;
-    unsigned long long* key = nullptr;
+    unsigned long long* key = nullptr;   // ... and a sweep's smallest hit key
     void* list = nullptr;         // per ray: its first listCap candidates (body, aabb entry)
     int listCap = 0;
     size_t listEntries = 0;

@@ -2793,8 +2793,8 @@ void solve_launch(const DevWorld& w, DevPairs& P, int nPairs, DevRows& R, Solver
 void solve_launch_learn(const DevWorld& w, DevPairs& P, int nPairs, DevRows& R, SolverBuffers& sb, float dt,
                         cudaStream_t s, const Prof* prof, const SolverLearn& learn) {
     if (prof) prof->mark(PH_COLOUR, 0, s);
-    if (nPairs <= 0 || sb.nFinite <= 0 || sb.nParts <= 0) cudaMemsetAsync(w.ctr + C_ROWS, 0, sizeof(int), s);
     if (nPairs <= 0 || sb.nFinite <= 0 || sb.nParts <= 0) {
+        cudaMemsetAsync(w.ctr + C_ROWS, 0, sizeof(int), s);
         cudaMemsetAsync(sb.nColours, 0, sizeof(int), s);
         cudaMemsetAsync(sb.nCand, 0, sizeof(int), s);
         if (prof) { prof->mark(PH_COLOUR, 1, s); prof->mark(PH_SETUP, 0, s); }

@@ -6,8 +6,8 @@ namespace jbg {
 
 constexpr int MAX_COLOURS = 1024;     // grid-wide colours of cut manifolds
 constexpr int MAX_LOCAL = 128;        // colours of the manifolds internal to one part
-constexpr int MAX_SUB = 16;
-constexpr int COL_REG = 4;            // internal-colouring candidates a thread keeps in registers           // claim passes that grow one colour towards a maximal set
+constexpr int MAX_SUB = 16;           // claim passes that grow one colour towards a maximal set
+constexpr int COL_REG = 4;            // colouring candidates a thread keeps in registers
 constexpr int COL_LIST = 32;          // candidates a body's list holds
 constexpr unsigned COL_CUT = 1u << 31;   // a list entry of a cut candidate
 constexpr int COL_SWEEPS = 1 << 20;   // a thread's sweeps over its candidates before it gives up
@@ -153,7 +153,6 @@ struct SolverBuffers {
     int* flowOrder = nullptr;     // flow blocks in the order they are taken
     void* flowScan = nullptr;     // scan scratch of the buckets
     int* flowTop = nullptr;       // device scalars: next block, rows kept outside shared memory
-    int rowStride = 0;            // points a plane of the row arrays holds (4 x pair capacity)
     int nFlow = 0, flowCap = 0;
     int gridFlow = 0;
     int flowSmem = 0;             // dynamic shared memory of a flow block

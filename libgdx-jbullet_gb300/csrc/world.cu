@@ -209,7 +209,6 @@ int alloc_pair_work(jbgpu_world* w, int cap) {
         for (float4** n : {&R.n_nrm, &R.n_rp1, &R.n_rp2, &R.n_angA, &R.n_angB}) { *n = p; p += c4; }
         for (float4** f : {&R.f_nrm, &R.f_rp1, &R.f_rp2, &R.f_angA, &R.f_angB}) { *f = p; p += c8; }
     }
-    w->sb.rowStride = (int)std::min<size_t>(c4, 0x7fffffff);
     CK(dalloc(&R.slot_pair, cap)); CK(dalloc(&R.slot_desc, cap)); CK(dalloc(&R.slot_im, cap));
     CK(dalloc(&R.slot_pt0, cap)); CK(dalloc(&R.pt_key, c4));
     SolverBuffers& S = w->sb;
@@ -417,7 +416,7 @@ int sync_planes(jbgpu_world* w) {
     for (int k = 0; k < nw; k++) { start[k] = (int)list.size(); list.insert(list.end(), per[k].begin(), per[k].end()); }
     start[nw] = (int)list.size();
     dfree(B.planeList); dfree(B.planeStart); dfree(B.wstart); dfree(B.wend); dfree(B.wroot); dfree(B.bounds); dfree(B.total);
-    dfree(B.segLong); dfree(B.list.body); dfree(B.list.pos); dfree(B.list.end); dfree(B.kept);
+    dfree(B.segLong); dfree(B.list.body); dfree(B.list.end); dfree(B.kept);
     CK(dalloc(&B.planeList, std::max<size_t>(1, list.size()))); CK(dalloc(&B.planeStart, nw + 1));
     CK(dalloc(&B.wstart, nw)); CK(dalloc(&B.wend, nw)); CK(dalloc(&B.wroot, nw)); CK(dalloc(&B.bounds, 6)); CK(dalloc(&B.total, 2));
     B.candBound = B.total + 1;
@@ -434,18 +433,14 @@ int sync_planes(jbgpu_world* w) {
     B.worldBits = nw > 1 ? bits : 0;
     w->nWorlds = nw;
     w->worldFinite = finite;
-    std::vector<int> pos(std::max(w->nBodies, 1)), end(nw + 1, 0), body(std::max(w->nBodies, 1)), bodies(nw, 0);
+    std::vector<int> end(nw + 1, 0), body(std::max(w->nBodies, 1)), bodies(nw, 0);
     for (int i = 0; i < w->nBodies; i++) bodies[w->hWorld[i]]++;
     for (int k = 0; k < nw; k++) end[k + 1] = end[k] + bodies[k];   // group starts, advanced to the ends below
-    for (int i = 0; i < w->nBodies; i++) {
-        pos[i] = end[w->hWorld[i]]++;
-        body[pos[i]] = i;
-    }
+    for (int i = 0; i < w->nBodies; i++) body[end[w->hWorld[i]]++] = i;
     B.direct = broadphase_direct(bodies, finite);
     if (B.direct) CK(dalloc(&B.kept, (size_t)DIRECT_CACHE * body.size()));
-    CK(dalloc(&B.list.body, body.size())); CK(dalloc(&B.list.pos, pos.size())); CK(dalloc(&B.list.end, nw));
+    CK(dalloc(&B.list.body, body.size())); CK(dalloc(&B.list.end, nw));
     CK(cudaMemcpyAsync(B.list.body, body.data(), sizeof(int) * body.size(), cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(B.list.pos, pos.data(), sizeof(int) * pos.size(), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(B.list.end, end.data(), sizeof(int) * nw, cudaMemcpyHostToDevice, s));
     CK(cudaStreamSynchronize(s));   // the lists above are this function's
     w->bb.built = w->bb.treeBuilt = false;
@@ -1396,7 +1391,7 @@ int jbgpu_world_destroy(jbgpu_world* w) {
     dfree(B.bvh.left); dfree(B.bvh.right); dfree(B.bvh.lo); dfree(B.bvh.hi); dfree(B.bvh.parent); dfree(B.bvh.leafParent);
     dfree(B.bvh.visit); dfree(B.bvh.node); dfree(B.tcount); dfree(B.tcache); dfree(B.wstart); dfree(B.wend); dfree(B.wroot);
     dfree(B.planeList); dfree(B.planeStart); dfree(B.cnt); dfree(B.off); dfree(B.offPrev); dfree(B.cursor); dfree(B.total); dfree(B.partners);
-    dfree(B.segLong); dfree(B.list.body); dfree(B.list.pos); dfree(B.list.end); dfree(B.kept);
+    dfree(B.segLong); dfree(B.list.body); dfree(B.list.end); dfree(B.kept);
     NarrowBuffers& N = w->nb;
     if (N.queue) cudaFree(N.queue);
     dfree(N.tierMode); dfree(N.ovfQueue); dfree(N.ovfQueue2); dfree(N.pairBucket); dfree(N.perm); dfree(N.blockOff);
