@@ -1142,22 +1142,27 @@ int query_prepare(const DevWorld& w, BroadphaseBuffers& bb, QueryBuffers& qb, bo
     return cudaGetLastError() == cudaSuccess ? JBGPU_OK : JBGPU_ERR_CUDA;
 }
 
+// Arrays that grow together lie in one allocation: each costs a first batch some 35 us.
+template <class T>
+static void carve(T*& array, char*& at, size_t bytes) {
+    array = (T*)at;
+    at += (bytes + 255) & ~(size_t)255;
+}
+
 static bool grow_ray_buffers(QueryBuffers& qb, int n, bool lists = false, int bodies = 0) {
     if (n > qb.capRays) {   // per-ray (per-sweep) buffers
-        void* old[] = {qb.slow, qb.rayCnt, qb.rayOff, qb.key, qb.scanScratch};
-        for (void* p : old)
-            if (p) cudaFree(p);
-        qb.slow = qb.rayCnt = qb.rayOff = nullptr;
-        qb.key = nullptr;
-        qb.scanScratch = nullptr;
+        if (qb.rayMem) cudaFree(qb.rayMem);
+        qb.rayMem = nullptr;
         const int c = n > 2 * qb.capRays ? n : 2 * qb.capRays;
         qb.capRays = 0;
-        if (cudaMalloc((void**)&qb.slow, sizeof(int) * (size_t)c) != cudaSuccess ||
-            cudaMalloc((void**)&qb.rayCnt, sizeof(int) * (size_t)c) != cudaSuccess ||
-            cudaMalloc((void**)&qb.rayOff, sizeof(int) * (size_t)c) != cudaSuccess ||
-            cudaMalloc((void**)&qb.key, sizeof(unsigned long long) * (size_t)c) != cudaSuccess ||
-            cudaMalloc(&qb.scanScratch, scan_scratch_bytes(c)) != cudaSuccess)
-            return false;
+        const size_t words = sizeof(int) * (size_t)c, scan = scan_scratch_bytes(c);
+        if (cudaMalloc(&qb.rayMem, 5 * words + scan + 5 * 256) != cudaSuccess) return false;
+        char* at = (char*)qb.rayMem;
+        carve(qb.key, at, 2 * words);
+        carve(qb.slow, at, words);
+        carve(qb.rayCnt, at, words);
+        carve(qb.rayOff, at, words);
+        carve(qb.scanScratch, at, scan);
         qb.capRays = c;
     }
     if (lists) {
@@ -1174,31 +1179,33 @@ static bool grow_ray_buffers(QueryBuffers& qb, int n, bool lists = false, int bo
         });
         if (!qb.listCap) return false;
     }
-    if (!qb.slowCount && (cudaMalloc((void**)&qb.slowCount, sizeof(int)) != cudaSuccess ||
-                          cudaMalloc((void**)&qb.candTotal, sizeof(int)) != cudaSuccess ||
-                          cudaMalloc((void**)&qb.castCount, sizeof(int) * (RAY_ROUNDS + 2)) != cudaSuccess ||
-                          cudaMalloc((void**)&qb.candTotal64, sizeof(unsigned long long)) != cudaSuccess))
-        return false;
+    if (!qb.slowCount) {
+        char* at = nullptr;
+        if (cudaMalloc((void**)&at, 4 * 256) != cudaSuccess) return false;
+        carve(qb.slowCount, at, sizeof(int));   // the allocation's address
+        carve(qb.candTotal, at, sizeof(int));
+        carve(qb.castCount, at, sizeof(int) * (RAY_ROUNDS + 2));
+        carve(qb.candTotal64, at, sizeof(unsigned long long));
+    }
     return true;
 }
 
 static bool grow_cand_buffers(QueryBuffers& qb, int total) {
     if (total > qb.capCand) {
-        void* old[] = {qb.cand, qb.hitA, qb.hitB, qb.candBody, qb.candF};
-        for (void* p : old)
-            if (p) cudaFree(p);
-        qb.cand = nullptr;
-        qb.hitA = qb.hitB = nullptr;
-        qb.candBody = nullptr;
-        qb.candF = nullptr;
+        if (qb.candMem) cudaFree(qb.candMem);
+        qb.candMem = nullptr;
         const int c = total > 2 * qb.capCand ? total : 2 * qb.capCand;
         qb.capCand = 0;
-        if (cudaMalloc((void**)&qb.cand, sizeof(RayCand) * (size_t)c) != cudaSuccess ||
-            cudaMalloc((void**)&qb.hitA, sizeof(float4) * (size_t)c) != cudaSuccess ||
-            cudaMalloc((void**)&qb.hitB, sizeof(float4) * (size_t)c) != cudaSuccess ||
-            cudaMalloc((void**)&qb.candBody, sizeof(RayEntry) * (size_t)c) != cudaSuccess ||
-            cudaMalloc((void**)&qb.candF, sizeof(float) * (size_t)c) != cudaSuccess)
+        const size_t m = (size_t)c;
+        if (cudaMalloc(&qb.candMem, (sizeof(RayCand) + 2 * sizeof(float4) + sizeof(RayEntry) + sizeof(float)) * m + 5 * 256) !=
+            cudaSuccess)
             return false;
+        char* at = (char*)qb.candMem;
+        carve(qb.cand, at, sizeof(RayCand) * m);
+        carve(qb.hitA, at, sizeof(float4) * m);
+        carve(qb.hitB, at, sizeof(float4) * m);
+        carve(qb.candBody, at, sizeof(RayEntry) * m);
+        carve(qb.candF, at, sizeof(float) * m);
         qb.capCand = c;
     }
     return true;
@@ -1769,9 +1776,8 @@ void ccd_free(CcdBuffers& cb) {
 }
 
 void query_free(QueryBuffers& qb) {
-    void* ps[] = {qb.qmin, qb.qmax, qb.node, qb.visit, qb.slow, qb.slowCount, qb.from, qb.to, qb.rayWorld, qb.hits,
-                  qb.rayCnt, qb.rayOff, qb.candTotal, qb.candTotal64, qb.key, qb.scanScratch, qb.cand, qb.hitA,
-                  qb.hitB, qb.list, qb.castCount, qb.candBody, qb.candF, qb.sweepMin, qb.sweepMax, qb.sweepPlane, qb.sweepFrom, qb.sweepTo};
+    void* ps[] = {qb.qmin, qb.qmax, qb.node, qb.visit, qb.rayMem, qb.slowCount, qb.candMem, qb.list, qb.from, qb.to,
+                  qb.rayWorld, qb.hits, qb.sweepMin, qb.sweepMax, qb.sweepPlane, qb.sweepFrom, qb.sweepTo};
     for (void* p : ps)
         if (p) cudaFree(p);
     qb = QueryBuffers();

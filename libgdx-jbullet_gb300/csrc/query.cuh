@@ -13,24 +13,26 @@ struct QueryBuffers {
     float4* node = nullptr;       // the broadphase tree's topology refit over qmin / qmax
     int* visit = nullptr;
     int capNodes = 0;
+    void* rayMem = nullptr;       // slow, rayCnt, rayOff, key, scanScratch
     int* slow = nullptr;          // rays for k_rays_slow (block lists that overflowed, the forced replay) or k_ray_long
-    int* slowCount = nullptr;     // rays replayed in body order
     int* rayCnt = nullptr;        // per ray (sweep): its candidates and their offset,
     int* rayOff = nullptr;
     unsigned long long* key = nullptr;   // ... and a sweep's smallest hit key
+    void* scanScratch = nullptr;
+    int capRays = 0;
     void* list = nullptr;         // per ray: its first listCap candidates (body, aabb entry)
     int listCap = 0;
     size_t listEntries = 0;
+    int* slowCount = nullptr;     // rays replayed in body order (the counters below lie behind it)
+    int* candTotal = nullptr;     // candidates of the batch
     int* castCount = nullptr;     // casts of each round
-    void* candBody = nullptr;     // (body, aabb entry) of the candidates of rays with more than listCap
-    float* candF = nullptr;       // per candidate: not cast, missed, or its smallest hit fraction
-    void* scanScratch = nullptr;
-    int* candTotal = nullptr;
-    unsigned long long* candTotal64 = nullptr;   // the same total in 64 bits (refuses overflowing batches)
-    int capRays = 0;
+    unsigned long long* candTotal64 = nullptr;   // the total in 64 bits (refuses overflowing batches)
+    void* candMem = nullptr;      // cand, hitA, hitB, candBody, candF
     void* cand = nullptr;         // (ray, body, aabb entry) candidates and their hits
     float4* hitA = nullptr;
     float4* hitB = nullptr;
+    void* candBody = nullptr;     // (body, aabb entry) of the candidates of rays with more than listCap
+    float* candF = nullptr;       // per candidate: not cast, missed, or its smallest hit fraction
     int capCand = 0;
     int replayAll = 0;            // verification: every ray takes the in-order replay
     float* from = nullptr;        // staging for host buffers
@@ -46,8 +48,8 @@ struct QueryBuffers {
     int capSweeps = 0;
 };
 
-// Query boxes for every body and, with `tree`, the refit tree over them; builds the broadphase
-// tree first when the body set changed since its last build.
+// Query boxes for every body and, with `tree`, the refit tree over them; when the body set changed, the
+// broadphase's order first and, with `tree`, its topology.
 int query_prepare(const DevWorld& w, BroadphaseBuffers& bb, QueryBuffers& qb, bool tree, cudaStream_t s);
 // Whether a batch of rays takes a block per ray (and needs no refit tree).
 bool query_rays_by_block(int bodies, int rays);
