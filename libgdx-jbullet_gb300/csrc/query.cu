@@ -12,15 +12,15 @@
 // a thread each, and replays the reference's loop over them in body order.
 //
 // Many rays: one thread per ray walks the broadphase tree (refit over the shapes' current aabbs)
-// and lists the objects whose aabb the ray enters before its end; then, in three rounds, the
-// nearest listed objects by aabb entry are cast, a thread per (ray, object) so that the warps run
-// one code path, and what the reference is sure to skip is dropped: once object i is past, its
-// closest fraction is at most max(hit of i, aabb entry of i) - either i was cast, or it was skipped
-// because the closest was below its entry already - so an object after i in body order whose entry
-// lies above that is skipped.  An object's cast does not depend on the hits before it, so the ray's
-// answer is the smallest hit by (fraction, body, triangle), j, among those cast - unless an object
-// before j in body order hit below j's aabb entry (then the order-dependent aabb test may have
-// skipped j): such rays replay their cast objects in body order.
+// and lists the objects whose aabb the ray enters before its end; then, in three rounds (or in one,
+// where rays have few candidates), the nearest listed objects by aabb entry are cast, a thread per
+// (ray, object) so that the warps run one code path, and what the reference is sure to skip is
+// dropped: once object i is past, its closest fraction is at most max(hit of i, aabb entry of i) -
+// either i was cast, or it was skipped because the closest was below its entry already - so an object
+// after i in body order whose entry lies above that is skipped.  An object's cast does not depend on
+// the hits before it, so the ray's answer is the smallest hit by (fraction, body, triangle), j, among
+// those cast - unless an object before j in body order hit below j's aabb entry (then the
+// order-dependent aabb test may have skipped j): such rays replay their cast objects in body order.
 #include "../../include/jbgpu.h"
 #include "gjk.cuh"
 #include "gridsync.cuh"
@@ -665,7 +665,7 @@ __device__ constexpr int ray_round_casts(int round) { return round == 0 ? 4 : 8;
 
 // A warp per ray: which of its candidates the next round casts - the nearest few by aabb entry that
 // are neither cast nor dropped (see the top of the file), in the last round all of them.
-__global__ void __launch_bounds__(256) k_ray_select(int n, int round, const int* cnt, const int* off, const RayEntry* list,
+__global__ void __launch_bounds__(256) k_ray_select(int n, int round, int rounds, const int* cnt, const int* off, const RayEntry* list,
                                                     int listCap, const RayEntry* all, float* candF, RayCast* casts,
                                                     int* castCount) {
     __shared__ int hBody[8][32], sWant[8], sBase;
@@ -702,7 +702,7 @@ __global__ void __launch_bounds__(256) k_ray_select(int n, int round, const int*
             if (hBody[warp][h] < body && hBound[warp][h] < enter) return false;
         return true;
     };
-    const bool pick = round + 1 < RAY_ROUNDS && m <= 32 * RAY_SORT;
+    const bool pick = round + 1 < rounds && m <= 32 * RAY_SORT;
     float en[RAY_SORT];
     int bo[RAY_SORT];
     int want = 0;
@@ -1300,8 +1300,13 @@ int query_rays(const DevWorld& w, const BroadphaseBuffers& bb, QueryBuffers& qb,
                                                            bb.planeStart, from, to, rayWorld, group, mask, qb.rayCnt,
                                                            qb.rayOff, list, cap, all, qb.slow, longCount);
         note_launch();
-        for (int round = 0; round < RAY_ROUNDS; round++) {
-            k_ray_select<<<gridn(n, 8), 256, 0, s>>>(n, round, qb.rayCnt, qb.rayOff, list, cap, all, qb.candF, casts,
+        // Rounds pay where rays have many candidates, or costly ones (triangle meshes).  At once / in rounds, us, by
+        // candidates a ray: 1.5 (50 bodies) 100,000 rays 272 / 345; 4.1 (2,000 bodies) 543 / 616; 4.9 (20,000 bodies)
+        // 680 / 750; 37 (4,000 hulls) 30,000 rays 1,619 / 1,236, 200,000 rays 8,103 / 5,104; a landscape with 20 bodies
+        // 100,000 rays 458 / 532, with 4,000 bodies (3.4) 200,000 rays 5,356 / 3,292.
+        const int rounds = total <= (bb.meshes ? 2LL : 6LL) * n ? 1 : RAY_ROUNDS;
+        for (int round = 0; round < rounds; round++) {
+            k_ray_select<<<gridn(n, 8), 256, 0, s>>>(n, round, rounds, qb.rayCnt, qb.rayOff, list, cap, all, qb.candF, casts,
                                                      qb.castCount);
             note_launch();
             k_ray_cast<<<std::min(gridn(total, RAY_THREADS), sms * 16), RAY_THREADS, 0, s>>>(
